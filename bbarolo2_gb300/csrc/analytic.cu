@@ -14,6 +14,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "anpix.cuh"
 #include "devmath.cuh"
 #include "kernels.h"
@@ -290,13 +292,13 @@ __global__ void __launch_bounds__(AN_WPB * 32) k_an_model(GridDev g, const AnSub
 }
 
 // ------------------------------------------------------------------------------ the model's float32 path
-// Sub-rings with one line on a linear channel map and a velocity independent of the height (anfast): one warp
-// per (member, azimuth sample).
+// Sub-rings with one line on a linear channel map and a velocity independent of the height (anfast), for each
+// (member, azimuth sample):
 //   pixels  lanes over heights, float32 with a rounding bound and exact fallbacks (sample_pixel), the reference's
 //           pixel of every height;
 //   runs    consecutive heights in one pixel (a ballot of the run starts), their weights by a segmented scan
 //           (float32), a run crossing a pass of 32 heights carried to the next pass;
-//   line    computed at the first run in the box: the velocity and its channel in float-float (the reference's
+//   line    the velocity and its channel in float-float (the reference's
 //           float64 _velgrid within 1e-6 of a channel boundary), the centre channel kc exact, then the
 //           channel-integrated profile over kc - K .. kc + K in float32: the edges relative to a reference
 //           velocity in float-float (so that (edge - v) / sig keeps ~1e-7), the normal CDF from the reference's
@@ -305,13 +307,16 @@ __global__ void __launch_bounds__(AN_WPB * 32) k_an_model(GridDev g, const AnSub
 //           products, each rounded to the unit 2^-e: exact and order-independent sums).
 #define ANF_WPB 8
 
+// (the integer part by an addition rounded down: the conversion instructions run at an eighth of the float32 rate;
+// no branch: outside the table the index is clamped and the value replaced)
 __device__ __forceinline__ float phi_f32(float t, const float *__restrict__ tab) {
     const float x = (t + 6.0f) * 512.0f;
-    if (!(x > 0.0f)) return 0.0f;
-    if (x >= (float)(PHI_N - 1)) return 1.0f;
-    const int k = (int)x;
-    const float t0 = __ldg(tab + k), t1 = __ldg(tab + k + 1);
-    return fmaf(x - (float)k, t1 - t0, t0);
+    const float y = fminf(fmaxf(x, 0.0f), 6144.9995f);              // (the largest float32 below the last entry)
+    const float f = __fadd_rd(y, 8388608.0f);
+    const int k = __float_as_int(f) - 0x4B000000;
+    const float t0 = tab[k], t1 = tab[k + 1];
+    const float v = fmaf(y - __fsub_rn(f, 8388608.0f), t1 - t0, t0);
+    return !(x > 0.0f) ? 0.0f : (x >= (float)(PHI_N - 1) ? 1.0f : v);
 }
 
 // The line of a float32-path sample: bbarolo/galmod.py:407 and :410 (_velgrid, _lround) in float-float (about 44
@@ -334,6 +339,53 @@ __device__ __forceinline__ long long fast_line_centre(const AnSub &S, const Grid
     return lround_ref(velgrid_exact(vplane, g, 0));
 }
 
+// The float32 nearest to q 2^-e: the two 23-bit halves of |q| < 2^46 are exact in float32 and joined by one FMA, so
+// there is one rounding and no float64 conversion (the float64 route, 3 instructions of the 1/64-rate pipe, held the
+// conversion of the models to 190 G values/s). Larger sums are shifted down first, the bits lost kept as a sticky one.
+__device__ __forceinline__ float fix_to_f32(long long q, int e) {
+    unsigned long long m = q < 0 ? 0ULL - (unsigned long long)q : (unsigned long long)q;
+    int x = -e;
+    if (m >> 46) {
+        m = (m >> 18) | ((m & 0x3ffffULL) != 0);
+        x += 18;
+    }
+    const float hi = __fsub_rn(__int_as_float(0x4B000000 | (int)(m >> 23)), 8388608.0f);
+    const float lo = __fsub_rn(__int_as_float(0x4B000000 | ((int)m & 0x7fffff)), 8388608.0f);
+    const float f = fmaf(hi, 8388608.0f, lo);
+    // (a power of two or a product outside the normal range: ldexpf's own rounding)
+    const float r = x > -126 && x < 80 ? __fmul_rn(f, __int_as_float((x + 127) << 23)) : ldexpf(f, x);
+    return q < 0 ? -r : r;
+}
+
+// What a warp needs of one of its 32 samples, staged in shared memory by the lane that set the sample up.
+struct __align__(16) AnfSample {
+    float vrh, vrl, invf, amp;        // the line: velocity about vref (float-float), 1 / sig, fixed-point amplitude
+    float bxf, byf, zP3, zQ3;         // the pixels (PixF); hwx < 0: every height takes the exact path
+    float hwx, hwy;
+    unsigned short k0, nk;            // the line's channels (an_smem_bytes keeps nz far below 65536)
+    int off;                          // the vertical samples
+    int nzz, sub, s, k;               // their number; index of the constants; sample (bit 31: second radius); member
+};
+
+#define ANF_RUNS 96                   // runs of a sample collected before their deposit (a pass adds at most 33)
+#define ANF_FIXMAX 1.7592186044416e13f // 2^44: below it f32_to_fix is f32_to_ll
+
+// f32_to_ll for |x| < ANF_FIXMAX without its branch and shift: adding 1.5 2^46 rounds x to a multiple of 2^23 held in
+// the low mantissa bits, the exact rest (at most 2^22) is rounded the same way.
+#define ANF_HI 1.0555311626649600e14f    // 1.5 2^46
+__device__ __forceinline__ unsigned long long f32_to_fix(float x) {
+    const float t = __fadd_rn(x, ANF_HI);
+    const float l = __fsub_rn(x, __fsub_rn(t, ANF_HI));
+    const int hi = __float_as_int(t) - __float_as_int(ANF_HI);
+    const int lo = __float_as_int(__fadd_rn(l, BB_MAGIC15)) - __float_as_int(BB_MAGIC15);
+    return (unsigned long long)((long long)hi * 8388608 + lo);
+}
+
+// The samples are set up 32 at a time, a lane each (constants, pixel coefficients, line); then the warp takes them one
+// after another: the profile over the lanes into shared memory; the heights, 32 a pass, into the list of the sample's
+// runs in the box; and the (run, channel) pairs laid end to end over the lanes, one 64-bit reduction each. At 27
+// channels and 20 runs that is about 550 instructions a sample, where a warp that set up and deposited a run at a time
+// took 1200 (40 ms for the thick gradient of 161 members, 160x160x128).
 __global__ void __launch_bounds__(ANF_WPB * 32, 4) k_an_model_fast(GridDev g, const AnSub *__restrict__ subs, int nsub,
                                                                 const int *__restrict__ sbase,
                                                                 const int *__restrict__ ssub,
@@ -350,190 +402,379 @@ __global__ void __launch_bounds__(ANF_WPB * 32, 4) k_an_model_fast(GridDev g, co
                                                                 const float *__restrict__ ptabf,
                                                                 const MemberDev *__restrict__ mem,
                                                                 unsigned long long *__restrict__ out64,
-                                                                long long mstride, int skip_thin) {
-    extern __shared__ float anf_smem[];                     // per warp: the CDF at the edges, the profile
+                                                                long long mstride) {
+    extern __shared__ __align__(16) uint8_t anf_smem[];     // samples, runs, the CDF table, profiles
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long gs = (long long)blockIdx.x * ANF_WPB + w;
-    AnSeg sg;
-    if (!an_seg(gs, astart, aseg, nseg, ntot, sbase, sg)) return;
-    const int k = sg.k;
-    const long long s = sg.s;
-    const int ir = ssub[s];
-    const AnSub &S = subs[(size_t)sg.src * nsub + ir];
-    if (!S.active || !S.anfast || (skip_thin && S.nzz == 1)) return;
-    const float2 cf = csf[s];
-    const bool rec = cf.x >= 0.0f;                          // (the sign of the float32 table is the float64 test's)
-    if (S.wzero & (rec ? 1 : 2)) return;
-    const int kr = (int)(s - sbase[ir]) >= S.naz ? 1 : 0;
-    const PixF px = pix_setup(S, kr, cf, zqf + S.zq_off, S.nzz);
-    const MemberDev &M = mem[k];
-    const int nz = g.nz, nzz = S.nzz, off = S.zq_off;
-    float *phe = anf_smem + (size_t)w * 2 * (nz + 2);
-    float *prof = phe + nz + 2;
-    unsigned long long *o64 = out64 + (size_t)k * mstride;
-    int k0 = 0, nk = -1;                                    // the line's channels (nk < 0: not computed yet)
-    auto line = [&]() {
-        ff v;
-        const long long kc = fast_line_centre(S, g, csff[s], cs + s, v);
-        long long a0 = kc - S.K, a1 = kc + S.K + 1;
-        if (a0 < 0) a0 = 0;
-        if (a1 > nz) a1 = nz;
-        if (a1 <= a0) {
-            nk = 0;
-            return;
-        }
-        k0 = (int)a0;
-        nk = (int)(a1 - a0);
-        const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
-        const float vrh = vr.hi, vrl = vr.lo;
-        const float amp = (float)sg.sign * ldexpf(S.af * (rec ? S.wrecf : S.wappf), M.fix_exp);
-        for (int j = lane; j <= nk; j += 32) {
-            const float2 e = __ldg(vef + k0 + j);
-            const float t = (__fsub_rn(e.x, vrh) + __fsub_rn(e.y, vrl)) * S.invf;
-            phe[j] = phi_f32(t, ptabf);
-        }
-        __syncwarp();
-        for (int j = lane; j < nk; j += 32) prof[j] = fabsf(phe[j + 1] - phe[j]) * __ldg(cd2if + k0 + j) * amp;
-        __syncwarp();
-    };
-    auto deposit = [&](int g0, int g1, float ws) {          // (warp-uniform arguments)
-        if (g0 < M.blo0 || g0 >= M.bhi0 || g1 < M.blo1 || g1 >= M.bhi1) return;
-        if (nk < 0) line();
-        if (nk == 0) return;
-        unsigned long long *o = o64 + ((size_t)(g1 - M.blo1) * M.bx + (size_t)(g0 - M.blo0)) * nz + k0;
-        for (int j = lane; j < nk; j += 32) {
-            const long long q = f32_to_ll(prof[j] * ws);
-            if (q) atomicAdd(o + j, (unsigned long long)q);
-        }
-    };
-    bool open = false;                                      // a run carried from the previous pass
-    int cg0 = 0, cg1 = 0;
-    float cws = 0.0f;
-    for (int base = 0; base < nzz; base += 32) {
-        const int cnt = min(32, nzz - base);
-        const bool valid = lane < cnt;
-        int g0 = 0x7fffffff, g1 = 0x7fffffff;
-        float wv = 0.0f;
-        if (valid) {
-            sample_pixel(S, px, kr, cs + s, nzz, nzz > 1 ? zqf[off + base + lane] : 0.f, zq + off + base + lane,
-                         g.cdelt0, g.cdelt1, g0, g1);
-            wv = wqf[off + base + lane];
-        }
-        const int pg0 = __shfl_up_sync(FULL, g0, 1), pg1 = __shfl_up_sync(FULL, g1, 1);
-        const bool start = valid && (lane == 0 ? (!open || g0 != cg0 || g1 != cg1) : (g0 != pg0 || g1 != pg1));
-        const unsigned smask = __ballot_sync(FULL, start);
-        if (open && (smask & 1u)) {                         // the carried run ended with the previous pass
-            deposit(cg0, cg1, cws);
-            open = false;
-        }
-        // segmented inclusive scan of the weights (a segment: from a run start to the lane before the next)
-        const unsigned upto = smask & (0xffffffffu >> (31 - lane));
-        const int head = upto ? 31 - __clz(upto) : 0;
-        float v = wv;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const float t = __shfl_up_sync(FULL, v, d);
-            if (lane - d >= head) v += t;
-        }
-        if (!upto && open) v += cws;                        // (the lanes that continue the carried run)
-        const bool nstart = lane < 31 && ((smask >> (lane + 1)) & 1u);
-        const bool last = lane == cnt - 1;
-        const bool final_pass = base + 32 >= nzz;
-        const bool done = valid && ((!last && nstart) || (last && final_pass));
-        unsigned dmask = __ballot_sync(FULL, done);
-        while (dmask) {
-            const int e = __ffs(dmask) - 1;
-            dmask &= dmask - 1;
-            deposit(__shfl_sync(FULL, g0, e), __shfl_sync(FULL, g1, e), __shfl_sync(FULL, v, e));
-        }
-        if (!final_pass) {
-            cg0 = __shfl_sync(FULL, g0, cnt - 1);
-            cg1 = __shfl_sync(FULL, g1, cnt - 1);
-            cws = __shfl_sync(FULL, v, cnt - 1);
-            open = true;
-        }
-    }
-}
-
-// The float32 path of the samples of thin sub-rings (one height, nzz = 1), 32 samples a warp: each lane sets up its
-// own sample (segment, pixel, box test, line centre, amplitude), then the warp deposits the samples in the box one
-// after another with its lanes over the channels. The same operations as k_an_model_fast on such a sample (one run
-// of one height: its weight is the height's), so the deposits are the same integers; the warp-uniform set-up that
-// k_an_model_fast repeats on 32 lanes for each sample is done once per lane here.
-__global__ void __launch_bounds__(ANF_WPB * 32, 4) k_an_model_thin(GridDev g, const AnSub *__restrict__ subs, int nsub,
-                                                                   const int *__restrict__ sbase,
-                                                                   const int *__restrict__ ssub,
-                                                                   const double2 *__restrict__ cs,
-                                                                   const float2 *__restrict__ csf,
-                                                                   const float4 *__restrict__ csff,
-                                                                   const long long *__restrict__ astart,
-                                                                   const int4 *__restrict__ aseg, int nseg,
-                                                                   long long ntot, const double *__restrict__ zq,
-                                                                   const float *__restrict__ zqf,
-                                                                   const float *__restrict__ wqf,
-                                                                   const float2 *__restrict__ vef,
-                                                                   const float *__restrict__ cd2if,
-                                                                   const float *__restrict__ ptabf,
-                                                                   const MemberDev *__restrict__ mem,
-                                                                   unsigned long long *__restrict__ out64,
-                                                                   long long mstride) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long gs = ((long long)blockIdx.x * ANF_WPB + w) * 32 + lane;
     const int nz = g.nz;
+    AnfSample *const sm = (AnfSample *)anf_smem + w * 32;
+    int2 *const run = (int2 *)(anf_smem + ANF_WPB * 32 * sizeof(AnfSample)) + w * ANF_RUNS;
+    float *const tab = (float *)(anf_smem + ANF_WPB * (32 * sizeof(AnfSample) + ANF_RUNS * sizeof(int2)));
+    float *const prof = tab + PHI_N + w * nz;
+    // (the lanes' channel edges are ~100 entries of the table apart: a gather, cheap in shared memory)
+    for (int i = threadIdx.x; i < PHI_N; i += ANF_WPB * 32) tab[i] = ptabf[i];
+    __syncthreads();
+    const long long gs = ((long long)blockIdx.x * ANF_WPB + w) * 32 + lane;
     bool ok = false;
-    int k0 = 0, nk = 0;
-    long long opix = 0;
-    float vrh = 0.0f, vrl = 0.0f, invf = 0.0f, amp = 0.0f, ws = 0.0f;
     AnSeg sg;
     if (an_seg(gs, astart, aseg, nseg, ntot, sbase, sg)) {
-        const long long s = sg.s;
-        const int ir = ssub[s];
+        const int s = (int)sg.s, ir = ssub[s];
         const AnSub &S = subs[(size_t)sg.src * nsub + ir];
         const float2 cf = csf[s];
-        const bool rec = cf.x >= 0.0f;
-        if (S.active && S.anfast && S.nzz == 1 && !(S.wzero & (rec ? 1 : 2))) {
-            const int kr = (int)(s - sbase[ir]) >= S.naz ? 1 : 0;
-            const PixF px = pix_setup(S, kr, cf, zqf + S.zq_off, 1);
-            int g0, g1;
-            sample_pixel(S, px, kr, cs + s, 1, 0.f, zq + S.zq_off, g.cdelt0, g.cdelt1, g0, g1);
-            const MemberDev &M = mem[sg.k];
-            if (g0 >= M.blo0 && g0 < M.bhi0 && g1 >= M.blo1 && g1 < M.bhi1) {
-                ff v;
-                const long long kc = fast_line_centre(S, g, csff[s], cs + s, v);
-                long long a0 = kc - S.K, a1 = kc + S.K + 1;
-                if (a0 < 0) a0 = 0;
-                if (a1 > nz) a1 = nz;
-                if (a1 > a0) {
-                    ok = true;
-                    k0 = (int)a0;
-                    nk = (int)(a1 - a0);
-                    const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
-                    vrh = vr.hi;
-                    vrl = vr.lo;
-                    invf = S.invf;
-                    amp = (float)sg.sign * ldexpf(S.af * (rec ? S.wrecf : S.wappf), M.fix_exp);
-                    ws = wqf[S.zq_off];
-                    opix = (long long)sg.k * mstride + ((long long)(g1 - M.blo1) * M.bx + (g0 - M.blo0)) * nz + k0;
-                }
+        const bool rec = cf.x >= 0.0f;                      // (the sign of the float32 table is the float64 test's)
+        if (S.active && S.anfast && !(S.wzero & (rec ? 1 : 2))) {
+            const int kr = s - sbase[ir] >= S.naz ? 1 : 0;
+            ff v;
+            const long long kc = fast_line_centre(S, g, csff[s], cs + s, v);
+            long long a0 = kc - S.K, a1 = kc + S.K + 1;
+            if (a0 < 0) a0 = 0;
+            if (a1 > nz) a1 = nz;
+            if (a1 > a0) {
+                ok = true;
+                AnfSample &o = sm[lane];
+                const PixF px = pix_setup(S, kr, cf, zqf + S.zq_off, S.nzz);
+                const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
+                o.vrh = vr.hi;
+                o.vrl = vr.lo;
+                o.invf = S.invf;
+                o.amp = (float)sg.sign * ldexpf(S.af * (rec ? S.wrecf : S.wappf), mem[sg.k].fix_exp);
+                o.bxf = px.bxf;
+                o.byf = px.byf;
+                o.zP3 = px.zP3;
+                o.zQ3 = px.zQ3;
+                o.hwx = px.fast ? px.hwx : -1.0f;
+                o.hwy = px.hwy;
+                o.k0 = (unsigned short)a0;
+                o.nk = (unsigned short)(a1 - a0);
+                o.off = S.zq_off;
+                o.nzz = S.nzz;
+                o.sub = sg.src * nsub + ir;
+                o.s = s | (kr << 31);
+                o.k = sg.k;
             }
         }
     }
     unsigned todo = __ballot_sync(FULL, ok);
-    while (todo) {
-        const int e = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const int ek0 = __shfl_sync(FULL, k0, e), enk = __shfl_sync(FULL, nk, e);
-        const float evh = __shfl_sync(FULL, vrh, e), evl = __shfl_sync(FULL, vrl, e);
-        const float einv = __shfl_sync(FULL, invf, e), eamp = __shfl_sync(FULL, amp, e);
-        const float ews = __shfl_sync(FULL, ws, e);
-        const long long eop = __shfl_sync(FULL, opix, e);
-        for (int j = lane; j < enk; j += 32) {
-            const float2 ea = __ldg(vef + ek0 + j), eb = __ldg(vef + ek0 + j + 1);
-            const float ta = (__fsub_rn(ea.x, evh) + __fsub_rn(ea.y, evl)) * einv;
-            const float tb = (__fsub_rn(eb.x, evh) + __fsub_rn(eb.y, evl)) * einv;
-            const float p = fabsf(phi_f32(tb, ptabf) - phi_f32(ta, ptabf)) * __ldg(cd2if + ek0 + j) * eamp;
-            const long long q = f32_to_ll(p * ews);
-            if (q) atomicAdd(out64 + eop + j, (unsigned long long)q);
+    __syncwarp();
+    for (; todo; todo &= todo - 1) {
+        const AnfSample &o = sm[__ffs(todo) - 1];
+        const int nk = o.nk, k0 = o.k0, nzz = o.nzz, off = o.off;
+        const PixF px{o.bxf, o.byf, o.zP3, o.zQ3, o.hwx, o.hwy, o.hwx > 0.0f};
+        const AnSub &S = subs[o.sub];
+        const double2 *cp = cs + (o.s & 0x7fffffff);
+        const int kr = (unsigned)o.s >> 31;
+        const MemberDev &M = mem[o.k];
+        const int blo0 = M.blo0, blo1 = M.blo1, bw = M.bx, bh = M.by;
+        unsigned long long *const o64 = out64 + (size_t)o.k * mstride + k0;
+        // the profile: a lane's upper edge is the next lane's lower one
+        bool big = false;
+        for (int j = lane; j - lane < nk; j += 31) {
+            const float2 e = __ldg(vef + k0 + min(j, nk));
+            const float ph = phi_f32((__fsub_rn(e.x, o.vrh) + __fsub_rn(e.y, o.vrl)) * o.invf, tab);
+            const float pn = __shfl_down_sync(FULL, ph, 1);
+            if (lane < 31 && j < nk) {
+                const float p = fabsf(pn - ph) * __ldg(cd2if + k0 + j) * o.amp;
+                prof[j] = p;
+                big |= !(fabsf(p) < 0.5f * ANF_FIXMAX);                          // (a weight is at most about 1)
+            }
+        }
+        big = __any_sync(FULL, big);
+        // the n runs of the list, their (run, channel) pairs over the lanes: 32 pairs on are dr runs and dj channels
+        int r0 = 0, j0 = lane, dr = 0, dj = 32;
+        while (j0 >= nk) {
+            j0 -= nk;
+            r0++;
+        }
+        while (dj >= nk) {
+            dj -= nk;
+            dr++;
+        }
+        auto deposit = [&](int n) {
+            const int2 *e = run + r0;
+            const int2 *const end = run + n;
+            int j = j0;
+            if (!big) {
+                while (e < end) {
+                    const int2 q = *e;
+                    atomicAdd(o64 + j + (long long)q.x * nz, f32_to_fix(prof[j] * __int_as_float(q.y)));
+                    j += dj;
+                    e += dr;
+                    if (j >= nk) {
+                        j -= nk;
+                        e++;
+                    }
+                }
+            } else {
+                while (e < end) {
+                    const int2 q = *e;
+                    atomicAdd(o64 + j + (long long)q.x * nz,
+                              (unsigned long long)f32_to_ll(prof[j] * __int_as_float(q.y)));
+                    j += dj;
+                    e += dr;
+                    if (j >= nk) {
+                        j -= nk;
+                        e++;
+                    }
+                }
+            }
+        };
+        bool open = false;                                  // a run carried from the previous pass
+        int cg0 = 0, cg1 = 0, nr = 0;
+        float cws = 0.0f;
+        for (int base = 0; base < nzz; base += 32) {
+            const int cnt = min(32, nzz - base);
+            const bool valid = lane < cnt;
+            int g0 = 0x7fffffff, g1 = 0x7fffffff;
+            float wv = 0.0f;
+            if (valid) {
+                sample_pixel(S, px, kr, cp, nzz, nzz > 1 ? __ldg(zqf + off + base + lane) : 0.f,
+                             zq + off + base + lane, g.cdelt0, g.cdelt1, g0, g1);
+                wv = __ldg(wqf + off + base + lane);
+            }
+            const int pg0 = __shfl_up_sync(FULL, g0, 1), pg1 = __shfl_up_sync(FULL, g1, 1);
+            const bool start = valid && (lane == 0 ? (!open || g0 != cg0 || g1 != cg1) : (g0 != pg0 || g1 != pg1));
+            const unsigned smask = __ballot_sync(FULL, start);
+            if (open && (smask & 1u)) {                     // the carried run ended with the previous pass
+                const int rx = cg0 - blo0, ry = cg1 - blo1;
+                if ((unsigned)rx < (unsigned)bw && (unsigned)ry < (unsigned)bh) {
+                    if (lane == 0) run[nr] = make_int2(ry * bw + rx, __float_as_int(cws));
+                    nr++;
+                }
+                open = false;
+            }
+            // segmented inclusive scan of the weights (a segment: from a run start to the lane before the next)
+            const unsigned upto = smask & (0xffffffffu >> (31 - lane));
+            const int head = upto ? 31 - __clz(upto) : 0;
+            float v = wv;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const float t = __shfl_up_sync(FULL, v, d);
+                if (lane - d >= head) v += t;
+            }
+            if (!upto && open) v += cws;                    // (the lanes that continue the carried run)
+            const bool nstart = lane < 31 && ((smask >> (lane + 1)) & 1u);
+            const bool last = lane == cnt - 1;
+            const bool final_pass = base + 32 >= nzz;
+            const bool done = valid && ((!last && nstart) || (last && final_pass));
+            const int rx = g0 - blo0, ry = g1 - blo1;
+            const bool put = done && (unsigned)rx < (unsigned)bw && (unsigned)ry < (unsigned)bh;
+            const unsigned pmask = __ballot_sync(FULL, put);
+            if (put) run[nr + __popc(pmask & ((1u << lane) - 1u))] = make_int2(ry * bw + rx, __float_as_int(v));
+            nr += __popc(pmask);
+            if (final_pass || nr > ANF_RUNS - 33) {
+                __syncwarp();
+                deposit(nr);
+                __syncwarp();
+                nr = 0;
+            }
+            if (!final_pass) {
+                cg0 = __shfl_sync(FULL, g0, cnt - 1);
+                cg1 = __shfl_sync(FULL, g1, cnt - 1);
+                cws = __shfl_sync(FULL, v, cnt - 1);
+                open = true;
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------ thin disks, by tiles of the sky
+// A batch whose sub-rings all have one height (nzz = 1) and the float32 path. Each sample falls in one pixel, so the
+// samples are listed by tile of pixels (k_ant_bin, a scan, k_ant_list) and a CTA takes a tile with all its channels:
+// it adds the deposits in shared memory (64-bit fixed point: any order) and writes the tile's float32 model. The sums
+// never leave the SM: no memset, no 64-bit model in HBM, no reductions in L2, no conversion pass. The deposits are
+// those of k_an_model_fast, integer for integer.
+#define ANT_NT 512
+#define ANT_BATCH 256                // samples of a tile in shared memory at a time
+
+// A sample as its tile deposits it: the line (velocity about vref in float-float, 1 / sig, amplitude in fixed-point
+// units), the weight of its height, its channels k0 .. k0 + nk and its pixel of the tile.
+struct __align__(16) AntSample {
+    float vrh, vrl, invf, amp, ws;
+    unsigned short k0, nk;
+    int pix, pad;
+};
+
+// one thread per sample of the batch's segments: the record, its tile (tiles of all members numbered from tile0[k];
+// -1: nothing to deposit) and its rank among the tile's samples (lanes of one tile count once)
+__global__ void __launch_bounds__(256) k_ant_bin(GridDev g, const AnSub *__restrict__ subs, int nsub,
+                                                 const int *__restrict__ sbase, const int *__restrict__ ssub,
+                                                 const double2 *__restrict__ cs, const float2 *__restrict__ csf,
+                                                 const float4 *__restrict__ csff, const long long *__restrict__ astart,
+                                                 const int4 *__restrict__ aseg, int nseg, long long ntot, int ltx,
+                                                 int lty, const int *__restrict__ tile0,
+                                                 const double *__restrict__ zq, const float *__restrict__ zqf,
+                                                 const float *__restrict__ wqf, const MemberDev *__restrict__ mem,
+                                                 AntSample *__restrict__ rec, int2 *__restrict__ where,
+                                                 int *__restrict__ count) {
+    const int lane = threadIdx.x & 31;
+    const long long gs = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    int tile = -1;
+    AnSeg sg;
+    if (an_seg(gs, astart, aseg, nseg, ntot, sbase, sg)) {
+        const int s = (int)sg.s, ir = ssub[s];
+        const AnSub &S = subs[(size_t)sg.src * nsub + ir];
+        const float2 cf = csf[s];
+        const bool rcd = cf.x >= 0.0f;                      // (the sign of the float32 table is the float64 test's)
+        if (S.active && !(S.wzero & (rcd ? 1 : 2))) {
+            const int kr = s - sbase[ir] >= S.naz ? 1 : 0;
+            const PixF px = pix_setup(S, kr, cf, zqf + S.zq_off, 1);
+            int g0, g1;
+            sample_pixel(S, px, kr, cs + s, 1, 0.f, zq + S.zq_off, g.cdelt0, g.cdelt1, g0, g1);
+            const MemberDev &M = mem[sg.k];
+            g0 -= M.blo0;
+            g1 -= M.blo1;
+            if ((unsigned)g0 < (unsigned)M.bx && (unsigned)g1 < (unsigned)M.by) {
+                ff v;
+                const long long kc = fast_line_centre(S, g, csff[s], cs + s, v);
+                long long a0 = kc - S.K, a1 = kc + S.K + 1;
+                if (a0 < 0) a0 = 0;
+                if (a1 > g.nz) a1 = g.nz;
+                if (a1 > a0) {
+                    const int ntx = (M.bx + (1 << ltx) - 1) >> ltx;
+                    tile = tile0[sg.k] + (g1 >> lty) * ntx + (g0 >> ltx);
+                    const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
+                    AntSample o;
+                    o.vrh = vr.hi;
+                    o.vrl = vr.lo;
+                    o.invf = S.invf;
+                    o.amp = (float)sg.sign * ldexpf(S.af * (rcd ? S.wrecf : S.wappf), M.fix_exp);
+                    o.ws = wqf[S.zq_off];
+                    o.k0 = (unsigned short)a0;
+                    o.nk = (unsigned short)(a1 - a0);
+                    o.pix = ((g1 & ((1 << lty) - 1)) << ltx) + (g0 & ((1 << ltx) - 1));
+                    o.pad = 0;
+                    rec[gs] = o;
+                }
+            }
+        }
+    }
+    // consecutive samples mostly share a tile: one atomic for each of the warp's tiles
+    const unsigned same = __match_any_sync(FULL, tile);
+    int r = 0;
+    if (tile >= 0 && lane == __ffs(same) - 1) r = atomicAdd(count + tile, __popc(same));
+    r = __shfl_sync(FULL, r, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
+    if (gs < ntot) where[gs] = make_int2(tile, r);
+}
+
+__global__ void k_ant_list(const int2 *__restrict__ where, long long ntot, const int *__restrict__ offset,
+                           int *__restrict__ order) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= ntot) return;
+    const int2 t = where[i];
+    if (t.x >= 0) order[offset[t.x] + t.y] = (int)i;
+}
+
+// The tiles of the members [kfirst, kfirst + nk) (tiles tile0[kfirst] .. tile0[kfirst + nk)), a CTA after another:
+// persistent, so that the CDF table is read into shared memory once. The channel edges of a batch of samples are laid
+// end to end and the warps take equal parts of them, a lane an edge (a lane's upper edge is the next lane's, so a
+// warp advances by 31): no lane idles for the samples' 5 to 100 channels, whatever they are. base64: member 0's sums
+// in its box, written with base_out (by a launch of member 0 alone), else added to the members with mbase >= 0.
+__global__ void __launch_bounds__(ANT_NT, 2) k_ant_tile(int nz, int ltx, int lty, const int *__restrict__ tile0,
+                                                        int kfirst, int nk, const int *__restrict__ offset,
+                                                        const int *__restrict__ count, const int *__restrict__ order,
+                                                        const AntSample *__restrict__ rec,
+                                                        const float2 *__restrict__ vef,
+                                                        const float *__restrict__ cd2if,
+                                                        const float *__restrict__ ptabf,
+                                                        const MemberDev *__restrict__ mem, float *__restrict__ model,
+                                                        double *__restrict__ model64, long long mstride,
+                                                        long long *__restrict__ base64, int base_out,
+                                                        const int *__restrict__ mbase) {
+    extern __shared__ __align__(16) unsigned long long ant_acc[];   // (pixel, channel); channel edges; factors; CDF
+    __shared__ AntSample rs[ANT_BATCH];
+    __shared__ int pre[ANT_BATCH + 1], wsum[ANT_BATCH / 32], nedge; // first edge of each sample
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int npix = 1 << (ltx + lty), tx = 1 << ltx, nacc = npix * nz;
+    float2 *const ved = (float2 *)(ant_acc + nacc);
+    float *const cdf = (float *)(ved + nz + 1), *const tab = cdf + nz;
+    float cdmax = 0.0f;
+    for (int i = tid; i < PHI_N; i += ANT_NT) tab[i] = ptabf[i];
+    for (int i = tid; i < nacc; i += ANT_NT) ant_acc[i] = 0;
+    for (int i = tid; i <= nz; i += ANT_NT) ved[i] = vef[i];
+    for (int i = tid; i < nz; i += ANT_NT) cdf[i] = cd2if[i];
+    for (int i = 0; i < nz; i++) cdmax = fmaxf(cdmax, fabsf(__ldg(cd2if + i)));
+    if (tid == 0) pre[0] = 0;
+    const int tend = tile0[kfirst + nk];
+    int k = kfirst;
+    for (int t = tile0[kfirst] + blockIdx.x; t < tend; t += gridDim.x) {
+        while (t >= tile0[k + 1]) k++;
+        const MemberDev &M = mem[k];
+        const int bx = M.bx, ntx = (bx + tx - 1) >> ltx, tl = t - tile0[k];
+        const int uy = tl / ntx, ux = (tl - uy * ntx) << ltx;
+        const int pw = min(tx, bx - ux), ph = min(1 << lty, M.by - (uy << lty));
+        const int n = count[t], o0 = offset[t];
+        for (int b0 = 0; b0 < n; b0 += ANT_BATCH) {
+            const int m = min(ANT_BATCH, n - b0);
+            __syncthreads();                                // (the batch or the tile before is done with)
+            int len = 0;
+            bool big = false;                               // (a deposit that may need f32_to_ll)
+            if (tid < m) {
+                const AntSample q = rec[order[o0 + b0 + tid]];
+                rs[tid] = q;
+                len = q.nk + 1;
+                big = !(fabsf(q.amp) * cdmax * q.ws < 0.5f * ANF_FIXMAX);
+            }
+            if (tid < ANT_BATCH) {
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(FULL, len, d);
+                    if (lane >= d) len += v;
+                }
+                if (lane == 31) wsum[w] = len;
+            }
+            __syncthreads();
+            if (tid < ANT_BATCH) {
+                for (int i = 0; i < w; i++) len += wsum[i];
+                pre[tid + 1] = tid < m - 1 ? len : 0x7fffffff;      // (the last sample has no end: nc stops it)
+                if (tid == m - 1) nedge = len;
+            }
+            big = __syncthreads_or(big);
+            const int ne = nedge, nwin = (ne + 30) / 31, per = (nwin + ANT_NT / 32 - 1) / (ANT_NT / 32);
+            const int w0 = w * per, w1 = min(nwin, w0 + per);
+            int pos = w0 * 31 + lane, e = 0;
+            if (w0 < w1) {
+                int hi = m - 1;                             // the sample of the lane's first edge
+                while (e < hi) {
+                    const int mid = (e + hi + 1) >> 1;
+                    if (pre[mid] <= pos) e = mid;
+                    else hi = mid - 1;
+                }
+            }
+            int first = pre[e], next = pre[e + 1];
+            for (int win = w0; win < w1; win++, pos += 31) {
+                while (pos >= next) {
+                    first = next;
+                    next = pre[++e + 1];
+                }
+                const AntSample &q = rs[e];
+                const int j = pos - first, nc = q.nk, c = q.k0 + min(j, nc);
+                const float2 ed = ved[c];
+                const float f = phi_f32((__fsub_rn(ed.x, q.vrh) + __fsub_rn(ed.y, q.vrl)) * q.invf, tab);
+                const float fn = __shfl_down_sync(FULL, f, 1);
+                if (lane < 31 && j < nc) {
+                    const float x = fabsf(fn - f) * cdf[c] * q.amp * q.ws;
+                    unsigned long long *const a = ant_acc + (q.pix * nz + c);
+                    if (!big) atomicAdd(a, f32_to_fix(x));
+                    else atomicAdd(a, (unsigned long long)f32_to_ll(x));
+                }
+            }
+        }
+        __syncthreads();
+        const long long *bas = !base_out && mbase[k] >= 0 ? base64 : nullptr;
+        const int e = M.fix_exp;
+        for (int p = w; p < npix; p += ANT_NT / 32) {       // a warp a pixel: lanes over channels
+            const int py = p >> ltx, pxx = p & (tx - 1);
+            if (pxx >= pw || py >= ph) continue;
+            const long long at = ((long long)((uy << lty) + py) * bx + ux + pxx) * nz;
+            float *out = model + (size_t)k * mstride + at;
+            for (int c = lane; c < nz; c += 32) {
+                unsigned long long q = ant_acc[p * nz + c];
+                ant_acc[p * nz + c] = 0;
+                if (base_out) base64[at + c] = (long long)q;
+                if (bas) q += (unsigned long long)bas[at + c];
+                out[c] = fix_to_f32((long long)q, e);
+                if (model64)
+                    model64[(size_t)k * mstride + at + c] = __dmul_rn((double)(long long)q, ldexp(1.0, -e));
+            }
         }
     }
 }
@@ -587,14 +828,14 @@ __global__ void k_fix_to_model(const long long *__restrict__ in, const MemberDev
     const int k = blockIdx.y;
     const MemberDev &M = mem[k];
     const long long n = (long long)M.by * M.bx * nz;
-    const double sc = ldexp(1.0, -M.fix_exp);
+    const int e = M.fix_exp;
+    const long long *src = in + (size_t)k * mstride;
     const long long *bas = mbase && mbase[k] >= 0 ? in + (size_t)mbase[k] * mstride : nullptr;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long q = in[(size_t)k * mstride + i];
+        long long q = src[i];
         if (bas) q = (long long)((unsigned long long)q + (unsigned long long)bas[i]);
-        const double v = __dmul_rn((double)q, sc);
-        model[(size_t)k * mstride + i] = (float)v;
-        if (model64) model64[(size_t)k * mstride + i] = v;
+        model[(size_t)k * mstride + i] = fix_to_f32(q, e);
+        if (model64) model64[(size_t)k * mstride + i] = __dmul_rn((double)q, ldexp(1.0, -e));
     }
 }
 
@@ -615,29 +856,64 @@ void launch_an_model(cudaStream_t s, const GridDev &g, const AnSub *subs, int ns
         ptab, mem, (unsigned long long *)out64, mstride, skip_fast);
 }
 
-size_t an_fast_smem_bytes(int nz) { return (size_t)ANF_WPB * 2 * (nz + 2) * sizeof(float); }
-
 void launch_an_model_fast(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase,
                           const int *ssub, const double *cs, const float *csf, const float *csff,
                           const long long *astart, const int *aseg, int nseg, long long ntot,
                           const double *zq, const float *zqf, const float *wqf, const float *vef, const float *cd2if,
-                          const float *ptabf, const MemberDev *mem, long long *out64, long long mstride, int thin,
-                          int thick) {
-    const long long nw = ntot;
-    if (nw == 0 || nseg == 0) return;
-    if (thin)
-        k_an_model_thin<<<(unsigned)((nw + 32 * ANF_WPB - 1) / (32 * ANF_WPB)), ANF_WPB * 32, 0, s>>>(
-            g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, (const float4 *)csff, astart,
-            (const int4 *)aseg, nseg, ntot, zq, zqf, wqf, (const float2 *)vef, cd2if, ptabf, mem,
-            (unsigned long long *)out64, mstride);
-    if (!thick) return;
-    const size_t smem = an_fast_smem_bytes(g.nz);
-    if (smem > 48 * 1024)
-        cudaFuncSetAttribute(k_an_model_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_an_model_fast<<<(unsigned)((nw + ANF_WPB - 1) / ANF_WPB), ANF_WPB * 32, smem, s>>>(
+                          const float *ptabf, const MemberDev *mem, long long *out64, long long mstride) {
+    if (ntot == 0 || nseg == 0) return;
+    const long long per = 32 * ANF_WPB;
+    const size_t smem = ANF_WPB * (32 * sizeof(AnfSample) + ANF_RUNS * sizeof(int2)) + (PHI_N + (size_t)ANF_WPB * g.nz) * 4;
+    cudaFuncSetAttribute(k_an_model_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_an_model_fast<<<(unsigned)((ntot + per - 1) / per), ANF_WPB * 32, smem, s>>>(
         g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, (const float4 *)csff, astart,
-        (const int4 *)aseg, nseg, ntot, zq, zqf, wqf,
-        (const float2 *)vef, cd2if, ptabf, mem, (unsigned long long *)out64, mstride, thin);
+        (const int4 *)aseg, nseg, ntot, zq, zqf, wqf, (const float2 *)vef, cd2if, ptabf, mem,
+        (unsigned long long *)out64, mstride);
+}
+
+// The tile of the thin batches, 2^ltx x 2^lty pixels: the largest whose sums and the CDF table leave room for two CTAs
+// on an SM (103 KB each beside the samples), else one that fits at all; smaller, down to 2 x 2, while the npix pixels
+// of the batch give the SMs fewer than 4 tiles each. False for more channels than a pixel's sums fit.
+#define ANT_TAB (PHI_N * 4 + 16)
+static size_t ant_smem(int nz, int ltx, int lty) { return ((size_t)nz << (ltx + lty)) * 8 + (size_t)nz * 12 + ANT_TAB; }
+bool an_tile_size(int nz, long long npix, int &ltx, int &lty) {
+    for (int most : {103 * 1024, AN_SMEM_MAX})
+        for (int l = 8; l >= (most == AN_SMEM_MAX ? 0 : 4); l--) {
+            ltx = (l + 1) / 2;
+            lty = l / 2;
+            if (ant_smem(nz, ltx, lty) > (size_t)most || (l > 2 && (npix >> l) < 4 * 152)) continue;
+            return nz < 65536;
+        }
+    return false;
+}
+
+void launch_ant_bin(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
+                    const double *cs, const float *csf, const float *csff, const long long *astart, const int *aseg,
+                    int nseg, long long ntot, int ltx, int lty, const int *tile0, const double *zq, const float *zqf,
+                    const float *wqf, const MemberDev *mem, void *rec, int *where, int *count) {
+    if (ntot == 0 || nseg == 0) return;
+    k_ant_bin<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(
+        g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, (const float4 *)csff, astart,
+        (const int4 *)aseg, nseg, ntot, ltx, lty, tile0, zq, zqf, wqf, mem, (AntSample *)rec, (int2 *)where, count);
+}
+
+void launch_ant_list(cudaStream_t s, const int *where, long long ntot, const int *offset, int *order) {
+    if (ntot == 0) return;
+    k_ant_list<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>((const int2 *)where, ntot, offset, order);
+}
+
+void launch_ant_tile(cudaStream_t s, int nz, int ltx, int lty, const int *tile0, int kfirst, int nk, int ntile,
+                     const int *offset, const int *count, const int *order, const void *rec, const float *vef,
+                     const float *cd2if, const float *ptabf, const MemberDev *mem, float *model, double *model64,
+                     long long mstride, long long *base64, int base_out, const int *mbase) {
+    if (nk <= 0 || ntile <= 0) return;
+    const size_t smem = ant_smem(nz, ltx, lty);
+    cudaFuncSetAttribute(k_ant_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ant_tile, ANT_NT, smem);
+    k_ant_tile<<<std::min(ntile, 152 * std::max(per, 1)), ANT_NT, smem, s>>>(
+        nz, ltx, lty, tile0, kfirst, nk, offset, count, order, (const AntSample *)rec, (const float2 *)vef, cd2if,
+        ptabf, mem, model, model64, mstride, base64, base_out, mbase);
 }
 
 void launch_an_maps(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,

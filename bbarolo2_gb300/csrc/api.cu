@@ -170,9 +170,18 @@ struct bbgpu_ctx {
     long long an_ntot = 0;
     std::vector<long long> h_astart;
     std::vector<int> h_aseg, h_mbase, asbase_host;
+    // thin batches: the tiles (an_ltx, an_lty; first tile of each member), the samples' records, tiles and lists
+    int an_ltx = 0, an_lty = 0;
+    std::vector<int> h_atile0;
+    int *d_awhere = nullptr, *d_acount = nullptr, *d_aorder = nullptr, *d_ascan = nullptr;
+    uint8_t *d_arec = nullptr;
+    size_t d_awhere_cap = 0, d_acount_cap = 0, d_aorder_cap = 0, d_arec_cap = 0, d_ascan_cap = 0;
+    // the tables of an_segments, one upload from pinned memory (ev_tab: it has left it): astart, aseg, mbase, atile0
+    uint8_t *h_atab = nullptr, *d_atab = nullptr;
+    size_t h_atab_cap = 0, d_atab_cap = 0;
+    cudaEvent_t ev_tab = nullptr;
     long long *d_astart = nullptr;
-    int *d_aseg = nullptr, *d_mbase = nullptr;
-    size_t d_astart_cap = 0, d_aseg_cap = 0, d_mbase_cap = 0;
+    int *d_aseg = nullptr, *d_mbase = nullptr, *d_atile0 = nullptr;
     std::vector<unsigned long long> h_chg; // per member: the sub-rings a replaying member deposits itself
     int nchw = 0;
     int *d_rp_rec = nullptr, *d_rp_n = nullptr;   // (2 ints a record; records per list of member 0)
@@ -199,7 +208,7 @@ struct bbgpu_ctx {
     // ANALYTIC batches: sub-ring constants per member, the sample table of the model's sub-rings, their vertical
     // grids (host cache mirrored on the device) and the fixed-point models
     AnSub *h_asub = nullptr, *d_asub = nullptr;
-    int an_thin = 0, an_thick = 0, an_exact = 1;   // the ANALYTIC kernels the uploaded batch needs
+    int an_thick = 0, an_exact = 1, an_tile = 0;   // the ANALYTIC kernels the uploaded batch needs
     size_t h_asub_cap = 0, d_asub_cap = 0;
     int *d_asbase = nullptr, *d_assub = nullptr;
     size_t d_asbase_cap = 0, d_assub_cap = 0;
@@ -557,13 +566,15 @@ extern "C" int bbgpu_ctx_destroy(bbgpu_ctx *ctx) {
                     (void *)ctx->d_cstart, (void *)ctx->d_base64, (void *)ctx->d_cseg, (void *)ctx->d_klist,
                     (void *)ctx->d_tsrc, (void *)ctx->d_blk, (void *)ctx->d_ktab, (void *)ctx->d_gflag,
                     (void *)ctx->d_rp_rec, (void *)ctx->d_rp_cnt, (void *)ctx->d_chg, (void *)ctx->d_rp_n,
-                    (void *)ctx->d_astart, (void *)ctx->d_aseg, (void *)ctx->d_mbase, (void *)ctx->d_tmask})
+                    (void *)ctx->d_atab, (void *)ctx->d_tmask, (void *)ctx->d_awhere, (void *)ctx->d_acount, (void *)ctx->d_aorder,
+                    (void *)ctx->d_ascan, (void *)ctx->d_arec})
         cudaFree(q);
     for (void *q : {(void *)ctx->d_asub, (void *)ctx->d_asbase, (void *)ctx->d_assub, (void *)ctx->d_acs,
                     (void *)ctx->d_azq, (void *)ctx->d_awq, (void *)ctx->d_model_fx, (void *)ctx->d_acsf,
                     (void *)ctx->d_azqf, (void *)ctx->d_awqf, (void *)ctx->d_acsff})
         cudaFree(q);
     cudaFreeHost(ctx->h_asub);
+    cudaFreeHost(ctx->h_atab);
     cudaFreeHost(ctx->h_reuse);
     cudaFreeHost(ctx->h_preuse);
     cudaFree(ctx->d_reuse);
@@ -573,6 +584,7 @@ extern "C" int bbgpu_ctx_destroy(bbgpu_ctx *ctx) {
     for (int i = 0; i <= NTIMER; i++)
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+    if (ctx->ev_tab) cudaEventDestroy(ctx->ev_tab);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -953,7 +965,6 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
     if ((rc = dgrow(ctx, &ctx->d_asub, &ctx->d_asub_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_mem, &ctx->d_mem_cap, (size_t)nb))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_model, &ctx->d_model_cap, (size_t)nb * ctx->mstride))) return rc;
-    if ((rc = dgrow(ctx, &ctx->d_model_fx, &ctx->d_model_fx_cap, (size_t)nb * ctx->mstride))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_partial, &ctx->d_partial_cap, (size_t)2 * nb * (ctx->npart ? ctx->npart : 1)))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_out2, &ctx->d_out2_cap, (size_t)2 * nb))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_out2, &ctx->h_out2_cap, (size_t)2 * nb))) return rc;
@@ -962,17 +973,26 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
     if (ctx->want64)
         if ((rc = dgrow(ctx, &ctx->d_model64, &ctx->d_model64_cap, (size_t)nb * ctx->mstride))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_reuse, &ctx->d_reuse_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
-    // which ANALYTIC kernels the batch needs: the float32 path of thin sub-rings (one height), of thick ones, the
-    // exact kernel for the others (a reused column is member 0's, whose flags count already)
-    ctx->an_thin = ctx->an_thick = ctx->an_exact = 0;
+    // which ANALYTIC kernels the batch needs: the tile kernels where every sub-ring is thin (one height) with the float32
+    // path, else the float32 path by samples, and the exact kernel for the sub-rings it does not take (a reused column
+    // is member 0's, whose flags count already). Thin disks: the tiles took less time than the samples (and the
+    // conversion pass these need) at every size tried, 63 against 65 us for one 64x64x64 member, 7.5 against 13.7 ms
+    // for 64 members of 256x256x192. A thick sub-ring's sample crosses many tiles, each of which would find its runs
+    // again: by samples only.
+    ctx->an_thick = ctx->an_exact = 0;
     for (size_t i = 0; i < (size_t)nb * nsub; i++) {
         if (ctx->h_reuse[i]) continue;
         const AnSub &S = ctx->h_asub[i];
         if (!S.active) continue;
         if (!S.anfast) ctx->an_exact = 1;
-        else if (S.nzz == 1) ctx->an_thin = 1;
-        else ctx->an_thick = 1;
+        else if (S.nzz > 1) ctx->an_thick = 1;
     }
+    long long npix = 0;
+    for (int k = 0; k < nb; k++) npix += (long long)ctx->mem_host[k].bx * ctx->mem_host[k].by;
+    ctx->an_tile = !ctx->an_thick && !ctx->an_exact && nb * ctx->ansamp < (1LL << 31) - 1 &&
+                   an_tile_size(g.nz, npix, ctx->an_ltx, ctx->an_lty);
+    if (!ctx->an_tile)
+        if ((rc = dgrow(ctx, &ctx->d_model_fx, &ctx->d_model_fx_cap, (size_t)nb * ctx->mstride))) return rc;
     CK(cudaMemcpyAsync(ctx->d_asub, ctx->h_asub, sizeof(AnSub) * (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_mem, ctx->h_mem, sizeof(MemberDev) * (size_t)nb, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_reuse, ctx->h_reuse, (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
@@ -1326,15 +1346,46 @@ static int an_segments(bbgpu_ctx *ctx) {
     ctx->an_ntot = tot;
     ctx->an_n2 = n2;
     int rc;
-    if ((rc = dgrow(ctx, &ctx->d_astart, &ctx->d_astart_cap, cs.size())) ||
-        (rc = dgrow(ctx, &ctx->d_aseg, &ctx->d_aseg_cap, sg.size() + 4)) ||
-        (rc = dgrow(ctx, &ctx->d_mbase, &ctx->d_mbase_cap, (size_t)nb)))
-        return rc;
     cudaStream_t s = ctx->stream;
-    CK(cudaMemcpyAsync(ctx->d_astart, cs.data(), sizeof(long long) * cs.size(), cudaMemcpyHostToDevice, s));
-    if (!sg.empty()) CK(cudaMemcpyAsync(ctx->d_aseg, sg.data(), sizeof(int) * sg.size(), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->d_mbase, mb.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, s));
-    CK(cudaStreamSynchronize(s));     // (the host vectors change with the next batch)
+    std::vector<int> &t0 = ctx->h_atile0;
+    t0.assign(1, 0);
+    if (ctx->an_tile) {
+        const int tx = 1 << ctx->an_ltx, ty = 1 << ctx->an_lty;
+        for (const MemberDev &M : ctx->mem_host)
+            t0.push_back(t0.back() + ((M.bx + tx - 1) / tx) * ((M.by + ty - 1) / ty));
+        const size_t nt = (size_t)t0[nb] + 1, n = (size_t)tot + 1;
+        if ((rc = dgrow(ctx, &ctx->d_acount, &ctx->d_acount_cap, 3 * nt)) ||
+            (rc = dgrow(ctx, &ctx->d_ascan, &ctx->d_ascan_cap, nt / 1024 + 2)) ||
+            (rc = dgrow(ctx, &ctx->d_awhere, &ctx->d_awhere_cap, 2 * n)) ||
+            (rc = dgrow(ctx, &ctx->d_aorder, &ctx->d_aorder_cap, n)) ||
+            (rc = dgrow(ctx, &ctx->d_arec, &ctx->d_arec_cap, ANT_REC * n)))
+            return rc;
+        if (n2)
+            if ((rc = dgrow(ctx, &ctx->d_base64, &ctx->d_base64_cap, (size_t)M0.bx * M0.by * ctx->g.nz + 1))) return rc;
+    }
+    // (the tables at 16-byte offsets of one buffer)
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (n + 15) & ~(size_t)15;
+        return at;
+    };
+    const size_t o_seg = place(sizeof(int) * sg.size()), o_start = place(sizeof(long long) * cs.size()),
+                 o_base = place(sizeof(int) * mb.size()), o_tile = place(sizeof(int) * t0.size());
+    if (!ctx->ev_tab) CK(cudaEventCreateWithFlags(&ctx->ev_tab, cudaEventDisableTiming));
+    CK(cudaEventSynchronize(ctx->ev_tab));                   // (the last upload has left the pinned buffer)
+    if ((rc = hgrow(ctx, &ctx->h_atab, &ctx->h_atab_cap, bytes))) return rc;
+    if ((rc = dgrow(ctx, &ctx->d_atab, &ctx->d_atab_cap, bytes))) return rc;
+    ctx->d_aseg = (int *)(ctx->d_atab + o_seg);
+    ctx->d_astart = (long long *)(ctx->d_atab + o_start);
+    ctx->d_mbase = (int *)(ctx->d_atab + o_base);
+    ctx->d_atile0 = (int *)(ctx->d_atab + o_tile);
+    if (!sg.empty()) memcpy(ctx->h_atab + o_seg, sg.data(), sizeof(int) * sg.size());
+    memcpy(ctx->h_atab + o_start, cs.data(), sizeof(long long) * cs.size());
+    memcpy(ctx->h_atab + o_base, mb.data(), sizeof(int) * mb.size());
+    memcpy(ctx->h_atab + o_tile, t0.data(), sizeof(int) * t0.size());
+    CK(cudaMemcpyAsync(ctx->d_atab, ctx->h_atab, bytes, cudaMemcpyHostToDevice, s));
+    CK(cudaEventRecord(ctx->ev_tab, s));
     ctx->an_dirty = false;
     return 0;
 }
@@ -1523,21 +1574,47 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
             int rc = an_segments(ctx);
             if (rc) return rc;
         }
-        CK(cudaMemsetAsync(ctx->d_model_fx, 0, sizeof(long long) * (size_t)ctx->nb * ctx->mstride, s));
-        launch_an_model_fast(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_acsf,
-                             (const float *)ctx->d_acsff, ctx->d_astart, ctx->d_aseg, ctx->an_nseg, ctx->an_ntot,
-                             ctx->d_azq, ctx->d_azqf, ctx->d_awqf, (const float *)ctx->d_vef, ctx->d_cd2if,
-                             ctx->d_ptabf, ctx->d_mem, ctx->d_model_fx, ctx->mstride, ctx->an_thin, ctx->an_thick);
-        CKL();
-        if (ctx->an_exact) {
-            launch_an_model(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_astart,
-                            ctx->d_aseg, ctx->an_nseg, ctx->an_ntot, ctx->d_azq, ctx->d_awq, ctx->d_vedges,
-                            ctx->d_cd2i, ctx->d_ptab, ctx->d_mem, ctx->d_model_fx, ctx->mstride, 1);
+        if (ctx->an_tile) {
+            const std::vector<int> &t0 = ctx->h_atile0;
+            const int nt = t0[ctx->nb];
+            int *count = ctx->d_acount, *offset = count + nt + 1;
+            CK(cudaMemsetAsync(count, 0, sizeof(int) * (nt + 1), s));
+            launch_ant_bin(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_acsf,
+                           (const float *)ctx->d_acsff, ctx->d_astart, ctx->d_aseg, ctx->an_nseg, ctx->an_ntot,
+                           ctx->an_ltx, ctx->an_lty, ctx->d_atile0, ctx->d_azq, ctx->d_azqf, ctx->d_awqf, ctx->d_mem,
+                           ctx->d_arec, ctx->d_awhere, count);
+            CKL();
+            launch_scan_tiles(s, count, offset, offset + nt + 1, nt, ctx->d_ascan);
+            CKL();
+            launch_ant_list(s, ctx->d_awhere, ctx->an_ntot, offset, ctx->d_aorder);
+            CKL();
+            // (members that add member 0's sums: member 0 first)
+            const int first = ctx->an_n2 ? 1 : 0;
+            for (int pass = first ? 0 : 1; pass < 2; pass++) {
+                const int k0 = pass ? first : 0, nk = pass ? ctx->nb - first : 1;
+                launch_ant_tile(s, g.nz, ctx->an_ltx, ctx->an_lty, ctx->d_atile0, k0, nk, t0[k0 + nk] - t0[k0], offset,
+                                count, ctx->d_aorder, ctx->d_arec, (const float *)ctx->d_vef, ctx->d_cd2if,
+                                ctx->d_ptabf, ctx->d_mem, ctx->d_model, ctx->want64 ? ctx->d_model64 : nullptr,
+                                ctx->mstride, ctx->d_base64, pass ? 0 : 1, ctx->d_mbase);
+                CKL();
+            }
+        } else {
+            CK(cudaMemsetAsync(ctx->d_model_fx, 0, sizeof(long long) * (size_t)ctx->nb * ctx->mstride, s));
+            launch_an_model_fast(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_acsf,
+                                 (const float *)ctx->d_acsff, ctx->d_astart, ctx->d_aseg, ctx->an_nseg, ctx->an_ntot,
+                                 ctx->d_azq, ctx->d_azqf, ctx->d_awqf, (const float *)ctx->d_vef, ctx->d_cd2if,
+                                 ctx->d_ptabf, ctx->d_mem, ctx->d_model_fx, ctx->mstride);
+            CKL();
+            if (ctx->an_exact) {
+                launch_an_model(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_astart,
+                                ctx->d_aseg, ctx->an_nseg, ctx->an_ntot, ctx->d_azq, ctx->d_awq, ctx->d_vedges,
+                                ctx->d_cd2i, ctx->d_ptab, ctx->d_mem, ctx->d_model_fx, ctx->mstride, 1);
+                CKL();
+            }
+            launch_fix_to_model(s, ctx->d_model_fx, ctx->d_mem, ctx->nb, ctx->mstride, g.nz, ctx->d_model,
+                                ctx->want64 ? ctx->d_model64 : nullptr, ctx->an_n2 ? ctx->d_mbase : nullptr);
             CKL();
         }
-        launch_fix_to_model(s, ctx->d_model_fx, ctx->d_mem, ctx->nb, ctx->mstride, g.nz, ctx->d_model,
-                            ctx->want64 ? ctx->d_model64 : nullptr, ctx->an_n2 ? ctx->d_mbase : nullptr);
-        CKL();
         if (tm) CK(cudaEventRecord(ctx->ev[11], s));
     } else {
         const LayoutDev &L = ctx->cur->dev;

@@ -199,13 +199,29 @@ void launch_an_model(cudaStream_t s, const GridDev &g, const AnSub *subs, int ns
 // csf, zqf, wqf float32 copies of the sample and vertical tables, csff (float4 per sample) its cos and sin in
 // float-float, vef (nz + 1) float-float channel edges of line 0
 // relative to g.vref, ptabf the normal CDF table in float32
-size_t an_fast_smem_bytes(int nz);
 void launch_an_model_fast(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase,
                           const int *ssub, const double *cs, const float *csf, const float *csff,
                           const long long *astart, const int *aseg, int nseg, long long ntot,
                           const double *zq, const float *zqf, const float *wqf, const float *vef, const float *cd2if,
-                          const float *ptabf, const MemberDev *mem, long long *out64, long long mstride, int thin,
-                          int thick);
+                          const float *ptabf, const MemberDev *mem, long long *out64, long long mstride);
+// The same models where every sub-ring has one height and the float32 path (a thin disk), by tiles of 2^ltx x 2^lty
+// pixels (an_tile_size: for nz channels and the
+// npix pixels of a batch; false where a pixel's sums do not fit): the samples of the segments listed by
+// tile (launch_ant_bin: records rec of ANT_REC bytes, where (tile, rank), count per tile, zeroed by the caller; the
+// scan of the counts; launch_ant_list: order), then the tiles of the members kfirst .. kfirst + nk - 1 (ntile of them;
+// tile0[k]: member k's first tile, nb + 1 entries) deposit theirs and write the float32 model. base64: with base_out
+// (nk = 1) receives the member's sums, else it is added to the members with mbase >= 0.
+#define ANT_REC 32
+bool an_tile_size(int nz, long long npix, int &ltx, int &lty);
+void launch_ant_bin(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
+                    const double *cs, const float *csf, const float *csff, const long long *astart, const int *aseg,
+                    int nseg, long long ntot, int ltx, int lty, const int *tile0, const double *zq, const float *zqf,
+                    const float *wqf, const MemberDev *mem, void *rec, int *where, int *count);
+void launch_ant_list(cudaStream_t s, const int *where, long long ntot, const int *offset, int *order);
+void launch_ant_tile(cudaStream_t s, int nz, int ltx, int lty, const int *tile0, int kfirst, int nk, int ntile,
+                     const int *offset, const int *count, const int *order, const void *rec, const float *vef,
+                     const float *cd2if, const float *ptabf, const MemberDev *mem, float *model, double *model64,
+                     long long mstride, long long *base64, int base_out, const int *mbase);
 void launch_an_maps(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
                     const double *cs, long long nsamp, const double *zq, const double *wq, const long long *widx,
                     const double *wval, const MemberDev &M, long long *maps64);

@@ -240,6 +240,7 @@ struct bbgpu_ctx {
     void *d_bimg = nullptr;               // its B operand image for conv_variant
     size_t d_bimg_cap = 0;
     int bimg_variant = 0;
+    void *d_wsjump = nullptr;             // GALWIND's streams: the jumps of k_ws_gen, the ziggurat's fn
     CUtensorMap *d_tmaps = nullptr;       // per member: TMA descriptor of its model
     int *d_tcq = nullptr;                 // the next work item of a tensor-core convolution launch
     size_t d_tmaps_cap = 0;
@@ -549,7 +550,7 @@ extern "C" int bbgpu_ctx_destroy(bbgpu_ctx *ctx) {
     cudaFree(ctx->d_sub); cudaFree(ctx->d_mem); cudaFree(ctx->d_pix); cudaFree(ctx->d_bucket);
     cudaFree(ctx->d_tcount); cudaFree(ctx->d_toff); cudaFree(ctx->d_tcur); cudaFree(ctx->d_model); cudaFree(ctx->d_scan);
     cudaFree(ctx->d_smooth); cudaFree(ctx->d_model64); cudaFree(ctx->d_partial); cudaFree(ctx->d_out2);
-    cudaFree(ctx->d_bimg); cudaFree(ctx->d_tmaps); cudaFree(ctx->d_tcq);
+    cudaFree(ctx->d_bimg); cudaFree(ctx->d_wsjump); cudaFree(ctx->d_tmaps); cudaFree(ctx->d_tcq);
     for (auto &v : ctx->pool)
         for (auto &b : v) cudaFree(b.p);
     if (ctx->gexec) cudaGraphExecDestroy(ctx->gexec);
@@ -2041,15 +2042,32 @@ static int an_upload(bbgpu_ctx *ctx, DevBufs &B, const std::vector<AnSub> &subs,
     return 0;
 }
 
-// The clouds of one or more chunks of shells (each parsed from its own stream) placed and deposited in one pass:
-// the fixed-point sums are exact, so the chunks' deposits add in any order; out += the sum of the chunks.
-static int wind_mc_run(bbgpu_ctx *ctx, double *out, std::vector<WindClouds> &chunks, int blo0, int blo1, int bhi0,
-                       int bhi1) {
-    const int by = bhi1 - blo1, bx = bhi0 - blo0;
-    const size_t n = (size_t)by * bx * ctx->g.nz;
+// A wind's chunks of shells: their constants and clouds, and the fixed-point unit of the deposits (2^E above their total
+// flux: exact sums, so that the chunks' deposits add in any order). false: nothing to deposit.
+struct WindRun {
+    int blo0, blo1, bhi0, bhi1;
+    double scale, unit;
+    size_t n;                              // values of the box
+    unsigned long long *acc = nullptr;
+};
+
+static bool wind_unit(const bbgpu_ctx *ctx, double total, WindRun &R) {
+    double rs = 0., cmax = 0.;
+    for (int l = 0; l < ctx->g.nlines; l++) rs += fabs(ctx->g.relint[l]);
+    for (double c : ctx->h_cd2i) cmax = std::max(cmax, fabs(c));
+    const double bound = total * rs * cmax;
+    if (!(bound > 0) || !std::isfinite(bound)) return false;
+    int E = 0;
+    frexp(bound * 1.0000001, &E);
+    R.scale = ldexp(1.0, 62 - E);
+    R.unit = ldexp(1.0, E - 62);
+    return true;
+}
+
+// The clouds of one or more chunks parsed on the host, placed and deposited in one pass.
+static int wind_clouds_run(bbgpu_ctx *ctx, std::vector<WindClouds> &chunks, DevBufs &B, const WindRun &R) {
     // the chunks' arrays go to the device at their offsets (shell indices and deviate offsets shifted)
     size_t nsh = 0, ncl = 0, nhz = 0, nsl = 0;
-    double total = 0.;
     for (WindClouds &c : chunks) {
         for (int &v : c.shell) v += (int)nsh;
         for (long long &v : c.nbase) v += (long long)nhz;
@@ -2058,43 +2076,19 @@ static int wind_mc_run(bbgpu_ctx *ctx, double *out, std::vector<WindClouds> &chu
         ncl += c.shell.size();
         nhz += c.hz.size();
         nsl += c.slow.size();
-        total += c.total;
     }
-    if (ncl == 0) return BBGPU_OK;
-    // fixed-point unit: 2^E above the total flux of the deposits
-    double rs = 0., cmax = 0.;
-    for (int l = 0; l < ctx->g.nlines; l++) rs += fabs(ctx->g.relint[l]);
-    for (double c : ctx->h_cd2i) cmax = std::max(cmax, fabs(c));
-    const double bound = total * rs * cmax;
-    if (!(bound > 0) || !std::isfinite(bound)) return BBGPU_OK;
-    int E = 0;
-    frexp(bound * 1.0000001, &E);
-    const double scale = ldexp(1.0, 62 - E), unit = ldexp(1.0, E - 62);
     WindShell *d_sh = nullptr;
     int *d_shell = nullptr, *d_hz = nullptr;
     double *d_geo = nullptr, *d_slow = nullptr;
     long long *d_nb = nullptr, *d_sb = nullptr;
-    unsigned long long *d_acc = nullptr;
-    auto release = [&]() {
-        cudaFree(d_sh); cudaFree(d_shell); cudaFree(d_hz); cudaFree(d_geo); cudaFree(d_slow); cudaFree(d_nb);
-        cudaFree(d_sb); cudaFree(d_acc);
-    };
-    bool ok = cudaMalloc(&d_sh, sizeof(WindShell) * nsh) == cudaSuccess &&
-              cudaMalloc(&d_shell, sizeof(int) * ncl) == cudaSuccess &&
-              cudaMalloc(&d_geo, sizeof(double) * 5 * ncl) == cudaSuccess &&
-              cudaMalloc(&d_hz, sizeof(int) * std::max<size_t>(nhz, 1)) == cudaSuccess &&
-              cudaMalloc(&d_slow, sizeof(double) * std::max<size_t>(nsl, 1)) == cudaSuccess &&
-              cudaMalloc(&d_nb, sizeof(long long) * ncl) == cudaSuccess &&
-              cudaMalloc(&d_sb, sizeof(long long) * ncl) == cudaSuccess &&
-              cudaMalloc(&d_acc, sizeof(unsigned long long) * n) == cudaSuccess;
-    if (!ok) {
-        cudaGetLastError();
-        release();
+    if (!B.get(&d_sh, sizeof(WindShell) * nsh) || !B.get(&d_shell, sizeof(int) * ncl) ||
+        !B.get(&d_geo, sizeof(double) * 5 * ncl) || !B.get(&d_hz, sizeof(int) * nhz) ||
+        !B.get(&d_slow, sizeof(double) * nsl) || !B.get(&d_nb, sizeof(long long) * ncl) ||
+        !B.get(&d_sb, sizeof(long long) * ncl))
         return fail(ctx, BBGPU_ERR_NOMEM, "galmod_wind: device allocation failed");
-    }
     cudaStream_t s = ctx->stream;
-    ok = cudaMemsetAsync(d_acc, 0, sizeof(unsigned long long) * n, s) == cudaSuccess;
     size_t o_sh = 0, o_cl = 0, o_hz = 0, o_sl = 0;
+    bool ok = true;
     for (const WindClouds &c : chunks) {
         auto up = [&](void *dst, const void *src, size_t bytes) {
             return !bytes || cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
@@ -2113,21 +2107,228 @@ static int wind_mc_run(bbgpu_ctx *ctx, double *out, std::vector<WindClouds> &chu
     }
     if (ok) {
         launch_wind_mc(s, d_sh, d_shell, d_geo, d_nb, d_sb, d_hz, d_slow, ctx->d_zig, (long long)ncl, ctx->g,
-                       ctx->d_cd2i, blo0, blo1, bhi0, bhi1, scale, d_acc);
+                       ctx->d_cd2i, R.blo0, R.blo1, R.bhi0, R.bhi1, R.scale, R.acc);
         ctx->launches++;
         ok = cudaGetLastError() == cudaSuccess;
     }
-    std::vector<unsigned long long> acc;
-    if (ok) {
-        acc.resize(n);
-        ok = cudaMemcpyAsync(acc.data(), d_acc, sizeof(unsigned long long) * n, cudaMemcpyDeviceToHost, s) ==
-                 cudaSuccess &&
-             cudaStreamSynchronize(s) == cudaSuccess;
+    // (the host arrays are the caller's: the copies complete first)
+    if (cudaStreamSynchronize(s) != cudaSuccess || !ok) return fail(ctx, BBGPU_ERR_CUDA, "galmod_wind: CUDA failure");
+    return 0;
+}
+
+// The clouds of the chunks with their streams followed on the device (galwind.cu), M draws a cloud: rounds of at most
+// WS_WORDS words (0.5 GB), a chunk that is longer continued in the next. The words asked for leave 4% for the
+// deviates that take more than one (3.6% on average); a chunk that needs more takes another round. Of the words 2.75%
+// leave the ziggurat's one-word path: room for 4%.
+#define WS_WORDS (64 << 20)
+#define WS_MIN 20000
+static int wind_stream_run(bbgpu_ctx *ctx, const std::vector<WindClouds> &chunks,
+                           const std::vector<std::vector<long long>> &first,
+                           const std::vector<std::vector<WindCloudLaw>> &law, const std::vector<uint64_t> &seed0, int M,
+                           DevBufs &B, const WindRun &R) {
+    const GridDev &g = ctx->g;
+    cudaStream_t s = ctx->stream;
+    const int nch = (int)chunks.size();
+    if (!ctx->d_wsjump) {
+        std::vector<uint64_t> tab((size_t)32 * 256);
+        bbh_stream_jumps(WS_SEG, tab.data());
+        std::vector<int64_t> kn(128);
+        std::vector<double> wn(128), fn(128);
+        bbh_zig_tables(kn.data(), wn.data(), fn.data());
+        uint8_t *p = nullptr;
+        CK(cudaMalloc(&p, tab.size() * 8 + 128 * 8));
+        ctx->d_wsjump = p;
+        CK(cudaMemcpy(p, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(p + tab.size() * 8, fn.data(), 128 * 8, cudaMemcpyHostToDevice));
     }
-    release();
-    if (!ok) return fail(ctx, BBGPU_ERR_CUDA, "galmod_wind: CUDA failure");
-    for (size_t i = 0; i < n; i++)
-        if (acc[i]) out[i] += (double)(long long)acc[i] * unit;
+    const double *d_fn = (const double *)((const uint8_t *)ctx->d_wsjump + (size_t)32 * 256 * 8);
+    std::vector<WindShell> shells;
+    std::vector<WindCloudLaw> laws;
+    std::vector<long long> sfirst;
+    std::vector<int> shell0;
+    for (int c = 0; c < nch; c++) {
+        shell0.push_back((int)shells.size());
+        shells.insert(shells.end(), chunks[c].shells.begin(), chunks[c].shells.end());
+        laws.insert(laws.end(), law[c].begin(), law[c].end());
+        sfirst.insert(sfirst.end(), first[c].begin(), first[c].end() - 1);
+    }
+    const int nsh = (int)shells.size();
+    struct Point {
+        long long seg = 0;                 // the segment of the next word, and the place in it
+        WsStart at{0, 0, 0};
+    };
+    std::vector<Point> pt(nch);
+    const long long blkw = (long long)WS_BLK * WS_SEG;
+    for (bool left = true; left;) {
+        std::vector<WindJob> jobs;
+        std::vector<int> chunk;
+        int nseg = 0, nblk = 0, ngrp = 0;
+        long long ncl = 0;
+        for (int c = 0; c < nch; c++) {
+            const long long kend = first[c].back(), k0 = (pt[c].at.draw + M - 1) / M;
+            if (k0 >= kend) continue;
+            const double draws = (double)(kend * M - pt[c].at.draw);
+            const long long want = (long long)((draws * 1.04 + pt[c].at.skip + 4096.) / (double)blkw) + 1;
+            const long long nb = std::min(want, ((long long)WS_WORDS - (long long)nseg * WS_SEG) / blkw);
+            if (nb < 1) break;
+            WindJob J{};
+            J.s0 = seed0[2 * c];
+            J.s1 = seed0[2 * c + 1];
+            J.segbase = pt[c].seg;
+            J.k0 = k0;
+            J.cl0 = ncl;
+            J.start = pt[c].at;
+            J.seg0 = nseg;
+            J.blk0 = nblk;
+            J.nblk = (int)nb;
+            J.grp0 = ngrp;
+            ngrp += ((int)nb + WS_GRP - 1) / WS_GRP;
+            J.shell0 = shell0[c];
+            J.nshell = (int)chunks[c].shells.size();
+            J.ncl = (int)std::min(kend - k0, nb * blkw / M + 2);
+            jobs.push_back(J);
+            chunk.push_back(c);
+            nseg += (int)nb * WS_BLK + 1;
+            nblk += (int)nb;
+            ncl += J.ncl;
+        }
+        if (jobs.empty()) break;
+        const int njob = (int)jobs.size(), cap = nseg * (WS_SEG / 25) + 1024;
+        WindJob *d_job = nullptr;
+        WindShell *d_sh = nullptr;
+        WindCloudLaw *d_law = nullptr;
+        long long *d_first = nullptr, *d_fix = nullptr;
+        unsigned long long *d_words = nullptr;
+        unsigned *d_mask = nullptr, *d_fpos = nullptr, *d_spec = nullptr;
+        int *d_cnt = nullptr, *d_err = nullptr;
+        unsigned char *d_fext = nullptr;
+        double *d_fval = nullptr;
+        WsStart *d_start = nullptr, *d_end = nullptr, *d_group = nullptr;
+        uint8_t *d_cloud = nullptr;
+        const size_t keep = B.i;
+        if (!B.get(&d_job, sizeof(WindJob) * njob) || !B.get(&d_sh, sizeof(WindShell) * nsh) ||
+            !B.get(&d_law, sizeof(WindCloudLaw) * nsh) || !B.get(&d_first, sizeof(long long) * nsh) ||
+            !B.get(&d_fix, sizeof(long long) * (size_t)nsh * g.nlines * g.nz) ||
+            !B.get(&d_words, sizeof(uint64_t) * (size_t)nseg * WS_SEG) ||
+            !B.get(&d_mask, sizeof(unsigned) * (size_t)nseg * (WS_SEG / 32)) ||
+            !B.get(&d_fpos, sizeof(unsigned) * (size_t)cap) || !B.get(&d_fext, (size_t)cap) ||
+            !B.get(&d_fval, sizeof(double) * (size_t)cap) ||
+            !B.get(&d_cnt, sizeof(int) * (3 * (size_t)nseg + nseg / 1024 + 8)) || !B.get(&d_err, sizeof(int)) ||
+            !B.get(&d_spec, sizeof(unsigned) * (size_t)nblk * M) || !B.get(&d_start, sizeof(WsStart) * (size_t)nblk) ||
+            !B.get(&d_end, sizeof(WsStart) * njob) ||
+            !B.get(&d_group, sizeof(WsStart) * (size_t)ngrp * (M + 1)) || !B.get(&d_cloud, 8 * (size_t)ncl))
+            return fail(ctx, BBGPU_ERR_NOMEM, "galmod_wind: device allocation failed");
+        B.i = keep;                        // (the next round's buffers are these)
+        CK(cudaMemcpyAsync(d_job, jobs.data(), sizeof(WindJob) * njob, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d_sh, shells.data(), sizeof(WindShell) * nsh, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d_law, laws.data(), sizeof(WindCloudLaw) * nsh, cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(d_first, sfirst.data(), sizeof(long long) * nsh, cudaMemcpyHostToDevice, s));
+        CK(cudaMemsetAsync(d_err, 0, sizeof(int), s));
+        int *nfail = d_cnt, *foff = d_cnt + nseg, *fcur = foff + nseg, *scr = fcur + nseg;
+        launch_ws_flux(s, d_sh, nsh, g, ctx->d_cd2i, R.scale, d_fix);
+        launch_ws_words(s, d_job, njob, nseg, ctx->d_wsjump, ctx->d_zig, d_fn, d_words, d_mask, nfail, foff, fcur, scr,
+                        d_fpos, d_fext, d_fval, cap, d_err);
+        launch_ws_clouds(s, d_job, njob, nblk, ngrp, ncl, M, foff, d_fpos, d_fext, d_fval, cap, d_spec, d_group,
+                         d_start, d_end, d_cloud, d_words, (unsigned)nseg * WS_SEG, ctx->d_zig, d_sh, d_law, d_first, d_err, g, R.blo0,
+                         R.blo1, R.bhi0, R.bhi1, d_fix, R.acc);
+        CKL();
+        ctx->launches += nseg > 16384 ? 12 : 10;
+        std::vector<WsStart> ends(njob);
+        int err = 0;
+        CK(cudaMemcpyAsync(ends.data(), d_end, sizeof(WsStart) * njob, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        if (err) return fail(ctx, BBGPU_ERR_KERNEL, "galmod_wind: a velocity deviate could not be followed");
+        left = false;
+        for (int j = 0; j < njob; j++) {
+            Point &p = pt[chunk[j]];
+            const long long word = (jobs[j].segbase + (long long)jobs[j].nblk * WS_BLK) * WS_SEG + ends[j].skip;
+            p.seg = word / WS_SEG;
+            p.at = ends[j];
+            p.at.skip = (int)(word % WS_SEG);
+        }
+        for (int c = 0; c < nch; c++)
+            if ((pt[c].at.draw + M - 1) / M < first[c].back()) left = true;
+    }
+    return 0;
+}
+
+// The chunks [lo[c], hi[c]) of the shells of sr, each with its stream: out (by, bx, nz) += their model, or with cube
+// out (nz, by, bx) = it.
+static int wind_mc_run(bbgpu_ctx *ctx, double *out, bool cube, const double *sr, int nsub, int nch, const int *lo,
+                       const int *hi, const uint64_t *seeds, double sep, const int64_t *nv, WindRun R, int threads) {
+    const int by = R.bhi1 - R.blo1, bx = R.bhi0 - R.blo0;
+    R.n = (size_t)by * bx * ctx->g.nz;
+    cudaStream_t s = ctx->stream;
+    std::vector<WindClouds> W(nch);
+    std::vector<std::vector<long long>> first(nch);
+    std::vector<std::vector<WindCloudLaw>> law(nch);
+    std::vector<uint64_t> seed0(2 * (size_t)nch);
+    double total = 0.;
+    long long ncl = 0;
+    int M = 0;
+    bool same = true;                      // (the shells have the same number of velocity samples)
+    for (int c = 0; c < nch; c++) {
+        if (bbh_wind_shells(&W[c], first[c], law[c], seeds[c], &seed0[2 * c], sr, nsub, lo[c], hi[c], sep, nv, &ctx->g))
+            return fail(ctx, BBGPU_ERR_ARG, "galmod_wind: cloud or velocity-sample counts out of range");
+        for (const WindShell &h : W[c].shells) {
+            same = same && (M == 0 || M == h.nvr + 3);
+            M = h.nvr + 3;
+        }
+        total += W[c].total;
+        ncl += first[c].back();
+    }
+    if (ncl == 0 || !wind_unit(ctx, total, R)) {
+        if (cube) memset(out, 0, sizeof(double) * R.n);
+        return BBGPU_OK;
+    }
+    DevBufs B(ctx, 5);
+    struct Trim {                          // (what a large model took goes back at the end of its call)
+        std::vector<PoolBuf> &v;
+        ~Trim() {
+            size_t sum = 0;
+            for (PoolBuf &b : v) sum += b.cap;
+            if (sum <= ((size_t)2 << 30)) return;
+            for (PoolBuf &b : v) cudaFree(b.p);
+            v.clear();
+        }
+    } trim{ctx->pool[5]};
+    double *d_out = nullptr;
+    if (!B.get(&R.acc, sizeof(uint64_t) * R.n) || !B.get(&d_out, cube ? sizeof(double) * R.n : 8))
+        return fail(ctx, BBGPU_ERR_NOMEM, "galmod_wind: device allocation failed");
+    CK(cudaMemsetAsync(R.acc, 0, sizeof(uint64_t) * R.n, s));
+    int rc = 0;
+    // (from WS_MIN draws on the device's dozen launches cost less than the host's 15 ns a draw and its uploads)
+    if (same && M <= WS_MAXM && ncl * M >= WS_MIN) {
+        rc = wind_stream_run(ctx, W, first, law, seed0, M, B, R);
+    } else {
+        // the chunks' streams parsed on host threads (each chunk its own stream), then one device pass
+        std::vector<int> err(nch, 0);
+        const int nt = std::max(1, std::min(threads, nch));
+        std::vector<std::thread> pool;
+        for (int t = 0; t < nt; t++)
+            pool.emplace_back([&, t]() {
+                for (int c = t; c < nch; c += nt)
+                    err[c] = bbh_wind_clouds(&W[c], seeds[c], sr, nsub, lo[c], hi[c], sep, nv, &ctx->g);
+            });
+        for (std::thread &th : pool) th.join();
+        for (int e : err)
+            if (e) return fail(ctx, BBGPU_ERR_ARG, "galmod_wind: cloud or velocity-sample counts out of range");
+        rc = wind_clouds_run(ctx, W, B, R);
+    }
+    if (rc) return rc;
+    if (cube) {
+        launch_ws_cube(s, R.acc, (long long)by * bx, ctx->g.nz, R.unit, d_out);
+        CKL();
+        CK(cudaMemcpyAsync(out, d_out, sizeof(double) * R.n, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        return BBGPU_OK;
+    }
+    std::vector<unsigned long long> acc(R.n);
+    CK(cudaMemcpyAsync(acc.data(), R.acc, sizeof(uint64_t) * R.n, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    for (size_t i = 0; i < R.n; i++)
+        if (acc[i]) out[i] += (double)(long long)acc[i] * R.unit;
     return BBGPU_OK;
 }
 
@@ -2145,39 +2346,39 @@ extern "C" int bbgpu_galmod_wind(bbgpu_ctx *ctx, double *out, const double *sr, 
     if (ring_lo < 0 || ring_hi > nsub || ring_lo > ring_hi) return fail(ctx, BBGPU_ERR_ARG, "galmod_wind: shells");
     CK(cudaSetDevice(ctx->device));
     if (bhi1 <= blo1 || bhi0 <= blo0 || ring_hi == ring_lo) return BBGPU_OK;
-    std::vector<WindClouds> W(1);
-    if (bbh_wind_clouds(&W[0], seed, sr, nsub, ring_lo, ring_hi, sep, nv, &ctx->g))
-        return fail(ctx, BBGPU_ERR_ARG, "galmod_wind: cloud or velocity-sample counts out of range");
-    return wind_mc_run(ctx, out, W, blo0, blo1, bhi0, bhi1);
+    return wind_mc_run(ctx, out, false, sr, nsub, 1, &ring_lo, &ring_hi, &seed, sep, nv,
+                       WindRun{blo0, blo1, bhi0, bhi1, 0., 0., 0}, 1);
+}
+
+static int galwind_chunks(bbgpu_ctx *ctx, double *out, bool cube, const double *sr, int nsub, int nchunks,
+                          const int *chunk_lo, const int *chunk_hi, const uint64_t *seeds, double sep,
+                          const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1, int threads) {
+    if (!ctx) return BBGPU_ERR_ARG;
+    int rc = wind_args(ctx, out, sr, nv, sep);
+    if (rc) return rc;
+    if (nchunks < 0 || (nchunks && (!chunk_lo || !chunk_hi || !seeds)))
+        return fail(ctx, BBGPU_ERR_ARG, "galwind: chunks");
+    for (int c = 0; c < nchunks; c++)
+        if (chunk_lo[c] < 0 || chunk_hi[c] > nsub || chunk_lo[c] > chunk_hi[c])
+            return fail(ctx, BBGPU_ERR_ARG, "galwind: a chunk outside the shells");
+    CK(cudaSetDevice(ctx->device));
+    if (bhi1 <= blo1 || bhi0 <= blo0) return BBGPU_OK;
+    return wind_mc_run(ctx, out, cube, sr, nsub, nchunks, chunk_lo, chunk_hi, seeds, sep, nv,
+                       WindRun{blo0, blo1, bhi0, bhi1, 0., 0., 0}, threads);
 }
 
 extern "C" int bbgpu_galwind_spherical(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int nchunks,
                                        const int *chunk_lo, const int *chunk_hi, const uint64_t *seeds, double sep,
                                        const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1, int threads) {
-    if (!ctx) return BBGPU_ERR_ARG;
-    int rc = wind_args(ctx, out, sr, nv, sep);
-    if (rc) return rc;
-    if (nchunks < 0 || (nchunks && (!chunk_lo || !chunk_hi || !seeds)))
-        return fail(ctx, BBGPU_ERR_ARG, "galwind_spherical: chunks");
-    for (int c = 0; c < nchunks; c++)
-        if (chunk_lo[c] < 0 || chunk_hi[c] > nsub || chunk_lo[c] > chunk_hi[c])
-            return fail(ctx, BBGPU_ERR_ARG, "galwind_spherical: a chunk outside the shells");
-    CK(cudaSetDevice(ctx->device));
-    if (bhi1 <= blo1 || bhi0 <= blo0 || nchunks == 0) return BBGPU_OK;
-    // the chunks' streams parsed on host threads (each chunk its own stream), then one device pass
-    std::vector<WindClouds> W(nchunks);
-    std::vector<int> err(nchunks, 0);
-    const int nt = std::max(1, std::min(threads, nchunks));
-    std::vector<std::thread> pool;
-    for (int t = 0; t < nt; t++)
-        pool.emplace_back([&, t]() {
-            for (int c = t; c < nchunks; c += nt)
-                err[c] = bbh_wind_clouds(&W[c], seeds[c], sr, nsub, chunk_lo[c], chunk_hi[c], sep, nv, &ctx->g);
-        });
-    for (std::thread &th : pool) th.join();
-    for (int e : err)
-        if (e) return fail(ctx, BBGPU_ERR_ARG, "galwind_spherical: cloud or velocity-sample counts out of range");
-    return wind_mc_run(ctx, out, W, blo0, blo1, bhi0, bhi1);
+    return galwind_chunks(ctx, out, false, sr, nsub, nchunks, chunk_lo, chunk_hi, seeds, sep, nv, blo0, blo1, bhi0,
+                          bhi1, threads);
+}
+
+extern "C" int bbgpu_galwind_cube(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int nchunks,
+                                  const int *chunk_lo, const int *chunk_hi, const uint64_t *seeds, double sep,
+                                  const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1, int threads) {
+    return galwind_chunks(ctx, out, true, sr, nsub, nchunks, chunk_lo, chunk_hi, seeds, sep, nv, blo0, blo1, bhi0,
+                          bhi1, threads);
 }
 
 extern "C" int bbgpu_galmod_analytic(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,

@@ -177,6 +177,88 @@ uint64_t bbh_layout_key(uint64_t seed, int ltype, int nsub, const int *nc, const
     return h;
 }
 
+namespace {
+int64_t wind_count(const GridDev *g, const double *sr, int nsub, int ir, double sep) {
+    return lround_ref(g->cdens * pow(sr[(size_t)4 * nsub + ir], (double)g->cmode) * 2 * M_PI * sr[ir] * sep / g->pixarea);
+}
+
+// the constants of shell ir with nc clouds
+WindShell wind_shell(const GridDev *g, const double *sr, int nsub, int ir, double sep, int64_t nc, int64_t nv) {
+    auto SRV = [&](int row) { return sr[(size_t)row * nsub + ir]; };
+    WindShell s{};
+    s.vrot = SRV(1);
+    s.vsph = SRV(2);
+    s.vdisp = sqrt(SRV(3) * SRV(3) + g->sig_instr * g->sig_instr);
+    s.vsys = SRV(10);
+    s.sinc = sin(SRV(5));
+    s.cinc = cos(SRV(5));
+    const double pa = SRV(6);
+    s.spa = sin(pa) * cos(g->crota2) + cos(pa) * sin(g->crota2);
+    s.cpa = cos(pa) * cos(g->crota2) - sin(pa) * sin(g->crota2);
+    s.xpos = SRV(8);
+    s.ypos = SRV(9);
+    s.nvr = (int)nv;
+    s.fluxsc = SRV(4) * 2 * M_PI * SRV(0) * sep / (double)(nc * nv);
+    return s;
+}
+}  // namespace
+
+int bbh_wind_shells(WindClouds *W, std::vector<long long> &first, std::vector<WindCloudLaw> &law, uint64_t seed,
+                    uint64_t *seed0, const double *sr, int nsub, int lo, int hi, double sep, const int64_t *nv,
+                    const GridDev *g) {
+    if (!W || !sr || !nv || lo < 0 || hi > nsub || lo > hi) return -1;
+    *W = WindClouds();
+    first.assign(1, 0);
+    law.clear();
+    Stream st(seed);
+    seed0[0] = st.s0;
+    seed0[1] = st.s1;
+    for (int ir = lo; ir < hi; ir++) {
+        const int64_t nc = wind_count(g, sr, nsub, ir, sep);
+        if (nc < 0 || nc > (1LL << 31) || nv[ir] < 1 || nv[ir] > (1 << 20)) return -2;
+        if (nc == 0) continue;
+        const double rtmp = sr[ir];
+        W->shells.push_back(wind_shell(g, sr, nsub, ir, sep, nc, nv[ir]));
+        law.push_back({pow(rtmp - 0.5 * sep, 2.0), 2 * sep * rtmp, sr[(size_t)7 * nsub + ir] / 2.});
+        first.push_back(first.back() + nc);
+        W->total += (double)nc * (int)nv[ir] * fabs(W->shells.back().fluxsc);
+    }
+    return 0;
+}
+
+void bbh_stream_jumps(uint64_t n, uint64_t *tab) {
+    // columns (images of the state's bits) of one step, raised to n, then squared again and again
+    typedef std::vector<uint64_t> Mat;
+    auto apply = [](const Mat &m, const uint64_t *v, uint64_t *out) {
+        uint64_t a = 0, b = 0;
+        for (int i = 0; i < 128; i++)
+            if ((v[i >> 6] >> (i & 63)) & 1) {
+                a ^= m[2 * i];
+                b ^= m[2 * i + 1];
+            }
+        out[0] = a;
+        out[1] = b;
+    };
+    auto mul = [&](const Mat &m, const Mat &x) {
+        Mat r(256);
+        for (int i = 0; i < 128; i++) apply(m, &x[2 * i], &r[2 * i]);
+        return r;
+    };
+    Mat step(256), acc(256, 0);
+    for (int i = 0; i < 128; i++) {
+        Stream st(0);
+        st.s0 = i < 64 ? 1ULL << i : 0;
+        st.s1 = i < 64 ? 0 : 1ULL << (i - 64);
+        st.next();
+        step[2 * i] = st.s0;
+        step[2 * i + 1] = st.s1;
+        acc[2 * i + (i >> 6)] = 1ULL << (i & 63);
+    }
+    for (; n; n >>= 1, step = mul(step, step))
+        if (n & 1) acc = mul(step, acc);
+    for (int b = 0; b < 32; b++, acc = mul(acc, acc)) memcpy(tab + 256 * b, acc.data(), sizeof(uint64_t) * 256);
+}
+
 // Parses the stream of _galmod_wind (bbarolo/galmod.py:546-590): per shell its cloud count and constants (each
 // in the reference's float64 operation order, with the C library's sin and cos), per cloud the three uniforms
 // made into its radius, azimuth (cos, sin) and polar angle (sin, cos), and its velocity deviates (the first word of
@@ -187,9 +269,7 @@ int bbh_wind_clouds(WindClouds *W, uint64_t seed, const double *sr, int nsub, in
     *W = WindClouds();
     Stream st(seed);
     auto SRV = [&](int row, int ir) { return sr[(size_t)row * nsub + ir]; };
-    auto count = [&](int ir) {
-        return lround_ref(g->cdens * pow(SRV(4, ir), (double)g->cmode) * 2 * M_PI * SRV(0, ir) * sep / g->pixarea);
-    };
+    auto count = [&](int ir) { return wind_count(g, sr, nsub, ir, sep); };
     // (the arrays sized first: the clouds and deviates of every shell)
     size_t ncl = 0, nnrm = 0;
     for (int ir = lo; ir < hi; ir++) {
@@ -209,21 +289,8 @@ int bbh_wind_clouds(WindClouds *W, uint64_t seed, const double *sr, int nsub, in
         const double rtmp = SRV(0, ir);
         const int64_t nc = count(ir);
         if (nc == 0) continue;
-        WindShell s{};
-        s.vrot = SRV(1, ir);
-        s.vsph = SRV(2, ir);
         const double opentmp = SRV(7, ir) / 2.;
-        s.vdisp = sqrt(SRV(3, ir) * SRV(3, ir) + g->sig_instr * g->sig_instr);
-        s.vsys = SRV(10, ir);
-        s.sinc = sin(SRV(5, ir));
-        s.cinc = cos(SRV(5, ir));
-        const double pa = SRV(6, ir);
-        s.spa = sin(pa) * cos(g->crota2) + cos(pa) * sin(g->crota2);
-        s.cpa = cos(pa) * cos(g->crota2) - sin(pa) * sin(g->crota2);
-        s.xpos = SRV(8, ir);
-        s.ypos = SRV(9, ir);
-        s.nvr = (int)nv[ir];
-        s.fluxsc = SRV(4, ir) * 2 * M_PI * rtmp * sep / (double)(nc * nv[ir]);
+        const WindShell s = wind_shell(g, sr, nsub, ir, sep, nc, nv[ir]);
         const int si = (int)W->shells.size();
         W->shells.push_back(s);
         const double r_in2 = pow(rtmp - 0.5 * sep, 2.0);

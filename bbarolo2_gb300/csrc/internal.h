@@ -98,6 +98,11 @@ struct WindShell {
     int nvr, pad;
 };
 
+// how the clouds of a shell are drawn: rad = sqrt(r2 + rc |2u - 1|), ph = open |2u - 1|
+struct WindCloudLaw {
+    double r2, rc, open;
+};
+
 #ifdef __cplusplus
 struct WindClouds {
     std::vector<WindShell> shells;
@@ -117,6 +122,14 @@ extern "C++" {
 // and velocity deviates (all drawn, as the reference, also for clouds outside any box); 0 or a negative error
 int bbh_wind_clouds(WindClouds *W, uint64_t seed, const double *sr, int nsub, int lo, int hi, double sep,
                     const int64_t *nv, const GridDev *g);
+// ... or only its shells with clouds (W: shells, total): their constants, first cloud and clouds (shell i: clouds
+// first[i] .. first[i + 1]); seed0: the two words of the stream's first state
+int bbh_wind_shells(WindClouds *W, std::vector<long long> &first, std::vector<WindCloudLaw> &law, uint64_t seed,
+                    uint64_t *seed0, const double *sr, int nsub, int lo, int hi, double sep, const int64_t *nv,
+                    const GridDev *g);
+// the state 2^b n steps of the stream further as a linear map over GF(2): tab (32, 128, 2), the images of the 128
+// state bits for b = 0 .. 31
+void bbh_stream_jumps(uint64_t n, uint64_t *tab);
 void bbh_zig_tables(int64_t *kn, double *wn, double *fn);
 void bbh_phi_table(double *tab);      // 6146 entries
 int bbh_layout_build(LayoutHost *L, uint64_t seed, int ltype, int nsub, const int *nc, const int *nv,

@@ -297,3 +297,37 @@ void launch_wind_mc(cudaStream_t st, const WindShell *shells, const int *shell, 
                     const long long *nbase, const long long *sbase, const int *hz, const double *slow,
                     const ZigDev *zig, long long ncloud, const GridDev &g, const double *cd2i, int blo0, int blo1,
                     int bhi0, int bhi1, double scale, unsigned long long *acc);
+// The streams of GALWIND's chunks followed on the device: segments of WS_SEG words, blocks of WS_BLK segments.
+#define WS_SEG 512
+#define WS_BLK 2
+#define WS_GRP 32             // blocks of a group of the chain
+#define WS_MAXM 128           // draws a cloud (3 + velocity samples) the device follows
+// a point of a stream: words of the block already taken, place in the cloud's cycle of draws, draws before it
+struct WsStart {
+    int skip, slot;
+    long long draw;
+};
+// a part of a chunk's stream: the words from segment segbase of the stream on, as segments seg0 .. of the launch (its
+// blocks and one guard segment), blocks blk0 .. blk0 + nblk (groups grp0 ..), from `start`; its clouds k0 .. (at most ncl) as clouds
+// cl0 .. of the launch; the chunk's shells
+struct WindJob {
+    unsigned long long s0, s1;        // the stream's first state
+    long long segbase, k0, cl0;
+    WsStart start;
+    int seg0, blk0, nblk, grp0, shell0, nshell, ncl, pad;
+};
+// words, failing words and their deviates (cap of them; err set when there are more); then the clouds; jump: (32, 128)
+// pairs of bbh_stream_jumps(WS_SEG)
+void launch_ws_words(cudaStream_t st, const WindJob *jobs, int njob, int nseg, const void *jump, const ZigDev *zig,
+                     const double *fn, unsigned long long *words, unsigned *masks, int *nfail, int *foff, int *fcur,
+                     int *scratch, unsigned *fpos, unsigned char *fext, double *fval, int cap, int *err);
+void launch_ws_clouds(cudaStream_t st, const WindJob *jobs, int njob, int nblk, int ngrp, long long ncl, int M,
+                      const int *foff, const unsigned *fpos, const unsigned char *fext, const double *fval, int cap,
+                      unsigned *spec, WsStart *group, WsStart *start, WsStart *ends, void *cloud,
+                      const unsigned long long *words, unsigned nword, const ZigDev *zig, const WindShell *shells,
+                      const WindCloudLaw *law, const long long *sfirst, int *err, const GridDev &g, int blo0, int blo1,
+                      int bhi0, int bhi1, const long long *fix, unsigned long long *acc);
+// the fixed-point deposit of each (shell, line, channel); the sums as the cube (nz, by, bx)
+void launch_ws_flux(cudaStream_t st, const WindShell *shells, int nshell, const GridDev &g, const double *cd2i,
+                    double scale, long long *fix);
+void launch_ws_cube(cudaStream_t st, const unsigned long long *acc, long long npix, int nz, double unit, double *out);

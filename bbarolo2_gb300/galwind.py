@@ -111,12 +111,13 @@ class GalWindMC:
         return [c for c in np.array_split(np.arange(ns), n) if len(c)]
 
     def model(self, host_threads=None):
-        """The model cube (nz, ny, nx): the chunks' streams parsed on host_threads threads (default: as many as
-        the chunks, at most the host's cores), every cloud deposited in one device pass."""
+        """The model cube (nz, ny, nx): the chunks' streams followed on the device (parsed on host_threads threads,
+        default as many as the chunks and at most the host's cores, where the shells differ in their velocity
+        samples), every cloud deposited in one device pass."""
         import os
         from . import _lib
         c = self.cube
-        out = np.zeros((c.DimY(), c.DimX(), c.DimZ()))
+        out = np.empty((c.DimZ(), c.DimY(), c.DimX()))
         seed = int(self.par.ISEED) & 0xFFFFFFFF
         ch = self.chunks()
         lo = np.array([int(x[0]) for x in ch], dtype=np.int32)
@@ -124,7 +125,7 @@ class GalWindMC:
         seeds = np.array([(seed + 7919 * t) & 0xFFFFFFFF for t in range(len(ch))], dtype=np.uint64)
         nt = host_threads or min(len(ch), os.cpu_count() or 1)
         ctx = self.dm.ctx
-        ctx.check(ctx.L.bbgpu_galwind_spherical(ctx.h, _lib.ptr(out), _lib.ptr(self.sr), self.sr.shape[1], len(ch),
-                                                _lib.ptr(lo), _lib.ptr(hi), _lib.ptr(seeds), float(self.sep),
-                                                _lib.ptr(self.nv), 0, 0, c.DimX(), c.DimY(), int(nt)))
-        return np.ascontiguousarray(out.transpose(2, 0, 1))
+        ctx.check(ctx.L.bbgpu_galwind_cube(ctx.h, _lib.ptr(out), _lib.ptr(self.sr), self.sr.shape[1], len(ch),
+                                           _lib.ptr(lo), _lib.ptr(hi), _lib.ptr(seeds), float(self.sep),
+                                           _lib.ptr(self.nv), 0, 0, c.DimX(), c.DimY(), int(nt)))
+        return out

@@ -103,11 +103,16 @@ int bbgpu_galmod_mc(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int
 int bbgpu_galmod_wind(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
                       uint64_t seed, double sep, const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1);
 /* GalWind._spherical (bbarolo/galwind.py:301-331): the chunks [chunk_lo[c], chunk_hi[c]) of the shells, each with
- * its own stream seeds[c], their streams parsed on up to `threads` host threads, all clouds deposited in one pass;
+ * its own stream seeds[c] (followed on the device; where the shells differ in their velocity samples, parsed on up to
+ * `threads` host threads), all clouds deposited in one pass;
  * out += the sum of the chunks' models (the fixed-point sums are exact: the same as adding them one by one). */
 int bbgpu_galwind_spherical(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int nchunks,
                             const int *chunk_lo, const int *chunk_hi, const uint64_t *seeds, double sep,
                             const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1, int threads);
+/* The same as a cube: out (nz, bhi1-blo1, bhi0-blo0) float64 = the sum of the chunks' models. */
+int bbgpu_galwind_cube(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int nchunks, const int *chunk_lo,
+                       const int *chunk_hi, const uint64_t *seeds, double sep, const int64_t *nv, int blo0, int blo1,
+                       int bhi0, int bhi1, int threads);
 int bbgpu_galmod_analytic(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
                           int nzq, int blo0, int blo1, int bhi0, int bhi1);
 /* out (nr, bhi1-blo1, bhi0-blo0) float64 accumulated; widx (nsub, 2) int64 (-1: none), wval (nsub, 2). */

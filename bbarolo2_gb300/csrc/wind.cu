@@ -7,7 +7,8 @@
 //   k_wind_points    one thread per quadrature point: sky position, line-of-sight velocity and dispersion, the
 //                    un-normalised weight r^2 sin(theta) (bbarolo/windmodel.py:225-288);
 //   k_wind_cells     one warp per cell: its clipped volume, the weights normalised to it, the mean radius;
-//   k_wind_rawbox    one warp per cell: the pixels and channels that its points reach (windmodel.py:291-319);
+//   k_wind_rawbox    one warp per cell: the pixels and channels that its points reach (windmodel.py:291-319), from the
+//                    extreme positions and velocities;
 //   (host)           offsets of the raw boxes and of the beam-grown boxes: one read of ncell x 6 integers;
 //   k_wind_deposit   one warp per point, lanes over channels: the channel-integrated line (the tabulated normal
 //                    CDF) times the bilinear weights of the four nearest pixels, added to the raw box of the cell
@@ -61,7 +62,8 @@ struct bbgpu_wind {
     cudaStream_t s = nullptr;
     WindGridDev g{};
     int hx = 0, hy = 0, separable = 1;
-    double *d_vedges = nullptr, *d_ptab = nullptr;
+    double *d_vedges = nullptr;
+    double2 *d_ptab = nullptr;          // the CDF table: each entry and its step to the next
     float2 *d_kern = nullptr, *d_kx = nullptr, *d_ky = nullptr;     // the beam taps as float-float (hi, lo)
     // cells and their quadrature
     int ncell = 0;
@@ -97,14 +99,17 @@ struct bbgpu_wind {
 
 namespace {
 
-// bbarolo/galmod.py:183-191: the normal CDF at t from the table (512 entries per unit from -6)
-__device__ __forceinline__ double wphi(double t, const double *__restrict__ tab) {
+// bbarolo/galmod.py:183-191: the normal CDF at t from the table (512 entries per unit from -6; each entry and its step
+// to the next). Every float64 instruction costs 16 cycles of an SM here: the comparisons are integer ones on the bit
+// patterns, the integer part comes from an addition rounded down.
+__device__ __forceinline__ double wphi(double t, const double2 *__restrict__ tab) {
     const double x = __dmul_rn(__dadd_rn(t, 6.0), 512.0);
-    if (x <= 0.0) return 0.0;
-    const long long k = (long long)x;
-    if (k >= WIND_PHI_N - 1) return 1.0;
-    const double t0 = tab[k], t1 = tab[k + 1];
-    return __dadd_rn(t0, __dmul_rn(__dsub_rn(x, (double)k), __dsub_rn(t1, t0)));
+    const long long b = __double_as_longlong(x);
+    if (b <= 0) return 0.0;                                          // (x <= 0 or a NaN with its sign bit set)
+    if (b >= __double_as_longlong((double)(WIND_PHI_N - 1))) return b > 0x7ff0000000000000ll ? 0.0 : 1.0;
+    const double y = __dadd_rd(x, 4503599627370496.0);               // 2^52: the integer part in the low bits
+    const double2 e = tab[__double2loint(y)];
+    return __dadd_rn(e.x, __dmul_rn(__dsub_rn(x, __dsub_rn(y, 4503599627370496.0)), e.y));
 }
 
 // bbarolo/galmod.py:38-46
@@ -315,7 +320,27 @@ __device__ __forceinline__ int clamp30(long long v) {
     return (int)(v < -(1LL << 30) ? -(1LL << 30) : (v > (1LL << 30) ? (1LL << 30) : v));
 }
 
-// bbarolo/windmodel.py:291-319: one warp per cell; lim: the raw limits (the cube box grown by the beam)
+// doubles as 64-bit integers of the same order (no NaN): minima and maxima off the float64 pipe
+__device__ __forceinline__ long long dkey(double v) {
+    const long long b = __double_as_longlong(v);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double dkey_value(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ long long warp_min(long long v) {
+    for (int o = 16; o; o >>= 1) v = min(v, __shfl_xor_sync(FULLMASK, v, o));
+    return v;
+}
+__device__ __forceinline__ long long warp_max(long long v) {
+    for (int o = 16; o; o >>= 1) v = max(v, __shfl_xor_sync(FULLMASK, v, o));
+    return v;
+}
+
+// bbarolo/windmodel.py:291-319: one warp per cell; lim: the raw limits (the cube box grown by the beam). The pixel of
+// a point is monotonic in its position and, for points of one dispersion (a cell's, unless the shells' dispersions
+// differ across it) and |v| < c, its channel in its velocity, so the box follows from the extreme positions and
+// velocities (273 us for 3192 cells with a channel per point, most of it float64 divisions).
 __global__ void __launch_bounds__(256) k_wind_rawbox(const long long *__restrict__ qoff, int ncell,
                                                      const double *__restrict__ gx, const double *__restrict__ gy,
                                                      const double *__restrict__ vel, const double *__restrict__ sig,
@@ -324,28 +349,51 @@ __global__ void __launch_bounds__(256) k_wind_rawbox(const long long *__restrict
     const int k = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (k >= ncell) return;
-    int bx0 = 1 << 30, bx1 = -(1 << 30), by0 = 1 << 30, by1 = -(1 << 30), bk0 = 1 << 30, bk1 = -(1 << 30);
-    for (long long i = qoff[k] + lane; i < qoff[k + 1]; i += 32) {
-        const double x = gx[i], y = gy[i];
+    const long long i0 = qoff[k], i1 = qoff[k + 1], top = 0x7fffffffffffffffll;
+    long long lo[4] = {top, top, top, top}, hi[4] = {-top, -top, -top, -top};       // x, y, velocity, dispersion
+    bool nan = false;
+    for (long long i = i0 + lane; i < i1; i += 32) {
+        const double x = gx[i], y = gy[i], v = vel[i], sg = sig[i];
         if (!wpoint_ok(wpoint(w, wt, i), x, y)) continue;
-        const int ix = (int)floor(x), iy = (int)floor(y);
-        bx0 = min(bx0, ix);
-        bx1 = max(bx1, ix + 2);
-        by0 = min(by0, iy);
-        by1 = max(by1, iy + 2);
-        const long long K = (long long)__ddiv_rn(__dmul_rn(5.0, sig[i]), g.chmin) + 2;
-        for (int nl = 0; nl < g.nlines; nl++) {
-            const long long kc = wround(wvelgrid(vel[i], g, nl));
-            bk0 = min(bk0, clamp30(kc - K));
-            bk1 = max(bk1, clamp30(kc + K + 1));
+        const long long q[4] = {dkey(x), dkey(y), dkey(v), dkey(sg)};
+        nan |= v != v || sg != sg;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            lo[j] = min(lo[j], q[j]);
+            hi[j] = max(hi[j], q[j]);
         }
     }
-    bx0 = __reduce_min_sync(FULLMASK, bx0);
-    bx1 = __reduce_max_sync(FULLMASK, bx1);
-    by0 = __reduce_min_sync(FULLMASK, by0);
-    by1 = __reduce_max_sync(FULLMASK, by1);
-    bk0 = __reduce_min_sync(FULLMASK, bk0);
-    bk1 = __reduce_max_sync(FULLMASK, bk1);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        lo[j] = warp_min(lo[j]);
+        hi[j] = warp_max(hi[j]);
+    }
+    int bx0 = 1 << 30, bx1 = -(1 << 30), by0 = 1 << 30, by1 = -(1 << 30), bk0 = 1 << 30, bk1 = -(1 << 30);
+    if (lo[0] <= hi[0]) {
+        bx0 = (int)floor(dkey_value(lo[0]));
+        bx1 = (int)floor(dkey_value(hi[0])) + 2;
+        by0 = (int)floor(dkey_value(lo[1]));
+        by1 = (int)floor(dkey_value(hi[1])) + 2;
+        const double v0 = dkey_value(lo[2]), v1 = dkey_value(hi[2]);
+        const bool mono = lo[3] == hi[3] && !__any_sync(FULLMASK, nan) &&
+                          (g.axtyp == 4 || (v0 > -0.9 * W_C_MS && v1 < 0.9 * W_C_MS));
+        auto reach = [&](double v, double sg) {
+            const long long K = (long long)__ddiv_rn(__dmul_rn(5.0, sg), g.chmin) + 2;
+            for (int nl = 0; nl < g.nlines; nl++) {
+                const long long kc = wround(wvelgrid(v, g, nl));
+                bk0 = min(bk0, clamp30(kc - K));
+                bk1 = max(bk1, clamp30(kc + K + 1));
+            }
+        };
+        if (mono) {
+            reach(lane & 1 ? v1 : v0, dkey_value(lo[3]));
+        } else {
+            for (long long i = i0 + lane; i < i1; i += 32)
+                if (wpoint_ok(wpoint(w, wt, i), gx[i], gy[i])) reach(vel[i], sig[i]);
+        }
+        bk0 = __reduce_min_sync(FULLMASK, bk0);
+        bk1 = __reduce_max_sync(FULLMASK, bk1);
+    }
     if (lane) return;
     long long o[6] = {std::max((long long)bx0, lim.x0), std::min((long long)bx1, lim.x1),
                       std::max((long long)by0, lim.y0), std::min((long long)by1, lim.y1),
@@ -364,7 +412,7 @@ template <class Put>
 __device__ __forceinline__ void deposit_point(long long i, double wi, const double *__restrict__ gx,
                                               const double *__restrict__ gy, const double *__restrict__ vel,
                                               const double *__restrict__ sig, const long long *B,
-                                              const double *__restrict__ vedges, const double *__restrict__ ptab,
+                                              const double *__restrict__ vedges, const double2 *__restrict__ ptab,
                                               const WindGridDev &g, int lane, Put put) {
     const int x0 = (int)B[0], x1 = (int)B[1], y0 = (int)B[2], y1 = (int)B[3], k0 = (int)B[4], k1 = (int)B[5];
     const int bx = x1 - x0, by = y1 - y0;
@@ -423,8 +471,9 @@ __global__ void __launch_bounds__(512) k_wind_deposit_cell(const long long *__re
                                                            const long long *__restrict__ rbox,
                                                            const long long *__restrict__ roffs,
                                                            const double *__restrict__ vedges,
-                                                           const double *__restrict__ ptab, WindGridDev g,
-                                                           long long maxvals, double *__restrict__ rbuf) {
+                                                           const double2 *__restrict__ ptab, WindGridDev g,
+                                                           long long maxvals, double *__restrict__ rbuf,
+                                                           float2 *__restrict__ rff, int *__restrict__ bexp) {
     extern __shared__ unsigned long long acc[];
     __shared__ double red[16];
     const int k = blockIdx.x;
@@ -490,8 +539,8 @@ __global__ void __launch_bounds__(512) k_wind_deposit_cell(const long long *__re
                 const double pn = wphi(__dmul_rn(__dsub_rn(ve[kz + 1], v), inv), ptab);
                 const double f = __dsub_rn(pn, pp);
                 pp = pn;
-                const double pv = __dmul_rn(amp, f >= 0 ? f : -f);
-                if (pv == 0.) continue;
+                const double pv = __dmul_rn(amp, fabs(f));
+                if ((__double_as_longlong(pv) & 0x7fffffffffffffffll) == 0) continue;
                 unsigned long long *plane = acc + (size_t)(kz - k0) * by * bx;
                 for (int c = 0; c < nc; c++)
                     atomicAdd(plane + o4[c], (unsigned long long)__double2ll_rn(pv * c4[c]));
@@ -499,8 +548,38 @@ __global__ void __launch_bounds__(512) k_wind_deposit_cell(const long long *__re
         }
     }
     __syncthreads();
-    double *out = rbuf + roffs[k];
-    for (int j = threadIdx.x; j < size; j += blockDim.x) out[j] = (double)(long long)acc[j] * unit;
+    if (!rff) {
+        double *out = rbuf + roffs[k];
+        for (int j = threadIdx.x; j < size; j += blockDim.x) out[j] = (double)(long long)acc[j] * unit;
+        return;
+    }
+    // for the convolution (k_wind_to_ff): the sums times 2^-b, 2^b above the largest, as float-float (the leading 24
+    // bits and those of the rest, from the integers)
+    unsigned long long m = 0;
+    auto mag = [](unsigned long long v) { return (long long)v < 0 ? 0ull - v : v; };
+    for (int j = threadIdx.x; j < size; j += blockDim.x) m = max(m, mag(acc[j]));
+    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(FULLMASK, m, o));
+    unsigned long long *const rm = (unsigned long long *)red;
+    if (lane == 0) rm[wid] = m;
+    __syncthreads();
+    for (int j = 0; j < nw; j++) m = max(m, rm[j]);
+    const int b = 64 - __clzll((long long)m);
+    if (threadIdx.x == 0) bexp[k] = m ? b + E - 62 : 0;
+    float2 *const out = rff + roffs[k];
+    for (int j = threadIdx.x; j < size; j += blockDim.x) {
+        const unsigned long long q = mag(acc[j]);
+        const int sh = 64 - __clzll((long long)q);                   // q < 2^sh
+        float2 v = make_float2(0.f, 0.f);
+        if (q) {
+            const unsigned long long l = q << (64 - sh);             // the leading bit at the top
+            const float h = (float)(unsigned)(l >> 40);              // 24 bits, exact
+            const float r = (float)(unsigned)((l >> 8) & 0xffffffffull);
+            const float s0 = scalbnf(1.0f, sh - b - 24);
+            v = make_float2(h * s0, r * (s0 * 2.3283064365386963e-10f));
+            if ((long long)acc[j] < 0) v = make_float2(-v.x, -v.y);
+        }
+        out[j] = v;
+    }
 }
 
 // one warp per point of the cells whose raw box holds more than maxvals values: float64 atomics in global memory
@@ -511,7 +590,7 @@ __global__ void __launch_bounds__(256) k_wind_deposit(const int *__restrict__ pc
                                                       const long long *__restrict__ rbox,
                                                       const long long *__restrict__ roffs,
                                                       const double *__restrict__ vedges,
-                                                      const double *__restrict__ ptab, WindGridDev g,
+                                                      const double2 *__restrict__ ptab, WindGridDev g,
                                                       long long maxvals, double *__restrict__ rbuf) {
     const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -552,13 +631,15 @@ __device__ __forceinline__ float2 ff_norm(float ah, float al) {
     return make_float2(h, __fsub_rn(al, __fsub_rn(h, ah)));
 }
 
-// one CTA per raw box: its values times 2^-E (2^E above the box's largest magnitude) as float-float, and E
+// one CTA per raw box of more than maxvals values: its values times 2^-E (2^E above the box's largest magnitude) as
+// float-float, and E (the others: k_wind_deposit_cell)
 __global__ void __launch_bounds__(256) k_wind_to_ff(const double *__restrict__ rbuf, const long long *__restrict__ roffs,
-                                                    float2 *__restrict__ rff, int *__restrict__ bexp) {
+                                                    long long maxvals, float2 *__restrict__ rff,
+                                                    int *__restrict__ bexp) {
     __shared__ unsigned long long red[8];
     const int k = blockIdx.x;
     const long long j0 = roffs[k], j1 = roffs[k + 1];
-    if (j1 == j0) return;
+    if (j1 - j0 <= maxvals) return;
     unsigned long long m = 0;
     for (long long j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
         const unsigned long long a = (unsigned long long)__double_as_longlong(rbuf[j]) & 0x7fffffffffffffffull;
@@ -579,59 +660,82 @@ __global__ void __launch_bounds__(256) k_wind_to_ff(const double *__restrict__ r
     if (threadIdx.x == 0) bexp[k] = E;
 }
 
-// bbarolo/windmodel.py:380-393, the x pass of a separable beam: tmp (box k: raw channels x raw rows x grown columns)
+// The separable beam in two passes, WIND_R outputs of a thread along the pass's axis: a value is read once for the
+// outputs that it reaches, the (row, output block) items laid over the threads (a warp a row of 37 outputs, a load for
+// every tap, took 528 and 985 us for the 42.6 M values of 2211 boxes; 394 and 546 so). Each sum still runs over its
+// taps in the reference's order. The taps of a pass are in shared memory.
+#define WIND_R 8
+
+// bbarolo/windmodel.py:380-393, the x pass: tmp (box k: raw channels x raw rows x grown columns)
 __global__ void __launch_bounds__(256) k_wind_conv_x(const float2 *__restrict__ rff, const long long *__restrict__ roffs,
                                                      const long long *__restrict__ rbox,
                                                      const long long *__restrict__ box,
                                                      const long long *__restrict__ toffs,
                                                      const float2 *__restrict__ kx, int hx, float2 *__restrict__ tmp) {
+    __shared__ float2 tap[512];
     const int k = blockIdx.x;
     if (toffs[k + 1] == toffs[k]) return;
+    for (int i = threadIdx.x; i <= 2 * hx; i += blockDim.x) tap[i] = kx[i];
+    __syncthreads();
     const long long *R = rbox + 6 * (size_t)k, *B = box + 6 * (size_t)k;
-    const int rx0 = (int)R[0], rx1 = (int)R[1], rby = (int)(R[3] - R[2]), rbz = (int)(R[5] - R[4]);
-    const int rbx = rx1 - rx0, x0 = (int)B[0], bx = (int)(B[1] - B[0]);
-    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) * gridDim.y;
+    const int rx0 = (int)R[0], rx1 = (int)R[1], rows = (int)((R[3] - R[2]) * (R[5] - R[4]));
+    const int rbx = rx1 - rx0, x0 = (int)B[0], bx = (int)(B[1] - B[0]), nb = (bx + WIND_R - 1) / WIND_R;
     const float2 *src = rff + roffs[k];
     float2 *dst = tmp + toffs[k];
-    for (int row = (threadIdx.x >> 5) + (blockDim.x >> 5) * blockIdx.y; row < rbz * rby; row += nw) {
+    for (int it = blockIdx.y * blockDim.x + threadIdx.x; it < rows * nb; it += gridDim.y * blockDim.x) {
+        const int row = it / nb, c0 = (it - row * nb) * WIND_R, xo = x0 + c0;
         const float2 *a = src + (size_t)row * rbx - rx0;
-        float2 *o = dst + (size_t)row * bx;
-        for (int c = lane; c < bx; c += 32) {
-            const int xx = x0 + c;
-            const int xa = max(rx0, xx - hx), xb = min(rx1 - 1, xx + hx);
-            float ah = 0.f, al = 0.f;
-            for (int x = xa; x <= xb; x++) ff_fma(ah, al, a[x], kx[xx - x + hx]);
-            o[c] = ff_norm(ah, al);
+        const int xa = max(rx0, xo - hx), xb = min(rx1 - 1, xo + WIND_R - 1 + hx);
+        float ah[WIND_R] = {}, al[WIND_R] = {};
+        for (int x = xa; x <= xb; x++) {
+            const float2 v = a[x];
+            const int j = xo - x + hx;
+#pragma unroll
+            for (int r = 0; r < WIND_R; r++)
+                if ((unsigned)(j + r) <= (unsigned)(2 * hx)) ff_fma(ah[r], al[r], v, tap[j + r]);
         }
+        float2 *o = dst + (size_t)row * bx + c0;
+#pragma unroll
+        for (int r = 0; r < WIND_R; r++)
+            if (c0 + r < bx) o[r] = ff_norm(ah[r], al[r]);
     }
 }
 
-// bbarolo/windmodel.py:394-401, the y pass of a separable beam: buf (box k, float64) from tmp
+// bbarolo/windmodel.py:394-401, the y pass: buf (box k, float64) from tmp
 __global__ void __launch_bounds__(256) k_wind_conv_y(const float2 *__restrict__ tmp, const long long *__restrict__ toffs,
                                                      const long long *__restrict__ rbox,
                                                      const long long *__restrict__ box,
                                                      const long long *__restrict__ offs,
                                                      const int *__restrict__ bexp, const float2 *__restrict__ ky,
                                                      int hy, double *__restrict__ buf) {
+    __shared__ float2 tap[512];
     const int k = blockIdx.x;
     if (offs[k + 1] == offs[k] || toffs[k + 1] == toffs[k]) return;
+    for (int i = threadIdx.x; i <= 2 * hy; i += blockDim.x) tap[i] = ky[i];
+    __syncthreads();
     const long long *R = rbox + 6 * (size_t)k, *B = box + 6 * (size_t)k;
     const int ry0 = (int)R[2], ry1 = (int)R[3], rby = ry1 - ry0;
     const int bx = (int)(B[1] - B[0]), by = (int)(B[3] - B[2]), bz = (int)(B[5] - B[4]), y0 = (int)B[2];
-    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) * gridDim.y;
+    const int nb = (by + WIND_R - 1) / WIND_R;
     const double sc = ldexp(1.0, bexp[k]);
     const float2 *src = tmp + toffs[k];
     double *dst = buf + offs[k];
-    for (int row = (threadIdx.x >> 5) + (blockDim.x >> 5) * blockIdx.y; row < bz * by; row += nw) {
-        const int kz = row / by, yy = y0 + (row - kz * by);
-        const int ya = max(ry0, yy - hy), yb = min(ry1 - 1, yy + hy);
-        const float2 *t = src + (size_t)kz * rby * bx;
-        double *o = dst + (size_t)row * bx;
-        for (int c = lane; c < bx; c += 32) {
-            float ah = 0.f, al = 0.f;
-            for (int y = ya; y <= yb; y++) ff_fma(ah, al, t[(size_t)(y - ry0) * bx + c], ky[yy - y + hy]);
-            o[c] = __dmul_rn(__dadd_rn((double)ah, (double)al), sc);
+    for (int it = blockIdx.y * blockDim.x + threadIdx.x; it < bz * nb * bx; it += gridDim.y * blockDim.x) {
+        const int zb = it / bx, c = it - zb * bx, kz = zb / nb, r0 = (zb - kz * nb) * WIND_R, yo = y0 + r0;
+        const float2 *t = src + ((size_t)kz * rby - ry0) * bx + c;
+        const int ya = max(ry0, yo - hy), yb = min(ry1 - 1, yo + WIND_R - 1 + hy);
+        float ah[WIND_R] = {}, al[WIND_R] = {};
+        for (int y = ya; y <= yb; y++) {
+            const float2 v = t[(size_t)y * bx];
+            const int j = yo - y + hy;
+#pragma unroll
+            for (int r = 0; r < WIND_R; r++)
+                if ((unsigned)(j + r) <= (unsigned)(2 * hy)) ff_fma(ah[r], al[r], v, tap[j + r]);
         }
+        double *o = dst + ((size_t)kz * by + r0) * bx + c;
+#pragma unroll
+        for (int r = 0; r < WIND_R; r++)
+            if (r0 + r < by) o[(size_t)r * bx] = __dmul_rn(__dadd_rn((double)ah[r], (double)al[r]), sc);
     }
 }
 
@@ -713,26 +817,29 @@ __global__ void __launch_bounds__(256) k_wind_lists(int pass, const double *__re
     // (the tests as integers on the bit patterns: |v| >= t for t >= 0, v != 0 and W != 0, off the float64 pipe)
     const unsigned long long t = (unsigned long long)__double_as_longlong(thr[k]);
     const double *col = buf + offs[k];
-    for (int row = threadIdx.x >> 5; row < by * bz; row += nw) {
-        const int zr = row / by, yr = row - zr * by;
-        const int z = (int)B[4] + zr, y = (int)B[2] + yr;
-        const double *a = col + (size_t)row * bx;
-        const double *wr = W + ((size_t)z * ny + y) * nx + B[0];
-        const int vrow = ((z - (int)lim.k0) * ly + (y - (int)lim.y0)) * lx + (int)(B[0] - lim.x0);
+    // (four rows in flight: the values are read once, latency is what it costs; W only where the value passes)
+    for (int row0 = (threadIdx.x >> 5) * 4; row0 < by * bz; row0 += nw * 4)
         for (int x = lane; x < bx; x += 32) {
-            const double v = a[x];
-            const unsigned long long av = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
-            const unsigned long long aw = (unsigned long long)__double_as_longlong(wr[x]) & 0x7fffffffffffffffull;
-            if (av == 0 || av < t || av > 0x7ff0000000000000ull || aw == 0) continue;
-            if (pass == 0) {
-                atomicAdd(cnt + vrow + x, 1);
-            } else {
-                const int j = atomicAdd(cursor + vrow + x, 1);
-                ecell[j] = k;
-                eval[j] = v;
+            double v[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) v[q] = row0 + q < by * bz ? col[(size_t)(row0 + q) * bx + x] : 0.;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                const unsigned long long av = (unsigned long long)__double_as_longlong(v[q]) & 0x7fffffffffffffffull;
+                if (av == 0 || av < t || av > 0x7ff0000000000000ull) continue;
+                const int zr = (row0 + q) / by, z = (int)B[4] + zr, y = (int)B[2] + (row0 + q) - zr * by;
+                const double wv = W[((size_t)z * ny + y) * nx + B[0] + x];
+                if (((unsigned long long)__double_as_longlong(wv) & 0x7fffffffffffffffull) == 0) continue;
+                const int vox = ((z - (int)lim.k0) * ly + (y - (int)lim.y0)) * lx + (int)(B[0] - lim.x0) + x;
+                if (pass == 0) {
+                    atomicAdd(cnt + vox, 1);
+                } else {
+                    const int j = atomicAdd(cursor + vox, 1);
+                    ecell[j] = k;
+                    eval[j] = v[q];
+                }
             }
         }
-    }
 }
 
 // bbarolo/windmodel.py:530-554: one warp per voxel of lim: b[k] += A_k Wd over its entries and, for every pair of
@@ -756,16 +863,20 @@ __global__ void __launch_bounds__(256) k_wind_lists_gram(const int *__restrict__
     const double w = W[cv], d = Wd[cv];
     const int j0 = start[i];
     for (int p = lane; p < n; p += 32) atomicAdd(b + ecell[j0 + p], __dmul_rn(eval[j0 + p], d));
-    for (int p = 0; p < n; p++) {
-        const int kp = ecell[j0 + p];
-        const double ap = eval[j0 + p];
-        for (int q = p + lane; q < n; q += 32) {
-            const int kq = ecell[j0 + q];
-            const double aq = eval[j0 + q];
-            // (the reference's order: the weight times the value of the lower cell, times the other)
-            if (kp <= kq) atomicAdd(G + (size_t)kp * ncell + kq, __dmul_rn(__dmul_rn(w, ap), aq));
-            else atomicAdd(G + (size_t)kq * ncell + kp, __dmul_rn(__dmul_rn(w, aq), ap));
+    // its pairs p <= q laid end to end over the lanes (row by row of the triangle left most lanes idle: 1.05 ms for
+    // 71.5 M pairs of lists of 25 entries, 0.43 so)
+    for (int p = 0, q = lane; p < n; q += 32) {
+        while (q >= n && p < n) {
+            p++;
+            q += p - n;
         }
+        if (p >= n) break;
+        const int kp = ecell[j0 + p], kq = ecell[j0 + q];
+        const double ap = eval[j0 + p], aq = eval[j0 + q];
+        // (the reference's order: the weight times the value of the lower cell, times the other)
+        const bool low = kp <= kq;
+        atomicAdd(G + (size_t)(low ? kp : kq) * ncell + (low ? kq : kp),
+                  __dmul_rn(__dmul_rn(w, low ? ap : aq), low ? aq : ap));
     }
 }
 
@@ -832,9 +943,10 @@ int grow(bbgpu_wind *w, T **p, size_t &cap, size_t n) {
 }  // namespace
 
 // PHI table (bbarolo/galmod.py:176-180) for the wind engine: 0.5 erfc(-t/sqrt 2) at t = -6 + k/512
-static void wind_phi_table(std::vector<double> &t) {
+static void wind_phi_table(std::vector<double2> &t) {
     t.resize(WIND_PHI_N);
-    for (int k = 0; k < WIND_PHI_N; k++) t[k] = 0.5 * erfc(-(-6.0 + k / 512.0) / sqrt(2.0));
+    for (int k = 0; k < WIND_PHI_N; k++) t[k].x = 0.5 * erfc(-(-6.0 + k / 512.0) / sqrt(2.0));
+    for (int k = 0; k < WIND_PHI_N; k++) t[k].y = k + 1 < WIND_PHI_N ? t[k + 1].x - t[k].x : 0.0;
 }
 
 extern "C" int bbgpu_wind_create(bbgpu_wind **out, int device, const bbgpu_wind_grid *g, const double *lfreq0,
@@ -861,7 +973,7 @@ extern "C" int bbgpu_wind_create(bbgpu_wind **out, int device, const bbgpu_wind_
     w->hx = hx;
     w->hy = hy;
     w->separable = separable ? 1 : 0;
-    std::vector<double> ptab;
+    std::vector<double2> ptab;
     wind_phi_table(ptab);
     const size_t nk = (size_t)(2 * hy + 1) * (2 * hx + 1), ne = (size_t)g->nlines * (g->nz + 1);
     bool ok = cudaStreamCreateWithFlags(&w->s, cudaStreamNonBlocking) == cudaSuccess &&
@@ -869,7 +981,7 @@ extern "C" int bbgpu_wind_create(bbgpu_wind **out, int device, const bbgpu_wind_
               cudaMalloc(&w->d_kx, sizeof(float2) * (2 * hx + 1)) == cudaSuccess &&
               cudaMalloc(&w->d_ky, sizeof(float2) * (2 * hy + 1)) == cudaSuccess &&
               cudaMalloc(&w->d_vedges, sizeof(double) * ne) == cudaSuccess &&
-              cudaMalloc(&w->d_ptab, sizeof(double) * WIND_PHI_N) == cudaSuccess &&
+              cudaMalloc(&w->d_ptab, sizeof(double2) * WIND_PHI_N) == cudaSuccess &&
               cudaMalloc(&w->d_rad, sizeof(double) * 4 * WIND_MAXRAD) == cudaSuccess;
     auto split = [](const double *v, size_t n) {
         std::vector<float2> o(n);
@@ -884,7 +996,7 @@ extern "C" int bbgpu_wind_create(bbgpu_wind **out, int device, const bbgpu_wind_
     const std::vector<float2> ky2 = separable ? split(ky, 2 * hy + 1) : std::vector<float2>(2 * hy + 1);
     ok = ok && cudaMemcpy(w->d_kern, k2.data(), sizeof(float2) * nk, cudaMemcpyHostToDevice) == cudaSuccess &&
          cudaMemcpy(w->d_vedges, vedges, sizeof(double) * ne, cudaMemcpyHostToDevice) == cudaSuccess &&
-         cudaMemcpy(w->d_ptab, ptab.data(), sizeof(double) * WIND_PHI_N, cudaMemcpyHostToDevice) == cudaSuccess;
+         cudaMemcpy(w->d_ptab, ptab.data(), sizeof(double2) * WIND_PHI_N, cudaMemcpyHostToDevice) == cudaSuccess;
     if (ok && separable)
         ok = cudaMemcpy(w->d_kx, kx2.data(), sizeof(float2) * (2 * hx + 1), cudaMemcpyHostToDevice) == cudaSuccess &&
              cudaMemcpy(w->d_ky, ky2.data(), sizeof(float2) * (2 * hy + 1), cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1154,9 +1266,9 @@ extern "C" int bbgpu_wind_boxes(bbgpu_wind *w, const int64_t *lim, const double 
     if (!rc) rc = cuda_check(w, cudaMemcpyAsync(w->d_toffs, w->h_toffs.data(), sizeof(long long) * (n + 1),
                                                 cudaMemcpyHostToDevice, w->s), "up");
     if (rc) return rc;
+    long long big = 0;
     if (rtot) {
         // cells whose raw box fits in shared memory: one CTA each; the others: float64 atomics in global memory
-        long long big = 0;
         for (int k = 0; k < n; k++) big = std::max(big, w->h_roffs[k + 1] - w->h_roffs[k]);
         const long long maxvals = std::min(big, (long long)WIND_SMEM_VALS);
         if (big > maxvals) {        // (the global path accumulates: its boxes start at zero; the others are written)
@@ -1166,7 +1278,7 @@ extern "C" int bbgpu_wind_boxes(bbgpu_wind *w, const int64_t *lim, const double 
         if (maxvals > 0) {
             k_wind_deposit_cell<<<n, 512, sizeof(unsigned long long) * maxvals, w->s>>>(
                 w->d_qoff, w->d_gx, w->d_gy, w->d_vel, w->d_sig, w->d_w, wt, w->d_rbox, w->d_roffs, w->d_vedges,
-                w->d_ptab, w->g, maxvals, w->d_rbuf);
+                w->d_ptab, w->g, maxvals, w->d_rbuf, conv ? w->d_rff : nullptr, w->d_bexp);
             w->launches++;
         }
         if (big > maxvals) {
@@ -1179,18 +1291,21 @@ extern "C" int bbgpu_wind_boxes(bbgpu_wind *w, const int64_t *lim, const double 
     }
     if (conv && tot) {
         const dim3 cg((unsigned)n, 4);
-        k_wind_to_ff<<<n, 256, 0, w->s>>>(w->d_rbuf, w->d_roffs, w->d_rff, w->d_bexp);
+        if (big > WIND_SMEM_VALS) {
+            k_wind_to_ff<<<n, 256, 0, w->s>>>(w->d_rbuf, w->d_roffs, WIND_SMEM_VALS, w->d_rff, w->d_bexp);
+            w->launches++;
+        }
         if (w->separable) {
             if (ttot)
                 k_wind_conv_x<<<cg, 256, 0, w->s>>>(w->d_rff, w->d_roffs, w->d_rbox, w->d_box, w->d_toffs,
                                                     w->d_kx, hx, w->d_tmp);
             k_wind_conv_y<<<cg, 256, 0, w->s>>>(w->d_tmp, w->d_toffs, w->d_rbox, w->d_box, w->d_offs, w->d_bexp,
                                                 w->d_ky, hy, w->d_buf);
-            w->launches += 3;
+            w->launches += 2;
         } else {
             k_wind_conv_2d<<<cg, 256, 0, w->s>>>(w->d_rff, w->d_roffs, w->d_rbox, w->d_box, w->d_offs, w->d_bexp,
                                                  w->d_kern, hy, hx, w->d_buf);
-            w->launches += 2;
+            w->launches++;
         }
     }
     rc = cuda_check(w, cudaGetLastError(), "wind deposit/convolution");

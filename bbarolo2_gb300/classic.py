@@ -19,8 +19,9 @@ from dataclasses import dataclass
 
 import numpy as np
 
+from . import _lib
 from .galfit import _norm, context
-from .galmod import arcsconv
+from .galmod import arcsconv, ring_rows_batch, seed32, subrings_batch
 
 TINY = 1.0e-10
 NORMCODE = {"LOCAL": 0, "AZIM": 1, "AZIMUTHAL": 1, "NONE": 2}
@@ -285,13 +286,25 @@ class ClassicFit:
     def _residual(self, dring, data_yxz, noise, normtype):
         """The CLASSIC residual of the model of one ring (``Galfit.getFuncValue``, ``bbarolo/galfit.py:736-749``):
         its MC model and sparse convolution on the device, then ``_norm`` on the device."""
-        blo, bhi = self.model.box(dring)
-        mod = np.ascontiguousarray(self.model.array(dring, blo, bhi, final=False, layout="yxz"), np.float64)
-        p = self.par
-        return _norm(mod, data_yxz, self.mask_yxz, blo[0], blo[1], dring.xpos[-1] - blo[0], dring.ypos[-1] - blo[1],
-                     dring.phi[-1], dring.inc[-1], dring.radii[0] / self.pixscale, dring.radii[-1] / self.pixscale,
-                     float(p.WFUNC), SIDECODE.get(p.SIDE, 0), p.FTYPE, self.chan_noise, noise, float(p.BWEIGHT),
-                     normtype, None, None, None, None, None, 0, 0., ctx=self.ctx)
+        m, st, p = self.model, self.model.setup, self.par
+        blo, bhi = m.box(dring)
+        if st.galmodtype != "MC":
+            mod = np.ascontiguousarray(m.array(dring, blo, bhi, final=False, layout="yxz"), np.float64)
+            return _norm(mod, data_yxz, self.mask_yxz, blo[0], blo[1], dring.xpos[-1] - blo[0],
+                         dring.ypos[-1] - blo[1], dring.phi[-1], dring.inc[-1], dring.radii[0] / self.pixscale,
+                         dring.radii[-1] / self.pixscale, float(p.WFUNC), SIDECODE.get(p.SIDE, 0), p.FTYPE,
+                         self.chan_noise, noise, float(p.BWEIGHT), normtype, None, None, None, None, None, 0, 0.,
+                         ctx=self.ctx)
+        sr, nv = (a[0] for a in subrings_batch(st, dring, ring_rows_batch([dring])))
+        k = m.cfield
+        out = np.empty(1)
+        self.ctx.check(self.ctx.L.bbgpu_classic_residual(
+            self.ctx.h, _lib.ptr(sr), sr.shape[1], seed32(st.iseed) & 0xFFFFFFFFFFFFFFFF, _lib.ptr(nv), blo[0], blo[1],
+            bhi[0], bhi[1], _lib.ptr(k), 0 if k is None else k.shape[0], 0 if k is None else k.shape[1],
+            float(m.scalefactor), dring.xpos[-1] - blo[0], dring.ypos[-1] - blo[1], dring.phi[-1], dring.inc[-1],
+            dring.radii[0] / self.pixscale, dring.radii[-1] / self.pixscale, float(p.WFUNC), SIDECODE.get(p.SIDE, 0),
+            int(p.FTYPE), noise, float(p.BWEIGHT), normtype, _lib.ptr(out)))
+        return float(out[0])
 
     def _start(self, ir, stage):
         """The coroutine of ring ir and its state, or None (ring skipped: too few pixels of the mask)."""
@@ -331,6 +344,11 @@ class ClassicFit:
             noise = noise * scaling
         data_yxz = np.ascontiguousarray(np.asarray(data, np.float32).transpose(1, 2, 0))
         normtype = NORMCODE[self.norms[stage - 1]]
+        dny, dnx, nz = data_yxz.shape
+        chan_noise = np.ascontiguousarray(self.chan_noise, np.float64)
+        self.ctx.check(self.ctx.L.bbgpu_classic_set(self.ctx.h, _lib.ptr(data_yxz),
+                                                    _lib.ptr(self.mask_yxz.view(np.uint8)), dny, dnx, nz,
+                                                    _lib.ptr(chan_noise)))
         nr = self.inr.nr
         start = self.par.STARTRAD if self.par.STARTRAD < nr else 0
         order = list(range(start, nr)) if rings is None else list(rings)

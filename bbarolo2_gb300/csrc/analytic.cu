@@ -136,7 +136,6 @@ __device__ __forceinline__ void an_runs(const AnSub &S, const double *__restrict
 struct AnWarp {
     int sgx[32], sgy[32], rg0[33], rg1[33];
     double rws[33];
-    int k0[BBGPU_MAXL], nk[BBGPU_MAXL];
 };
 
 // The (member, sample) of warp gs of a batch, by segments of warps: segment i (warps astart[i] .. astart[i + 1])
@@ -180,13 +179,21 @@ __device__ __forceinline__ bool an_sample(long long s, int src, int nsub, const 
     return true;
 }
 
-// Models: out64 (per member: box (by, bx, nz), stride mstride) += fixed-point deposits.
+// Models: out64 (per member: box (by, bx, nz), stride mstride) += fixed-point deposits. Every value is the reference's
+// float64 one; what does not decide a value is kept off the float64 pipe (16 cycles of an SM an instruction): the
+// pixels in float32 with a rounding bound (sample_pixel), the profile times cd2i once a sample and the amplitude times
+// the run's weight, in fixed-point units (a power of two: exact), once a run, so that a deposit is one multiplication
+// and one conversion, its (run, channel) pairs over the lanes. One 160x160x128 model: 3.6 ms with the pixels in
+// float64, the runs found by one lane and four float64 operations a deposit, 1.42 ms so.
+#define AN_RUNS 96
 __global__ void __launch_bounds__(AN_WPB * 32) k_an_model(GridDev g, const AnSub *__restrict__ subs, int nsub,
                                                           const int *__restrict__ sbase, const int *__restrict__ ssub,
                                                           const double2 *__restrict__ cs,
+                                                          const float2 *__restrict__ csf,
                                                           const long long *__restrict__ astart,
                                                           const int4 *__restrict__ aseg, int nseg, long long ntot,
                                                           const double *__restrict__ zq, const double *__restrict__ wq,
+                                                          const float *__restrict__ zqf,
                                                           const double *__restrict__ vedges,
                                                           const double *__restrict__ cd2i,
                                                           const double *__restrict__ ptab,
@@ -194,7 +201,8 @@ __global__ void __launch_bounds__(AN_WPB * 32) k_an_model(GridDev g, const AnSub
                                                           unsigned long long *__restrict__ out64, long long mstride,
                                                           int skip_fast) {
     extern __shared__ double an_smem[];
-    __shared__ AnWarp wsm[AN_WPB];
+    __shared__ double rws[AN_WPB][AN_RUNS];                 // per warp: the runs of a sample (weight; pixel of the box)
+    __shared__ int rpix[AN_WPB][AN_RUNS];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const long long gs = (long long)blockIdx.x * AN_WPB + w;
     AnSeg sg;
@@ -210,42 +218,136 @@ __global__ void __launch_bounds__(AN_WPB * 32) k_an_model(GridDev g, const AnSub
     const MemberDev &M = mem[k];
     const int nz = g.nz, nl_n = g.nlines;
     double *pe = an_smem + (size_t)w * nl_n * (nz + 2);
-    AnWarp &W = wsm[w];
     // (a negative unit: the deposits of member 0's constants taken out of a difference, rounded symmetrically)
     const double fscale = sg.sign < 0 ? -ldexp(1.0, M.fix_exp) : ldexp(1.0, M.fix_exp);
     unsigned long long *o64 = out64 + (size_t)k * mstride;
-    const double x = __dmul_rn(R, caz);
-    const double yb = __dmul_rn(__dmul_rn(R, saz), S.cinc);
-    const double xs = __dmul_rn(x, S.spa), xc = __dmul_rn(x, S.cpa);
     // bbarolo/galmod.py:407
     const double vplane = __dadd_rn(__dadd_rn(S.vsys, __dmul_rn(__dadd_rn(__dmul_rn(S.vrot, caz), __dmul_rn(S.vrad, saz)),
                                                                 S.sinc)),
                                     __dmul_rn(S.vvert, S.cinc));
     const double *zqs = zq + S.zq_off, *wqs = wq + S.zq_off;
     if (!S.zdep) {
+        const int nzz = S.nzz, kr = (int)(sg.s - sbase[ssub[sg.s]]) >= S.naz ? 1 : 0;
+        const PixF px = pix_setup(S, kr, csf[sg.s], zqf + S.zq_off, nzz);
+        const double2 *cp = cs + sg.s;
         bool ready = false;
-        auto emit = [&](int g0, int g1, double ws) {
-            if (g0 < M.blo0 || g0 >= M.bhi0 || g1 < M.blo1 || g1 >= M.bhi1) return;
+        int lk0[BBGPU_MAXL], lnk[BBGPU_MAXL];
+        auto deposit = [&](int n) {                    // the n runs of the list (bbarolo/galmod.py:422-428)
             if (!ready) {
                 for (int nl = 0; nl < nl_n; nl++) {
-                    int k0, nk;
-                    an_profile(g, nl, vplane, S, vedges, ptab, pe + (size_t)nl * (nz + 2), k0, nk);
-                    W.k0[nl] = k0;
-                    W.nk[nl] = nk;
+                    double *f = pe + (size_t)nl * (nz + 2);
+                    an_profile(g, nl, vplane, S, vedges, ptab, f, lk0[nl], lnk[nl]);
+                    // (the profile in place of the CDF: a lane's value before the next lane's edge is overwritten)
+                    for (int j0 = 0; j0 < lnk[nl]; j0 += 32) {
+                        const int j = j0 + lane;
+                        double v = 0.0;
+                        if (j < lnk[nl]) v = __dmul_rn(fabs(__dsub_rn(f[j + 1], f[j])), cd2i[lk0[nl] + j]);
+                        __syncwarp();
+                        if (j < lnk[nl]) f[j] = v;
+                        __syncwarp();
+                    }
                 }
                 ready = true;
             }
-            unsigned long long *o = o64 + ((size_t)(g1 - M.blo1) * M.bx + (size_t)(g0 - M.blo0)) * nz;
             for (int nl = 0; nl < nl_n; nl++) {
-                if (W.nk[nl] == 0) continue;
-                const double aw = __dmul_rn(__dmul_rn(S.a[nl], wside), ws);
-                an_add(o, pe + (size_t)nl * (nz + 2), cd2i, W.k0[nl], W.nk[nl], aw, fscale);
+                const int nk = lnk[nl];
+                if (nk == 0) continue;
+                const double *f = pe + (size_t)nl * (nz + 2);
+                const double aw0 = __dmul_rn(S.a[nl], wside);
+                double aw[AN_RUNS / 32];
+#pragma unroll
+                for (int i = 0; i < AN_RUNS / 32; i++)
+                    aw[i] = i * 32 + lane < n ? __dmul_rn(__dmul_rn(aw0, rws[w][i * 32 + lane]), fscale) : 0.0;
+                int r = 0, j = lane;
+                while (j >= nk) {
+                    j -= nk;
+                    r++;
+                }
+                for (int i0 = 0; i0 < n * nk; i0 += 32) {
+                    double a = __shfl_sync(FULL, aw[0], r & 31);
+#pragma unroll
+                    for (int i = 1; i < AN_RUNS / 32; i++) {
+                        const double b = __shfl_sync(FULL, aw[i], r & 31);
+                        if ((r >> 5) == i) a = b;
+                    }
+                    if (r < n) {
+                        const long long q = __double2ll_rn(__dmul_rn(a, f[j]));
+                        if (q) atomicAdd(o64 + (size_t)rpix[w][r] * nz + lk0[nl] + j, (unsigned long long)q);
+                    }
+                    j += 32;
+                    while (j >= nk) {
+                        j -= nk;
+                        r++;
+                    }
+                }
             }
-            __syncwarp();
         };
-        an_runs(S, zqs, wqs, g.cdelt0, g.cdelt1, xs, xc, yb, W.sgx, W.sgy, W.rg0, W.rg1, W.rws, emit);
+        bool open = false;                             // a run carried from the previous pass
+        int cg0 = 0, cg1 = 0, nr = 0;
+        double cws = 0.0;
+        for (int base = 0; base < nzz; base += 32) {
+            const int cnt = min(32, nzz - base);
+            const bool valid = lane < cnt;
+            int g0 = 0x7fffffff, g1 = 0x7fffffff;
+            if (valid)
+                sample_pixel(S, px, kr, cp, nzz, nzz > 1 ? zqf[S.zq_off + base + lane] : 0.f, zqs + base + lane, g.cdelt0,
+                             g.cdelt1, g0, g1);
+            const int pg0 = __shfl_up_sync(FULL, g0, 1), pg1 = __shfl_up_sync(FULL, g1, 1);
+            const bool start = valid && (lane == 0 ? (!open || g0 != cg0 || g1 != cg1) : (g0 != pg0 || g1 != pg1));
+            const unsigned smask = __ballot_sync(FULL, start);
+            if (open && (smask & 1u)) {                // the carried run ended with the previous pass
+                const int rx = cg0 - M.blo0, ry = cg1 - M.blo1;
+                if ((unsigned)rx < (unsigned)M.bx && (unsigned)ry < (unsigned)M.by) {
+                    if (lane == 0) {
+                        rpix[w][nr] = ry * M.bx + rx;
+                        rws[w][nr] = cws;
+                    }
+                    nr++;
+                }
+                open = false;
+            }
+            const bool last = lane == cnt - 1, final_pass = base + 32 >= nzz;
+            const bool end = valid && (last || ((smask >> (lane + 1)) & 1u));
+            // the run's weight, its heights added in their order (bbarolo/galmod.py:416-418)
+            const unsigned upto = smask & (0xffffffffu >> (31 - lane));
+            double ws = 0.0;
+            if (end) {
+                int t = 0;
+                if (upto) {
+                    t = 31 - __clz(upto);
+                    ws = wqs[base + t++];
+                } else {
+                    ws = cws;
+                }
+                for (; t <= lane; t++) ws = __dadd_rn(ws, wqs[base + t]);
+            }
+            const int rx = g0 - M.blo0, ry = g1 - M.blo1;
+            const bool put = end && (!last || final_pass) && (unsigned)rx < (unsigned)M.bx && (unsigned)ry < (unsigned)M.by;
+            const unsigned pmask = __ballot_sync(FULL, put);
+            if (put) {
+                const int at = nr + __popc(pmask & ((1u << lane) - 1u));
+                rpix[w][at] = ry * M.bx + rx;
+                rws[w][at] = ws;
+            }
+            nr += __popc(pmask);
+            if (nr > 0 && (final_pass || nr > AN_RUNS - 33)) {
+                __syncwarp();
+                deposit(nr);
+                __syncwarp();
+                nr = 0;
+            }
+            if (!final_pass) {
+                cg0 = __shfl_sync(FULL, g0, cnt - 1);
+                cg1 = __shfl_sync(FULL, g1, cnt - 1);
+                cws = __shfl_sync(FULL, ws, cnt - 1);
+                open = true;
+            }
+        }
         return;
     }
+    const double x = __dmul_rn(R, caz);
+    const double yb = __dmul_rn(__dmul_rn(R, saz), S.cinc);
+    const double xs = __dmul_rn(x, S.spa), xc = __dmul_rn(x, S.cpa);
     // bbarolo/galmod.py:430-463: the velocity depends on |z|; the samples at +z and -z share a profile
     const int nzz = S.nzz;
     for (int kz = 0; kz < (nzz + 1) / 2; kz++) {
@@ -844,16 +946,16 @@ __global__ void k_fix_to_model(const long long *__restrict__ in, const MemberDev
 size_t an_smem_bytes(int nz, int nlines) { return (size_t)AN_WPB * nlines * (nz + 2) * sizeof(double); }
 
 void launch_an_model(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
-                     const double *cs, const long long *astart, const int *aseg, int nseg, long long ntot,
-                     const double *zq, const double *wq, const double *vedges, const double *cd2i, const double *ptab,
+                     const double *cs, const float *csf, const long long *astart, const int *aseg, int nseg,
+                     long long ntot, const double *zq, const double *wq, const float *zqf, const double *vedges, const double *cd2i, const double *ptab,
                      const MemberDev *mem, long long *out64, long long mstride, int skip_fast) {
     const long long nw = ntot;
     if (nw == 0 || nseg == 0) return;
     const size_t smem = an_smem_bytes(g.nz, g.nlines);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_an_model, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_an_model, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_an_model<<<(unsigned)((nw + AN_WPB - 1) / AN_WPB), AN_WPB * 32, smem, s>>>(
-        g, subs, nsub, sbase, ssub, (const double2 *)cs, astart, (const int4 *)aseg, nseg, ntot, zq, wq, vedges, cd2i,
-        ptab, mem, (unsigned long long *)out64, mstride, skip_fast);
+        g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, astart, (const int4 *)aseg, nseg, ntot, zq,
+        wq, zqf, vedges, cd2i, ptab, mem, (unsigned long long *)out64, mstride, skip_fast);
 }
 
 void launch_an_model_fast(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase,

@@ -240,6 +240,12 @@ struct bbgpu_ctx {
     void *d_bimg = nullptr;               // its B operand image for conv_variant
     size_t d_bimg_cap = 0;
     int bimg_variant = 0;
+    // CLASSIC: the data, mask and channel noise of a fit (bbgpu_classic_set); pinned pixel weights and sums
+    float *d_cdata = nullptr;
+    uint8_t *d_cmask = nullptr;
+    double *d_cnoise = nullptr, *h_cpix = nullptr;
+    size_t d_cdata_cap = 0, d_cmask_cap = 0, d_cnoise_cap = 0, h_cpix_cap = 0;
+    int cny = 0, cnx = 0;
     void *d_wsjump = nullptr;             // GALWIND's streams: the jumps of k_ws_gen, the ziggurat's fn
     CUtensorMap *d_tmaps = nullptr;       // per member: TMA descriptor of its model
     int *d_tcq = nullptr;                 // the next work item of a tensor-core convolution launch
@@ -550,6 +556,7 @@ extern "C" int bbgpu_ctx_destroy(bbgpu_ctx *ctx) {
     cudaFree(ctx->d_sub); cudaFree(ctx->d_mem); cudaFree(ctx->d_pix); cudaFree(ctx->d_bucket);
     cudaFree(ctx->d_tcount); cudaFree(ctx->d_toff); cudaFree(ctx->d_tcur); cudaFree(ctx->d_model); cudaFree(ctx->d_scan);
     cudaFree(ctx->d_smooth); cudaFree(ctx->d_model64); cudaFree(ctx->d_partial); cudaFree(ctx->d_out2);
+    cudaFree(ctx->d_cdata); cudaFree(ctx->d_cmask); cudaFree(ctx->d_cnoise); cudaFreeHost(ctx->h_cpix);
     cudaFree(ctx->d_bimg); cudaFree(ctx->d_wsjump); cudaFree(ctx->d_tmaps); cudaFree(ctx->d_tcq);
     for (auto &v : ctx->pool)
         for (auto &b : v) cudaFree(b.p);
@@ -1607,9 +1614,10 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
                                  ctx->d_ptabf, ctx->d_mem, ctx->d_model_fx, ctx->mstride);
             CKL();
             if (ctx->an_exact) {
-                launch_an_model(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_astart,
-                                ctx->d_aseg, ctx->an_nseg, ctx->an_ntot, ctx->d_azq, ctx->d_awq, ctx->d_vedges,
-                                ctx->d_cd2i, ctx->d_ptab, ctx->d_mem, ctx->d_model_fx, ctx->mstride, 1);
+                launch_an_model(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_acsf,
+                                ctx->d_astart, ctx->d_aseg, ctx->an_nseg, ctx->an_ntot, ctx->d_azq, ctx->d_awq,
+                                ctx->d_azqf, ctx->d_vedges, ctx->d_cd2i, ctx->d_ptab, ctx->d_mem, ctx->d_model_fx,
+                                ctx->mstride, 1);
                 CKL();
             }
             launch_fix_to_model(s, ctx->d_model_fx, ctx->d_mem, ctx->nb, ctx->mstride, g.nz, ctx->d_model,
@@ -1655,11 +1663,27 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
             }
             if (tm) CK(cudaEventRecord(ctx->ev[10], s));
         } else {
+            // (a float64 model: the pixel-owned kernel leaves its sums, with the clouds of a tile shared by CTAs, and
+            // they are converted after it; where it does not apply, the general kernel writes the float64 model
+            // itself: for a single ring of 64x64x64, 98 us against 20 + 3)
+            const bool sums = ctx->want64 && ctx->nb == 1 && mc_deposit_shares(ctx->lean, false, ctx->tx, ctx->ty);
+            if (sums) {
+                int rc = dgrow(ctx, &ctx->d_base64, &ctx->d_base64_cap, (size_t)ctx->mstride + 1);
+                if (rc) return rc;
+            }
             launch_mc_deposit(s, g, L, ctx->d_sub, ctx->nsub, ctx->d_mem, ctx->mem_host.data(), ctx->nb, ctx->tx,
                               ctx->ty, ctx->d_toff, ctx->d_tcount, ctx->d_bucket, ctx->d_zig, ctx->d_cd2if,
-                              ctx->d_cd2i, ctx->d_model, ctx->mstride, ctx->want64 ? ctx->d_model64 : nullptr,
-                              ctx->d_err, ctx->lean);
+                              ctx->d_cd2i, ctx->d_model, ctx->mstride,
+                              ctx->want64 && !sums ? ctx->d_model64 : nullptr, ctx->d_err, ctx->lean, nullptr, 0, 0,
+                              sums ? ctx->d_base64 : nullptr, nullptr, Replay{nullptr, nullptr, nullptr, nullptr, 0, nullptr},
+                              sums ? mc_deposit_split(ctx->ntile_total) : 1);
             CKL();
+            if (sums) {
+                const MemberDev &M = ctx->mem_host[0];
+                launch_mc_sums64(s, ctx->d_base64, (long long)M.bx * M.by * g.nz, g.nz, ctx->d_cd2i, ctx->d_cd2if,
+                                 M.fix_exp, ctx->d_model64, ctx->d_model);
+                CKL();
+            }
             if (tm) {
                 CK(cudaEventRecord(ctx->ev[8], s));
                 CK(cudaEventRecord(ctx->ev[9], s));
@@ -1841,6 +1865,57 @@ extern "C" int bbgpu_eval_model(bbgpu_ctx *ctx, int k, int smoothed, float *out,
 }
 
 // ------------------------------------------------------------------------------------------- reference kernels
+// Scratch buffers of a stand-alone call: the i-th buffer of call site `tag` is kept in the context and reused by
+// the next call of that site (grown when too small), so that a call allocates nothing once warm (a cudaFree would
+// also wait for the whole device). The calls of a context run in order on its stream, so reuse is safe.
+struct DevBufs {
+    bbgpu_ctx *ctx;
+    int tag;
+    size_t i = 0;
+    DevBufs(bbgpu_ctx *c, int t) : ctx(c), tag(t) {}
+    template <class T>
+    bool get(T **out, size_t n) {
+        std::vector<PoolBuf> &v = ctx->pool[tag];
+        if (i == v.size()) v.push_back(PoolBuf{});
+        PoolBuf &b = v[i++];
+        const size_t need = n ? n : 1;
+        if (b.cap < need) {
+            if (b.p) cudaFree(b.p);
+            b.p = nullptr;
+            b.cap = 0;
+            const size_t want = need + need / 4;
+            if (cudaMalloc(&b.p, want) != cudaSuccess) {
+                cudaGetLastError();
+                return false;
+            }
+            b.cap = want;
+        }
+        *out = (T *)b.p;
+        return true;
+    }
+};
+
+// The Monte-Carlo model of the sub-rings [ring_lo, ring_hi) in the box on the device: float64 (by, bx, nz) in
+// ctx->d_model64 (queued on the context's stream; the error flag is check_err's).
+static int galmod_mc_dev(bbgpu_ctx *ctx, const double *sr, int nsub, int ring_lo, int ring_hi, uint64_t seed,
+                         const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1) {
+    // sub-rings [ring_lo, ring_hi) with a stream seeded by seed: the table restricted to them
+    const int ns = ring_hi - ring_lo;
+    std::vector<double> s2((size_t)BBGPU_NSR * ns);
+    std::vector<int64_t> nv2(ns);
+    for (int r = 0; r < BBGPU_NSR; r++)
+        for (int i = 0; i < ns; i++) s2[(size_t)r * ns + i] = sr[(size_t)r * nsub + ring_lo + i];
+    for (int i = 0; i < ns; i++) nv2[i] = nv[ring_lo + i];
+    bbgpu_eval_desc d{};
+    d.blo0 = blo0; d.blo1 = blo1; d.bhi0 = bhi0; d.bhi1 = bhi1; d.seed = seed;
+    ctx->want64 = true;
+    int rc = batch_prepare(ctx, BBGPU_MC, 1, ns, s2.data(), nv2.data(), &d, false);
+    if (!rc) rc = batch_run(ctx, false);
+    ctx->want64 = false;
+    ctx->uploaded = ctx->ran = false;
+    return rc;
+}
+
 extern "C" int bbgpu_galmod_mc(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
                                uint64_t seed, const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1) {
     if (ctx) ctx->gen++;
@@ -1848,32 +1923,48 @@ extern "C" int bbgpu_galmod_mc(bbgpu_ctx *ctx, double *out, const double *sr, in
     if (!out || !sr || !nv || ring_lo < 0 || ring_hi > nsub || ring_lo > ring_hi)
         return fail(ctx, BBGPU_ERR_ARG, "galmod_mc: invalid arguments");
     CK(cudaSetDevice(ctx->device));
-    // sub-rings [ring_lo, ring_hi) with a stream seeded by seed: the table restricted to them
-    int ns = ring_hi - ring_lo;
-    std::vector<double> s2((size_t)BBGPU_NSR * (ns ? ns : 1));
-    std::vector<int64_t> nv2(ns ? ns : 1);
-    for (int r = 0; r < BBGPU_NSR; r++)
-        for (int i = 0; i < ns; i++) s2[(size_t)r * ns + i] = sr[(size_t)r * nsub + ring_lo + i];
-    for (int i = 0; i < ns; i++) nv2[i] = nv[ring_lo + i];
-    int by = bhi1 - blo1, bx = bhi0 - blo0;
-    if (ns == 0 || by <= 0 || bx <= 0) return BBGPU_OK;
-    bbgpu_eval_desc d{};
-    d.blo0 = blo0; d.blo1 = blo1; d.bhi0 = bhi0; d.bhi1 = bhi1; d.seed = seed;
-    ctx->want64 = true;
-    int rc = batch_prepare(ctx, BBGPU_MC, 1, ns, s2.data(), nv2.data(), &d, false);
-    if (rc) return rc;
-    rc = batch_run(ctx, false);
-    ctx->want64 = false;
-    if (rc) return rc;
-    rc = check_err(ctx);
+    const int by = bhi1 - blo1, bx = bhi0 - blo0;
+    if (ring_hi == ring_lo || by <= 0 || bx <= 0) return BBGPU_OK;
+    int rc = galmod_mc_dev(ctx, sr, nsub, ring_lo, ring_hi, seed, nv, blo0, blo1, bhi0, bhi1);
+    if (!rc) rc = check_err(ctx);
     if (rc) return rc;
     size_t n = (size_t)by * bx * ctx->g.nz;
     std::vector<double> tmp(n);
     CK(cudaMemcpy(tmp.data(), ctx->d_model64, n * sizeof(double), cudaMemcpyDeviceToHost));
     for (size_t i = 0; i < n; i++) out[i] += tmp[i];
-    ctx->uploaded = ctx->ran = false;
     return BBGPU_OK;
 }
+
+// The "same" convolution of a (ny, nx, nz) float32 model on the device with the context's beam: b (the same layout).
+static int conv_dev(bbgpu_ctx *ctx, DevBufs &B, const float *a, float *b, int nz, int ny, int nx, double scale,
+                    int threshold) {
+    GridDev g = ctx->g;
+    g.scalefactor = threshold ? scale : 1.0;
+    MemberDev M{};
+    M.blo0 = 0; M.blo1 = 0; M.bhi0 = nx; M.bhi1 = ny; M.bx = nx; M.by = ny;
+    MemberDev *dm = nullptr;
+    double *dp = nullptr;
+    const int npart = conv_resid_npart(&M, 1, nz);
+    if (!B.get(&dm, sizeof M) || !B.get(&dp, 2 * sizeof(double) * (npart ? npart : 1)))
+        return fail(ctx, BBGPU_ERR_NOMEM, "convolve: allocation failed");
+    CK(cudaMemcpyAsync(dm, &M, sizeof M, cudaMemcpyHostToDevice, ctx->stream));
+    launch_conv_resid(ctx->stream, g, dm, &M, 1, a, (long long)nz * ny * nx, nz, ctx->d_taps, ctx->ky, ctx->kx,
+                      ctx->kxw, b, threshold ? 1 : 2, 0, dp);
+    CKL();
+    return 0;
+}
+
+// (what a large cube took goes back at the end of its call)
+struct PoolTrim {
+    std::vector<PoolBuf> &v;
+    ~PoolTrim() {
+        size_t sum = 0;
+        for (PoolBuf &b : v) sum += b.cap;
+        if (sum <= ((size_t)2 << 30)) return;
+        for (PoolBuf &b : v) cudaFree(b.p);
+        v.clear();
+    }
+};
 
 extern "C" int bbgpu_convolve(bbgpu_ctx *ctx, const double *in, double *out, int nz, int ny, int nx, double scale,
                               int threshold) {
@@ -1882,41 +1973,24 @@ extern "C" int bbgpu_convolve(bbgpu_ctx *ctx, const double *in, double *out, int
     if (!in || !out || nz < 1 || ny < 1 || nx < 1) return fail(ctx, BBGPU_ERR_ARG, "convolve: invalid arguments");
     if (!ctx->kernel_set) return fail(ctx, BBGPU_ERR_STATE, "convolve before set_kernel");
     CK(cudaSetDevice(ctx->device));
-    size_t n = (size_t)nz * ny * nx;
+    const size_t n = (size_t)nz * ny * nx;
+    PoolTrim trim{ctx->pool[6]};
+    DevBufs B(ctx, 6);
     double *d64 = nullptr;
     float *a = nullptr, *b = nullptr;
-    MemberDev *dm = nullptr;
-    int rc = 0;
-    GridDev g = ctx->g;
-    g.scalefactor = threshold ? scale : 1.0;
-    MemberDev M{};
-    M.blo0 = 0; M.blo1 = 0; M.bhi0 = nx; M.bhi1 = ny; M.bx = nx; M.by = ny;
+    if (!B.get(&d64, n * sizeof(double)) || !B.get(&a, n * sizeof(float)) || !B.get(&b, n * sizeof(float)))
+        return fail(ctx, BBGPU_ERR_NOMEM, "convolve: allocation failed");
     cudaStream_t s = ctx->stream;
-    if (cudaMalloc(&d64, n * sizeof(double)) != cudaSuccess || cudaMalloc(&a, n * sizeof(float)) != cudaSuccess ||
-        cudaMalloc(&b, n * sizeof(float)) != cudaSuccess || cudaMalloc(&dm, sizeof M) != cudaSuccess) {
-        cudaGetLastError();
-        rc = fail(ctx, BBGPU_ERR_NOMEM, "convolve: allocation failed");
-    }
-    int npart = conv_resid_npart(&M, 1, nz);
-    double *dp = nullptr;
-    if (!rc && cudaMalloc(&dp, 2 * sizeof(double) * (npart ? npart : 1)) != cudaSuccess) {
-        cudaGetLastError();
-        rc = fail(ctx, BBGPU_ERR_NOMEM, "convolve: allocation failed");
-    }
-    if (!rc) {
-        cudaMemcpyAsync(d64, in, n * sizeof(double), cudaMemcpyHostToDevice, s);
-        cudaMemcpyAsync(dm, &M, sizeof M, cudaMemcpyHostToDevice, s);
-        launch_zyx64_to_yxz32(s, d64, a, nz, ny, nx);
-        launch_conv_resid(s, g, dm, &M, 1, a, (long long)n, nz, ctx->d_taps, ctx->ky, ctx->kx, ctx->kxw, b,
-                          threshold ? 1 : 2, 0, dp);
-        launch_yxz32_to_zyx64(s, b, d64, nz, ny, nx);
-        ctx->launches += 3;
-        cudaMemcpyAsync(out, d64, n * sizeof(double), cudaMemcpyDeviceToHost, s);
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) rc = fail(ctx, BBGPU_ERR_CUDA, "convolve: %s", cudaGetErrorString(e));
-    }
-    cudaFree(d64); cudaFree(a); cudaFree(b); cudaFree(dm); cudaFree(dp);
-    return rc;
+    CK(cudaMemcpyAsync(d64, in, n * sizeof(double), cudaMemcpyHostToDevice, s));
+    launch_zyx64_to_yxz32(s, d64, a, nz, ny, nx);
+    CKL();
+    int rc = conv_dev(ctx, B, a, b, nz, ny, nx, scale, threshold);
+    if (rc) return rc;
+    launch_yxz32_to_zyx64(s, b, d64, nz, ny, nx);
+    CKL();
+    CK(cudaMemcpyAsync(out, d64, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    return BBGPU_OK;
 }
 
 static int sumsq_common(bbgpu_ctx *ctx, const double *model, const float *data, const uint8_t *mask, int maskmode,
@@ -1978,42 +2052,12 @@ extern "C" int bbgpu_residuals_fracerr(bbgpu_ctx *ctx, const double *model, cons
     return sumsq_common(ctx, model, data, mask, maskmode, region, nz, ny, nx, sigma2, eps2, out2);
 }
 
-// A scoped set of device buffers freed at the end of a stand-alone entry point.
-// Scratch buffers of a stand-alone call: the i-th buffer of call site `tag` is kept in the context and reused by
-// the next call of that site (grown when too small), so that a call allocates nothing once warm (a cudaFree would
-// also wait for the whole device). The calls of a context run in order on its stream, so reuse is safe.
-struct DevBufs {
-    bbgpu_ctx *ctx;
-    int tag;
-    size_t i = 0;
-    DevBufs(bbgpu_ctx *c, int t) : ctx(c), tag(t) {}
-    template <class T>
-    bool get(T **out, size_t n) {
-        std::vector<PoolBuf> &v = ctx->pool[tag];
-        if (i == v.size()) v.push_back(PoolBuf{});
-        PoolBuf &b = v[i++];
-        const size_t need = n ? n : 1;
-        if (b.cap < need) {
-            if (b.p) cudaFree(b.p);
-            b.p = nullptr;
-            b.cap = 0;
-            const size_t want = need + need / 4;
-            if (cudaMalloc(&b.p, want) != cudaSuccess) {
-                cudaGetLastError();
-                return false;
-            }
-            b.cap = want;
-        }
-        *out = (T *)b.p;
-        return true;
-    }
-};
-
 // The azimuthal samples and sub-ring constants of one ANALYTIC call, on the device.
 struct AnDev {
     AnSub *subs = nullptr;
     int *sbase = nullptr, *ssub = nullptr;
     double *cs = nullptr, *zq = nullptr, *wq = nullptr;
+    float *csf = nullptr, *zqf = nullptr;  // (float32 copies: the pixels' fast path)
     long long nsamp = 0;
 };
 
@@ -2026,14 +2070,19 @@ static int an_upload(bbgpu_ctx *ctx, DevBufs &B, const std::vector<AnSub> &subs,
     if (!B.get(&D.subs, sizeof(AnSub) * (subs.size() ? subs.size() : 1)) || !B.get(&D.sbase, sizeof(int) * sbase.size()) ||
         !B.get(&D.ssub, sizeof(int) * ssub.size()) || !B.get(&D.cs, sizeof(double) * cs.size()) ||
         !B.get(&D.zq, sizeof(double) * (zq.size() ? zq.size() : 1)) ||
-        !B.get(&D.wq, sizeof(double) * (wq.size() ? wq.size() : 1)))
+        !B.get(&D.wq, sizeof(double) * (wq.size() ? wq.size() : 1)) || !B.get(&D.csf, sizeof(float) * cs.size()) ||
+        !B.get(&D.zqf, sizeof(float) * (zq.size() ? zq.size() : 1)))
         return fail(ctx, BBGPU_ERR_NOMEM, "analytic: allocation failed");
     cudaStream_t s = ctx->stream;
     CK(cudaMemcpyAsync(D.subs, subs.data(), sizeof(AnSub) * subs.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(D.sbase, sbase.data(), sizeof(int) * sbase.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(D.ssub, ssub.data(), sizeof(int) * ssub.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(D.cs, cs.data(), sizeof(double) * cs.size(), cudaMemcpyHostToDevice, s));
+    std::vector<float> csf, zqf(zq.begin(), zq.end());
+    bbh_an_samples_f32(cs, csf);
+    CK(cudaMemcpyAsync(D.csf, csf.data(), sizeof(float) * csf.size(), cudaMemcpyHostToDevice, s));
     if (zq.size()) {
+        CK(cudaMemcpyAsync(D.zqf, zqf.data(), sizeof(float) * zqf.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(D.zq, zq.data(), sizeof(double) * zq.size(), cudaMemcpyHostToDevice, s));
         CK(cudaMemcpyAsync(D.wq, wq.data(), sizeof(double) * wq.size(), cudaMemcpyHostToDevice, s));
     }
@@ -2283,16 +2332,7 @@ static int wind_mc_run(bbgpu_ctx *ctx, double *out, bool cube, const double *sr,
         return BBGPU_OK;
     }
     DevBufs B(ctx, 5);
-    struct Trim {                          // (what a large model took goes back at the end of its call)
-        std::vector<PoolBuf> &v;
-        ~Trim() {
-            size_t sum = 0;
-            for (PoolBuf &b : v) sum += b.cap;
-            if (sum <= ((size_t)2 << 30)) return;
-            for (PoolBuf &b : v) cudaFree(b.p);
-            v.clear();
-        }
-    } trim{ctx->pool[5]};
+    PoolTrim trim{ctx->pool[5]};
     double *d_out = nullptr;
     if (!B.get(&R.acc, sizeof(uint64_t) * R.n) || !B.get(&d_out, cube ? sizeof(double) * R.n : 8))
         return fail(ctx, BBGPU_ERR_NOMEM, "galmod_wind: device allocation failed");
@@ -2381,20 +2421,12 @@ extern "C" int bbgpu_galwind_cube(bbgpu_ctx *ctx, double *out, const double *sr,
                           bhi1, threads);
 }
 
-extern "C" int bbgpu_galmod_analytic(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
-                                     int nzq, int blo0, int blo1, int bhi0, int bhi1) {
-    if (ctx) ctx->gen++;
-    if (!ctx) return BBGPU_ERR_ARG;
-    if (!out || !sr || ring_lo < 0 || ring_hi > nsub || ring_lo > ring_hi || blo0 > bhi0 || blo1 > bhi1)
-        return fail(ctx, BBGPU_ERR_ARG, "galmod_analytic: invalid arguments");
-    if (!ctx->grid_set) return fail(ctx, BBGPU_ERR_STATE, "galmod_analytic before set_grid");
-    if (!ctx->d_vedges) return fail(ctx, BBGPU_ERR_STATE, "galmod_analytic: set_grid was given no channel edges");
+// The ANALYTIC model of the sub-rings [ring_lo, ring_hi) in the box on the device: its fixed-point sums (by, bx, nz) in
+// units of 2^-e, and its member (device).
+static int galmod_analytic_dev(bbgpu_ctx *ctx, DevBufs &B, const double *sr, int nsub, int ring_lo, int ring_hi, int nzq,
+                               int blo0, int blo1, int bhi0, int bhi1, long long **o64, MemberDev **dm, int *exp2) {
     const GridDev &g = ctx->g;
-    if (an_smem_bytes(g.nz, g.nlines) > AN_SMEM_MAX)
-        return fail(ctx, BBGPU_ERR_ARG, "galmod_analytic: %d channels x %d lines above the device limit", g.nz, g.nlines);
-    CK(cudaSetDevice(ctx->device));
     const int ns = ring_hi - ring_lo, by = bhi1 - blo1, bx = bhi0 - blo0;
-    if (ns == 0 || by == 0 || bx == 0) return BBGPU_OK;
     std::vector<double> s2((size_t)BBGPU_NSR * ns);
     for (int r = 0; r < BBGPU_NSR; r++)
         for (int i = 0; i < ns; i++) s2[(size_t)r * ns + i] = sr[(size_t)r * nsub + ring_lo + i];
@@ -2404,37 +2436,109 @@ extern "C" int bbgpu_galmod_analytic(bbgpu_ctx *ctx, double *out, const double *
                               subs.data(), zc);
     const std::vector<double> &zq = zc.zq, &wq = zc.wq;
     if (e == -10000) return fail(ctx, BBGPU_ERR_ARG, "galmod_analytic: the total flux is not finite");
-    DevBufs B(ctx, 0);
     AnDev D;
     int rc = an_upload(ctx, B, subs, s2.data(), ns, zq, wq, D);
     if (rc) return rc;
     const size_t n = (size_t)by * bx * g.nz;
-    long long *o64 = nullptr;
-    MemberDev *dm = nullptr;
-    if (!B.get(&o64, n * sizeof(long long)) || !B.get(&dm, sizeof(MemberDev)))
+    long long *ast = nullptr;
+    int *asg = nullptr;
+    if (!B.get(o64, n * sizeof(long long)) || !B.get(dm, sizeof(MemberDev)) || !B.get(&ast, 2 * sizeof(long long)) ||
+        !B.get(&asg, 4 * sizeof(int)))
         return fail(ctx, BBGPU_ERR_NOMEM, "galmod_analytic: allocation failed");
     MemberDev M{};
     M.blo0 = blo0; M.blo1 = blo1; M.bhi0 = bhi0; M.bhi1 = bhi1; M.bx = bx; M.by = by; M.fix_exp = e;
     cudaStream_t s = ctx->stream;
-    CK(cudaMemcpyAsync(dm, &M, sizeof M, cudaMemcpyHostToDevice, s));
-    CK(cudaMemsetAsync(o64, 0, n * sizeof(long long), s));
-    long long *ast = nullptr;
-    int *asg = nullptr;
-    if (!B.get(&ast, 2 * sizeof(long long)) || !B.get(&asg, 4 * sizeof(int)))
-        return fail(ctx, BBGPU_ERR_NOMEM, "galmod_analytic: allocation failed");
     const long long hst[2] = {0, D.nsamp};
     const int hsg[4] = {0, 0, -1, 1};                   // (the member's own samples)
+    CK(cudaMemcpyAsync(*dm, &M, sizeof M, cudaMemcpyHostToDevice, s));
+    CK(cudaMemsetAsync(*o64, 0, n * sizeof(long long), s));
     CK(cudaMemcpyAsync(ast, hst, sizeof hst, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(asg, hsg, sizeof hsg, cudaMemcpyHostToDevice, s));
-    launch_an_model(s, g, D.subs, ns, D.sbase, D.ssub, D.cs, ast, asg, 1, D.nsamp, D.zq, D.wq, ctx->d_vedges,
-                    ctx->d_cd2i, ctx->d_ptab, dm, o64, (long long)n, 0);
+    launch_an_model(s, g, D.subs, ns, D.sbase, D.ssub, D.cs, D.csf, ast, asg, 1, D.nsamp, D.zq, D.wq, D.zqf,
+                    ctx->d_vedges, ctx->d_cd2i, ctx->d_ptab, *dm, *o64, (long long)n, 0);
     CKL();
+    *exp2 = e;
+    return 0;
+}
+
+static int analytic_args(bbgpu_ctx *ctx, const double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
+                         int blo0, int blo1, int bhi0, int bhi1) {
+    if (!out || !sr || ring_lo < 0 || ring_hi > nsub || ring_lo > ring_hi || blo0 > bhi0 || blo1 > bhi1)
+        return fail(ctx, BBGPU_ERR_ARG, "galmod_analytic: invalid arguments");
+    if (!ctx->grid_set) return fail(ctx, BBGPU_ERR_STATE, "galmod_analytic before set_grid");
+    if (!ctx->d_vedges) return fail(ctx, BBGPU_ERR_STATE, "galmod_analytic: set_grid was given no channel edges");
+    if (an_smem_bytes(ctx->g.nz, ctx->g.nlines) > AN_SMEM_MAX)
+        return fail(ctx, BBGPU_ERR_ARG, "galmod_analytic: %d channels x %d lines above the device limit", ctx->g.nz,
+                    ctx->g.nlines);
+    return 0;
+}
+
+extern "C" int bbgpu_galmod_analytic(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
+                                     int nzq, int blo0, int blo1, int bhi0, int bhi1) {
+    if (ctx) ctx->gen++;
+    if (!ctx) return BBGPU_ERR_ARG;
+    int rc = analytic_args(ctx, out, sr, nsub, ring_lo, ring_hi, blo0, blo1, bhi0, bhi1);
+    if (rc) return rc;
+    CK(cudaSetDevice(ctx->device));
+    if (ring_hi == ring_lo || bhi1 == blo1 || bhi0 == blo0) return BBGPU_OK;
+    DevBufs B(ctx, 0);
+    long long *o64 = nullptr;
+    MemberDev *dm = nullptr;
+    int e = 0;
+    rc = galmod_analytic_dev(ctx, B, sr, nsub, ring_lo, ring_hi, nzq, blo0, blo1, bhi0, bhi1, &o64, &dm, &e);
+    if (rc) return rc;
+    const size_t n = (size_t)(bhi1 - blo1) * (bhi0 - blo0) * ctx->g.nz;
     std::vector<long long> h(n);
-    CK(cudaMemcpyAsync(h.data(), o64, n * sizeof(long long), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    CK(cudaMemcpyAsync(h.data(), o64, n * sizeof(long long), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
     const double sc = ldexp(1.0, -e);
     for (size_t i = 0; i < n; i++) out[i] += (double)h[i] * sc;
     return BBGPU_OK;
+}
+
+// The convolved model as a cube: the model built, converted to float32 (what bbgpu_convolve does to its input),
+// convolved and turned to (nz, by, bx) on the device, one copy back.
+extern "C" int bbgpu_model_cube(bbgpu_ctx *ctx, int galmodtype, double *out, const double *sr, int nsub, uint64_t seed,
+                                const int64_t *nv, int nzq, int blo0, int blo1, int bhi0, int bhi1, double scale) {
+    if (ctx) ctx->gen++;
+    if (!ctx) return BBGPU_ERR_ARG;
+    if (galmodtype != BBGPU_MC && galmodtype != BBGPU_ANALYTIC)
+        return fail(ctx, BBGPU_ERR_ARG, "model_cube: galmodtype %d not supported", galmodtype);
+    if (!out || !sr || nsub < 1 || blo0 >= bhi0 || blo1 >= bhi1 || (galmodtype == BBGPU_MC && !nv))
+        return fail(ctx, BBGPU_ERR_ARG, "model_cube: invalid arguments");
+    if (!ctx->kernel_set) return fail(ctx, BBGPU_ERR_STATE, "model_cube before set_kernel");
+    int rc = 0;
+    if (galmodtype == BBGPU_ANALYTIC && (rc = analytic_args(ctx, out, sr, nsub, 0, nsub, blo0, blo1, bhi0, bhi1)))
+        return rc;
+    CK(cudaSetDevice(ctx->device));
+    const int nz = ctx->g.nz, by = bhi1 - blo1, bx = bhi0 - blo0;
+    const size_t n = (size_t)by * bx * nz;
+    PoolTrim trim{ctx->pool[7]};
+    DevBufs B(ctx, 7);
+    double *d64 = nullptr;
+    float *a = nullptr, *b = nullptr;
+    if (!B.get(&d64, n * sizeof(double)) || !B.get(&a, n * sizeof(float)) || !B.get(&b, n * sizeof(float)))
+        return fail(ctx, BBGPU_ERR_NOMEM, "model_cube: allocation failed");
+    cudaStream_t s = ctx->stream;
+    if (galmodtype == BBGPU_ANALYTIC) {
+        long long *o64 = nullptr;
+        MemberDev *dm = nullptr;
+        int e = 0;
+        rc = galmod_analytic_dev(ctx, B, sr, nsub, 0, nsub, nzq, blo0, blo1, bhi0, bhi1, &o64, &dm, &e);
+        if (rc) return rc;
+        launch_fix_to_model(s, o64, dm, 1, (long long)n, nz, a, nullptr);
+    } else {
+        rc = galmod_mc_dev(ctx, sr, nsub, 0, nsub, seed, nv, blo0, blo1, bhi0, bhi1);
+        if (rc) return rc;
+        launch_f64_to_f32(s, ctx->d_model64, (long long)n, a);
+    }
+    CKL();
+    rc = conv_dev(ctx, B, a, b, nz, by, bx, scale, 1);
+    if (rc) return rc;
+    launch_yxz32_to_zyx64(s, b, d64, nz, by, bx);
+    CKL();
+    CK(cudaMemcpyAsync(out, d64, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+    return check_err(ctx);                              // (waits for the stream)
 }
 
 extern "C" int bbgpu_ring_maps_analytic(bbgpu_ctx *ctx, double *out, int nr, const double *sr, int nsub,
@@ -2526,12 +2630,11 @@ extern "C" int bbgpu_norm(bbgpu_ctx *ctx, double *model, int bsy, int bsx, int n
     // the box of the data and mask ("yxz"), contiguous
     std::vector<float> dbox(n ? n : 1);
     std::vector<uint8_t> mbox(n ? n : 1);
-    for (int y = 0; y < bsy; y++)
-        for (int x = 0; x < bsx; x++) {
-            const size_t src = (((size_t)(y + blo1)) * dnx + (size_t)(x + blo0)) * nz;
-            memcpy(&dbox[((size_t)y * bsx + x) * nz], data + src, sizeof(float) * nz);
-            memcpy(&mbox[((size_t)y * bsx + x) * nz], mask + src, nz);
-        }
+    for (int y = 0; y < bsy && n; y++) {
+        const size_t src = (((size_t)(y + blo1)) * dnx + (size_t)blo0) * nz, dst = (size_t)y * bsx * nz;
+        memcpy(&dbox[dst], data + src, sizeof(float) * (size_t)bsx * nz);
+        memcpy(&mbox[dst], mask + src, (size_t)bsx * nz);
+    }
     DevBufs B(ctx, 3);
     double *dm = nullptr, *dw = nullptr, *dcn = nullptr, *dpre = nullptr, *dthr = nullptr, *dpart = nullptr,
            *dP = nullptr;
@@ -2566,7 +2669,7 @@ extern "C" int bbgpu_norm(bbgpu_ctx *ctx, double *model, int bsy, int bsx, int n
     std::vector<double> part((size_t)np * 4 + 1);
     double factor = 1.0;
     if (normtype == 1 && np) {
-        launch_norm_sums(s, dm, dd, dk, din, bsy, bsx, nz, dpart);
+        launch_norm_sums(s, dm, dd, dk, bsx, 0, 0, din, bsy, bsx, nz, dpart);
         CKL();
         CK(cudaMemcpyAsync(part.data(), dpart, (size_t)np * 2 * 8, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -2578,8 +2681,8 @@ extern "C" int bbgpu_norm(bbgpu_ctx *ctx, double *model, int bsy, int bsx, int n
         factor = ms != 0 ? os / ms : 0.0;
     }
     if (np) {
-        launch_norm_pix(s, dm, dd, dk, din, dw, bsy, bsx, nz, ftype, dcn, data_noise, normtype, factor, dP, dilo, dihi,
-                        ky, dthr, dpart);
+        launch_norm_pix(s, dm, dd, dk, bsx, 0, 0, din, dw, bsy, bsx, nz, ftype, dcn, data_noise, normtype, factor, dP,
+                        dilo, dihi, ky, dthr, dpart);
         CKL();
         CK(cudaMemcpyAsync(part.data(), dpart, (size_t)np * 4 * 8, cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(model, dm, n * 8, cudaMemcpyDeviceToHost, s));
@@ -2594,6 +2697,106 @@ extern "C" int bbgpu_norm(bbgpu_ctx *ctx, double *model, int bsy, int bsx, int n
     }
     if (nt - nb == 0) *out = INFINITY;
     else *out = pow(1 + (double)nb / (double)nt, bweight) * minfunc / (double)(nt - nb);
+    return BBGPU_OK;
+}
+
+// CLASSIC: the data, mask ("yxz") and channel noise of a fit, kept for bbgpu_classic_residual.
+extern "C" int bbgpu_classic_set(bbgpu_ctx *ctx, const float *data, const uint8_t *mask, int dny, int dnx, int nz,
+                                 const double *chan_noise) {
+    if (ctx) ctx->gen++;
+    if (!ctx) return BBGPU_ERR_ARG;
+    if (!data || !mask || !chan_noise || dny < 1 || dnx < 1 || nz < 1 || !ctx->grid_set || nz != ctx->g.nz)
+        return fail(ctx, BBGPU_ERR_ARG, "classic_set: invalid arguments");
+    CK(cudaSetDevice(ctx->device));
+    const size_t n = (size_t)dny * dnx * nz;
+    int rc;
+    if ((rc = dgrow(ctx, &ctx->d_cdata, &ctx->d_cdata_cap, n)) || (rc = dgrow(ctx, &ctx->d_cmask, &ctx->d_cmask_cap, n)) ||
+        (rc = dgrow(ctx, &ctx->d_cnoise, &ctx->d_cnoise_cap, (size_t)nz)))
+        return rc;
+    CK(cudaMemcpyAsync(ctx->d_cdata, data, sizeof(float) * n, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_cmask, mask, n, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(ctx->d_cnoise, chan_noise, sizeof(double) * nz, cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    ctx->cny = dny;
+    ctx->cnx = dnx;
+    return BBGPU_OK;
+}
+
+// One CLASSIC evaluation (Galfit.getFuncValue, bbarolo/galfit.py:736-749) without its round trips: the Monte-Carlo
+// model of the ring, its sparse convolution (kernel: ky = 0, none) and _norm on the device, the kernels and the order
+// of the sums those of bbgpu_galmod_mc, bbgpu_conv_sparse and bbgpu_norm, of which each copied the box to the host and
+// back.
+extern "C" int bbgpu_classic_residual(bbgpu_ctx *ctx, const double *sr, int nsub, uint64_t seed, const int64_t *nv,
+                                      int blo0, int blo1, int bhi0, int bhi1, const double *kernel, int ky, int kx,
+                                      double scale, double x0, double y0, double phi, double inc, double r1, double r2,
+                                      double wpow, int side, int ftype, double data_noise, double bweight,
+                                      int normtype, double *out) {
+    if (ctx) ctx->gen++;
+    if (!ctx) return BBGPU_ERR_ARG;
+    const int bsx = bhi0 - blo0, bsy = bhi1 - blo1, nz = ctx->g.nz;
+    if (!sr || !nv || !out || nsub < 0 || blo0 < 0 || blo1 < 0 || bsx < 0 || bsy < 0 || ky < 0 || kx < 0 || (ky && !kernel))
+        return fail(ctx, BBGPU_ERR_ARG, "classic_residual: invalid arguments");
+    if (!ctx->d_cdata) return fail(ctx, BBGPU_ERR_STATE, "classic_residual before classic_set");
+    if (bhi0 > ctx->cnx || bhi1 > ctx->cny) return fail(ctx, BBGPU_ERR_ARG, "classic_residual: box outside the data");
+    CK(cudaSetDevice(ctx->device));
+    *out = INFINITY;
+    const int np = bsx * bsy;
+    if (np == 0) return BBGPU_OK;                       // (no voxel counts)
+    const size_t n = (size_t)np * nz;
+    cudaStream_t s = ctx->stream;
+    DevBufs B(ctx, 3);
+    double *dm = nullptr, *dk = nullptr, *dw = nullptr, *dpart = nullptr;
+    uint8_t *din = nullptr;
+    if (!B.get(&dm, n * 8) || !B.get(&dk, std::max((size_t)ky * kx, (size_t)1) * 8) || !B.get(&dpart, (size_t)np * 4 * 8) ||
+        !B.get(&dw, (size_t)np * 9))
+        return fail(ctx, BBGPU_ERR_NOMEM, "classic_residual: allocation failed");
+    din = (uint8_t *)(dw + np);
+    int rc;
+    if ((rc = hgrow(ctx, &ctx->h_cpix, &ctx->h_cpix_cap, (size_t)np * 4 + (np + 7) / 8))) return rc;
+    // the model, and beside it the ring's pixels and weights (host: the reference's float64 and C library calls); the
+    // pinned buffer takes them there and the pixels' sums back
+    if (nsub) {
+        if ((rc = galmod_mc_dev(ctx, sr, nsub, 0, nsub, seed, nv, blo0, blo1, bhi0, bhi1))) return rc;
+    }
+    const double *model = ctx->d_model64;
+    if (!nsub) {
+        CK(cudaMemsetAsync(dm, 0, n * 8, s));
+    } else if (ky) {
+        CK(cudaMemcpyAsync(dk, kernel, (size_t)ky * kx * 8, cudaMemcpyHostToDevice, s));
+        launch_conv_sparse(s, model, dm, bsy, bsx, nz, dk, ky, kx, scale);
+        CKL();
+    } else {
+        CK(cudaMemcpyAsync(dm, model, n * 8, cudaMemcpyDeviceToDevice, s));
+    }
+    bbh_norm_footprint(bsy, bsx, x0, y0, phi, inc, r1, r2, wpow, side, 0, 0.0, (uint8_t *)(ctx->h_cpix + np), ctx->h_cpix);
+    CK(cudaMemcpyAsync(dw, ctx->h_cpix, (size_t)np * 9, cudaMemcpyHostToDevice, s));
+    double *part = ctx->h_cpix;
+    double factor = 1.0;
+    if (normtype == 1) {
+        launch_norm_sums(s, dm, ctx->d_cdata, ctx->d_cmask, ctx->cnx, blo0, blo1, din, bsy, bsx, nz, dpart);
+        CKL();
+        CK(cudaMemcpyAsync(part, dpart, (size_t)np * 2 * 8, cudaMemcpyDeviceToHost, s));
+        CK(cudaStreamSynchronize(s));
+        double ms = 0.0, os = 0.0;
+        for (int p = 0; p < np; p++) {
+            ms += part[2 * p];
+            os += part[2 * p + 1];
+        }
+        factor = ms != 0 ? os / ms : 0.0;
+    }
+    launch_norm_pix(s, dm, ctx->d_cdata, ctx->d_cmask, ctx->cnx, blo0, blo1, din, dw, bsy, bsx, nz, ftype, ctx->d_cnoise,
+                    data_noise, normtype, factor, nullptr, nullptr, nullptr, 0, nullptr, dpart);
+    CKL();
+    CK(cudaMemcpyAsync(part, dpart, (size_t)np * 4 * 8, cudaMemcpyDeviceToHost, s));
+    if ((rc = check_err(ctx))) return rc;               // (waits for the stream)
+    double minfunc = 0.0;
+    long long nb = 0, nt = 0;
+    for (int p = 0; p < np; p++) {
+        minfunc += part[4 * p];
+        nb += (long long)part[4 * p + 1];
+        nt += (long long)part[4 * p + 2];
+    }
+    if (nt - nb != 0) *out = pow(1 + (double)nb / (double)nt, bweight) * minfunc / (double)(nt - nb);
     return BBGPU_OK;
 }
 

@@ -26,16 +26,26 @@ __global__ void k_conv_sparse(const double *__restrict__ model, double *__restri
     const long long p = i / nz;
     const int x = (int)(p % nx), y = (int)(p / nx);
     const int hy = ky / 2, hx = kx / 2;
+    // (most voxels of a single ring's box are empty: their terms add nothing and cost no float64 operation; the values
+    // of eight taps are loaded before the first is used)
     double s = 0.0;
     for (int j = ky - 1; j >= 0; j--) {
         const int yy = y - j + hy;
         if (yy < 0 || yy >= ny) continue;
-        for (int q = kx - 1; q >= 0; q--) {
-            const double kv = kern[j * kx + q];
-            if (kv == 0.0) continue;
-            const int xx = x - q + hx;
-            if (xx < 0 || xx >= nx) continue;
-            s = __dadd_rn(s, __dmul_rn(kv, model[((size_t)yy * nx + xx) * nz + z]));
+        const double *row = model + (size_t)yy * nx * nz + z;
+        for (int q0 = kx - 1; q0 >= 0; q0 -= 8) {
+            double m[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int xx = x - (q0 - u) + hx;
+                m[u] = q0 - u >= 0 && xx >= 0 && xx < nx ? __ldg(row + (size_t)xx * nz) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if ((__double_as_longlong(m[u]) << 1) != 0) {
+                    const double kv = __ldg(kern + j * kx + q0 - u);
+                    if (kv != 0.0) s = __dadd_rn(s, __dmul_rn(kv, m[u]));
+                }
         }
     }
     out[i] = s < 1.E-12 ? 0.0 : (scale != 1.0 ? __dmul_rn(s, scale) : s);
@@ -57,16 +67,17 @@ __global__ void k_norm_prefix(const double *__restrict__ pre, double *__restrict
 
 // _norm, pass 1 (NORM AZIM): sums of the model and of the data in the mask over the pixels of the ring.
 __global__ void k_norm_sums(const double *__restrict__ model, const float *__restrict__ data,
-                            const uint8_t *__restrict__ mask, const uint8_t *__restrict__ inside, int bsy, int bsx,
-                            int nz, double *__restrict__ part) {
+                            const uint8_t *__restrict__ mask, int dnx, int x0, int y0,
+                            const uint8_t *__restrict__ inside, int bsy, int bsx, int nz, double *__restrict__ part) {
     __shared__ double sm[256], so[256];
     const int p = blockIdx.x;           // pixel
+    const size_t dq = ((size_t)(p / bsx + y0) * dnx + p % bsx + x0) * nz;
     double a = 0.0, b = 0.0;
     if (inside[p])
         for (int z = threadIdx.x; z < nz; z += blockDim.x) {
             const size_t q = (size_t)p * nz + z;
             a += model[q];
-            if (mask[q]) b += data[q];
+            if (mask[dq + z]) b += data[dq + z];
         }
     sm[threadIdx.x] = a;
     so[threadIdx.x] = b;
@@ -91,7 +102,7 @@ __global__ void k_norm_sums(const double *__restrict__ model, const float *__res
 // factor); the sum over channels is a fixed tree (the reference's running sum over all voxels differs from it
 // by rounding only).
 __global__ void k_norm_pix(double *__restrict__ model, const float *__restrict__ data, const uint8_t *__restrict__ mask,
-                           const uint8_t *__restrict__ inside, const double *__restrict__ wmap, int bsy, int bsx, int nz,
+                           int dnx, int x0, int y0, const uint8_t *__restrict__ inside, const double *__restrict__ wmap, int bsy, int bsx, int nz,
                            int ftype, const double *__restrict__ chan_noise, double data_noise, int normtype,
                            double factor_azim, const double *__restrict__ P, const long long *__restrict__ ilo,
                            const long long *__restrict__ ihi, int ky, const double *__restrict__ thr,
@@ -101,6 +112,7 @@ __global__ void k_norm_pix(double *__restrict__ model, const float *__restrict__
     __shared__ int s_ca, s_cb;
     const int p = blockIdx.x;
     const int y = p / bsx, x = p - y * bsx;
+    const size_t dq = ((size_t)(y + y0) * dnx + x + x0) * nz;
     if (!inside[p]) {
         if (threadIdx.x == 0) { part[4 * p] = 0.0; part[4 * p + 1] = 0.0; part[4 * p + 2] = 0.0; part[4 * p + 3] = 0.0; }
         return;
@@ -114,8 +126,8 @@ __global__ void k_norm_pix(double *__restrict__ model, const float *__restrict__
             for (int z = 0; z < nz; z++) {
                 const size_t q = (size_t)p * nz + z;
                 a = __dadd_rn(a, model[q]);
-                const double o = data[q];
-                if (o > 0 && mask[q]) b = __dadd_rn(b, o);
+                const double o = data[dq + z];
+                if (o > 0 && mask[dq + z]) b = __dadd_rn(b, o);
             }
             f = a != 0 ? __ddiv_rn(b, a) : 0.0;
         }
@@ -130,7 +142,7 @@ __global__ void k_norm_pix(double *__restrict__ model, const float *__restrict__
     if (trunc)
         for (int z = threadIdx.x; z < nz; z += blockDim.x) {
             const size_t q = (size_t)p * nz + z;
-            if (model[q] != 0 && !mask[q]) { atomicMin(&s_ca, z); atomicMax(&s_cb, z); }
+            if (model[q] != 0 && !mask[dq + z]) { atomicMin(&s_ca, z); atomicMax(&s_cb, z); }
         }
     __syncthreads();
     const int ca = s_ca, cb = s_cb;
@@ -141,10 +153,10 @@ __global__ void k_norm_pix(double *__restrict__ model, const float *__restrict__
     for (int z = threadIdx.x; z < nz; z += blockDim.x) {
         const size_t q = (size_t)p * nz + z;
         if (normtype != 2) model[q] = __dmul_rn(model[q], factor);
-        const double o = data[q];
+        const double o = data[dq + z];
         const double obs = o > 0 ? o : data_noise;
         const double mod = model[q];
-        if (!mask[q]) {
+        if (!mask[dq + z]) {
             if (mod == 0) continue;
             if (trunc) {
                 // lam: the rows' sums of pre over the kernel footprint, from the running sums (reference order)
@@ -202,10 +214,10 @@ void launch_conv_sparse(cudaStream_t s, const double *model, double *out, int ny
     k_conv_sparse<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(model, out, ny, nx, nz, kern, ky, kx, scale);
 }
 
-void launch_norm_sums(cudaStream_t s, const double *model, const float *data, const uint8_t *mask,
-                      const uint8_t *inside, int bsy, int bsx, int nz, double *part) {
+void launch_norm_sums(cudaStream_t s, const double *model, const float *data, const uint8_t *mask, int dnx, int x0,
+                      int y0, const uint8_t *inside, int bsy, int bsx, int nz, double *part) {
     if (bsy * bsx == 0) return;
-    k_norm_sums<<<bsy * bsx, 128, 0, s>>>(model, data, mask, inside, bsy, bsx, nz, part);
+    k_norm_sums<<<bsy * bsx, 128, 0, s>>>(model, data, mask, dnx, x0, y0, inside, bsy, bsx, nz, part);
 }
 
 void launch_norm_prefix(cudaStream_t s, const double *pre, double *P, int bsy, int bsx, int nz) {
@@ -214,11 +226,11 @@ void launch_norm_prefix(cudaStream_t s, const double *pre, double *P, int bsy, i
     k_norm_prefix<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(pre, P, bsy, bsx, nz);
 }
 
-void launch_norm_pix(cudaStream_t s, double *model, const float *data, const uint8_t *mask, const uint8_t *inside,
-                     const double *wmap, int bsy, int bsx, int nz, int ftype, const double *chan_noise,
+void launch_norm_pix(cudaStream_t s, double *model, const float *data, const uint8_t *mask, int dnx, int x0, int y0,
+                     const uint8_t *inside, const double *wmap, int bsy, int bsx, int nz, int ftype, const double *chan_noise,
                      double data_noise, int normtype, double factor_azim, const double *P, const long long *ilo,
                      const long long *ihi, int ky, const double *thr, double *part) {
     if (bsy * bsx == 0) return;
-    k_norm_pix<<<bsy * bsx, 128, 0, s>>>(model, data, mask, inside, wmap, bsy, bsx, nz, ftype, chan_noise, data_noise,
+    k_norm_pix<<<bsy * bsx, 128, 0, s>>>(model, data, mask, dnx, x0, y0, inside, wmap, bsy, bsx, nz, ftype, chan_noise, data_noise,
                                         normtype, factor_azim, P, ilo, ihi, ky, thr, part);
 }

@@ -545,12 +545,13 @@ void bbh_norm_footprint(int bsy, int bsx, double x0, double y0, double phi, doub
             const double ys = -(x - x0) * cphi - (y - y0) * sphi;
             const double yr = ys / cinc;
             const double r = sqrt(xr * xr + yr * yr);
-            double th = r < 0.1 ? 0.0 : atan2(yr, xr) / F;
+            double th;
             if (foot == 1) {
                 if (!(fabs(xr) >= r1 && fabs(xr) <= r2 && fabs(ys) <= hmax)) continue;
                 th = xr >= 0 ? 0.0 : 180.0;
-            } else if (!(r >= r1 && r <= r2)) {
-                continue;
+            } else {
+                if (!(r >= r1 && r <= r2)) continue;
+                th = r < 0.1 ? 0.0 : atan2(yr, xr) / F;
             }
             if (side == 1 && !(fabs(th) <= 90.0)) continue;
             if (side == 2 && !(fabs(th) >= 90.0)) continue;

@@ -60,6 +60,14 @@ struct ZigDev {
 void launch_mc_bin(cudaStream_t s, const GridDev &g, const LayoutDev &L, const SubMC *sub, int nsub,
                    const MemberDev *mem, const long long *cstart, const int *cseg, int nseg, long long ntot, int tx,
                    int ty, int *pix, int *tile_count, int *err);
+// float64 and float32 values of n fixed-point sums (unit 2^-e, times cd2i of the channel)
+void launch_mc_sums64(cudaStream_t s, const long long *sums, long long n, int nz, const double *cd2i,
+                      const float *cd2if, int e, double *out, float *model);
+// The CTAs that share a tile's clouds in the pixel-owned deposit of one member with ntile tiles (argument split;
+// they add their sums to base64, and no float32 model is written).
+// Measured: one ring of a 64x64x64 cube (9 tiles, 20 k clouds) 81 us with one CTA a tile, 20 us with 16; from 304
+// tiles on the chip is full (two CTAs per SM) and a split would only repeat the tiles' zeroing and output.
+int mc_deposit_split(int ntile);
 // Exclusive scan of n list counts into offsets (and cursors); scratch holds (n + 1023) / 1024 ints.
 void launch_scan_tiles(cudaStream_t s, const int *count, int *offset, int *cursor, int n, int *scratch);
 // bucket: 32-byte entries (Entry in mc.cu), one per in-box (member, cloud)
@@ -108,7 +116,7 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
                        const int *offset, const int *count, const void *bucket, const ZigDev *zig,
                        const float *cd2if, const double *cd2i, float *model, long long mstride, double *model64,
                        int *err, int lean, const int *klist = nullptr, int nk = 0, int delta = 0,
-                       long long *base64 = nullptr, int *tsrc = nullptr, Replay rp = Replay{nullptr, nullptr, nullptr, nullptr, 0, nullptr});
+                       long long *base64 = nullptr, int *tsrc = nullptr, Replay rp = Replay{nullptr, nullptr, nullptr, nullptr, 0, nullptr}, int split = 1);
 
 // ---- convolution + residual (conv.cu)
 // The taps of a beam kernel (ky, kx) as the conv kernels read them: flipped, float32, rows padded to the
@@ -170,17 +178,19 @@ void launch_prep_deff(cudaStream_t s, const float *data, const uint8_t *mask, co
 int launch_sumsq64(cudaStream_t s, const double *model, const float *data, const uint8_t *mask, int maskmode,
                    const uint8_t *region, int nz, int ny, int nx, double sigma2, double eps2, double *partial,
                    int maxblocks);
+void launch_f64_to_f32(cudaStream_t s, const double *in, long long n, float *out);
 void launch_zyx64_to_yxz32(cudaStream_t s, const double *in, float *out, int nz, int ny, int nx);
 void launch_yxz32_to_zyx64(cudaStream_t s, const float *in, double *out, int nz, int ny, int nx);
 
 // ---- CLASSIC (classic.cu)
 void launch_conv_sparse(cudaStream_t s, const double *model, double *out, int ny, int nx, int nz, const double *kern,
                         int ky, int kx, double scale);
-void launch_norm_sums(cudaStream_t s, const double *model, const float *data, const uint8_t *mask,
-                      const uint8_t *inside, int bsy, int bsx, int nz, double *part);
+void launch_norm_sums(cudaStream_t s, const double *model, const float *data, const uint8_t *mask, int dnx, int x0,
+                      int y0, const uint8_t *inside, int bsy, int bsx, int nz, double *part);
+// data and mask: the pixel (x, y) of the box is pixel (x0 + x, y0 + y) of rows of dnx pixels
 void launch_norm_prefix(cudaStream_t s, const double *pre, double *P, int bsy, int bsx, int nz);
-void launch_norm_pix(cudaStream_t s, double *model, const float *data, const uint8_t *mask, const uint8_t *inside,
-                     const double *wmap, int bsy, int bsx, int nz, int ftype, const double *chan_noise,
+void launch_norm_pix(cudaStream_t s, double *model, const float *data, const uint8_t *mask, int dnx, int x0, int y0,
+                     const uint8_t *inside, const double *wmap, int bsy, int bsx, int nz, int ftype, const double *chan_noise,
                      double data_noise, int normtype, double factor_azim, const double *P, const long long *ilo,
                      const long long *ihi, int ky, const double *thr, double *part);
 
@@ -192,9 +202,10 @@ size_t an_smem_bytes(int nz, int nlines);
 // astart[i + 1], ntot = astart[nseg]) is aseg[4i .. 4i + 4) = (member whose model takes the deposits, member whose
 // constants make them, sub-ring (-1: every sample of the table), sign of the deposits).
 void launch_an_model(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
-                     const double *cs, const long long *astart, const int *aseg, int nseg, long long ntot,
-                     const double *zq, const double *wq, const double *vedges, const double *cd2i, const double *ptab,
-                     const MemberDev *mem, long long *out64, long long mstride, int skip_fast);
+                     const double *cs, const float *csf, const long long *astart, const int *aseg, int nseg,
+                     long long ntot, const double *zq, const double *wq, const float *zqf, const double *vedges,
+                     const double *cd2i, const double *ptab, const MemberDev *mem, long long *out64, long long mstride,
+                     int skip_fast);
 // the float32 path of the ANALYTIC model (sub-rings with anfast; launch_an_model with skip_fast does the others):
 // csf, zqf, wqf float32 copies of the sample and vertical tables, csff (float4 per sample) its cos and sin in
 // float-float, vef (nz + 1) float-float channel edges of line 0

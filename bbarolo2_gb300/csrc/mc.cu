@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(256, PX_MINB) k_mc_deposit_px(GridDev g, Layou
             any |= (rp.tmask[(size_t)t * rp.nchw + threadIdx.x] & rp.chg[(size_t)k * rp.nchw + threadIdx.x]) != 0;
         if (!__syncthreads_or(any)) {
             if (tsrc && threadIdx.x == 0) tsrc[mem[k].tile_off + t] = delta == 1 ? 0 : k;
-            if (delta == 1) return;
+            if (delta == 1 || gridDim.z > 1) return;
             for (int lp = warp; lp < TP; lp += 8) {
                 const int py = y0 + lp / tx, px = x0 + lp % tx;
                 if (py >= by || px >= bx) continue;
@@ -1148,8 +1148,13 @@ __global__ void __launch_bounds__(256, PX_MINB) k_mc_deposit_px(GridDev g, Layou
     const int grp = lane / LPP, q = lane % LPP;
     const int lp = warp + 8 * grp;
     const bool own = lp < TP;
-    const int beg = own ? offset[lbase + 8 * warp + grp] : 0;
-    const int n = own ? count[lbase + 8 * warp + grp] : 0;
+    int beg = own ? offset[lbase + 8 * warp + grp] : 0;
+    int n = own ? count[lbase + 8 * warp + grp] : 0;
+    if (gridDim.z > 1) {                                    // this CTA's part of the pixel's clouds
+        const int e0 = (int)((long long)n * blockIdx.z / gridDim.z);
+        n = (int)((long long)n * (blockIdx.z + 1) / gridDim.z) - e0;
+        beg += e0;
+    }
     const int rowoff = (own ? lp : 0) * RS + 2 * grp;
     PxDefer *qe = qall + warp * PX_QCAP;
     int *qn = qns + warp;
@@ -1236,7 +1241,10 @@ __global__ void __launch_bounds__(256, PX_MINB) k_mc_deposit_px(GridDev g, Layou
         const unsigned long long *src = tile + (size_t)p * RS + 2 * (p >> 3);
         const size_t v0 = ((size_t)py * bx + px) * nz;
         float *o = mout + v0;
-        if (delta == 1) {
+        if (gridDim.z > 1) {
+            for (int z = lane; z < nz; z += 32)
+                if (src[z]) atomicAdd(&wbase[v0 + z], src[z]);
+        } else if (delta == 1) {
             for (int z = lane; z < nz; z += 32) o[z] = ll_to_f32((long long)(src[z] + base64[v0 + z])) * chs[z];
         } else {
             for (int z = lane; z < nz; z += 32) o[z] = ll_to_f32((long long)src[z]) * chs[z];
@@ -1263,6 +1271,17 @@ __global__ void k_fill_submc(SubMC *__restrict__ sub, int nsub, int nb, const si
         }
     }
     sub[i] = S;
+}
+
+// The models of one member from its fixed-point sums (as k_mc_deposit_px writes its own).
+__global__ void k_mc_sums64(const long long *__restrict__ sums, long long n, int nz, const double *__restrict__ cd2i,
+                            const float *__restrict__ cd2if, int e, double *__restrict__ out,
+                            float *__restrict__ model) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const long long q = sums[i];
+    model[i] = ll_to_f32(q) * ldexpf(cd2if[i % nz], -e);
+    out[i] = q ? ldexp((double)q * cd2i[i % nz], -e) : 0.0;
 }
 
 // A plain copy of member 0's entry into the entries marked reused (structures of 8-byte words).
@@ -1464,7 +1483,7 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
                        const int *offset, const int *count, const void *bucket, const ZigDev *zig,
                        const float *cd2if, const double *cd2i, float *model, long long mstride, double *model64,
                        int *err, int lean, const int *klist, int nk, int delta, long long *base64, int *tsrc,
-                       Replay rp) {
+                       Replay rp, int split) {
     int maxt = 0;
     for (int k = 0; k < nb; k++) maxt = max(maxt, mem_host[k].ntx * mem_host[k].nty);
     if (maxt == 0 || nb == 0 || (klist && nk == 0)) return;
@@ -1487,6 +1506,10 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
             // pixel-owned deposit: 8 (TP 64) or 4 (TP 32) pixels per warp
             const size_t smem_px = px_smem(g, TP);
             unsigned long long *b64 = (unsigned long long *)base64;
+            if (split > 1 && base64 && !delta && !klist && nb == 1) {
+                cudaMemsetAsync(base64, 0, sizeof(long long) * (size_t)mem_host[0].bx * mem_host[0].by * g.nz, s);
+                grid.z = split;
+            }
             if (TP == 64)
                 k_mc_deposit_px<32><<<grid, 256, smem_px, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count,
                                                                (const Entry *)bucket, zig, cd2if, model, mstride,
@@ -1503,6 +1526,13 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
     }
     k_mc_deposit<<<grid, 256, smem, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count, (const Entry *)bucket, zig, cd2if,
                                         cd2i, model, mstride, model64, err);
+}
+
+int mc_deposit_split(int ntile) { return max(1, min(16, 304 / max(ntile, 1))); }
+
+void launch_mc_sums64(cudaStream_t s, const long long *sums, long long n, int nz, const double *cd2i,
+                      const float *cd2if, int e, double *out, float *model) {
+    if (n) k_mc_sums64<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(sums, n, nz, cd2i, cd2if, e, out, model);
 }
 
 void launch_fill_submc(cudaStream_t s, SubMC *sub, int nsub, int nb, const signed char *reused, const MemberDev *mem,

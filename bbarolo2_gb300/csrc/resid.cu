@@ -75,6 +75,11 @@ __global__ void k_sumsq64(const double *__restrict__ model, const float *__restr
 }
 
 // (nz, ny, nx) float64 -> (ny, nx, nz) float32 and back
+__global__ void k_f64_to_f32(const double *__restrict__ in, long long n, float *__restrict__ out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = (float)in[i];
+}
+
 __global__ void k_zyx64_to_yxz32(const double *__restrict__ in, float *__restrict__ out, int nz, int ny, int nx) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long n = (long long)nz * ny * nx;
@@ -110,6 +115,10 @@ int launch_sumsq64(cudaStream_t s, const double *model, const float *data, const
     if (nbk < 1) nbk = 1;
     k_sumsq64<<<nbk, 256, 0, s>>>(model, data, mask, maskmode, region, nz, ny, nx, sigma2, eps2, partial);
     return nbk;
+}
+
+void launch_f64_to_f32(cudaStream_t s, const double *in, long long n, float *out) {
+    if (n) k_f64_to_f32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(in, n, out);
 }
 
 void launch_zyx64_to_yxz32(cudaStream_t s, const double *in, float *out, int nz, int ny, int nx) {

@@ -150,6 +150,10 @@ class DiskModel:
             blo, bhi = (0, 0), (self.cin.DimX(), self.cin.DimY())
         if final:
             rings = model_rings(rings, self.ringmode if ringmode is None else ringmode, self.setup.radsep)
+            if self.cfield is not None:
+                cube = self._cube(rings, blo, bhi, seed, galmodtype)
+                if cube is not None:
+                    return cube if layout == "zyx" else np.ascontiguousarray(cube.transpose(1, 2, 0))
         mod = self.build(rings, blo, bhi, seed=seed, galmodtype=galmodtype, layout="yxz")
         if self.cfield is not None:
             if final:
@@ -162,6 +166,25 @@ class DiskModel:
         if layout == "zyx":
             return np.ascontiguousarray(mod.transpose(2, 0, 1))
         return mod
+
+    def _cube(self, rings, blo, bhi, seed, galmodtype):
+        """The convolved model (nz, by, bx) of rings (used as nodes), built and convolved in one device call; None
+        for an empty model or box."""
+        st = self.setup
+        gtype = (galmodtype or st.galmodtype).upper()
+        sr, nv = st.subrings(rings)
+        if not sr.shape[1] or bhi[0] <= blo[0] or bhi[1] <= blo[1]:
+            return None
+        out = np.empty((st.nsubs, bhi[1] - blo[1], bhi[0] - blo[0]))
+        sr, nv = np.ascontiguousarray(sr, np.float64), np.ascontiguousarray(nv, np.int64)
+        an = gtype == "ANALYTIC"
+        nzq = 1 if not np.any(sr[6] > 0) else ZSAMPLES_MAX
+        s = 0 if an else seed32(st.iseed if seed is None else seed)
+        self.ctx.check(self.ctx.L.bbgpu_model_cube(self.ctx.h, _lib.ANALYTIC if an else _lib.MC, _lib.ptr(out),
+                                                   _lib.ptr(sr), sr.shape[1], int(s) & 0xFFFFFFFFFFFFFFFF, _lib.ptr(nv),
+                                                   nzq, int(blo[0]), int(blo[1]), int(bhi[0]), int(bhi[1]),
+                                                   float(self.scalefactor)))
+        return out
 
     def convolve(self, mod, layout="zyx", workers=1):
         """A dense model (ny, nx, nz) convolved with the beam, values below 1e-12 set to zero, times the scale

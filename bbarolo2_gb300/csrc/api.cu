@@ -334,6 +334,7 @@ static int upload_layout(bbgpu_ctx *ctx, LayoutEntry &E) {
     D.ncloud = H.ncloud;
     D.nsub = H.nsub;
     D.nsubcloud = H.nsubcloud;
+    for (int ir = 0; ir < H.nsub; ir++) D.maxnv = std::max(D.maxnv, (int)H.nv[ir]);
     D.nslow = H.nslow;
     size_t nc = (size_t)(H.ncloud ? H.ncloud : 1);
     std::vector<float4> cf(nc);

@@ -26,6 +26,7 @@ struct LayoutDev {
     double *slow_val;    // slow normal values
     long long *sub_base; // per sub-ring: first sub-cloud
     int *nvs;            // per sub-ring: velocity samples per cloud
+    int maxnv;           // the largest of nvs
     int *cloud_base;     // per sub-ring: first cloud
 };
 

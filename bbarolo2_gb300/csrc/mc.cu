@@ -768,6 +768,26 @@ __device__ __forceinline__ void px_entry(const Entry *__restrict__ bucket, int b
     }
 }
 
+// two float32 operations an instruction, each half rounded as the scalar one
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // this lane's (up to) SPL sorted samples of the cloud, 16-byte loads (the runs are padded to 4 samples with NaN;
 // the samples past the cloud are NaN as well)
 template <int SPL>
@@ -847,13 +867,12 @@ __device__ __forceinline__ void px_flush(const GridDev &g, const LayoutDev &L, c
 // a centre out of range counts its samples one by one, with the exact channels where needed.
 // The lowest non-empty bin (the lane's first run, which the previous lane may share) is added after the group's
 // lanes have merged equal ones; the other bins at once.
-template <int SPL>
+template <int LPP, int SPL>
 __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, const ZigDev *zig,
                                          const SubMC *__restrict__ subk, const SubMC *__restrict__ sub0,
                                          const PxCloud &p, const float4 (&w)[SPL / 4],
                                          int i0, int q, unsigned long long *tile, int rowoff, PxDefer *qe, int *qn,
                                          const unsigned long long *inc, int *err) {
-    constexpr int LPP = 128 / SPL;
     const int nz = g.nz;
     unsigned long long *row = tile + rowoff;
     const int m = min(SPL, p.nv - i0);                      // this lane's samples (<= 0: none)
@@ -861,11 +880,13 @@ __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, c
     const float hw = 0.5f - p.eps;
     const float tc = p.tc, sg = p.sg;
     const long long fix = p.fix;
-    // f = sample x sg + (tc + 1/2): the half folded into the centre (one rounding in place of another, within the
-    // same bound); samples past the cloud are NaN, which fail the test below and add the empty increment
-    const float tc5 = tc + 0.5f;
-    const float fl0 = floorf(fmaf(w[0].x, sg, tc5)) - 1.0f;
-    const float fl0m = fl0 - 12582912.0f;                  // (exact: an integer below 2^24 in magnitude)
+    // v = sample x sg + tc, its nearest integer r by adding and subtracting 1.5 2^23 (a tie fails the test below, as
+    // does a sample past the cloud: NaN), two samples an instruction. |v| < 2^22 wherever a sample can pass: the
+    // cloud's bound eps holds |v| EPS_REL, and passing takes eps < 1/2
+    const unsigned long long sg2 = pack2(sg, sg), tc2 = pack2(tc, tc);
+    const unsigned long long magic2 = pack2(12582912.0f, 12582912.0f), nmagic2 = pack2(-12582912.0f, -12582912.0f);
+    const unsigned long long neg2 = pack2(-1.0f, -1.0f);
+    const int base = __float_as_int(__fadd_rn(fmaf(w[0].x, sg, tc), 12582912.0f)) - 1;
     const float hwf = fastc ? hw : -1.0f;                  // (a centre out of range: no sample passes)
     // straight-line code: each sample adds inc[min(channel - c0, 30)] (bins 0..10 five bits each, a channel
     // beyond them one unit of bits 55..63; index 31: a sample left out)
@@ -873,16 +894,19 @@ __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, c
     unsigned need = 0;
     int dlast = 0;
 #pragma unroll
-    for (int s = 0; s < SPL / 4; s++) {
-        const float vv[4] = {w[s].x, w[s].y, w[s].z, w[s].w};
+    for (int s = 0; s < SPL / 2; s++) {
+        const float4 &q4 = w[s >> 1];
+        const unsigned long long v2 = fma2((s & 1) ? pack2(q4.z, q4.w) : pack2(q4.x, q4.y), sg2, tc2);
+        const unsigned long long t2 = add2(v2, magic2);
+        const unsigned long long e2 = fma2(add2(t2, nmagic2), neg2, v2);
+        float t[2], d2[2];
+        unpack2(t2, t[0], t[1]);
+        unpack2(e2, d2[0], d2[1]);
 #pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int i = 4 * s + e;
-            const float f = fmaf(vv[e], sg, tc5);
-            const float fl = floorf(f);
-            const bool ok = fabsf(f - fl - 0.5f) <= hwf;
-            const int d = __float_as_int(fl - fl0m) - 0x4B400000;      // (exact: small integers)
-            need |= ok ? 0u : 1u << i;
+        for (int e = 0; e < 2; e++) {
+            const bool ok = fabsf(d2[e]) <= hwf;
+            const int d = __float_as_int(t[e]) - base;
+            need |= ok ? 0u : 1u << (2 * s + e);
             H += inc[ok ? min((unsigned)d, 30u) : 31u];
             if (SPL == 32) dlast = ok ? d : dlast;
         }
@@ -895,19 +919,24 @@ __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, c
             qe[slot] = PxDefer{p.c, p.pb, p.nv, i0 + __ffs(need) - 1, fix, rowoff, p.src0};
         }
         if (H) {
-            const int c0 = (int)fl0;
+            const int c0 = base - 0x4B400000;
             const int ntake = m - (need ? 1 : 0);
             const int blo = (__ffsll((long long)H) - 1) / 5;
             // all 32 samples in one channel: 32 overflows its five bits into a single carry bit of H
             const bool one = SPL == 32 && ntake == 32 && H == 1ull << (5 * dlast + 5);
             fch = c0 + (one ? dlast : blo);
             fcnt = one ? 32 : (int)((H >> (5 * blo)) & 31);
-#pragma unroll
-            for (int b = 0; b < 11; b++) {
+            auto put = [&](int b) {
                 const int cnt = (int)((H >> (5 * b)) & 31);
                 const int ch = c0 + b;
-                const bool put = !one & (cnt != 0) & (b != blo) & ((unsigned)ch < (unsigned)nz);
-                if (put) row[ch] += (unsigned long long)(fix * (long long)cnt);
+                const bool yes = !one & (cnt != 0) & (b != blo) & ((unsigned)ch < (unsigned)nz);
+                if (yes) row[ch] += (unsigned long long)(fix * (long long)cnt);
+            };
+#pragma unroll
+            for (int b = 0; b < 6; b++) put(b);
+            if (H >> 30) {
+#pragma unroll
+                for (int b = 6; b < 11; b++) put(b);
             }
         }
     } else {
@@ -950,10 +979,14 @@ __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, c
 // by groups of LPP = 128 / SPL lanes: warp w owns the pixels lp = w + 8 grp of the tile (TP = 8 x 32 / LPP
 // pixels), and a group takes the clouds of its pixel one after another, so a warp advances 32 / LPP clouds at a
 // time. Lane q of a group counts the samples SPL q .. SPL q + SPL - 1 of the cloud in their sorted order (float32
-// channels within the rounding bound of the cloud); the samples of the next cloud are loaded during the count.
+// channels within the rounding bound of the cloud). SPL is the smallest of a few multiples of 4 that holds the
+// layout's clouds in LPP lanes: the count is straight-line code over SPL samples, empty ones included.
 // The channels are monotone along the sorted samples, so the lanes of a group can only meet on the channel of a
 // run that crosses from one lane's samples into the next lane's: every lane's channels but its lowest are added
 // at once (distinct channels), and the lowest ones after a segmented scan over the group's lanes.
+// The instructions a sample bound it: with the nearest integer by two additions (two samples an instruction) for a
+// floor, and the samples loaded when they are counted (loading them a cloud ahead spilled registers at three CTAs per
+// SM): 61 models of 101x97x75 1.32 -> 0.73 ms, base point and 160 steps of 160x160x128 2.61 -> 2.08 ms.
 // A sample within the bound of a half-integer (about one in a thousand) waits in the warp's queue; when the
 // queue fills, its exact float64 channels are computed a lane each and added with shared-memory atomics.
 // Rows: stride nz + 2 G sums (G pixels per warp) and a skew of 2 grp sums, so that equal channels of the warp's
@@ -1074,7 +1107,7 @@ __global__ void __launch_bounds__(256) k_replay_records(GridDev g, LayoutDev L, 
     if (lane == 0) nrec[l] = nr;
 }
 
-template <int SPL>
+template <int LPP, int SPL>
 __global__ void __launch_bounds__(256, PX_MINB) k_mc_deposit_px(GridDev g, LayoutDev L, const SubMC *__restrict__ sub,
                                                               int nsub, const MemberDev *__restrict__ mem, int tx,
                                                               int ty, const int *__restrict__ offset,
@@ -1086,7 +1119,6 @@ __global__ void __launch_bounds__(256, PX_MINB) k_mc_deposit_px(GridDev g, Layou
                                                               const int *__restrict__ klist, int delta,
                                                               unsigned long long *__restrict__ base64,
                                                               int *__restrict__ tsrc, Replay rp, int *err) {
-    constexpr int LPP = 128 / SPL;
     extern __shared__ unsigned long long tile[];           // TP rows of fixed-point sums, queues, nz scales
     __shared__ unsigned long long inc[32];                 // the histogram increments of px_count
     const int k = klist ? klist[blockIdx.x] : blockIdx.x;
@@ -1216,21 +1248,15 @@ __global__ void __launch_bounds__(256, PX_MINB) k_mc_deposit_px(GridDev g, Layou
     const int i0 = SPL * q;                                 // this lane's samples: i0 .. min(i0 + SPL, nv) - 1
     // software pipeline: the samples of the next cloud and the entry after it are loaded during a count
     PxCloud ca, cb;
-    float4 wa[SPL / 4], wb[SPL / 4];
     px_entry(bucket, beg, n, 0, ca);
-    px_samples<SPL>(L, ca, i0, wa);
-    px_entry(bucket, beg, n, 1, cb);
     for (int j = 0; j < nj; j++) {
-        px_samples<SPL>(L, cb, i0, wb);
-        PxCloud cn;
-        px_entry(bucket, beg, n, j + 2, cn);
-        px_count<SPL>(g, L, zig, subk, sub, ca, wa, i0, q, tile, rowoff, qe, qn, inc, err);
+        float4 wa[SPL / 4];
+        px_samples<SPL>(L, ca, i0, wa);
+        px_entry(bucket, beg, n, j + 1, cb);
+        px_count<LPP, SPL>(g, L, zig, subk, sub, ca, wa, i0, q, tile, rowoff, qe, qn, inc, err);
         __syncwarp();
         if (*qn > PX_QCAP - 32) px_flush(g, L, zig, subk, sub, qe, qn, tile, lane, err);
         ca = cb;
-        cb = cn;
-#pragma unroll
-        for (int s = 0; s < SPL / 4; s++) wa[s] = wb[s];
     }
     __syncwarp();
     if (*qn) px_flush(g, L, zig, subk, sub, qe, qn, tile, lane, err);
@@ -1462,20 +1488,10 @@ bool mc_deposit_shares(int lean, bool model64, int tx, int ty) {
     return lean && !model64 && (tx * ty == 64 || tx * ty == 32);
 }
 
-// dynamic shared memory of the pixel-owned deposit (TP pixels a tile), the kernel configured for it once
+// dynamic shared memory of the pixel-owned deposit (TP pixels a tile)
 static size_t px_smem(const GridDev &g, int TP) {
-    const size_t smem_px = (size_t)TP * (g.nz + TP / 4) * sizeof(unsigned long long) +
-                           (size_t)8 * PX_QCAP * sizeof(PxDefer) + 8 * sizeof(int) + (size_t)g.nz * sizeof(float);
-    static size_t cfg32 = 0, cfg16 = 0;
-    size_t &cfg = TP == 64 ? cfg32 : cfg16;
-    if (smem_px > 48 * 1024 && smem_px > cfg) {
-        if (TP == 64)
-            cudaFuncSetAttribute(k_mc_deposit_px<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_px);
-        else
-            cudaFuncSetAttribute(k_mc_deposit_px<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_px);
-        cfg = smem_px;
-    }
-    return smem_px;
+    return (size_t)TP * (g.nz + TP / 4) * sizeof(unsigned long long) + (size_t)8 * PX_QCAP * sizeof(PxDefer) +
+           8 * sizeof(int) + (size_t)g.nz * sizeof(float);
 }
 
 void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, const SubMC *sub, int nsub,
@@ -1510,14 +1526,28 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
                 cudaMemsetAsync(base64, 0, sizeof(long long) * (size_t)mem_host[0].bx * mem_host[0].by * g.nz, s);
                 grid.z = split;
             }
-            if (TP == 64)
-                k_mc_deposit_px<32><<<grid, 256, smem_px, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count,
-                                                               (const Entry *)bucket, zig, cd2if, model, mstride,
-                                                               klist, delta, b64, tsrc, rp, err);
-            else
-                k_mc_deposit_px<16><<<grid, 256, smem_px, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count,
-                                                               (const Entry *)bucket, zig, cd2if, model, mstride,
-                                                               klist, delta, b64, tsrc, rp, err);
+            // samples a lane: the fewest that hold the layout's clouds (61 models of 101x97x75, 75 samples a cloud:
+            // 0.73 ms with 20, 1.05 ms with 32)
+#define PX(LPP, SPL)                                                                                                  \
+    {                                                                                                                 \
+        static size_t cfg = 0;                                                                                        \
+        if (smem_px > 48 * 1024 && smem_px > cfg) {                                                                   \
+            cudaFuncSetAttribute(k_mc_deposit_px<LPP, SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_px);\
+            cfg = smem_px;                                                                                            \
+        }                                                                                                             \
+        k_mc_deposit_px<LPP, SPL><<<grid, 256, smem_px, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count,             \
+                                                             (const Entry *)bucket, zig, cd2if, model, mstride,       \
+                                                             klist, delta, b64, tsrc, rp, err);                       \
+    }
+            if (TP == 64) {
+                if (L.maxnv <= 64) PX(4, 16)
+                else if (L.maxnv <= 80) PX(4, 20)
+                else if (L.maxnv <= 96) PX(4, 24)
+                else PX(4, 32)
+            } else {
+                PX(8, 16)
+            }
+#undef PX
             return;
         }
         k_mc_deposit_lean<<<grid, 256, smem, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count, (const Entry *)bucket,

@@ -18,6 +18,7 @@
 
 #include "anpix.cuh"
 #include "devmath.cuh"
+#include "f32x2.cuh"
 #include "kernels.h"
 
 #define PHI_N 6146
@@ -483,6 +484,105 @@ __device__ __forceinline__ unsigned long long f32_to_fix(float x) {
     return (unsigned long long)((long long)hi * 8388608 + lo);
 }
 
+// The set-up of sample s (constants S = subs[sub], radius kr) by its lane; false if its line has no channel in the band.
+__device__ __forceinline__ bool anf_setup(const GridDev &g, const AnSub &S, int sub, int s, int kr, float2 cf,
+                                          const float4 *__restrict__ csff, const double2 *__restrict__ cs,
+                                          const float *__restrict__ zqf, AnfSample &o) {
+    ff v;
+    const long long kc = fast_line_centre(S, g, csff[s], cs + s, v);
+    long long a0 = kc - S.K, a1 = kc + S.K + 1;
+    if (a0 < 0) a0 = 0;
+    if (a1 > g.nz) a1 = g.nz;
+    if (a1 <= a0) return false;
+    const PixF px = pix_setup(S, kr, cf, zqf + S.zq_off, S.nzz);
+    const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
+    o.vrh = vr.hi;
+    o.vrl = vr.lo;
+    o.invf = S.invf;
+    o.bxf = px.bxf;
+    o.byf = px.byf;
+    o.zP3 = px.zP3;
+    o.zQ3 = px.zQ3;
+    o.hwx = px.fast ? px.hwx : -1.0f;
+    o.hwy = px.hwy;
+    o.k0 = (unsigned short)a0;
+    o.nk = (unsigned short)(a1 - a0);
+    o.off = S.zq_off;
+    o.nzz = S.nzz;
+    o.sub = sub;
+    o.s = s | (kr << 31);
+    return true;
+}
+
+// The runs of a sample's heights in the box (bw, bh from blo0, blo1), 32 heights a pass, collected in the warp's list
+// run (pixel, weight); flush(n) takes the n of a full list and the last ones.
+template <class F>
+__device__ __forceinline__ void anf_runs(const GridDev &g, const AnfSample &o, const AnSub &S,
+                                         const double2 *__restrict__ cs, const double *__restrict__ zq,
+                                         const float *__restrict__ zqf, const float *__restrict__ wqf, int blo0,
+                                         int blo1, int bw, int bh, int lane, int2 *run, F flush) {
+    const PixF px{o.bxf, o.byf, o.zP3, o.zQ3, o.hwx, o.hwy, o.hwx > 0.0f};
+    const int nzz = o.nzz, off = o.off;
+    const double2 *cp = cs + (o.s & 0x7fffffff);
+    const int kr = (unsigned)o.s >> 31;
+    bool open = false;                                  // a run carried from the previous pass
+    int cg0 = 0, cg1 = 0, nr = 0;
+    float cws = 0.0f;
+    for (int base = 0; base < nzz; base += 32) {
+        const int cnt = min(32, nzz - base);
+        const bool valid = lane < cnt;
+        int g0 = 0x7fffffff, g1 = 0x7fffffff;
+        float wv = 0.0f;
+        if (valid) {
+            sample_pixel(S, px, kr, cp, nzz, nzz > 1 ? __ldg(zqf + off + base + lane) : 0.f,
+                         zq + off + base + lane, g.cdelt0, g.cdelt1, g0, g1);
+            wv = __ldg(wqf + off + base + lane);
+        }
+        const int pg0 = __shfl_up_sync(FULL, g0, 1), pg1 = __shfl_up_sync(FULL, g1, 1);
+        const bool start = valid && (lane == 0 ? (!open || g0 != cg0 || g1 != cg1) : (g0 != pg0 || g1 != pg1));
+        const unsigned smask = __ballot_sync(FULL, start);
+        if (open && (smask & 1u)) {                     // the carried run ended with the previous pass
+            const int rx = cg0 - blo0, ry = cg1 - blo1;
+            if ((unsigned)rx < (unsigned)bw && (unsigned)ry < (unsigned)bh) {
+                if (lane == 0) run[nr] = make_int2(ry * bw + rx, __float_as_int(cws));
+                nr++;
+            }
+            open = false;
+        }
+        // segmented inclusive scan of the weights (a segment: from a run start to the lane before the next)
+        const unsigned upto = smask & (0xffffffffu >> (31 - lane));
+        const int head = upto ? 31 - __clz(upto) : 0;
+        float v = wv;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const float t = __shfl_up_sync(FULL, v, d);
+            if (lane - d >= head) v += t;
+        }
+        if (!upto && open) v += cws;                    // (the lanes that continue the carried run)
+        const bool nstart = lane < 31 && ((smask >> (lane + 1)) & 1u);
+        const bool last = lane == cnt - 1;
+        const bool final_pass = base + 32 >= nzz;
+        const bool done = valid && ((!last && nstart) || (last && final_pass));
+        const int rx = g0 - blo0, ry = g1 - blo1;
+        const bool put = done && (unsigned)rx < (unsigned)bw && (unsigned)ry < (unsigned)bh;
+        const unsigned pmask = __ballot_sync(FULL, put);
+        if (put) run[nr + __popc(pmask & ((1u << lane) - 1u))] = make_int2(ry * bw + rx, __float_as_int(v));
+        nr += __popc(pmask);
+        if (final_pass || nr > ANF_RUNS - 33) {
+            __syncwarp();
+            flush(nr);
+            __syncwarp();
+            nr = 0;
+        }
+        if (!final_pass) {
+            cg0 = __shfl_sync(FULL, g0, cnt - 1);
+            cg1 = __shfl_sync(FULL, g1, cnt - 1);
+            cws = __shfl_sync(FULL, v, cnt - 1);
+            open = true;
+        }
+    }
+}
+
 // The samples are set up 32 at a time, a lane each (constants, pixel coefficients, line); then the warp takes them one
 // after another: the profile over the lanes into shared memory; the heights, 32 a pass, into the list of the sample's
 // runs in the box; and the (run, channel) pairs laid end to end over the lanes, one 64-bit reduction each. At 27
@@ -524,34 +624,10 @@ __global__ void __launch_bounds__(ANF_WPB * 32, 4) k_an_model_fast(GridDev g, co
         const float2 cf = csf[s];
         const bool rec = cf.x >= 0.0f;                      // (the sign of the float32 table is the float64 test's)
         if (S.active && S.anfast && !(S.wzero & (rec ? 1 : 2))) {
-            const int kr = s - sbase[ir] >= S.naz ? 1 : 0;
-            ff v;
-            const long long kc = fast_line_centre(S, g, csff[s], cs + s, v);
-            long long a0 = kc - S.K, a1 = kc + S.K + 1;
-            if (a0 < 0) a0 = 0;
-            if (a1 > nz) a1 = nz;
-            if (a1 > a0) {
-                ok = true;
-                AnfSample &o = sm[lane];
-                const PixF px = pix_setup(S, kr, cf, zqf + S.zq_off, S.nzz);
-                const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
-                o.vrh = vr.hi;
-                o.vrl = vr.lo;
-                o.invf = S.invf;
-                o.amp = (float)sg.sign * ldexpf(S.af * (rec ? S.wrecf : S.wappf), mem[sg.k].fix_exp);
-                o.bxf = px.bxf;
-                o.byf = px.byf;
-                o.zP3 = px.zP3;
-                o.zQ3 = px.zQ3;
-                o.hwx = px.fast ? px.hwx : -1.0f;
-                o.hwy = px.hwy;
-                o.k0 = (unsigned short)a0;
-                o.nk = (unsigned short)(a1 - a0);
-                o.off = S.zq_off;
-                o.nzz = S.nzz;
-                o.sub = sg.src * nsub + ir;
-                o.s = s | (kr << 31);
-                o.k = sg.k;
+            ok = anf_setup(g, S, sg.src * nsub + ir, s, s - sbase[ir] >= S.naz ? 1 : 0, cf, csff, cs, zqf, sm[lane]);
+            if (ok) {
+                sm[lane].amp = (float)sg.sign * ldexpf(S.af * (rec ? S.wrecf : S.wappf), mem[sg.k].fix_exp);
+                sm[lane].k = sg.k;
             }
         }
     }
@@ -559,11 +635,8 @@ __global__ void __launch_bounds__(ANF_WPB * 32, 4) k_an_model_fast(GridDev g, co
     __syncwarp();
     for (; todo; todo &= todo - 1) {
         const AnfSample &o = sm[__ffs(todo) - 1];
-        const int nk = o.nk, k0 = o.k0, nzz = o.nzz, off = o.off;
-        const PixF px{o.bxf, o.byf, o.zP3, o.zQ3, o.hwx, o.hwy, o.hwx > 0.0f};
+        const int nk = o.nk, k0 = o.k0;
         const AnSub &S = subs[o.sub];
-        const double2 *cp = cs + (o.s & 0x7fffffff);
-        const int kr = (unsigned)o.s >> 31;
         const MemberDev &M = mem[o.k];
         const int blo0 = M.blo0, blo1 = M.blo1, bw = M.bx, bh = M.by;
         unsigned long long *const o64 = out64 + (size_t)o.k * mstride + k0;
@@ -619,60 +692,253 @@ __global__ void __launch_bounds__(ANF_WPB * 32, 4) k_an_model_fast(GridDev g, co
                 }
             }
         };
-        bool open = false;                                  // a run carried from the previous pass
-        int cg0 = 0, cg1 = 0, nr = 0;
-        float cws = 0.0f;
-        for (int base = 0; base < nzz; base += 32) {
-            const int cnt = min(32, nzz - base);
-            const bool valid = lane < cnt;
-            int g0 = 0x7fffffff, g1 = 0x7fffffff;
-            float wv = 0.0f;
-            if (valid) {
-                sample_pixel(S, px, kr, cp, nzz, nzz > 1 ? __ldg(zqf + off + base + lane) : 0.f,
-                             zq + off + base + lane, g.cdelt0, g.cdelt1, g0, g1);
-                wv = __ldg(wqf + off + base + lane);
-            }
-            const int pg0 = __shfl_up_sync(FULL, g0, 1), pg1 = __shfl_up_sync(FULL, g1, 1);
-            const bool start = valid && (lane == 0 ? (!open || g0 != cg0 || g1 != cg1) : (g0 != pg0 || g1 != pg1));
-            const unsigned smask = __ballot_sync(FULL, start);
-            if (open && (smask & 1u)) {                     // the carried run ended with the previous pass
-                const int rx = cg0 - blo0, ry = cg1 - blo1;
-                if ((unsigned)rx < (unsigned)bw && (unsigned)ry < (unsigned)bh) {
-                    if (lane == 0) run[nr] = make_int2(ry * bw + rx, __float_as_int(cws));
-                    nr++;
+        anf_runs(g, o, S, cs, zq, zqf, wqf, blo0, blo1, bw, bh, lane, run, deposit);
+    }
+}
+
+// ------------------------------------------------------------------ members that are member 0 but for the fluxes
+// A member whose sub-rings are member 0's but for the density (a step of a geometry parameter of one ring, whose flux
+// normalisation moves every ring's) has member 0's runs and profiles: only the amplitudes differ. Member 0's runs are
+// listed by pixel and block of 32 channels beside the profiles of their samples (k_an_records: counted, then placed),
+// and a warp takes a list and 16 members: it reads each run and its profile once and adds the 16 members' deposits in
+// registers. The deposits are k_an_model_fast's, integer for integer, without its reductions in L2 (15 SM cycles a
+// warp of deposits against 3); the model is written in float32. The sub-rings that differ are deposited by
+// k_an_model_fast beforehand and added here. Bound by the float32 pipe (five packed operations for two deposits) and
+// the issue slots: 80 members of 160x160x128 4.8 ms, against 12.2 ms by their samples; with 64-bit sums 6.9 ms, with
+// six operations and single runs 6.6 ms.
+struct __align__(16) AnRun {
+    int s;                // the sample, whose profile is prof[s kw ..]
+    float w;              // the weight of the run
+    unsigned kn;          // first channel | channels << 16
+    unsigned hb;          // 2 sub-ring + (receding 0, approaching 1) | upper half: a bound of profile x weight (a
+                          // bfloat16, rounded up)
+};
+#define ANR_MG 16                     // members of a warp
+#define ANR_D 8                       // profiles on their way
+
+template <bool PLACE>
+__global__ void __launch_bounds__(ANF_WPB * 32) k_an_records(GridDev g, const AnSub *__restrict__ subs,
+                                                             const int *__restrict__ sbase,
+                                                             const int *__restrict__ ssub,
+                                                             const double2 *__restrict__ cs,
+                                                             const float2 *__restrict__ csf,
+                                                             const float4 *__restrict__ csff, long long ns,
+                                                             const unsigned long long *__restrict__ act,
+                                                             const double *__restrict__ zq,
+                                                             const float *__restrict__ zqf,
+                                                             const float *__restrict__ wqf,
+                                                             const float2 *__restrict__ vef,
+                                                             const float *__restrict__ cd2if,
+                                                             const float *__restrict__ ptabf,
+                                                             const MemberDev *__restrict__ mem, int *__restrict__ count,
+                                                             AnRun *__restrict__ runs, float *__restrict__ prof,
+                                                             int kw) {
+    __shared__ AnfSample sm_[ANF_WPB][32];
+    __shared__ int2 run_[ANF_WPB][ANF_RUNS];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    AnfSample *const sm = sm_[w];
+    int2 *const run = run_[w];
+    const long long s0 = ((long long)blockIdx.x * ANF_WPB + w) * 32 + lane;
+    bool ok = false;
+    if (s0 < ns) {
+        const int s = (int)s0, ir = ssub[s];
+        const AnSub &S = subs[ir];
+        const float2 cf = csf[s];
+        const int half = cf.x >= 0.0f ? 0 : 1;
+        if (((act[ir >> 6] >> (ir & 63)) & 1ull) && !(S.wzero & (1 << half))) {
+            ok = anf_setup(g, S, ir, s, s - sbase[ir] >= S.naz ? 1 : 0, cf, csff, cs, zqf, sm[lane]);
+            sm[lane].k = 2 * ir + half;
+        }
+    }
+    const MemberDev &M = mem[0];
+    const int blo0 = M.blo0, blo1 = M.blo1, bw = M.bx, bh = M.by, nzb = (g.nz + 31) / 32;
+    unsigned todo = __ballot_sync(FULL, ok);
+    __syncwarp();
+    for (; todo; todo &= todo - 1) {
+        const AnfSample &o = sm[__ffs(todo) - 1];
+        const int nk = o.nk, k0 = o.k0, s = o.s & 0x7fffffff;
+        float top = 0.0f;
+        if (PLACE) {
+            for (int j = lane; j - lane < nk; j += 31) {    // (the profile as k_an_model_fast's, before the amplitude)
+                const float2 e = __ldg(vef + k0 + min(j, nk));
+                const float ph = phi_f32((__fsub_rn(e.x, o.vrh) + __fsub_rn(e.y, o.vrl)) * o.invf, ptabf);
+                const float pn = __shfl_down_sync(FULL, ph, 1);
+                if (lane < 31 && j < nk) {
+                    const float p = fabsf(pn - ph) * __ldg(cd2if + k0 + j);
+                    prof[(size_t)s * kw + j] = p;
+                    top = fmaxf(top, fabsf(p));
                 }
-                open = false;
             }
-            // segmented inclusive scan of the weights (a segment: from a run start to the lane before the next)
-            const unsigned upto = smask & (0xffffffffu >> (31 - lane));
-            const int head = upto ? 31 - __clz(upto) : 0;
-            float v = wv;
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const float t = __shfl_up_sync(FULL, v, d);
-                if (lane - d >= head) v += t;
+            for (int d = 16; d > 0; d >>= 1) top = fmaxf(top, __shfl_xor_sync(FULL, top, d));
+        }
+        anf_runs(g, o, subs[o.sub], cs, zq, zqf, wqf, blo0, blo1, bw, bh, lane, run, [&](int n) {
+            for (int r = lane; r < n; r += 32) {
+                const int2 q = run[r];
+                const float w = __int_as_float(q.y);
+                const unsigned b = (__float_as_uint(top * fabsf(w)) & 0xffff0000u) + 0x10000u;
+                for (int zb = k0 >> 5; zb <= (k0 + nk - 1) >> 5; zb++) {
+                    const int at = atomicAdd(count + q.x * nzb + zb, 1);
+                    if (PLACE) runs[at] = AnRun{s, w, (unsigned)k0 | ((unsigned)nk << 16), (unsigned)o.k | b};
+                }
             }
-            if (!upto && open) v += cws;                    // (the lanes that continue the carried run)
-            const bool nstart = lane < 31 && ((smask >> (lane + 1)) & 1u);
-            const bool last = lane == cnt - 1;
-            const bool final_pass = base + 32 >= nzz;
-            const bool done = valid && ((!last && nstart) || (last && final_pass));
-            const int rx = g0 - blo0, ry = g1 - blo1;
-            const bool put = done && (unsigned)rx < (unsigned)bw && (unsigned)ry < (unsigned)bh;
-            const unsigned pmask = __ballot_sync(FULL, put);
-            if (put) run[nr + __popc(pmask & ((1u << lane) - 1u))] = make_int2(ry * bw + rx, __float_as_int(v));
-            nr += __popc(pmask);
-            if (final_pass || nr > ANF_RUNS - 33) {
-                __syncwarp();
-                deposit(nr);
-                __syncwarp();
-                nr = 0;
+        });
+    }
+}
+
+// The members' amplitudes of (sub-ring, side): amp[2 sub-ring + side][member of klist] (padded to ANR_MG; 0 where the
+// member deposits the sub-ring itself, chg, or has none), and the largest of each group of ANR_MG.
+__global__ void k_an_amps(const AnSub *__restrict__ subs, int nsub, const MemberDev *__restrict__ mem,
+                          const int *__restrict__ klist, int n3, int ng, const unsigned long long *__restrict__ chg,
+                          int nchw, float *__restrict__ amp, float *__restrict__ top) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int np = ng * ANR_MG, ih = (int)(i / np), m = (int)(i - (long long)ih * np), ir = ih >> 1;
+    float a = 0.0f;
+    if (ir < nsub && m < n3) {
+        const int k = klist[m];
+        const AnSub &S = subs[(size_t)k * nsub + ir];
+        if (S.active && !((chg[(size_t)m * nchw + (ir >> 6)] >> (ir & 63)) & 1ull) && !(S.wzero & (1 << (ih & 1))))
+            a = ldexpf(S.af * ((ih & 1) ? S.wappf : S.wrecf), mem[k].fix_exp);
+    }
+    float t = fabsf(a);
+#pragma unroll
+    for (int d = ANR_MG / 2; d > 0; d >>= 1) t = fmaxf(t, __shfl_xor_sync(FULL, t, d));
+    if (ir >= nsub) return;
+    amp[i] = a;
+    if (m % ANR_MG == 0) top[(size_t)ih * ng + m / ANR_MG] = t;
+}
+
+// f32_to_fix of two values x (|x| < ANF_FIXMAX / 2, packed float32 operations): t holds the multiple of 2^23 below x in
+// its low mantissa bits, q the rest rounded to an integer of at most 2^23. Sums of both stay within 32 bits for ANR_FLUSH
+// runs, each addition with the bias of its constant.
+#define ANR_FLUSH 256
+#define ANR_TOP (ANF_HI + 8388608.0f)                       // (exact: 24 bits)
+__device__ __forceinline__ void fix_parts(unsigned long long x, unsigned long long &t, unsigned long long &q) {
+    t = f32x2_add_rm(x, f32x2(ANF_HI, ANF_HI));
+    q = f32x2_add(x, f32x2_fma(t, f32x2(-1.0f, -1.0f), f32x2(ANR_TOP, ANR_TOP)));
+}
+
+// A CTA keeps the amplitudes of one group of members in shared memory and its warps take (pixel, 32 channels) after
+// (pixel, 32 channels).
+__global__ void __launch_bounds__(256, 3) k_an_replay(int nz, int ng, int nzb, int npix, int ntask, int na,
+                                                      const int *__restrict__ offset, const int *__restrict__ count,
+                                                      const int4 *__restrict__ runs, const float *__restrict__ prof,
+                                                      int kw, const float *__restrict__ amp,
+                                                      const float *__restrict__ top, const int *__restrict__ klist,
+                                                      int n3, const MemberDev *__restrict__ mem,
+                                                      const unsigned long long *__restrict__ own, long long mstride,
+                                                      float *__restrict__ model) {
+    extern __shared__ __align__(16) float anr_amp[];        // na x ANR_MG amplitudes, na bounds
+    __shared__ unsigned long long sum_[8][ANR_MG][32];      // sums beyond 32 bits, where there are any
+    __shared__ float ring_[8][ANR_D][32];                   // the profiles of the next runs
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, grp = blockIdx.x % ng;
+    float *const atop = anr_amp + na * ANR_MG;
+    for (int i = threadIdx.x; i < na * ANR_MG; i += 256)
+        anr_amp[i] = __ldg(amp + ((size_t)(i / ANR_MG) * ng + grp) * ANR_MG + i % ANR_MG);
+    for (int i = threadIdx.x; i < na; i += 256) atop[i] = __ldg(top + (size_t)i * ng + grp);
+    __syncthreads();
+    unsigned long long (*const sum)[32] = sum_[warp];
+    float (*const ring)[32] = ring_[warp];
+    for (int task = (blockIdx.x / ng) * 8 + warp; task < ntask; task += (gridDim.x / ng) * 8) {
+        // (the tasks of a warp are spread over the image: the same load for all)
+        const int zb = task / npix, pix = task - zb * npix, c = zb * 32 + lane;
+        const int o0 = offset[pix * nzb + zb], m = count[pix * nzb + zb];
+        unsigned hi[ANR_MG], lo[ANR_MG];
+#pragma unroll
+        for (int i = 0; i < ANR_MG; i++) hi[i] = lo[i] = 0;
+        int n = 0;                                          // deposits in hi and lo
+        bool wide = false;                                  // sum is in use
+        auto part = [&](int i) {
+            return (unsigned long long)((long long)(int)(hi[i] - (unsigned)n * (unsigned)__float_as_int(ANF_HI)) *
+                                            8388608 +
+                                        (long long)(lo[i] - (unsigned)n * 0x4B000000u));
+        };
+        auto flush = [&]() {
+#pragma unroll
+            for (int i = 0; i < ANR_MG; i++) {
+                sum[i][lane] = part(i) + (wide ? sum[i][lane] : 0ULL);
+                hi[i] = lo[i] = 0;
             }
-            if (!final_pass) {
-                cg0 = __shfl_sync(FULL, g0, cnt - 1);
-                cg1 = __shfl_sync(FULL, g1, cnt - 1);
-                cws = __shfl_sync(FULL, v, cnt - 1);
-                open = true;
+            wide = true;
+            n = 0;
+        };
+        auto list = [&](int b0) { return lane < m - b0 ? __ldg(runs + o0 + b0 + lane) : make_int4(0, 0, 0, 0); };
+        auto below = [&](const int4 &r) {
+            return __ballot_sync(FULL, __int_as_float(r.w & 0xffff0000) * atop[r.w & 0xffff] < 0.5f * ANF_FIXMAX);
+        };
+        int4 q = list(0), qn = list(32);
+        unsigned small = below(q);
+        // the profiles of runs e and e + 1 in this lane's channel, on their way to the ring (0 outside a profile)
+        auto fetch = [&](int e, const int4 &r) {
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                const int l = (e + u) & 31;
+                const int s = __shfl_sync(FULL, r.x, l), kn = __shfl_sync(FULL, r.z, l), j = c - (kn & 0xffff);
+                const bool in = (unsigned)j < ((unsigned)kn >> 16);
+                const unsigned d = (unsigned)__cvta_generic_to_shared(&ring[(e + u) & (ANR_D - 1)][lane]);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d),
+                             "l"(prof + (in ? (size_t)s * kw + j : 0)), "r"(in ? 4 : 0)
+                             : "memory");
+            }
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+#pragma unroll
+        for (int e = 0; e < ANR_D - 2; e += 2) fetch(e, q);
+        // (two runs a step: their parts join a sum in one three-operand addition; an odd last one is paired with an
+        // empty run)
+        for (int e = 0; e < m; e += 2) {
+            const int l = e & 31, en = e + ANR_D - 2;
+            if (l == 0 && e) {
+                q = qn;
+                qn = list(e + 32);
+                small = below(q);
+            }
+            fetch(en, (en ^ e) & 32 ? qn : q);
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(ANR_D / 2 - 1) : "memory");
+            const float b = ring[e & (ANR_D - 1)][lane], bb = ring[(e + 1) & (ANR_D - 1)][lane];
+            const float w = __int_as_float(__shfl_sync(FULL, q.y, l));
+            const float ww = __int_as_float(__shfl_sync(FULL, q.y, l + 1));
+            const float4 *a4 = (const float4 *)(anr_amp + (__shfl_sync(FULL, q.w, l) & 0xffff) * ANR_MG);
+            const float4 *aa4 = (const float4 *)(anr_amp + (__shfl_sync(FULL, q.w, l + 1) & 0xffff) * ANR_MG);
+            if (((small >> l) & 3u) == 3u) {
+                const unsigned long long b2 = f32x2(b, b), w2 = f32x2(w, w);
+                const unsigned long long bb2 = f32x2(bb, bb), ww2 = f32x2(ww, ww);
+#pragma unroll
+                for (int i = 0; i < ANR_MG; i += 4) {
+                    const float4 a = a4[i / 4], aa = aa4[i / 4];
+                    unsigned long long t, q2, tt, qq;
+                    fix_parts(f32x2_mul(f32x2_mul(b2, f32x2(a.x, a.y)), w2), t, q2);
+                    fix_parts(f32x2_mul(f32x2_mul(bb2, f32x2(aa.x, aa.y)), ww2), tt, qq);
+                    hi[i] += (unsigned)t + (unsigned)tt;
+                    lo[i] += (unsigned)q2 + (unsigned)qq;
+                    hi[i + 1] += (unsigned)(t >> 32) + (unsigned)(tt >> 32);
+                    lo[i + 1] += (unsigned)(q2 >> 32) + (unsigned)(qq >> 32);
+                    fix_parts(f32x2_mul(f32x2_mul(b2, f32x2(a.z, a.w)), w2), t, q2);
+                    fix_parts(f32x2_mul(f32x2_mul(bb2, f32x2(aa.z, aa.w)), ww2), tt, qq);
+                    hi[i + 2] += (unsigned)t + (unsigned)tt;
+                    lo[i + 2] += (unsigned)q2 + (unsigned)qq;
+                    hi[i + 3] += (unsigned)(t >> 32) + (unsigned)(tt >> 32);
+                    lo[i + 3] += (unsigned)(q2 >> 32) + (unsigned)(qq >> 32);
+                }
+                n += 2;
+                if (n == ANR_FLUSH) flush();
+            } else {
+                if (!wide) flush();
+                for (int i = 0; i < ANR_MG; i++) {
+                    sum[i][lane] += (unsigned long long)f32_to_ll(b * ((const float *)a4)[i] * w);
+                    sum[i][lane] += (unsigned long long)f32_to_ll(bb * ((const float *)aa4)[i] * ww);
+                }
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        if (c >= nz) continue;
+#pragma unroll
+        for (int i = 0; i < ANR_MG; i++) {
+            const int mi = grp * ANR_MG + i;
+            if (mi < n3) {
+                const int k = __ldg(klist + mi);
+                const size_t at = (size_t)k * mstride + (size_t)pix * nz + c;
+                model[at] = fix_to_f32((long long)(part(i) + (wide ? sum[i][lane] : 0ULL) + own[at]), mem[k].fix_exp);
             }
         }
     }
@@ -928,6 +1194,7 @@ __global__ void k_fix_to_model(const long long *__restrict__ in, const MemberDev
                                int nz, float *__restrict__ model, double *__restrict__ model64,
                                const int *__restrict__ mbase) {
     const int k = blockIdx.y;
+    if (mbase && mbase[k] == -2) return;                    // (k_an_replay wrote it)
     const MemberDev &M = mem[k];
     const long long n = (long long)M.by * M.bx * nz;
     const int e = M.fix_exp;
@@ -971,6 +1238,46 @@ void launch_an_model_fast(cudaStream_t s, const GridDev &g, const AnSub *subs, i
         g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, (const float4 *)csff, astart,
         (const int4 *)aseg, nseg, ntot, zq, zqf, wqf, (const float2 *)vef, cd2if, ptabf, mem,
         (unsigned long long *)out64, mstride);
+}
+
+void launch_an_records(cudaStream_t s, const GridDev &g, const AnSub *subs, const int *sbase, const int *ssub,
+                       const double *cs, const float *csf, const float *csff, long long ns,
+                       const unsigned long long *act, const double *zq, const float *zqf, const float *wqf,
+                       const float *vef, const float *cd2if, const float *ptabf, const MemberDev *mem, int nlist,
+                       int *count, int *scan, void *runs, float *prof, int kw) {
+    const unsigned grid = (unsigned)((ns + 32 * ANF_WPB - 1) / (32 * ANF_WPB));
+    int *const offset = count + nlist + 1, *const cursor = offset + nlist + 1;
+    cudaMemsetAsync(count, 0, sizeof(int) * (nlist + 1), s);
+    if (!grid) return;
+    k_an_records<false><<<grid, ANF_WPB * 32, 0, s>>>(g, subs, sbase, ssub, (const double2 *)cs, (const float2 *)csf,
+                                                      (const float4 *)csff, ns, act, zq, zqf, wqf, (const float2 *)vef,
+                                                      cd2if, ptabf, mem, count, nullptr, nullptr, kw);
+    launch_scan_tiles(s, count, offset, cursor, nlist, scan);
+    k_an_records<true><<<grid, ANF_WPB * 32, 0, s>>>(g, subs, sbase, ssub, (const double2 *)cs, (const float2 *)csf,
+                                                     (const float4 *)csff, ns, act, zq, zqf, wqf, (const float2 *)vef,
+                                                     cd2if, ptabf, mem, cursor, (AnRun *)runs, prof, kw);
+}
+
+int an_replay_groups(int n3) { return (n3 + ANR_MG - 1) / ANR_MG; }
+bool an_replay_fits(int nsub) { return nsub <= 640; }
+
+void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const MemberDev *mem, int npix,
+                      const int *klist, int n3, const unsigned long long *chg, int nchw, const int *count,
+                      const void *runs, const float *prof, int kw, float *amp, const long long *own, long long mstride,
+                      float *model) {
+    const int ng = an_replay_groups(n3), nzb = (g.nz + 31) / 32, ntask = npix * nzb;
+    const long long na = 2LL * nsub * ng * ANR_MG;
+    if (!na || !ntask) return;
+    float *const top = amp + na;
+    k_an_amps<<<(unsigned)((na + 255) / 256), 256, 0, s>>>(subs, nsub, mem, klist, n3, ng, chg, nchw, amp, top);
+    const size_t smem = (size_t)2 * nsub * (ANR_MG + 1) * sizeof(float);
+    cudaFuncSetAttribute(k_an_replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per = 1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_an_replay, 256, smem);
+    const int nc = std::max(1, std::min(152 * std::max(per, 1) / ng, (ntask + 7) / 8));
+    k_an_replay<<<nc * ng, 256, smem, s>>>(g.nz, ng, nzb, npix, ntask, 2 * nsub, count + ntask + 1, count,
+                                           (const int4 *)runs, prof, kw, amp, top, klist, n3, mem, (const unsigned long long *)own, mstride,
+                                           model);
 }
 
 // The tile of the thin batches, 2^ltx x 2^lty pixels: the largest whose sums and the CDF table leave room for two CTAs

@@ -167,6 +167,16 @@ struct bbgpu_ctx {
     // sums it adds (-1: none); rebuilt before a run when an_dirty
     bool an_dirty = true;
     int an_nseg = 0, an_n2 = 0;
+    // the members computed from member 0's runs with their own amplitudes (an_segments): their number, the floats of a
+    // sample's profile; the workspace of the runs and, per member and sub-ring, whether its column is member 0's but
+    // for the density
+    int an_n3 = 0, an_kw = 0;
+    std::vector<signed char> an_same_nd;
+    int *d_anrcount = nullptr, *d_anrscan = nullptr, *d_anklist = nullptr;
+    unsigned long long *d_anchg = nullptr;
+    uint8_t *d_anruns = nullptr;
+    float *d_anprof = nullptr, *d_anamp = nullptr;
+    size_t d_anrcount_cap = 0, d_anrscan_cap = 0, d_anruns_cap = 0, d_anprof_cap = 0, d_anamp_cap = 0;
     long long an_ntot = 0;
     std::vector<long long> h_astart;
     std::vector<int> h_aseg, h_mbase, asbase_host;
@@ -572,7 +582,8 @@ extern "C" int bbgpu_ctx_destroy(bbgpu_ctx *ctx) {
                     (void *)ctx->d_pwvalf, (void *)ctx->d_maps32, (void *)ctx->d_K, (void *)ctx->d_maps64,
                     (void *)ctx->d_pmem, (void *)ctx->d_mstart, (void *)ctx->d_mseg, (void *)ctx->d_uidx,
                     (void *)ctx->d_ubase, (void *)ctx->d_prof_of, (void *)ctx->d_pstatu, (void *)ctx->d_pxu,
-                    (void *)ctx->d_cstart, (void *)ctx->d_base64, (void *)ctx->d_cseg, (void *)ctx->d_klist,
+                    (void *)ctx->d_anrcount, (void *)ctx->d_anrscan, (void *)ctx->d_anruns, (void *)ctx->d_anprof,
+                    (void *)ctx->d_anamp, (void *)ctx->d_cstart, (void *)ctx->d_base64, (void *)ctx->d_cseg, (void *)ctx->d_klist,
                     (void *)ctx->d_tsrc, (void *)ctx->d_blk, (void *)ctx->d_ktab, (void *)ctx->d_gflag,
                     (void *)ctx->d_rp_rec, (void *)ctx->d_rp_cnt, (void *)ctx->d_chg, (void *)ctx->d_rp_n,
                     (void *)ctx->d_atab, (void *)ctx->d_tmask, (void *)ctx->d_awhere, (void *)ctx->d_acount, (void *)ctx->d_aorder,
@@ -626,9 +637,9 @@ extern "C" int bbgpu_shared_members(const bbgpu_ctx *ctx, int *profiles, int *mc
     const bool mc = ctx->galmodtype == BBGPU_MC && !ctx->mc_dirty;
     const bool an = ctx->galmodtype == BBGPU_ANALYTIC && !ctx->an_dirty;
     if (profiles) *profiles = ctx->prof_uploaded ? ctx->nu : 0;
-    if (mc_full) *mc_full = mc ? ctx->mc_n1 : (an ? ctx->nb - ctx->an_n2 : 0);
+    if (mc_full) *mc_full = mc ? ctx->mc_n1 : (an ? ctx->nb - ctx->an_n2 - ctx->an_n3 : 0);
     if (mc_delta) *mc_delta = mc ? ctx->mc_n2 : (an ? ctx->an_n2 : 0);
-    if (mc_replay) *mc_replay = mc ? ctx->mc_n3 : 0;
+    if (mc_replay) *mc_replay = mc ? ctx->mc_n3 : (an ? ctx->an_n3 : 0);
     return BBGPU_OK;
 }
 
@@ -878,6 +889,8 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
     ZgridCache &zc = ctx->azcache;
     if (zc.zq.size() > ((size_t)1 << 24)) zc.clear();
     int nzq0 = 1;
+    std::vector<uint16_t> dmask((size_t)nsub + 1);
+    ctx->an_same_nd.assign((size_t)nb * nsub, 0);
     for (int k = 0; k < nb; k++) {
         const bbgpu_eval_desc &d = descs[k];
         const double *s = sr + (size_t)k * BBGPU_NSR * nsub;
@@ -893,9 +906,15 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
             return fail(ctx, BBGPU_ERR_ARG, "eval: member %d: box outside the cube", k);
         signed char *ru = ctx->h_reuse + (size_t)k * nsub;
         memset(ru, 0, (size_t)nsub);
+        if (reuse) bbh_column_diff(s, sr, nsub, dmask.data());
         const int e = bbh_an_subs(s, nsub, &g, nzq, d.blo0, d.blo1, d.bhi0, d.bhi1, ctx->h_cd2i.data(), 0, nullptr,
                                   nullptr, ctx->h_asub + (size_t)k * nsub, zc, reuse ? sr : nullptr,
-                                  reuse ? ctx->h_asub : nullptr, reuse ? ru : nullptr);
+                                  reuse ? ctx->h_asub : nullptr, reuse ? ru : nullptr, reuse ? dmask.data() : nullptr);
+        if (reuse)
+            for (int ir = 0; ir < nsub; ir++)
+                ctx->an_same_nd[(size_t)k * nsub + ir] =
+                    ru[ir] || (!(dmask[ir] & ~(1u << 5)) &&
+                               ctx->h_asub[(size_t)k * nsub + ir].active == ctx->h_asub[ir].active);
         if (e == -10000) return fail(ctx, BBGPU_ERR_ARG, "eval: member %d: the total flux is not finite", k);
         if ((rc = member_desc(ctx, k, d, e, need_cube, ctx->mem_host[k]))) return rc;
         ctx->h_mem[k] = ctx->mem_host[k];
@@ -1304,8 +1323,14 @@ static int mc_segments(bbgpu_ctx *ctx) {
 // The (member, sample) segments of an ANALYTIC batch. A member k > 0 whose columns differ from member 0's in a
 // few sub-rings, with member 0's box and fixed-point exponent (with a flux normalisation: member 0's profile), is
 // computed as member 0's fixed-point sums plus the deposits of those sub-rings' samples with its constants, minus
-// the same samples with member 0's (exact: the sums are modulo 2^64, the deposits rounded symmetrically); every
-// other member deposits all its samples.
+// the same samples with member 0's (exact: the sums are modulo 2^64, the deposits rounded symmetrically). A member
+// whose columns are member 0's but for the density, except a few sub-rings, takes member 0's runs with its own fluxes
+// (k_an_replay: the same deposits) and deposits only the samples of those sub-rings; every other member deposits all
+// its samples. The runs are listed for AN_REPLAY_MIN members or more: at 160x160x128 the list takes
+// 0.27 ms and a group of 16 members, full or not, 0.96 ms, where a member by its samples takes 0.18 ms.
+#define AN_REPLAY_MIN 8
+#define AN_REPLAY_RUNS (1LL << 27)        // 2 GB of runs
+#define AN_REPLAY_PROF (1LL << 28)        // 1 GB of profiles
 static int an_segments(bbgpu_ctx *ctx) {
     const int nb = ctx->nb, nsub = ctx->nsub;
     const long long ns = ctx->ansamp;
@@ -1325,37 +1350,86 @@ static int an_segments(bbgpu_ctx *ctx) {
     const bool can = ctx->share && nb > 1 && (int)sb.size() == nsub + 1 &&
                      (!ctx->prof_uploaded || (int)ctx->prof_of_host.size() == nb);
     const MemberDev &M0 = ctx->mem_host[0];
-    int n2 = 0;
-    for (int k = 0; k < nb; k++) {
-        if (can && k > 0) {
-            const MemberDev &M = ctx->mem_host[k];
-            bool ok = M.blo0 == M0.blo0 && M.blo1 == M0.blo1 && M.bx == M0.bx && M.by == M0.by;
-            if (ok) ok = ctx->prof_uploaded ? ctx->prof_of_host[k] == 0 : M.fix_exp == M0.fix_exp;
-            if (ok) {
-                const signed char *ru = ctx->h_reuse + (size_t)k * nsub;
-                long long nch = 0;
-                for (int ir = 0; ir < nsub; ir++)
-                    if (!ru[ir]) nch += sb[ir + 1] - sb[ir];
-                if (2 * nch < ns) {
-                    for (int ir = 0; ir < nsub; ir++)
-                        if (!ru[ir]) {
-                            seg(k, k, ir, 1, sb[ir + 1] - sb[ir]);
-                            seg(k, 0, ir, -1, sb[ir + 1] - sb[ir]);
-                        }
-                    mb[k] = 0;
-                    n2++;
-                    continue;
-                }
-            }
+    // how a member is computed (0: all its samples; 2: difference from member 0; 3: member 0's runs with its fluxes)
+    std::vector<signed char> kind(nb, 0);
+    const AnSub *A0 = ctx->h_asub;
+    int n2 = 0, n3 = 0, kw = 0;
+    long long nrun = 0;                                      // (a bound of member 0's runs)
+    bool replay = can && !ctx->an_tile && !ctx->an_exact && !ctx->want64 && an_replay_fits(nsub);
+    if (replay) {
+        for (int ir = 0; ir < nsub; ir++) {
+            if (!A0[ir].active) continue;
+            nrun += (long long)(sb[ir + 1] - sb[ir]) * A0[ir].nzz;
+            kw = (int)std::max<long long>(kw, std::min<long long>(2 * A0[ir].K + 1, ctx->g.nz));
         }
-        seg(k, k, -1, 1, ns);
+        nrun *= an_run_blocks(kw);
+        replay = nrun <= AN_REPLAY_RUNS && ns * kw <= AN_REPLAY_PROF;
+    }
+    for (int k = 1; can && k < nb; k++) {
+        const MemberDev &M = ctx->mem_host[k];
+        if (M.blo0 != M0.blo0 || M.blo1 != M0.blo1 || M.bx != M0.bx || M.by != M0.by) continue;
+        const signed char *ru = ctx->h_reuse + (size_t)k * nsub, *sn = ctx->an_same_nd.data() + (size_t)k * nsub;
+        long long nch = 0, nnd = 0;
+        for (int ir = 0; ir < nsub; ir++) {
+            if (!ru[ir]) nch += sb[ir + 1] - sb[ir];
+            if (!sn[ir]) nnd += sb[ir + 1] - sb[ir];
+        }
+        if ((ctx->prof_uploaded ? ctx->prof_of_host[k] == 0 : M.fix_exp == M0.fix_exp) && 2 * nch < ns) {
+            kind[k] = 2;
+            n2++;
+        } else if (replay && 2 * nnd < ns) {
+            kind[k] = 3;
+            n3++;
+        }
+    }
+    if (n3 < AN_REPLAY_MIN) n3 = 0;
+    const int nchw = (nsub + 63) / 64;
+    std::vector<unsigned long long> chg;                     // member 0's active sub-rings, then per member its own
+    std::vector<int> kl;
+    if (n3) {
+        chg.assign((size_t)(n3 + 1) * nchw, 0ULL);
+        for (int ir = 0; ir < nsub; ir++)
+            if (A0[ir].active) chg[ir >> 6] |= 1ULL << (ir & 63);
+    }
+    for (int k = 0; k < nb; k++) {
+        if (kind[k] == 2) {
+            const signed char *ru = ctx->h_reuse + (size_t)k * nsub;
+            for (int ir = 0; ir < nsub; ir++)
+                if (!ru[ir]) {
+                    seg(k, k, ir, 1, sb[ir + 1] - sb[ir]);
+                    seg(k, 0, ir, -1, sb[ir + 1] - sb[ir]);
+                }
+            mb[k] = 0;
+        } else if (kind[k] == 3 && n3) {
+            const signed char *sn = ctx->an_same_nd.data() + (size_t)k * nsub;
+            kl.push_back(k);
+            for (int ir = 0; ir < nsub; ir++)
+                if (!sn[ir]) {
+                    seg(k, k, ir, 1, sb[ir + 1] - sb[ir]);
+                    chg[kl.size() * nchw + (ir >> 6)] |= 1ULL << (ir & 63);
+                }
+            mb[k] = -2;
+        } else {
+            seg(k, k, -1, 1, ns);
+        }
     }
     cs.push_back(tot);
     ctx->an_nseg = (int)cs.size() - 1;
     ctx->an_ntot = tot;
     ctx->an_n2 = n2;
+    ctx->an_n3 = n3;
+    ctx->an_kw = kw;
     int rc;
     cudaStream_t s = ctx->stream;
+    if (n3) {
+        const size_t np = (size_t)M0.bx * M0.by * ((ctx->g.nz + 31) / 32) + 1;
+        if ((rc = dgrow(ctx, &ctx->d_anrcount, &ctx->d_anrcount_cap, 3 * np)) ||
+            (rc = dgrow(ctx, &ctx->d_anrscan, &ctx->d_anrscan_cap, np / 1024 + 2)) ||
+            (rc = dgrow(ctx, &ctx->d_anruns, &ctx->d_anruns_cap, AN_RUN_BYTES * (size_t)(nrun + 1))) ||
+            (rc = dgrow(ctx, &ctx->d_anprof, &ctx->d_anprof_cap, (size_t)(ns * kw) + 1)) ||
+            (rc = dgrow(ctx, &ctx->d_anamp, &ctx->d_anamp_cap, 2 * (size_t)nsub * 17 * an_replay_groups(n3) + 1)))
+            return rc;
+    }
     std::vector<int> &t0 = ctx->h_atile0;
     t0.assign(1, 0);
     if (ctx->an_tile) {
@@ -1380,7 +1454,8 @@ static int an_segments(bbgpu_ctx *ctx) {
         return at;
     };
     const size_t o_seg = place(sizeof(int) * sg.size()), o_start = place(sizeof(long long) * cs.size()),
-                 o_base = place(sizeof(int) * mb.size()), o_tile = place(sizeof(int) * t0.size());
+                 o_base = place(sizeof(int) * mb.size()), o_tile = place(sizeof(int) * t0.size()),
+                 o_kl = place(sizeof(int) * kl.size()), o_chg = place(sizeof(unsigned long long) * chg.size());
     if (!ctx->ev_tab) CK(cudaEventCreateWithFlags(&ctx->ev_tab, cudaEventDisableTiming));
     CK(cudaEventSynchronize(ctx->ev_tab));                   // (the last upload has left the pinned buffer)
     if ((rc = hgrow(ctx, &ctx->h_atab, &ctx->h_atab_cap, bytes))) return rc;
@@ -1389,10 +1464,16 @@ static int an_segments(bbgpu_ctx *ctx) {
     ctx->d_astart = (long long *)(ctx->d_atab + o_start);
     ctx->d_mbase = (int *)(ctx->d_atab + o_base);
     ctx->d_atile0 = (int *)(ctx->d_atab + o_tile);
+    ctx->d_anklist = (int *)(ctx->d_atab + o_kl);
+    ctx->d_anchg = (unsigned long long *)(ctx->d_atab + o_chg);
     if (!sg.empty()) memcpy(ctx->h_atab + o_seg, sg.data(), sizeof(int) * sg.size());
     memcpy(ctx->h_atab + o_start, cs.data(), sizeof(long long) * cs.size());
     memcpy(ctx->h_atab + o_base, mb.data(), sizeof(int) * mb.size());
     memcpy(ctx->h_atab + o_tile, t0.data(), sizeof(int) * t0.size());
+    if (n3) {
+        memcpy(ctx->h_atab + o_kl, kl.data(), sizeof(int) * kl.size());
+        memcpy(ctx->h_atab + o_chg, chg.data(), sizeof(unsigned long long) * chg.size());
+    }
     CK(cudaMemcpyAsync(ctx->d_atab, ctx->h_atab, bytes, cudaMemcpyHostToDevice, s));
     CK(cudaEventRecord(ctx->ev_tab, s));
     ctx->an_dirty = false;
@@ -1621,8 +1702,25 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
                                 ctx->mstride, 1);
                 CKL();
             }
+            if (ctx->an_n3) {
+                const MemberDev &M0 = ctx->mem_host[0];
+                const int npix = M0.bx * M0.by;
+                launch_an_records(s, g, ctx->d_asub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_acsf,
+                                  (const float *)ctx->d_acsff, ctx->ansamp, ctx->d_anchg, ctx->d_azq, ctx->d_azqf,
+                                  ctx->d_awqf, (const float *)ctx->d_vef, ctx->d_cd2if, ctx->d_ptabf, ctx->d_mem,
+                                  npix * ((g.nz + 31) / 32),
+                                  ctx->d_anrcount, ctx->d_anrscan, ctx->d_anruns, ctx->d_anprof, ctx->an_kw);
+                CKL();
+                ctx->launches += 3;                          // (the second pass, the scan and the amplitudes)
+                const int nchw = (ctx->nsub + 63) / 64;
+                launch_an_replay(s, g, ctx->d_asub, ctx->nsub, ctx->d_mem, npix, ctx->d_anklist, ctx->an_n3,
+                                 ctx->d_anchg + nchw, nchw, ctx->d_anrcount, ctx->d_anruns, ctx->d_anprof, ctx->an_kw,
+                                 ctx->d_anamp, ctx->d_model_fx, ctx->mstride, ctx->d_model);
+                CKL();
+            }
             launch_fix_to_model(s, ctx->d_model_fx, ctx->d_mem, ctx->nb, ctx->mstride, g.nz, ctx->d_model,
-                                ctx->want64 ? ctx->d_model64 : nullptr, ctx->an_n2 ? ctx->d_mbase : nullptr);
+                                ctx->want64 ? ctx->d_model64 : nullptr,
+                                ctx->an_n2 || ctx->an_n3 ? ctx->d_mbase : nullptr);
             CKL();
         }
         if (tm) CK(cudaEventRecord(ctx->ev[11], s));

@@ -6,6 +6,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
 #include "kernels.h"
 
 namespace {
@@ -23,20 +24,6 @@ __device__ __forceinline__ void cp_async_zfill16(float *dst, const float *src, b
 __device__ __forceinline__ void cp_async_zfill4(float *dst, const float *src, bool ok) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src), "r"(ok ? 4 : 0) : "memory");
-}
-
-// Two float32 FMAs in one instruction, (lo, hi) of each register pair rounded as fmaf: the issue slots bound the
-// convolution, not the FMA pipe.
-__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a, unsigned long long b) {
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
 }
 
 // TS: the model of a pixel is looked up in a tile table (TileSrc): the table entries of the CTA's input region
@@ -204,7 +191,7 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
                 }
             }
 #pragma unroll
-            for (int x = 0; x < TO; x++) a2[x] = pack2(acc[0][x], 0.0f);
+            for (int x = 0; x < TO; x++) a2[x] = f32x2(acc[0][x], 0.0f);
             for (int i = 1; i < ky; i++) {
                 if (!filled(i)) continue;
                 const float *row = col + (size_t)i * W * ZB;
@@ -219,14 +206,14 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
 #pragma unroll
                 for (int j = 0; j < W; j++) {
                     const float w = row[j * ZB];
-                    const unsigned long long w2 = pack2(w, w);
+                    const unsigned long long w2 = f32x2(w, w);
 #pragma unroll
                     for (int x = 0; x < TO; x++)
-                        if (j - x >= 0 && j - x < KXW) fma2(a2[x], tp[j - x], w2);
+                        if (j - x >= 0 && j - x < KXW) a2[x] = f32x2_fma(tp[j - x], w2, a2[x]);
                 }
             }
 #pragma unroll
-            for (int x = 0; x < TO; x++) unpack2(a2[x], acc[0][x], acc[1][x]);
+            for (int x = 0; x < TO; x++) f32x2_get(a2[x], acc[0][x], acc[1][x]);
             if (filled(ky)) {
                 const float *row = col + (size_t)ky * W * ZB;
                 float tp[KXW];

@@ -216,6 +216,26 @@ void launch_an_model_fast(cudaStream_t s, const GridDev &g, const AnSub *subs, i
                           const long long *astart, const int *aseg, int nseg, long long ntot,
                           const double *zq, const float *zqf, const float *wqf, const float *vef, const float *cd2if,
                           const float *ptabf, const MemberDev *mem, long long *out64, long long mstride);
+// Members that are member 0 but for the densities of most sub-rings: member 0's runs by pixel (launch_an_records:
+// sub-rings in the bit mask act, all of the float32 path; a list for each pixel and 32 channels, nlist of them: count
+// 3 (nlist + 1) ints, scan nlist / 1024 + 2; runs AN_RUN_BYTES for each run and list, at most an_run_blocks(kw) for every sample and height; prof kw
+// floats a sample), then the float32 models of the
+// n3 members klist (launch_an_replay: chg the sub-rings that a member deposits itself, its sums own of
+// k_an_model_fast; amp (2 nsub) (16 + 1) an_replay_groups(n3) floats).
+#define AN_RUN_BYTES 16
+// (kw channels from any first one lie in at most this many blocks of 32)
+inline int an_run_blocks(int kw) { return (kw + 30) / 32 + 1; }
+int an_replay_groups(int n3);
+bool an_replay_fits(int nsub);          // (the amplitudes of 16 members in shared memory)
+void launch_an_records(cudaStream_t s, const GridDev &g, const AnSub *subs, const int *sbase, const int *ssub,
+                       const double *cs, const float *csf, const float *csff, long long ns,
+                       const unsigned long long *act, const double *zq, const float *zqf, const float *wqf,
+                       const float *vef, const float *cd2if, const float *ptabf, const MemberDev *mem, int nlist,
+                       int *count, int *scan, void *runs, float *prof, int kw);
+void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const MemberDev *mem, int npix,
+                      const int *klist, int n3, const unsigned long long *chg, int nchw, const int *count,
+                      const void *runs, const float *prof, int kw, float *amp, const long long *own, long long mstride,
+                      float *model);
 // The same models where every sub-ring has one height and the float32 path (a thin disk), by tiles of 2^ltx x 2^lty
 // pixels (an_tile_size: for nz channels and the
 // npix pixels of a batch; false where a pixel's sums do not fit): the samples of the segments listed by

@@ -30,6 +30,7 @@
 #include <algorithm>
 
 #include "devmath.cuh"
+#include "f32x2.cuh"
 #include "kernels.h"
 
 #define ERR_LAYOUT 1
@@ -768,26 +769,6 @@ __device__ __forceinline__ void px_entry(const Entry *__restrict__ bucket, int b
     }
 }
 
-// two float32 operations an instruction, each half rounded as the scalar one
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 // this lane's (up to) SPL sorted samples of the cloud, 16-byte loads (the runs are padded to 4 samples with NaN;
 // the samples past the cloud are NaN as well)
 template <int SPL>
@@ -883,9 +864,9 @@ __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, c
     // v = sample x sg + tc, its nearest integer r by adding and subtracting 1.5 2^23 (a tie fails the test below, as
     // does a sample past the cloud: NaN), two samples an instruction. |v| < 2^22 wherever a sample can pass: the
     // cloud's bound eps holds |v| EPS_REL, and passing takes eps < 1/2
-    const unsigned long long sg2 = pack2(sg, sg), tc2 = pack2(tc, tc);
-    const unsigned long long magic2 = pack2(12582912.0f, 12582912.0f), nmagic2 = pack2(-12582912.0f, -12582912.0f);
-    const unsigned long long neg2 = pack2(-1.0f, -1.0f);
+    const unsigned long long sg2 = f32x2(sg, sg), tc2 = f32x2(tc, tc);
+    const unsigned long long magic2 = f32x2(12582912.0f, 12582912.0f), nmagic2 = f32x2(-12582912.0f, -12582912.0f);
+    const unsigned long long neg2 = f32x2(-1.0f, -1.0f);
     const int base = __float_as_int(__fadd_rn(fmaf(w[0].x, sg, tc), 12582912.0f)) - 1;
     const float hwf = fastc ? hw : -1.0f;                  // (a centre out of range: no sample passes)
     // straight-line code: each sample adds inc[min(channel - c0, 30)] (bins 0..10 five bits each, a channel
@@ -896,12 +877,12 @@ __device__ __forceinline__ void px_count(const GridDev &g, const LayoutDev &L, c
 #pragma unroll
     for (int s = 0; s < SPL / 2; s++) {
         const float4 &q4 = w[s >> 1];
-        const unsigned long long v2 = fma2((s & 1) ? pack2(q4.z, q4.w) : pack2(q4.x, q4.y), sg2, tc2);
-        const unsigned long long t2 = add2(v2, magic2);
-        const unsigned long long e2 = fma2(add2(t2, nmagic2), neg2, v2);
+        const unsigned long long v2 = f32x2_fma((s & 1) ? f32x2(q4.z, q4.w) : f32x2(q4.x, q4.y), sg2, tc2);
+        const unsigned long long t2 = f32x2_add(v2, magic2);
+        const unsigned long long e2 = f32x2_fma(f32x2_add(t2, nmagic2), neg2, v2);
         float t[2], d2[2];
-        unpack2(t2, t[0], t[1]);
-        unpack2(e2, d2[0], d2[1]);
+        f32x2_get(t2, t[0], t[1]);
+        f32x2_get(e2, d2[0], d2[1]);
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const bool ok = fabsf(d2[e]) <= hwf;

@@ -473,15 +473,15 @@ struct __align__(16) AnfSample {
 #define ANF_RUNS 96                   // runs of a sample collected before their deposit (a pass adds at most 33)
 #define ANF_FIXMAX 1.7592186044416e13f // 2^44: below it f32_to_fix is f32_to_ll
 
-// f32_to_ll for |x| < ANF_FIXMAX without its branch and shift: adding 1.5 2^46 rounds x to a multiple of 2^23 held in
-// the low mantissa bits, the exact rest (at most 2^22) is rounded the same way.
+// f32_to_ll for |x| < ANF_FIXMAX without its branch and shift: adding 1.5 2^46 rounded down leaves the multiple of 2^23
+// below x in the low mantissa bits of t, and the rest, at most 2^23, is rounded to an integer in the low bits of q.
 #define ANF_HI 1.0555311626649600e14f    // 1.5 2^46
+#define ANF_TOP (ANF_HI + 8388608.0f)    // (exact: 24 bits)
 __device__ __forceinline__ unsigned long long f32_to_fix(float x) {
-    const float t = __fadd_rn(x, ANF_HI);
-    const float l = __fsub_rn(x, __fsub_rn(t, ANF_HI));
-    const int hi = __float_as_int(t) - __float_as_int(ANF_HI);
-    const int lo = __float_as_int(__fadd_rn(l, BB_MAGIC15)) - __float_as_int(BB_MAGIC15);
-    return (unsigned long long)((long long)hi * 8388608 + lo);
+    const float t = __fadd_rd(x, ANF_HI);
+    const float q = __fadd_rn(x, __fsub_rn(ANF_TOP, t));
+    return (unsigned long long)((long long)(__float_as_int(t) - __float_as_int(ANF_HI)) * 8388608 +
+                                (__float_as_int(q) - 0x4B000000));
 }
 
 // The set-up of sample s (constants S = subs[sub], radius kr) by its lane; false if its line has no channel in the band.
@@ -812,10 +812,9 @@ __global__ void k_an_amps(const AnSub *__restrict__ subs, int nsub, const Member
 // its low mantissa bits, q the rest rounded to an integer of at most 2^23. Sums of both stay within 32 bits for ANR_FLUSH
 // runs, each addition with the bias of its constant.
 #define ANR_FLUSH 256
-#define ANR_TOP (ANF_HI + 8388608.0f)                       // (exact: 24 bits)
 __device__ __forceinline__ void fix_parts(unsigned long long x, unsigned long long &t, unsigned long long &q) {
     t = f32x2_add_rm(x, f32x2(ANF_HI, ANF_HI));
-    q = f32x2_add(x, f32x2_fma(t, f32x2(-1.0f, -1.0f), f32x2(ANR_TOP, ANR_TOP)));
+    q = f32x2_add(x, f32x2_fma(t, f32x2(-1.0f, -1.0f), f32x2(ANF_TOP, ANF_TOP)));
 }
 
 // A CTA keeps the amplitudes of one group of members in shared memory and its warps take (pixel, 32 channels) after
@@ -944,38 +943,36 @@ __global__ void __launch_bounds__(256, 3) k_an_replay(int nz, int ng, int nzb, i
     }
 }
 
-// ------------------------------------------------------------------------------ thin disks, by tiles of the sky
+// ------------------------------------------------------------------------------ thin disks, by pixels
 // A batch whose sub-rings all have one height (nzz = 1) and the float32 path. Each sample falls in one pixel, so the
-// samples are listed by tile of pixels (k_ant_bin, a scan, k_ant_list) and a CTA takes a tile with all its channels:
-// it adds the deposits in shared memory (64-bit fixed point: any order) and writes the tile's float32 model. The sums
-// never leave the SM: no memset, no 64-bit model in HBM, no reductions in L2, no conversion pass. The deposits are
+// samples are listed by pixel (k_ant_bin, a scan, k_ant_list) and a warp takes a pixel with all its channels: it adds
+// the deposits to a row of sums in shared memory that no other warp touches (64-bit fixed point: any order) and writes
+// the pixel's float32 model. No memset, no 64-bit model in HBM, no atomics on sums, no conversion pass. The deposits are
 // those of k_an_model_fast, integer for integer.
-#define ANT_NT 512
-#define ANT_BATCH 256                // samples of a tile in shared memory at a time
+#define ANT_NT 256
 
-// A sample as its tile deposits it: the line (velocity about vref in float-float, 1 / sig, amplitude in fixed-point
-// units), the weight of its height, its channels k0 .. k0 + nk and its pixel of the tile.
+// A sample as its pixel's warp deposits it: the line (velocity about vref in float-float, 1 / sig, amplitude in fixed-point
+// units), the weight of its height and its channels k0 .. k0 + nk.
 struct __align__(16) AntSample {
     float vrh, vrl, invf, amp, ws;
     unsigned short k0, nk;
-    int pix, pad;
+    int pad[2];
 };
 
-// one thread per sample of the batch's segments: the record, its tile (tiles of all members numbered from tile0[k];
-// -1: nothing to deposit) and its rank among the tile's samples (lanes of one tile count once)
+// one thread per sample of the batch's segments: the record, its pixel (pixels of all members numbered from pix0[k];
+// -1: nothing to deposit) and its rank among the pixel's samples (lanes of one pixel count once)
 __global__ void __launch_bounds__(256) k_ant_bin(GridDev g, const AnSub *__restrict__ subs, int nsub,
                                                  const int *__restrict__ sbase, const int *__restrict__ ssub,
                                                  const double2 *__restrict__ cs, const float2 *__restrict__ csf,
                                                  const float4 *__restrict__ csff, const long long *__restrict__ astart,
-                                                 const int4 *__restrict__ aseg, int nseg, long long ntot, int ltx,
-                                                 int lty, const int *__restrict__ tile0,
-                                                 const double *__restrict__ zq, const float *__restrict__ zqf,
+                                                 const int4 *__restrict__ aseg, int nseg, long long ntot,
+                                                 const int *__restrict__ pix0, const double *__restrict__ zq, const float *__restrict__ zqf,
                                                  const float *__restrict__ wqf, const MemberDev *__restrict__ mem,
                                                  AntSample *__restrict__ rec, int2 *__restrict__ where,
                                                  int *__restrict__ count) {
     const int lane = threadIdx.x & 31;
     const long long gs = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int tile = -1;
+    int pix = -1;
     AnSeg sg;
     if (an_seg(gs, astart, aseg, nseg, ntot, sbase, sg)) {
         const int s = (int)sg.s, ir = ssub[s];
@@ -997,8 +994,7 @@ __global__ void __launch_bounds__(256) k_ant_bin(GridDev g, const AnSub *__restr
                 if (a0 < 0) a0 = 0;
                 if (a1 > g.nz) a1 = g.nz;
                 if (a1 > a0) {
-                    const int ntx = (M.bx + (1 << ltx) - 1) >> ltx;
-                    tile = tile0[sg.k] + (g1 >> lty) * ntx + (g0 >> ltx);
+                    pix = pix0[sg.k] + g1 * M.bx + g0;
                     const ff vr = ff_add(v, ff{-g.vrefh, -g.vrefl});
                     AntSample o;
                     o.vrh = vr.hi;
@@ -1008,19 +1004,18 @@ __global__ void __launch_bounds__(256) k_ant_bin(GridDev g, const AnSub *__restr
                     o.ws = wqf[S.zq_off];
                     o.k0 = (unsigned short)a0;
                     o.nk = (unsigned short)(a1 - a0);
-                    o.pix = ((g1 & ((1 << lty) - 1)) << ltx) + (g0 & ((1 << ltx) - 1));
-                    o.pad = 0;
+                    o.pad[0] = o.pad[1] = 0;
                     rec[gs] = o;
                 }
             }
         }
     }
-    // consecutive samples mostly share a tile: one atomic for each of the warp's tiles
-    const unsigned same = __match_any_sync(FULL, tile);
+    // consecutive samples often share a pixel: one atomic for each of the warp's pixels
+    const unsigned same = __match_any_sync(FULL, pix);
     int r = 0;
-    if (tile >= 0 && lane == __ffs(same) - 1) r = atomicAdd(count + tile, __popc(same));
+    if (pix >= 0 && lane == __ffs(same) - 1) r = atomicAdd(count + pix, __popc(same));
     r = __shfl_sync(FULL, r, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
-    if (gs < ntot) where[gs] = make_int2(tile, r);
+    if (gs < ntot) where[gs] = make_int2(pix, r);
 }
 
 __global__ void k_ant_list(const int2 *__restrict__ where, long long ntot, const int *__restrict__ offset,
@@ -1031,118 +1026,100 @@ __global__ void k_ant_list(const int2 *__restrict__ where, long long ntot, const
     if (t.x >= 0) order[offset[t.x] + t.y] = (int)i;
 }
 
-// The tiles of the members [kfirst, kfirst + nk) (tiles tile0[kfirst] .. tile0[kfirst + nk)), a CTA after another:
-// persistent, so that the CDF table is read into shared memory once. The channel edges of a batch of samples are laid
-// end to end and the warps take equal parts of them, a lane an edge (a lane's upper edge is the next lane's, so a
-// warp advances by 31): no lane idles for the samples' 5 to 100 channels, whatever they are. base64: member 0's sums
-// in its box, written with base_out (by a launch of member 0 alone), else added to the members with mbase >= 0.
-__global__ void __launch_bounds__(ANT_NT, 2) k_ant_tile(int nz, int ltx, int lty, const int *__restrict__ tile0,
-                                                        int kfirst, int nk, const int *__restrict__ offset,
-                                                        const int *__restrict__ count, const int *__restrict__ order,
-                                                        const AntSample *__restrict__ rec,
-                                                        const float2 *__restrict__ vef,
-                                                        const float *__restrict__ cd2if,
-                                                        const float *__restrict__ ptabf,
-                                                        const MemberDev *__restrict__ mem, float *__restrict__ model,
-                                                        double *__restrict__ model64, long long mstride,
-                                                        long long *__restrict__ base64, int base_out,
-                                                        const int *__restrict__ mbase) {
-    extern __shared__ __align__(16) unsigned long long ant_acc[];   // (pixel, channel); channel edges; factors; CDF
-    __shared__ AntSample rs[ANT_BATCH];
-    __shared__ int pre[ANT_BATCH + 1], wsum[ANT_BATCH / 32], nedge; // first edge of each sample
-    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const int npix = 1 << (ltx + lty), tx = 1 << ltx, nacc = npix * nz;
-    float2 *const ved = (float2 *)(ant_acc + nacc);
-    float *const cdf = (float *)(ved + nz + 1), *const tab = cdf + nz;
-    float cdmax = 0.0f;
-    for (int i = tid; i < PHI_N; i += ANT_NT) tab[i] = ptabf[i];
-    for (int i = tid; i < nacc; i += ANT_NT) ant_acc[i] = 0;
-    for (int i = tid; i <= nz; i += ANT_NT) ved[i] = vef[i];
-    for (int i = tid; i < nz; i += ANT_NT) cdf[i] = cd2if[i];
-    for (int i = 0; i < nz; i++) cdmax = fmaxf(cdmax, fabsf(__ldg(cd2if + i)));
-    if (tid == 0) pre[0] = 0;
-    const int tend = tile0[kfirst + nk];
+__device__ __host__ inline int ant_pitch(int nz) { return (nz + 3) & ~1; }     // (sums of a warp: 16-byte rows)
+
+// The pixels of the members [kfirst, kfirst + nk) (numbered pix0[kfirst] .. pix0[kfirst + nk)), a pixel a warp:
+// persistent, so that the CDF table is read into shared memory once. 32 samples at a time are gathered a lane each; of
+// a sample, a lane takes an edge of the line (its upper edge is the next lane's: 31 channels a step), always of a
+// channel that is the lane's number modulo 32, so that no lane touches another's sums. Bound by issue (about 90
+// instructions a step): 256 members of 256x256x192 7.3 ms (8.8 ms with 4-byte writes), where tiles of pixels with
+// shared-memory atomics, the samples' edges laid end to end, took 8.9 ms. A pixel without samples, four in five, is only
+// written. base64:
+// member 0's sums in its box, written with base_out (by a launch of member 0 alone), else added to the members with
+// mbase >= 0.
+__global__ void __launch_bounds__(ANT_NT) k_ant_pixel(int nz, const int *__restrict__ pix0, int kfirst, int nk,
+                                                      const int *__restrict__ offset, const int *__restrict__ count,
+                                                      const int *__restrict__ order,
+                                                      const AntSample *__restrict__ rec,
+                                                      const float2 *__restrict__ vef, const float *__restrict__ cd2if,
+                                                      const float *__restrict__ ptabf,
+                                                      const MemberDev *__restrict__ mem, float *__restrict__ model,
+                                                      double *__restrict__ model64, long long mstride,
+                                                      long long *__restrict__ base64, int base_out,
+                                                      const int *__restrict__ mbase) {
+    // samples, (upper edge in float-float, factor) of the channels, sums of each warp, CDF
+    extern __shared__ __align__(16) uint8_t ant_smem_[];
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    AntSample *const rs = (AntSample *)ant_smem_ + w * 32;
+    float4 *const chan = (float4 *)(ant_smem_ + nw * 32 * sizeof(AntSample));
+    unsigned long long *const rows = (unsigned long long *)(chan + nz + 1), *const row = rows + (size_t)w * ant_pitch(nz);
+    float *const tab = (float *)(rows + (size_t)nw * ant_pitch(nz));
+    for (int i = tid; i < PHI_N; i += blockDim.x) tab[i] = ptabf[i];
+    for (int i = tid; i <= nz; i += blockDim.x) {
+        const float2 e = vef[i];
+        chan[i] = make_float4(e.x, e.y, i < nz ? cd2if[i] : 0.0f, 0.0f);
+    }
+    for (int i = lane; i < nz; i += 32) row[i] = 0;
+    __syncthreads();
+    const int pend = pix0[kfirst + nk];
+    const bool vec = (nz & 3) == 0 && (mstride & 3) == 0 && ((uintptr_t)model & 15) == 0;
     int k = kfirst;
-    for (int t = tile0[kfirst] + blockIdx.x; t < tend; t += gridDim.x) {
-        while (t >= tile0[k + 1]) k++;
-        const MemberDev &M = mem[k];
-        const int bx = M.bx, ntx = (bx + tx - 1) >> ltx, tl = t - tile0[k];
-        const int uy = tl / ntx, ux = (tl - uy * ntx) << ltx;
-        const int pw = min(tx, bx - ux), ph = min(1 << lty, M.by - (uy << lty));
-        const int n = count[t], o0 = offset[t];
-        for (int b0 = 0; b0 < n; b0 += ANT_BATCH) {
-            const int m = min(ANT_BATCH, n - b0);
-            __syncthreads();                                // (the batch or the tile before is done with)
-            int len = 0;
-            bool big = false;                               // (a deposit that may need f32_to_ll)
-            if (tid < m) {
-                const AntSample q = rec[order[o0 + b0 + tid]];
-                rs[tid] = q;
-                len = q.nk + 1;
-                big = !(fabsf(q.amp) * cdmax * q.ws < 0.5f * ANF_FIXMAX);
-            }
-            if (tid < ANT_BATCH) {
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const int v = __shfl_up_sync(FULL, len, d);
-                    if (lane >= d) len += v;
-                }
-                if (lane == 31) wsum[w] = len;
-            }
-            __syncthreads();
-            if (tid < ANT_BATCH) {
-                for (int i = 0; i < w; i++) len += wsum[i];
-                pre[tid + 1] = tid < m - 1 ? len : 0x7fffffff;      // (the last sample has no end: nc stops it)
-                if (tid == m - 1) nedge = len;
-            }
-            big = __syncthreads_or(big);
-            const int ne = nedge, nwin = (ne + 30) / 31, per = (nwin + ANT_NT / 32 - 1) / (ANT_NT / 32);
-            const int w0 = w * per, w1 = min(nwin, w0 + per);
-            int pos = w0 * 31 + lane, e = 0;
-            if (w0 < w1) {
-                int hi = m - 1;                             // the sample of the lane's first edge
-                while (e < hi) {
-                    const int mid = (e + hi + 1) >> 1;
-                    if (pre[mid] <= pos) e = mid;
-                    else hi = mid - 1;
-                }
-            }
-            int first = pre[e], next = pre[e + 1];
-            for (int win = w0; win < w1; win++, pos += 31) {
-                while (pos >= next) {
-                    first = next;
-                    next = pre[++e + 1];
-                }
-                const AntSample &q = rs[e];
-                const int j = pos - first, nc = q.nk, c = q.k0 + min(j, nc);
-                const float2 ed = ved[c];
-                const float f = phi_f32((__fsub_rn(ed.x, q.vrh) + __fsub_rn(ed.y, q.vrl)) * q.invf, tab);
-                const float fn = __shfl_down_sync(FULL, f, 1);
-                if (lane < 31 && j < nc) {
-                    const float x = fabsf(fn - f) * cdf[c] * q.amp * q.ws;
-                    unsigned long long *const a = ant_acc + (q.pix * nz + c);
-                    if (!big) atomicAdd(a, f32_to_fix(x));
-                    else atomicAdd(a, (unsigned long long)f32_to_ll(x));
+    for (int t = pix0[kfirst] + blockIdx.x * nw + w; t < pend; t += gridDim.x * nw) {
+        while (t >= pix0[k + 1]) k++;
+        const int n = count[t], o0 = n ? offset[t] : 0;
+        int c0 = nz, c1 = 0;                                // the channels with deposits
+        for (int b0 = 0; b0 < n; b0 += 32) {
+            const int m = min(32, n - b0);
+            __syncwarp();                                   // (the samples before are done with)
+            if (lane < m) rs[lane] = rec[order[o0 + b0 + lane]];
+            __syncwarp();
+            for (int i = 0; i < m; i++) {
+                const AntSample q = rs[i];
+                const int ka = q.k0, kb = ka + q.nk;
+                c0 = min(c0, ka);
+                c1 = max(c1, kb);
+                for (int a = ka; a < kb; a += 31) {
+                    const int c = a + ((lane - a) & 31), ce = min(c, kb);
+                    const float4 ed = chan[ce];
+                    const float f = phi_f32((__fsub_rn(ed.x, q.vrh) + __fsub_rn(ed.y, q.vrl)) * q.invf, tab);
+                    const float fn = __shfl_sync(FULL, f, (lane + 1) & 31);
+                    if (c < min(kb, a + 31)) {
+                        const float x = fabsf(fn - f) * ed.z * q.amp * q.ws;
+                        row[c] += fabsf(x) < ANF_FIXMAX ? f32_to_fix(x) : (unsigned long long)f32_to_ll(x);
+                    }
                 }
             }
         }
-        __syncthreads();
+        const MemberDev &M = mem[k];
+        const long long at = (long long)(t - pix0[k]) * nz;
         const long long *bas = !base_out && mbase[k] >= 0 ? base64 : nullptr;
+        float *const out = model + (size_t)k * mstride + at;
+        double *const out64 = model64 ? model64 + (size_t)k * mstride + at : nullptr;
         const int e = M.fix_exp;
-        for (int p = w; p < npix; p += ANT_NT / 32) {       // a warp a pixel: lanes over channels
-            const int py = p >> ltx, pxx = p & (tx - 1);
-            if (pxx >= pw || py >= ph) continue;
-            const long long at = ((long long)((uy << lty) + py) * bx + ux + pxx) * nz;
-            float *out = model + (size_t)k * mstride + at;
-            for (int c = lane; c < nz; c += 32) {
-                unsigned long long q = ant_acc[p * nz + c];
-                ant_acc[p * nz + c] = 0;
-                if (base_out) base64[at + c] = (long long)q;
-                if (bas) q += (unsigned long long)bas[at + c];
-                out[c] = fix_to_f32((long long)q, e);
-                if (model64)
-                    model64[(size_t)k * mstride + at + c] = __dmul_rn((double)(long long)q, ldexp(1.0, -e));
+        if (vec && !base_out && !bas && !out64) {           // (16-byte writes, four channels a lane)
+            for (int c = 4 * lane; c < nz; c += 128) {
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (c < c1 && c + 4 > c0) {
+                    ulonglong2 *const r = (ulonglong2 *)(row + c);
+                    const ulonglong2 a = r[0], b = r[1];
+                    r[0] = r[1] = make_ulonglong2(0ULL, 0ULL);
+                    v = make_float4(fix_to_f32((long long)a.x, e), fix_to_f32((long long)a.y, e),
+                                    fix_to_f32((long long)b.x, e), fix_to_f32((long long)b.y, e));
+                }
+                *(float4 *)(out + c) = v;
             }
+            continue;
+        }
+        for (int c = lane; c < nz; c += 32) {
+            unsigned long long q = 0;
+            if (c >= c0 && c < c1) {
+                q = row[c];
+                row[c] = 0;
+            }
+            if (base_out) base64[at + c] = (long long)q;
+            if (bas) q += (unsigned long long)bas[at + c];
+            out[c] = q ? fix_to_f32((long long)q, e) : 0.0f;
+            if (out64) out64[c] = __dmul_rn((double)(long long)q, ldexp(1.0, -e));
         }
     }
 }
@@ -1280,30 +1257,25 @@ void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int n
                                            model);
 }
 
-// The tile of the thin batches, 2^ltx x 2^lty pixels: the largest whose sums and the CDF table leave room for two CTAs
-// on an SM (103 KB each beside the samples), else one that fits at all; smaller, down to 2 x 2, while the npix pixels
-// of the batch give the SMs fewer than 4 tiles each. False for more channels than a pixel's sums fit.
-#define ANT_TAB (PHI_N * 4 + 16)
-static size_t ant_smem(int nz, int ltx, int lty) { return ((size_t)nz << (ltx + lty)) * 8 + (size_t)nz * 12 + ANT_TAB; }
-bool an_tile_size(int nz, long long npix, int &ltx, int &lty) {
-    for (int most : {103 * 1024, AN_SMEM_MAX})
-        for (int l = 8; l >= (most == AN_SMEM_MAX ? 0 : 4); l--) {
-            ltx = (l + 1) / 2;
-            lty = l / 2;
-            if (ant_smem(nz, ltx, lty) > (size_t)most || (l > 2 && (npix >> l) < 4 * 152)) continue;
-            return nz < 65536;
-        }
-    return false;
+// shared memory of k_ant_pixel with nw warps a CTA; the warps that fit (8, or fewer for many channels; 0: none)
+static size_t ant_smem(int nz, int nw) {
+    return nw * (32 * sizeof(AntSample) + (size_t)ant_pitch(nz) * 8) + ((size_t)nz + 1) * 16 + PHI_N * 4;
+}
+int ant_warps(int nz) {
+    if (nz >= 65536) return 0;
+    for (int nw = ANT_NT / 32; nw > 0; nw >>= 1)
+        if (ant_smem(nz, nw) <= AN_SMEM_MAX) return nw;
+    return 0;
 }
 
 void launch_ant_bin(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
                     const double *cs, const float *csf, const float *csff, const long long *astart, const int *aseg,
-                    int nseg, long long ntot, int ltx, int lty, const int *tile0, const double *zq, const float *zqf,
+                    int nseg, long long ntot, const int *pix0, const double *zq, const float *zqf,
                     const float *wqf, const MemberDev *mem, void *rec, int *where, int *count) {
     if (ntot == 0 || nseg == 0) return;
     k_ant_bin<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(
         g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, (const float4 *)csff, astart,
-        (const int4 *)aseg, nseg, ntot, ltx, lty, tile0, zq, zqf, wqf, mem, (AntSample *)rec, (int2 *)where, count);
+        (const int4 *)aseg, nseg, ntot, pix0, zq, zqf, wqf, mem, (AntSample *)rec, (int2 *)where, count);
 }
 
 void launch_ant_list(cudaStream_t s, const int *where, long long ntot, const int *offset, int *order) {
@@ -1311,18 +1283,19 @@ void launch_ant_list(cudaStream_t s, const int *where, long long ntot, const int
     k_ant_list<<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>((const int2 *)where, ntot, offset, order);
 }
 
-void launch_ant_tile(cudaStream_t s, int nz, int ltx, int lty, const int *tile0, int kfirst, int nk, int ntile,
-                     const int *offset, const int *count, const int *order, const void *rec, const float *vef,
-                     const float *cd2if, const float *ptabf, const MemberDev *mem, float *model, double *model64,
-                     long long mstride, long long *base64, int base_out, const int *mbase) {
-    if (nk <= 0 || ntile <= 0) return;
-    const size_t smem = ant_smem(nz, ltx, lty);
-    cudaFuncSetAttribute(k_ant_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+void launch_ant_pixel(cudaStream_t s, int nz, const int *pix0, int kfirst, int nk, int npix, const int *offset,
+                      const int *count, const int *order, const void *rec, const float *vef, const float *cd2if,
+                      const float *ptabf, const MemberDev *mem, float *model, double *model64, long long mstride,
+                      long long *base64, int base_out, const int *mbase) {
+    const int nw = ant_warps(nz);
+    if (nk <= 0 || npix <= 0 || !nw) return;
+    const size_t smem = ant_smem(nz, nw);
+    cudaFuncSetAttribute(k_ant_pixel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ant_tile, ANT_NT, smem);
-    k_ant_tile<<<std::min(ntile, 152 * std::max(per, 1)), ANT_NT, smem, s>>>(
-        nz, ltx, lty, tile0, kfirst, nk, offset, count, order, (const AntSample *)rec, (const float2 *)vef, cd2if,
-        ptabf, mem, model, model64, mstride, base64, base_out, mbase);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ant_pixel, 32 * nw, smem);
+    k_ant_pixel<<<std::min((npix + nw - 1) / nw, 152 * std::max(per, 1)), 32 * nw, smem, s>>>(
+        nz, pix0, kfirst, nk, offset, count, order, (const AntSample *)rec, (const float2 *)vef, cd2if, ptabf, mem,
+        model, model64, mstride, base64, base_out, mbase);
 }
 
 void launch_an_maps(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,

@@ -180,18 +180,17 @@ struct bbgpu_ctx {
     long long an_ntot = 0;
     std::vector<long long> h_astart;
     std::vector<int> h_aseg, h_mbase, asbase_host;
-    // thin batches: the tiles (an_ltx, an_lty; first tile of each member), the samples' records, tiles and lists
-    int an_ltx = 0, an_lty = 0;
-    std::vector<int> h_atile0;
+    // thin batches: the first pixel of each member, the samples' records, pixels and lists
+    std::vector<int> h_apix0;
     int *d_awhere = nullptr, *d_acount = nullptr, *d_aorder = nullptr, *d_ascan = nullptr;
     uint8_t *d_arec = nullptr;
     size_t d_awhere_cap = 0, d_acount_cap = 0, d_aorder_cap = 0, d_arec_cap = 0, d_ascan_cap = 0;
-    // the tables of an_segments, one upload from pinned memory (ev_tab: it has left it): astart, aseg, mbase, atile0
+    // the tables of an_segments, one upload from pinned memory (ev_tab: it has left it): astart, aseg, mbase, apix0
     uint8_t *h_atab = nullptr, *d_atab = nullptr;
     size_t h_atab_cap = 0, d_atab_cap = 0;
     cudaEvent_t ev_tab = nullptr;
     long long *d_astart = nullptr;
-    int *d_aseg = nullptr, *d_mbase = nullptr, *d_atile0 = nullptr;
+    int *d_aseg = nullptr, *d_mbase = nullptr, *d_apix0 = nullptr;
     std::vector<unsigned long long> h_chg; // per member: the sub-rings a replaying member deposits itself
     int nchw = 0;
     int *d_rp_rec = nullptr, *d_rp_n = nullptr;   // (2 ints a record; records per list of member 0)
@@ -218,7 +217,7 @@ struct bbgpu_ctx {
     // ANALYTIC batches: sub-ring constants per member, the sample table of the model's sub-rings, their vertical
     // grids (host cache mirrored on the device) and the fixed-point models
     AnSub *h_asub = nullptr, *d_asub = nullptr;
-    int an_thick = 0, an_exact = 1, an_tile = 0;   // the ANALYTIC kernels the uploaded batch needs
+    int an_thick = 0, an_exact = 1, an_pixel = 0;   // the ANALYTIC kernels the uploaded batch needs
     size_t h_asub_cap = 0, d_asub_cap = 0;
     int *d_asbase = nullptr, *d_assub = nullptr;
     size_t d_asbase_cap = 0, d_assub_cap = 0;
@@ -1001,12 +1000,12 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
     if (ctx->want64)
         if ((rc = dgrow(ctx, &ctx->d_model64, &ctx->d_model64_cap, (size_t)nb * ctx->mstride))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_reuse, &ctx->d_reuse_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
-    // which ANALYTIC kernels the batch needs: the tile kernels where every sub-ring is thin (one height) with the float32
-    // path, else the float32 path by samples, and the exact kernel for the sub-rings it does not take (a reused column
-    // is member 0's, whose flags count already). Thin disks: the tiles took less time than the samples (and the
-    // conversion pass these need) at every size tried, 63 against 65 us for one 64x64x64 member, 7.5 against 13.7 ms
-    // for 64 members of 256x256x192. A thick sub-ring's sample crosses many tiles, each of which would find its runs
-    // again: by samples only.
+    // which ANALYTIC kernels the batch needs: by pixels where every sub-ring is thin (one height) with the float32 path,
+    // else the float32 path by samples, and the exact kernel for the sub-rings it does not take (a reused column is
+    // member 0's, whose flags count already). Thin disks: by pixels took less time than by samples (and the conversion
+    // pass these need) at every size tried, an evaluation of one 64x64x64 member 279 against 288 us, of 64 members of
+    // 256x256x192 4.8 against 8.6 ms. A thick sub-ring's sample has a run in many pixels: to list them costs as much as
+    // to deposit them.
     ctx->an_thick = ctx->an_exact = 0;
     for (size_t i = 0; i < (size_t)nb * nsub; i++) {
         if (ctx->h_reuse[i]) continue;
@@ -1017,9 +1016,9 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
     }
     long long npix = 0;
     for (int k = 0; k < nb; k++) npix += (long long)ctx->mem_host[k].bx * ctx->mem_host[k].by;
-    ctx->an_tile = !ctx->an_thick && !ctx->an_exact && nb * ctx->ansamp < (1LL << 31) - 1 &&
-                   an_tile_size(g.nz, npix, ctx->an_ltx, ctx->an_lty);
-    if (!ctx->an_tile)
+    ctx->an_pixel = !ctx->an_thick && !ctx->an_exact && nb * ctx->ansamp < (1LL << 31) - 1 && npix < (1LL << 30) &&
+                    ant_warps(g.nz) > 0;
+    if (!ctx->an_pixel)
         if ((rc = dgrow(ctx, &ctx->d_model_fx, &ctx->d_model_fx_cap, (size_t)nb * ctx->mstride))) return rc;
     CK(cudaMemcpyAsync(ctx->d_asub, ctx->h_asub, sizeof(AnSub) * (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_mem, ctx->h_mem, sizeof(MemberDev) * (size_t)nb, cudaMemcpyHostToDevice, ctx->stream));
@@ -1355,7 +1354,7 @@ static int an_segments(bbgpu_ctx *ctx) {
     const AnSub *A0 = ctx->h_asub;
     int n2 = 0, n3 = 0, kw = 0;
     long long nrun = 0;                                      // (a bound of member 0's runs)
-    bool replay = can && !ctx->an_tile && !ctx->an_exact && !ctx->want64 && an_replay_fits(nsub);
+    bool replay = can && !ctx->an_pixel && !ctx->an_exact && !ctx->want64 && an_replay_fits(nsub);
     if (replay) {
         for (int ir = 0; ir < nsub; ir++) {
             if (!A0[ir].active) continue;
@@ -1430,14 +1429,12 @@ static int an_segments(bbgpu_ctx *ctx) {
             (rc = dgrow(ctx, &ctx->d_anamp, &ctx->d_anamp_cap, 2 * (size_t)nsub * 17 * an_replay_groups(n3) + 1)))
             return rc;
     }
-    std::vector<int> &t0 = ctx->h_atile0;
+    std::vector<int> &t0 = ctx->h_apix0;
     t0.assign(1, 0);
-    if (ctx->an_tile) {
-        const int tx = 1 << ctx->an_ltx, ty = 1 << ctx->an_lty;
-        for (const MemberDev &M : ctx->mem_host)
-            t0.push_back(t0.back() + ((M.bx + tx - 1) / tx) * ((M.by + ty - 1) / ty));
+    if (ctx->an_pixel) {
+        for (const MemberDev &M : ctx->mem_host) t0.push_back(t0.back() + M.bx * M.by);
         const size_t nt = (size_t)t0[nb] + 1, n = (size_t)tot + 1;
-        if ((rc = dgrow(ctx, &ctx->d_acount, &ctx->d_acount_cap, 3 * nt)) ||
+        if ((rc = dgrow(ctx, &ctx->d_acount, &ctx->d_acount_cap, 2 * nt)) ||
             (rc = dgrow(ctx, &ctx->d_ascan, &ctx->d_ascan_cap, nt / 1024 + 2)) ||
             (rc = dgrow(ctx, &ctx->d_awhere, &ctx->d_awhere_cap, 2 * n)) ||
             (rc = dgrow(ctx, &ctx->d_aorder, &ctx->d_aorder_cap, n)) ||
@@ -1454,7 +1451,7 @@ static int an_segments(bbgpu_ctx *ctx) {
         return at;
     };
     const size_t o_seg = place(sizeof(int) * sg.size()), o_start = place(sizeof(long long) * cs.size()),
-                 o_base = place(sizeof(int) * mb.size()), o_tile = place(sizeof(int) * t0.size()),
+                 o_base = place(sizeof(int) * mb.size()), o_pix = place(sizeof(int) * t0.size()),
                  o_kl = place(sizeof(int) * kl.size()), o_chg = place(sizeof(unsigned long long) * chg.size());
     if (!ctx->ev_tab) CK(cudaEventCreateWithFlags(&ctx->ev_tab, cudaEventDisableTiming));
     CK(cudaEventSynchronize(ctx->ev_tab));                   // (the last upload has left the pinned buffer)
@@ -1463,13 +1460,13 @@ static int an_segments(bbgpu_ctx *ctx) {
     ctx->d_aseg = (int *)(ctx->d_atab + o_seg);
     ctx->d_astart = (long long *)(ctx->d_atab + o_start);
     ctx->d_mbase = (int *)(ctx->d_atab + o_base);
-    ctx->d_atile0 = (int *)(ctx->d_atab + o_tile);
+    ctx->d_apix0 = (int *)(ctx->d_atab + o_pix);
     ctx->d_anklist = (int *)(ctx->d_atab + o_kl);
     ctx->d_anchg = (unsigned long long *)(ctx->d_atab + o_chg);
     if (!sg.empty()) memcpy(ctx->h_atab + o_seg, sg.data(), sizeof(int) * sg.size());
     memcpy(ctx->h_atab + o_start, cs.data(), sizeof(long long) * cs.size());
     memcpy(ctx->h_atab + o_base, mb.data(), sizeof(int) * mb.size());
-    memcpy(ctx->h_atab + o_tile, t0.data(), sizeof(int) * t0.size());
+    memcpy(ctx->h_atab + o_pix, t0.data(), sizeof(int) * t0.size());
     if (n3) {
         memcpy(ctx->h_atab + o_kl, kl.data(), sizeof(int) * kl.size());
         memcpy(ctx->h_atab + o_chg, chg.data(), sizeof(unsigned long long) * chg.size());
@@ -1664,17 +1661,17 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
             int rc = an_segments(ctx);
             if (rc) return rc;
         }
-        if (ctx->an_tile) {
-            const std::vector<int> &t0 = ctx->h_atile0;
+        if (ctx->an_pixel) {
+            const std::vector<int> &t0 = ctx->h_apix0;
             const int nt = t0[ctx->nb];
             int *count = ctx->d_acount, *offset = count + nt + 1;
             CK(cudaMemsetAsync(count, 0, sizeof(int) * (nt + 1), s));
             launch_ant_bin(s, g, ctx->d_asub, ctx->nsub, ctx->d_asbase, ctx->d_assub, ctx->d_acs, ctx->d_acsf,
                            (const float *)ctx->d_acsff, ctx->d_astart, ctx->d_aseg, ctx->an_nseg, ctx->an_ntot,
-                           ctx->an_ltx, ctx->an_lty, ctx->d_atile0, ctx->d_azq, ctx->d_azqf, ctx->d_awqf, ctx->d_mem,
+                           ctx->d_apix0, ctx->d_azq, ctx->d_azqf, ctx->d_awqf, ctx->d_mem,
                            ctx->d_arec, ctx->d_awhere, count);
             CKL();
-            launch_scan_tiles(s, count, offset, offset + nt + 1, nt, ctx->d_ascan);
+            launch_scan_tiles(s, count, offset, nullptr, nt, ctx->d_ascan);
             CKL();
             launch_ant_list(s, ctx->d_awhere, ctx->an_ntot, offset, ctx->d_aorder);
             CKL();
@@ -1682,10 +1679,10 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
             const int first = ctx->an_n2 ? 1 : 0;
             for (int pass = first ? 0 : 1; pass < 2; pass++) {
                 const int k0 = pass ? first : 0, nk = pass ? ctx->nb - first : 1;
-                launch_ant_tile(s, g.nz, ctx->an_ltx, ctx->an_lty, ctx->d_atile0, k0, nk, t0[k0 + nk] - t0[k0], offset,
-                                count, ctx->d_aorder, ctx->d_arec, (const float *)ctx->d_vef, ctx->d_cd2if,
-                                ctx->d_ptabf, ctx->d_mem, ctx->d_model, ctx->want64 ? ctx->d_model64 : nullptr,
-                                ctx->mstride, ctx->d_base64, pass ? 0 : 1, ctx->d_mbase);
+                launch_ant_pixel(s, g.nz, ctx->d_apix0, k0, nk, t0[k0 + nk] - t0[k0], offset, count, ctx->d_aorder,
+                                 ctx->d_arec, (const float *)ctx->d_vef, ctx->d_cd2if, ctx->d_ptabf, ctx->d_mem,
+                                 ctx->d_model, ctx->want64 ? ctx->d_model64 : nullptr, ctx->mstride, ctx->d_base64,
+                                 pass ? 0 : 1, ctx->d_mbase);
                 CKL();
             }
         } else {

@@ -69,7 +69,7 @@ void launch_mc_sums64(cudaStream_t s, const long long *sums, long long n, int nz
 // Measured: one ring of a 64x64x64 cube (9 tiles, 20 k clouds) 81 us with one CTA a tile, 20 us with 16; from 304
 // tiles on the chip is full (two CTAs per SM) and a split would only repeat the tiles' zeroing and output.
 int mc_deposit_split(int ntile);
-// Exclusive scan of n list counts into offsets (and cursors); scratch holds (n + 1023) / 1024 ints.
+// Exclusive scan of n list counts into offsets (and cursors, where not null); scratch holds (n + 1023) / 1024 ints.
 void launch_scan_tiles(cudaStream_t s, const int *count, int *offset, int *cursor, int n, int *scratch);
 // bucket: 32-byte entries (Entry in mc.cu), one per in-box (member, cloud)
 #define ENTRY_BYTES 32
@@ -236,28 +236,27 @@ void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int n
                       const int *klist, int n3, const unsigned long long *chg, int nchw, const int *count,
                       const void *runs, const float *prof, int kw, float *amp, const long long *own, long long mstride,
                       float *model);
-// The same models where every sub-ring has one height and the float32 path (a thin disk), by tiles of 2^ltx x 2^lty
-// pixels (an_tile_size: for nz channels and the
-// npix pixels of a batch; false where a pixel's sums do not fit): the samples of the segments listed by
-// tile (launch_ant_bin: records rec of ANT_REC bytes, where (tile, rank), count per tile, zeroed by the caller; the
-// scan of the counts; launch_ant_list: order), then the tiles of the members kfirst .. kfirst + nk - 1 (ntile of them;
-// tile0[k]: member k's first tile, nb + 1 entries) deposit theirs and write the float32 model. base64: with base_out
-// (nk = 1) receives the member's sums, else it is added to the members with mbase >= 0.
+// The same models where every sub-ring has one height and the float32 path (a thin disk), by pixels (ant_warps(nz) > 0:
+// a pixel's sums fit in shared memory): the samples of the segments listed by pixel (launch_ant_bin: records rec of
+// ANT_REC bytes, where (pixel, rank), count per pixel, zeroed by the caller; the scan of the counts; launch_ant_list:
+// order), then the pixels of the members kfirst .. kfirst + nk - 1 (npix of them; pix0[k]: member k's first pixel, nb + 1
+// entries) deposit theirs and write the float32 model. base64: with base_out (nk = 1) receives the member's sums, else
+// it is added to the members with mbase >= 0.
 #define ANT_REC 32
-bool an_tile_size(int nz, long long npix, int &ltx, int &lty);
+int ant_warps(int nz);
 void launch_ant_bin(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
                     const double *cs, const float *csf, const float *csff, const long long *astart, const int *aseg,
-                    int nseg, long long ntot, int ltx, int lty, const int *tile0, const double *zq, const float *zqf,
-                    const float *wqf, const MemberDev *mem, void *rec, int *where, int *count);
+                    int nseg, long long ntot, const int *pix0, const double *zq, const float *zqf, const float *wqf,
+                    const MemberDev *mem, void *rec, int *where, int *count);
 void launch_ant_list(cudaStream_t s, const int *where, long long ntot, const int *offset, int *order);
-void launch_ant_tile(cudaStream_t s, int nz, int ltx, int lty, const int *tile0, int kfirst, int nk, int ntile,
-                     const int *offset, const int *count, const int *order, const void *rec, const float *vef,
-                     const float *cd2if, const float *ptabf, const MemberDev *mem, float *model, double *model64,
-                     long long mstride, long long *base64, int base_out, const int *mbase);
+void launch_ant_pixel(cudaStream_t s, int nz, const int *pix0, int kfirst, int nk, int npix, const int *offset,
+                      const int *count, const int *order, const void *rec, const float *vef, const float *cd2if,
+                      const float *ptabf, const MemberDev *mem, float *model, double *model64, long long mstride,
+                      long long *base64, int base_out, const int *mbase);
 void launch_an_maps(cudaStream_t s, const GridDev &g, const AnSub *subs, int nsub, const int *sbase, const int *ssub,
                     const double *cs, long long nsamp, const double *zq, const double *wq, const long long *widx,
                     const double *wval, const MemberDev &M, long long *maps64);
-// mbase (nullable): per member, the member whose fixed-point sums are added (-1: none)
+// mbase (nullable): per member, the member whose fixed-point sums are added (-1: none; -2: the member is left out)
 void launch_fix_to_model(cudaStream_t s, const long long *in, const MemberDev *mem, int nb, long long mstride, int nz,
                          float *model, double *model64, const int *mbase = nullptr);
 

@@ -1378,7 +1378,7 @@ __global__ void __launch_bounds__(1024) k_scan_one(const int *__restrict__ count
     for (int i = 0; i < SCAN_ONE / 1024; i++) {
         if (b + i < e) {
             offset[b + i] = run;
-            cursor[b + i] = run;
+            if (cursor) cursor[b + i] = run;
         }
         run += c[i];
     }
@@ -1411,7 +1411,7 @@ __global__ void k_scan_c(const int *__restrict__ count, int n, const int *__rest
     const int ex = x - v + (wid > 0 ? r[wid - 1] : 0) + bsum[blockIdx.x];
     if (i < n) {
         offset[i] = ex;
-        cursor[i] = ex;
+        if (cursor) cursor[i] = ex;
     }
 }
 

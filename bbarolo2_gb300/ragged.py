@@ -50,17 +50,21 @@ class GalaxyBatch:
     def upload(self, rows_list, seed=None):
         """The host set-up and upload of every galaxy's ring sets (rows_list[i]: (B_i, 17, nr_i)); returns the
         boxes per galaxy."""
+        return [self._upload(item, rows, seed) for item, rows in self._pairs(rows_list)]
+
+    def _pairs(self, rows_list):
         if len(rows_list) != len(self.items):
             raise ValueError("one array of ring sets per galaxy")
+        return zip(self.items, rows_list)
+
+    def _upload(self, item, rows, seed):
+        dm, like, rings = item
         code = _lib.ANALYTIC if self.galmodtype == "ANALYTIC" else _lib.MC
-        boxes = []
-        for (dm, like, rings), rows in zip(self.items, rows_list):
-            sr, nv, descs, bx = like.prepare(rows, rings, seed)
-            ctx = dm.ctx
-            ctx.check(ctx.L.bbgpu_eval_upload(ctx.h, code, sr.shape[0], sr.shape[2], _lib.ptr(sr), _lib.ptr(nv),
-                                              _lib.ptr(descs)))
-            boxes.append(bx)
-        return boxes
+        sr, nv, descs, bx = like.prepare(rows, rings, seed)
+        ctx = dm.ctx
+        ctx.check(ctx.L.bbgpu_eval_upload(ctx.h, code, sr.shape[0], sr.shape[2], _lib.ptr(sr), _lib.ptr(nv),
+                                          _lib.ptr(descs)))
+        return bx
 
     def run(self):
         """Queues every galaxy's evaluation of its uploaded ring sets (no result is read)."""
@@ -78,7 +82,10 @@ class GalaxyBatch:
         return out
 
     def evaluate(self, rows_list, seed=None):
-        """log L of every galaxy's ring sets: uploads, queues and reads them all."""
-        boxes = self.upload(rows_list, seed)
-        self.run()
+        """log L of every galaxy's ring sets: each galaxy's evaluation is queued as soon as its ring sets are uploaded,
+        so that the set-up of the next runs beside it; then all are read."""
+        boxes = []
+        for item, rows in self._pairs(rows_list):
+            boxes.append(self._upload(item, rows, seed))
+            item[0].ctx.check(item[0].ctx.L.bbgpu_eval_run(item[0].ctx.h))
         return self.download(boxes)

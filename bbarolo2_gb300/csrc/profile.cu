@@ -35,6 +35,9 @@
 #define EPS_REL 3.814697265625e-06f
 #define GRAM_TP 128         // pixels per CTA of k_prof_gram
 
+// row pitch of the factor of k_prof_solve (odd: a column's elements in different banks)
+static __host__ __device__ inline int prof_solve_pitch(int n) { return n | 1; }
+
 namespace {
 
 // ------------------------------------------------------------------------------------------- ring maps
@@ -372,23 +375,36 @@ __global__ void k_prof_gram_reduce(const double *__restrict__ part, int ntile, i
 }
 
 // ------------------------------------------------------------------------------------------- NNLS
-// Shared state of one member's solve (one CTA, PS_THREADS threads).
-#define PS_THREADS 128
+// Shared state of one member's solve (one CTA: PS_UPDATE threads that eliminate and a warp for the pivots). A solve is
+// a serial chain of small steps, and the float64 pipe takes 16 cycles of the SM an instruction whatever its lanes hold:
+// the elimination spreads elements (not rows) over the lanes, the pivots' reciprocals are one warp's, taken while the
+// others update, the right-hand side is eliminated with the matrix, and what a single thread would do serially is a
+// warp's ballots and shuffles.
+// 81 solves of 41 unknowns 153 us; 422 us with rows over the warps, a reciprocal in every warp, dot products for the
+// substitutions and a thread for the passive set.
+#define PS_UPDATE 128
+#define PS_THREADS (PS_UPDATE + 32)
 
 struct Solver {
-    int n;
+    int n, fs;
     double *H;      // n x n (the normal matrix of the current system)
-    double *F;      // factor of the passive block, n x n
+    double *F;      // factor of the passive block and its right-hand side, (n + 1) x fs
     double *g;      // right-hand side
     double *x, *z, *w;
     int *P, *idx;   // passive flags, passive indices
     int *blocked;
     int *sflag;     // shared scalars
     double *sval;
-    double *rs;     // 1 / sqrt of the pivots of the factorisation
+    double *rs;     // 1 / pivots of the factorisation
+    double *l;      // the current column over its pivot
 };
 
-// Cholesky of H[P,P] into F and solve F F^T z_P = g_P; false if the block is not positive definite.
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
+    return v;
+}
+
 // 1 / d for d > 0 in float64 without a division: a float32 seed and two Newton steps (within an ulp or two of
 // the quotient; float64 division is slow on this part)
 __device__ __forceinline__ double rcp_newton(double d) {
@@ -398,78 +414,76 @@ __device__ __forceinline__ double rcp_newton(double d) {
     return y;
 }
 
+// the pivot c: its reciprocal, or the flag of a block that is not positive definite
+__device__ __forceinline__ void take_pivot(Solver &S, int c, double d) {
+    if (d > 0.0) S.rs[c] = d > 1e-30 && d < 1e30 ? rcp_newton(d) : 1.0 / d;
+    else S.sflag[0] = 0;
+}
+
+// H[P,P] z_P = g_P by elimination (L D L^T); false if the block is not positive definite. F holds L[r][c] D[c] below the
+// diagonal, and as row p the right-hand side.
 __device__ bool chol_solve(Solver &S, int p) {
-    const int tid = threadIdx.x;
-    const int n = S.n;
+    const int tid = threadIdx.x, n = S.n, fs = S.fs;
     for (int e = tid; e < p * p; e += blockDim.x) {
         const int a = e / p, b = e - a * p;
-        S.F[a * n + b] = S.H[S.idx[a] * n + S.idx[b]];
+        if (b <= a) S.F[a * fs + b] = S.H[S.idx[a] * n + S.idx[b]];
     }
+    for (int b = tid; b < p; b += blockDim.x) S.F[p * fs + b] = S.g[S.idx[b]];
     if (tid == 0) S.sflag[0] = 1;
     __syncthreads();
-    // right-looking elimination on the unscaled columns (one barrier a column): the trailing block takes
-    // F[r][c] F[q][c] / F[c][c]; the columns are scaled to the Cholesky factor at the end, L[r][c] = F[r][c] /
-    // sqrt(F[c][c]), the diagonal sqrt(F[c][c]) (the same products as the scaled form, in another order)
+    if (tid == 0) take_pivot(S, 0, S.F[0]);
+    __syncthreads();
+    const int ty = tid >> 3, tx = tid & 7;
     for (int c = 0; c < p; c++) {
-        const double d = S.F[c * n + c];
-        if (!(d > 0.0)) {
-            if (tid == 0) S.sflag[0] = 0;
-            if (tid == 0) S.F[c * n + c] = 1.0;
-            __syncthreads();
-            continue;
-        }
-        const double inv = (d > 1e-30 && d < 1e30) ? rcp_newton(d) : 1.0 / d;
-        // the trailing block's lower triangle: rows on the warps, columns on the lanes
-        const int nwarp = blockDim.x >> 5, wid = tid >> 5, ln = tid & 31;
-        for (int r = c + 1 + wid; r < p; r += nwarp) {
-            const double frc = S.F[r * n + c] * inv;
-            for (int q = c + 1 + ln; q <= r; q += 32) S.F[r * n + q] -= frc * S.F[q * n + c];
+        if (!S.sflag[0]) return false;                      // (the same for all: read between two barriers)
+        const double inv = S.rs[c];
+        for (int r = c + 1 + tid; r <= p; r += blockDim.x) S.l[r] = S.F[r * fs + c] * inv;
+        __syncthreads();
+        if (tid < PS_UPDATE) {
+            // the rows after the next pivot's, 16 at a time, 8 columns at a time
+            for (int r = c + 2 + ty; r <= p; r += PS_UPDATE / 8) {
+                const double lr = S.l[r];
+                for (int q = c + 1 + tx; q <= r && q < p; q += 8) S.F[r * fs + q] -= lr * S.F[q * fs + c];
+            }
+        } else if (tid == PS_UPDATE) {
+            const int r = c + 1;
+            if (r < p) {
+                const double d = S.F[r * fs + r] - S.l[r] * S.F[r * fs + c];
+                S.F[r * fs + r] = d;
+                take_pivot(S, r, d);
+            }
         }
         __syncthreads();
     }
-    for (int c = tid; c < p; c += blockDim.x) {
-        const double d = S.F[c * n + c];
-        S.rs[c] = d > 0.0 ? 1.0 / sqrt(d) : 1.0;
-    }
-    __syncthreads();
     for (int e = tid; e < p * p; e += blockDim.x) {
         const int r = e / p, c = e - r * p;
-        if (r > c) S.F[r * n + c] *= S.rs[c];
+        if (c < r) S.F[r * fs + c] *= S.rs[c];
+        else if (c == r) S.z[r] = S.F[p * fs + r] * S.rs[r];
     }
     __syncthreads();
-    for (int c = tid; c < p; c += blockDim.x) {
-        const double d = S.F[c * n + c];
-        S.F[c * n + c] = d > 0.0 ? sqrt(d) : 1.0;
-    }
-    __syncthreads();
-    const bool ok = S.sflag[0] != 0;
-    // forward then back substitution (one warp; lanes over the dot products)
     if (tid < 32) {
-        for (int r = 0; r < p; r++) {
-            double acc = 0.0;
-            for (int q = tid; q < r; q += 32) acc += S.F[r * n + q] * S.z[q];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(FULL, acc, o);
-            if (tid == 0) S.z[r] = (S.g[S.idx[r]] - acc) * S.rs[r];   // (F[r][r] = 1 / rs[r])
-            __syncwarp();
-        }
-        for (int r = p - 1; r >= 0; r--) {
-            double acc = 0.0;
-            for (int q = r + 1 + tid; q < p; q += 32) acc += S.F[q * n + r] * S.z[q];
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(FULL, acc, o);
-            if (tid == 0) S.z[r] = (S.z[r] - acc) * S.rs[r];
+        for (int r = p - 1; r > 0; r--) {
+            const double x = S.z[r];
+            for (int q = tid; q < r; q += 32) S.z[q] -= S.F[r * fs + q] * x;
             __syncwarp();
         }
     }
     __syncthreads();
-    return ok;
+    return true;
 }
 
+// the passive indices in ascending order; their number
 __device__ int gather_passive(Solver &S) {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         int p = 0;
-        for (int j = 0; j < S.n; j++)
-            if (S.P[j]) S.idx[p++] = j;
-        S.sflag[1] = p;
+        for (int b = 0; b < S.n; b += 32) {
+            const int j = b + threadIdx.x;
+            const bool in = j < S.n && S.P[j];
+            const unsigned m = __ballot_sync(FULL, in);
+            if (in) S.idx[p + __popc(m & ((1u << threadIdx.x) - 1u))] = j;
+            p += __popc(m);
+        }
+        if (threadIdx.x == 0) S.sflag[1] = p;
     }
     __syncthreads();
     return S.sflag[1];
@@ -491,45 +505,64 @@ __device__ int nnls(Solver &S) {
         if (p == 0) break;
         if (!chol_solve(S, p)) {
             status = 1;
+            __syncthreads();
             for (int j = tid; j < n; j += blockDim.x) S.P[j] = 0;
             __syncthreads();
             break;
         }
-        if (tid == 0) {
-            int bad = 0;
-            for (int a = 0; a < p; a++)
+        if (tid < 32) {
+            bool bad = false;
+            for (int a = tid; a < p; a += 32)
                 if (!(S.z[a] > 0.0)) {
                     S.P[S.idx[a]] = 0;
-                    bad = 1;
+                    bad = true;
                 }
+            bad = __any_sync(FULL, bad);
             if (!bad)
-                for (int a = 0; a < p; a++) S.x[S.idx[a]] = S.z[a];
-            S.sflag[2] = bad;
+                for (int a = tid; a < p; a += 32) S.x[S.idx[a]] = S.z[a];
+            if (tid == 0) S.sflag[2] = bad;
         }
         __syncthreads();
         if (!S.sflag[2]) break;
     }
-    double gmax = 0.0;
-    for (int j = 0; j < n; j++) gmax = fmax(gmax, fabs(S.g[j]));
-    const double tol = 1e-12 * (gmax > 0 ? gmax : 1.0);
+    double tol = 0.0;                                       // (the first warp's)
+    if (tid < 32) {
+        double gmax = 0.0;
+        for (int j = tid; j < n; j += 32) gmax = fmax(gmax, fabs(S.g[j]));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) gmax = fmax(gmax, __shfl_xor_sync(FULL, gmax, o));
+        tol = 1e-12 * (gmax > 0 ? gmax : 1.0);
+    }
     for (int outer = 0; outer < 3 * n; outer++) {
         // w = g - H x
         for (int j = tid; j < n; j += blockDim.x) {
             double acc = S.g[j];
-            for (int q = 0; q < n; q++) acc -= S.H[j * n + q] * S.x[q];
+            for (int q = 0; q < n; q++) acc -= S.H[q * n + j] * S.x[q];
             S.w[j] = acc;
         }
         __syncthreads();
-        if (tid == 0) {
+        if (tid < 32) {
+            // the largest w of the free components, the first of equal ones
             int t = -1;
             double best = tol;
-            for (int j = 0; j < n; j++)
+            for (int j = tid; j < n; j += 32)
                 if (!S.P[j] && !S.blocked[j] && S.w[j] > best) {
                     best = S.w[j];
                     t = j;
                 }
-            S.sflag[3] = t;
-            if (t >= 0) S.P[t] = 1;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double b2 = __shfl_xor_sync(FULL, best, o);
+                const int t2 = __shfl_xor_sync(FULL, t, o);
+                if (t2 >= 0 && (t < 0 || b2 > best || (b2 == best && t2 < t))) {
+                    best = b2;
+                    t = t2;
+                }
+            }
+            if (tid == 0) {
+                S.sflag[3] = t;
+                if (t >= 0) S.P[t] = 1;
+            }
         }
         __syncthreads();
         const int t = S.sflag[3];
@@ -538,6 +571,7 @@ __device__ int nnls(Solver &S) {
             const int p = gather_passive(S);
             if (!chol_solve(S, p)) {
                 status |= 1;
+                __syncthreads();
                 if (tid == 0) {
                     S.P[t] = 0;
                     S.blocked[t] = 1;
@@ -545,33 +579,40 @@ __device__ int nnls(Solver &S) {
                 __syncthreads();
                 break;
             }
-            if (tid == 0) {
-                int allpos = 1, tpos = 1;
-                for (int a = 0; a < p; a++)
+            if (tid < 32) {
+                bool neg = false, tneg = false;
+                for (int a = tid; a < p; a += 32)
                     if (!(S.z[a] > 0.0)) {
-                        allpos = 0;
-                        if (S.idx[a] == t) tpos = 0;
+                        neg = true;
+                        tneg |= S.idx[a] == t;
                     }
-                if (allpos) {
-                    for (int j = 0; j < n; j++) S.x[j] = 0.0;
-                    for (int a = 0; a < p; a++) S.x[S.idx[a]] = S.z[a];
-                    for (int j = 0; j < n; j++) S.blocked[j] = 0;
-                    S.sflag[4] = 1;
-                } else if (inner == 0 && !tpos) {
+                neg = __any_sync(FULL, neg);
+                tneg = __any_sync(FULL, tneg);
+                if (!neg) {
+                    for (int j = tid; j < n; j += 32) {
+                        S.x[j] = 0.0;
+                        S.blocked[j] = 0;
+                    }
+                    __syncwarp();
+                    for (int a = tid; a < p; a += 32) S.x[S.idx[a]] = S.z[a];
+                } else if (inner == 0 && tneg) {
                     // the entering variable is not positive in the least squares: numerically at its bound
-                    S.P[t] = 0;
-                    S.blocked[t] = 1;
-                    S.sflag[4] = 1;
+                    if (tid == 0) {
+                        S.P[t] = 0;
+                        S.blocked[t] = 1;
+                    }
                 } else {
                     double alpha = 2.0;
-                    for (int a = 0; a < p; a++)
+                    for (int a = tid; a < p; a += 32)
                         if (!(S.z[a] > 0.0)) {
                             const int j = S.idx[a];
                             const double den = S.x[j] - S.z[a];
                             const double al = den > 0.0 ? S.x[j] / den : 0.0;
                             alpha = fmin(alpha, al);
                         }
-                    for (int a = 0; a < p; a++) {
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) alpha = fmin(alpha, __shfl_xor_sync(FULL, alpha, o));
+                    for (int a = tid; a < p; a += 32) {
                         const int j = S.idx[a];
                         S.x[j] += alpha * (S.z[a] - S.x[j]);
                         if (!(S.x[j] > 0.0)) {
@@ -579,8 +620,8 @@ __device__ int nnls(Solver &S) {
                             S.P[j] = 0;
                         }
                     }
-                    S.sflag[4] = 0;
                 }
+                if (tid == 0) S.sflag[4] = !neg || (inner == 0 && tneg);
             }
             __syncthreads();
             if (S.sflag[4]) break;
@@ -589,15 +630,17 @@ __device__ int nnls(Solver &S) {
     return status | 2;
 }
 
-// H = G + sum_i wi^2 L_i^T L_i (L_i: the 3 weights of second difference i at columns lc[i][0..2])
-__device__ void build_H(Solver &S, const double *G, const int *lc, const double *lv, const double *wr, int nrow) {
-    // H = G + sum over the prior rows i of w_i^2 lv_i lv_i^T (columns lc_i); each entry takes its terms in the
-    // order of the rows (i, then a, then b), a thread an entry
+// H = G + sum_i wi^2 L_i^T L_i (L_i: the 3 weights of second difference i at columns lc[i][0..2]): each entry takes its
+// terms in the order of the rows (i, then a, then b), a thread an entry; rows from span[2 j] to span[2 j + 1] hold
+// column j
+__device__ void build_H(Solver &S, const double *G, const int *lc, const double *lv, const double *wr, int nrow,
+                        const int *span) {
     const int n = S.n;
     for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
         const int j = e / n, q = e - j * n;
         double h = G[e];
-        for (int i = 0; i < nrow; i++) {
+        const int i1 = nrow ? min(span[2 * j + 1], span[2 * q + 1]) : -1;
+        for (int i = nrow ? max(span[2 * j], span[2 * q]) : 0; i <= i1; i++) {
             const int c0 = lc[3 * i], c1 = lc[3 * i + 1], c2 = lc[3 * i + 2];
             if ((c0 != j && c1 != j && c2 != j) || (c0 != q && c1 != q && c2 != q)) continue;
             const double w2 = wr[i] * wr[i];
@@ -623,76 +666,88 @@ __global__ void __launch_bounds__(PS_THREADS) k_prof_solve(const double *__restr
     const int n = pc.n, k = blockIdx.x, tid = threadIdx.x;
     Solver S;
     S.n = n;
+    S.fs = prof_solve_pitch(n);
     double *G = psm;
     S.H = G + n * n;
     S.F = S.H + n * n;
-    S.g = S.F + n * n;
+    S.g = S.F + (n + 1) * S.fs;
     S.x = S.g + n;
     S.z = S.x + n;
     S.w = S.z + n;
     double *wr = S.w + n;                       // n weights of the prior rows
     double *x0 = wr + n;
     S.rs = x0 + n;
-    S.sval = S.rs + n;
+    S.l = S.rs + n;
+    S.sval = S.l + n + 1;
     S.P = (int *)(S.sval + 8);
     S.idx = S.P + n;
     S.blocked = S.idx + n;
-    S.sflag = S.blocked + n;
+    int *span = S.blocked + n;
+    S.sflag = span + 2 * n;
     const int nent = n * (n + 1) / 2;
     const double *ghk = gh + (size_t)k * (nent + n);
-    for (int e = tid; e < nent; e += blockDim.x) {
+    for (int e = tid; e < n * n; e += blockDim.x) {
         // packed upper row-major: row i holds (i, i..n-1)
-        int i = 0, rem = e;
-        while (rem >= n - i) {
-            rem -= n - i;
-            i++;
-        }
-        const int j = i + rem;
-        G[i * n + j] = ghk[e];
-        G[j * n + i] = ghk[e];
+        const int a = e / n, b = e - a * n, i = min(a, b), j = max(a, b);
+        G[e] = ghk[i * n - i * (i - 1) / 2 + j - i];
     }
     for (int j = tid; j < n; j += blockDim.x) {
         S.g[j] = ghk[nent + j];
         S.P[j] = p0[j];
+        span[2 * j] = n;
+        span[2 * j + 1] = -1;
     }
     __syncthreads();
     int st = 0;
     const int nrow = n - 2;
     if (!(pc.smooth != 0.0) || n < 3) {
-        build_H(S, G, lc, lv, wr, 0);
+        build_H(S, G, lc, lv, wr, 0, span);
         st = nnls(S);
     } else {
-        double traa = 0.0;
-        for (int j = 0; j < n; j++) traa += G[j * n + j];
-        const double srel = sqrt(0.1 * traa / fmax(pc.norm, 1e-300));
+        for (int i = tid; i < nrow; i += blockDim.x)
+            for (int a = 0; a < 3; a++) {
+                atomicMin(&span[2 * lc[3 * i + a]], i);
+                atomicMax(&span[2 * lc[3 * i + a] + 1], i);
+            }
+        if (tid < 32) {
+            double traa = 0.0;
+            for (int j = tid; j < n; j += 32) traa += G[j * n + j];
+            traa = warp_sum(traa);
+            if (tid == 0) S.sval[3] = sqrt(0.1 * traa / fmax(pc.norm, 1e-300));
+        }
+        __syncthreads();
+        const double srel = S.sval[3];
         for (int i = tid; i < nrow; i += blockDim.x) wr[i] = srel;
         __syncthreads();
-        build_H(S, G, lc, lv, wr, nrow);
+        build_H(S, G, lc, lv, wr, nrow, span);
         st = nnls(S);
         for (int j = tid; j < n; j += blockDim.x) x0[j] = S.x[j];
         __syncthreads();
         // the reduced chi2 of the first solution, sum (b - A x0)^2 = b.b - 2 x0.h + x0^T G x0: the terms of each a
-        // by a thread (S.w), then summed in the order of a by thread 0
+        // by a thread (S.w), then summed by a warp
         for (int a = tid; a < n; a += blockDim.x) {
             double r = 0.0;
-            for (int b = 0; b < n; b++) r += G[a * n + b] * x0[b];
+            for (int b = 0; b < n; b++) r += G[b * n + a] * x0[b];
             S.w[a] = x0[a] * r;
         }
         __syncthreads();
-        if (tid == 0) {
-            double xm = 0.0;
-            for (int j = 0; j < n - 1; j++) xm += x0[j];
-            xm /= (double)(n - 1);
-            S.sval[0] = xm;
-            double xh = 0.0, xgx = 0.0;
-            for (int a = 0; a < n; a++) {
+        if (tid < 32) {
+            double xm = 0.0, xh = 0.0, xgx = 0.0;
+            for (int a = tid; a < n; a += 32) {
+                if (a < n - 1) xm += x0[a];
                 xh += x0[a] * S.g[a];
                 xgx += S.w[a];
             }
-            const double chi2 = (pc.bb - 2.0 * xh + xgx) / fmax((double)(pc.m - n), 1.0);
-            const double corr = fmax(pc.corr, 1.0) * fmax(chi2, 1.0);
-            S.sval[1] = sqrt(corr) * pc.d * pc.d / pc.smooth;
-            S.sval[2] = sqrt(pc.floor_) * srel;
+            xm = warp_sum(xm) / (double)(n - 1);
+            xh = warp_sum(xh);
+            xgx = warp_sum(xgx);
+            if (tid == 0) {
+                S.sval[0] = xm;
+                const double chi2 = (pc.bb - 2.0 * xh + xgx) / fmax((double)(pc.m - n), 1.0);
+                const double corr = fmax(pc.corr, 1.0) * fmax(chi2, 1.0);
+                S.sval[1] = sqrt(corr) * pc.d * pc.d / pc.smooth;
+                S.sval[2] = sqrt(pc.floor_) * srel;
+            }
         }
         __syncthreads();
         if (S.sval[0] > 0) {
@@ -709,7 +764,7 @@ __global__ void __launch_bounds__(PS_THREADS) k_prof_solve(const double *__restr
         if (S.sval[0] > 0) {
             for (int j = tid; j < n; j += blockDim.x) S.P[j] = x0[j] > 0.0;
             __syncthreads();
-            build_H(S, G, lc, lv, wr, nrow);
+            build_H(S, G, lc, lv, wr, nrow, span);
             st |= nnls(S);
         }
     }
@@ -894,7 +949,9 @@ void launch_prof_gram64(cudaStream_t s, const double *A, const ProfBox &box, con
     prof_gram<double>(s, A, box, nullptr, nullptr, b, m, ent_i, ent_j, nent, 1, part, gh, KRows{});
 }
 
-size_t prof_solve_smem(int n) { return (size_t)(3 * n * n + 7 * n + 8) * sizeof(double) + (size_t)(4 * n + 8) * sizeof(int); }
+size_t prof_solve_smem(int n) {
+    return (size_t)(2 * n * n + (n + 1) * prof_solve_pitch(n) + 8 * n + 9) * sizeof(double) + (size_t)(5 * n + 8) * sizeof(int);
+}
 
 void launch_prof_solve(cudaStream_t s, const double *gh, const ProfConst &pc, const int *lc, const double *lv,
                        const int *ord, const unsigned char *near, const int *p0, int nb, double *x, int *pout,

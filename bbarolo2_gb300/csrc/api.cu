@@ -1022,10 +1022,12 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
         if ((rc = dgrow(ctx, &ctx->d_model_fx, &ctx->d_model_fx_cap, (size_t)nb * ctx->mstride))) return rc;
     CK(cudaMemcpyAsync(ctx->d_asub, ctx->h_asub, sizeof(AnSub) * (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_mem, ctx->h_mem, sizeof(MemberDev) * (size_t)nb, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_reuse, ctx->h_reuse, (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
-    launch_fill_copy(ctx->stream, ctx->d_asub, sizeof(AnSub), nsub, nb, ctx->d_reuse);
-    CKL();
-    ctx->h2d += (long long)((sizeof(AnSub) + 1) * (size_t)nb * nsub + sizeof(MemberDev) * (size_t)nb);
+    if (nb > 1) {
+        CK(cudaMemcpyAsync(ctx->d_reuse, ctx->h_reuse, (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
+        launch_fill_copy(ctx->stream, ctx->d_asub, sizeof(AnSub), nsub, nb, ctx->d_reuse);
+        CKL();
+    }
+    ctx->h2d += (long long)((sizeof(AnSub) + (nb > 1)) * (size_t)nb * nsub + sizeof(MemberDev) * (size_t)nb);
     ctx->uploaded = true;
     ctx->ran = false;
     return 0;
@@ -1128,10 +1130,12 @@ static int batch_prepare(bbgpu_ctx *ctx, int galmodtype, int nb, int nsub, const
     if ((rc = dgrow(ctx, &ctx->d_reuse, &ctx->d_reuse_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
     CK(cudaMemcpyAsync(ctx->d_sub, ctx->h_sub, sizeof(SubMC) * (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_mem, ctx->h_mem, sizeof(MemberDev) * (size_t)nb, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->d_reuse, ctx->h_reuse, (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
-    launch_fill_submc(ctx->stream, ctx->d_sub, nsub, nb, ctx->d_reuse, ctx->d_mem, g.nlines);
-    CKL();
-    ctx->h2d = (long long)((sizeof(SubMC) + 1) * (size_t)nb * nsub + sizeof(MemberDev) * (size_t)nb);
+    if (nb > 1) {
+        CK(cudaMemcpyAsync(ctx->d_reuse, ctx->h_reuse, (size_t)nb * nsub, cudaMemcpyHostToDevice, ctx->stream));
+        launch_fill_submc(ctx->stream, ctx->d_sub, nsub, nb, ctx->d_reuse, ctx->d_mem, g.nlines);
+        CKL();
+    }
+    ctx->h2d = (long long)((sizeof(SubMC) + (nb > 1)) * (size_t)nb * nsub + sizeof(MemberDev) * (size_t)nb);
     ctx->uploaded = true;
     ctx->ran = false;
     return 0;
@@ -1493,7 +1497,8 @@ static int mc_lists(bbgpu_ctx *ctx, cudaStream_t s, bool tm) {
     CKL();
     if (tm) CK(cudaEventRecord(ctx->ev[6], s));
     launch_mc_scatter(s, L, ctx->d_sub, ctx->nsub, ctx->d_mem, ctx->d_cstart, ctx->d_cseg, ctx->mc_nseg,
-                      ctx->mc_ntot, ctx->tx, ctx->ty, ctx->d_pix, ctx->d_tcur, ctx->d_bucket, 1);
+                      ctx->mc_ntot, ctx->tx, ctx->ty, ctx->d_pix, ctx->d_tcur, ctx->d_bucket,
+                      ctx->prof_uploaded ? 1 : 0);
     CKL();
     if (ctx->mc_records) {
         const MemberDev &M0 = ctx->mem_host[0];
@@ -1727,9 +1732,11 @@ static int batch_run(bbgpu_ctx *ctx, bool do_resid) {
             int rc = mc_lists(ctx, s, tm);
             if (rc) return rc;
         }
-        launch_entry_fix(s, ctx->d_sub, ctx->d_toff, ctx->d_tcount, ctx->ntile_total * NOWN, ctx->mc_ntot,
-                         ctx->d_bucket);
-        CKL();
+        if (ctx->prof_uploaded) {
+            launch_entry_fix(s, ctx->d_sub, ctx->d_toff, ctx->d_tcount, ctx->ntile_total * NOWN, ctx->mc_ntot,
+                             ctx->d_bucket);
+            CKL();
+        }
         if (tm) CK(cudaEventRecord(ctx->ev[7], s));
         if (ctx->mc_n2 || ctx->mc_n3) {
             launch_mc_deposit(s, g, L, ctx->d_sub, ctx->nsub, ctx->d_mem, ctx->mem_host.data(), ctx->nb, ctx->tx,
@@ -3225,9 +3232,11 @@ extern "C" int bbgpu_eval_upload_profile(bbgpu_ctx *ctx, int nsm, const double *
     if ((rc = dgrow(ctx, &ctx->d_ppart, &ctx->d_ppart_cap, (size_t)2 * nb * (npart ? npart : 1)))) return rc;
     if ((rc = dgrow(ctx, &ctx->d_preuse, &ctx->d_preuse_cap, (size_t)nb * nsm))) return rc;
     CK(cudaMemcpyAsync(ctx->d_psub, ctx->h_psub, sizeof(AnSub) * (size_t)nb * nsm, cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(ctx->d_preuse, ctx->h_preuse, (size_t)nb * nsm, cudaMemcpyHostToDevice, s));
-    launch_fill_copy(s, ctx->d_psub, sizeof(AnSub), nsm, nb, ctx->d_preuse);
-    CKL();
+    if (nb > 1) {
+        CK(cudaMemcpyAsync(ctx->d_preuse, ctx->h_preuse, (size_t)nb * nsm, cudaMemcpyHostToDevice, s));
+        launch_fill_copy(s, ctx->d_psub, sizeof(AnSub), nsm, nb, ctx->d_preuse);
+        CKL();
+    }
     CK(cudaMemcpyAsync(ctx->d_pwidx, wi.data(), sizeof(int) * wi.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(ctx->d_pwvalf, wvalf.data(), sizeof(float) * wvalf.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(ctx->d_pwval, wval, sizeof(double) * 2 * (size_t)nsm, cudaMemcpyHostToDevice, s));

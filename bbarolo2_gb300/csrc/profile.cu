@@ -9,7 +9,7 @@
 //                    (member, pixel, ring) ring-fastest in the likelihood box;
 //   k_maps_to_f32    x mean(cd2i) sum(relint) x scale factor, float32 (then the beam convolution of
 //                    k_conv_resid with the rings as channels);
-//   k_prof_gram      the normal equations of the weighted least squares: G = A^T A, h = A^T b over the pixels
+//   k_prof_gram_ff   the normal equations of the weighted least squares: G = A^T A, h = A^T b over the pixels
 //                    used (A = maps / rms), exact float64 products of the float32 maps, fixed-order sums;
 //   k_prof_solve     one CTA per member: solve_profile's two non-negative least-squares solves with the
 //                    smoothness prior, Lawson-Hanson on the normal equations (Cholesky of the passive set),
@@ -29,6 +29,7 @@
 
 #include "anpix.cuh"
 #include "devmath.cuh"
+#include "f32x2.cuh"
 #include "kernels.h"
 
 #define FULL 0xffffffffu
@@ -202,14 +203,12 @@ __global__ void k_prof_gather(const double *__restrict__ xu, const int *__restri
 
 // ------------------------------------------------------------------------------------------- Gram matrix
 // CTA (tile of GRAM_TP used pixels, member k). Entry e < n(n+1)/2: G[i][j] (i <= j, row-major packed upper),
-// then h[i]. The tile is staged in shared memory with the range of rings not zero at each pixel, so that each entry
-// sums its products over the band of rings that overlap there. Float32 maps: the maps as they are, the maps times
-// the pixel weights and the weighted data in float-float (hi + lo, about 46 bits), each product of a float-float and
-// a float32 map and its sum carried in float-float with error-free transformations (float32 units, no float64
-// pipe), the tile's sum converted to float64 at the end; float64 maps: float64 FMAs; the entries outside the union of the tile's bands (the used pixels come in compact blocks, so
-// the union is narrow) are zero without a loop. Partial sums per tile, summed over the tiles in order by
-// k_prof_gram_reduce.
+// then h[i]. The used pixels come in compact blocks, so that few rings have a pixel of a tile: the entries of the others
+// are zero without a loop. Float32 maps (k_prof_gram_ff): products and sums in float-float (hi + lo, about 46 bits)
+// with error-free transformations, no float64 pipe, the tile's sums converted to float64 at the end; float64 maps
+// (k_prof_gram): float64 FMAs. Partial sums per tile, summed over the tiles in order by k_prof_gram_reduce.
 // pix == nullptr: the pixels 0 .. npix_used - 1; wpix == nullptr: unit weights.
+
 // s = sh + sl += (xh + xl) b: the product by TwoProduct (the float32 product and its exact error) plus xl b, the
 // sum by TwoSum (operations rounded one by one: no contraction)
 __device__ __forceinline__ void ff_madd(float &sh, float &sl, float xh, float xl, float b) {
@@ -223,30 +222,9 @@ __device__ __forceinline__ void ff_madd(float &sh, float &sl, float xh, float xl
     sl = __fadd_rn(sl, __fadd_rn(err, e));
 }
 
-__device__ __forceinline__ void out_entry(double *part, int k, int t, int nent, int e, double v) {
-    part[((size_t)k * gridDim.x + t) * nent + e] = v;
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) k_prof_gram(const T *__restrict__ K, ProfBox box, const int *__restrict__ pix,
-                                                   const double *__restrict__ wpix, const double *__restrict__ wy,
-                                                   int npix_used, const int *__restrict__ ent_i,
-                                                   const int *__restrict__ ent_j, int nent,
-                                                   double *__restrict__ part, KRows kr) {
-    extern __shared__ double gsm[];
-    const int n = box.nrp;
-    constexpr bool FF = sizeof(T) == 4;
-    double *Kd = gsm;                                       // GRAM_TP x n maps
-    double *Kw = Kd + GRAM_TP * n;                          // GRAM_TP x n maps x pixel weight
-    double *wys = Kw + GRAM_TP * n;                         // GRAM_TP weighted data
-    float *Kf = (float *)gsm;                               // (FF: the maps; maps x weight, hi and lo; data, hi, lo)
-    float *Kwh = Kf + GRAM_TP * n, *Kwl = Kwh + GRAM_TP * n;
-    float *wyh = Kwl + GRAM_TP * n, *wyl = wyh + GRAM_TP;
-    int *lo = FF ? (int *)(wyl + GRAM_TP) : (int *)(wys + GRAM_TP), *hi = lo + GRAM_TP;   // rings not zero: lo .. hi
-    __shared__ int srow[GRAM_TP];                           // the row whose K holds each pixel
-    const int k = blockIdx.y, t = blockIdx.x;
-    const int p0 = t * GRAM_TP;
-    const int np = min(GRAM_TP, npix_used - p0);
+// The row whose K holds each pixel of the tile (srow); false if the tile has row 0's sums (gflag set).
+__device__ __forceinline__ bool gram_rows(const ProfBox &box, const int *__restrict__ pix, const KRows &kr, int k,
+                                          int t, int p0, int np, int *srow) {
     if (kr.ktab) {
         // a row's convolution left the tiles it shares with row 0 unwritten: K of row 0 there (the same values);
         // a tile of such pixels only has row 0's sums, taken by the reduction
@@ -275,40 +253,196 @@ __global__ void __launch_bounds__(256) k_prof_gram(const T *__restrict__ K, Prof
         own = __syncthreads_or(own);
         if (k != 0 && !own) {
             if (threadIdx.x == 0) kr.gflag[(size_t)k * gridDim.x + t] = 1;
-            return;
+            return false;
         }
         if (threadIdx.x == 0) kr.gflag[(size_t)k * gridDim.x + t] = 0;
     } else {
         for (int pp = threadIdx.x; pp < np; pp += blockDim.x) srow[pp] = k;
         __syncthreads();
     }
+    return true;
+}
+
+// (sh + sl) += (xh + xl) b for two b (packed float32 operations, each rounded by itself): the product by TwoProduct
+// (nxh, nxl = -xh, -xl: the error and the small term with their signs turned), the sum by TwoSum.
+__device__ __forceinline__ void ff_madd2(unsigned long long &sh, unsigned long long &sl, unsigned long long xh,
+                                         unsigned long long nxh, unsigned long long nxl, unsigned long long b) {
+    const unsigned long long m1 = f32x2(-1.0f, -1.0f);
+    const unsigned long long p = f32x2_mul(xh, b);
+    const unsigned long long ne = f32x2_fma(nxl, b, f32x2_fma(nxh, b, p));
+    const unsigned long long s = f32x2_add(sh, p);
+    const unsigned long long z = f32x2_fma(sh, m1, s);
+    const unsigned long long err = f32x2_add(f32x2_fma(f32x2_fma(z, m1, s), m1, sh), f32x2_fma(z, m1, p));
+    sh = s;
+    sl = f32x2_add(sl, f32x2_fma(ne, m1, err));
+}
+
+__device__ __forceinline__ int gram_pitch(int n) { return (n + 3) & ~3; }
+
+// The normal equations of float32 maps, a tile of GRAM_TP pixels a CTA: the maps, the maps times the pixel weights
+// (float-float) and the weighted data (float-float) in shared memory, the products and sums in float-float. Only the
+// rings that have a pixel of the tile enter (blo .. bhi): their 4 x 4 blocks on and above the diagonal go to the
+// threads, as many pixel groups as fit, 16 products for three 16-byte loads; the groups' sums are added in order. Only
+// what a pixel or an entry needs once touches the float64 pipe: the weights' halves and the final sums. 81 systems of 41
+// unknowns, 25600 pixels: 379 us (644 us with the weights split at every map value); an entry a thread with its pixels'
+// bands tested one by one, five loads a product, 650 us.
+__global__ void __launch_bounds__(256) k_prof_gram_ff(const float *__restrict__ K, ProfBox box,
+                                                      const int *__restrict__ pix, const double *__restrict__ wpix,
+                                                      const double *__restrict__ wy, int npix_used,
+                                                      const int *__restrict__ ent_i, const int *__restrict__ ent_j,
+                                                      int nent, double *__restrict__ part, KRows kr) {
+    extern __shared__ __align__(16) double gsm[];
+    __shared__ int srow[GRAM_TP], band[2];
+    __shared__ float2 pw[GRAM_TP];                          // the pixel weights, hi and lo
+    __shared__ long long soff[GRAM_TP];                     // each pixel's maps in K
+    __shared__ float2 hsum[256];
+    const int n = box.nrp, n4 = gram_pitch(n), tid = threadIdx.x;
+    float *Kf = (float *)gsm, *Kwh = Kf + GRAM_TP * n4, *Kwl = Kwh + GRAM_TP * n4;
+    float *wyh = Kwl + GRAM_TP * n4, *wyl = wyh + GRAM_TP;
+    const int k = blockIdx.y, t = blockIdx.x;
+    const int p0 = t * GRAM_TP;
+    const int np = min(GRAM_TP, npix_used - p0);
+    if (tid == 0) {
+        band[0] = n;
+        band[1] = -1;
+    }
+    if (!gram_rows(box, pix, kr, k, t, p0, np, srow)) return;
+    for (int i = tid; i < np; i += 256) {
+        const double w = wpix ? wpix[p0 + i] : 1.0, y = wy[p0 + i];
+        const float wh = (float)w, yh = (float)y;
+        pw[i] = make_float2(wh, (float)(w - (double)wh));
+        wyh[i] = yh;
+        wyl[i] = (float)(y - (double)yh);
+        soff[i] = ((long long)srow[i] * box.npix + (pix ? pix[p0 + i] : p0 + i)) * n;   // (this thread's srow)
+    }
+    __syncthreads();
+    int a = n, b = -1;
+    for (int r = tid & 31; r < n4; r += 32) {
+#pragma unroll 4
+        for (int pp = tid >> 5; pp < np; pp += 8) {
+            const int i = pp * n4 + r;
+            const float kv = r < n ? __ldg(K + soff[pp] + r) : 0.0f;
+            float ph = 0.0f, pl = 0.0f;
+            if (kv != 0.0f) {
+                // kv x w in float-float: kv x wh exactly (TwoProduct), plus kv x wl rounded
+                const float2 w = pw[pp];
+                ph = __fmul_rn(kv, w.x);
+                pl = __fadd_rn(__fmaf_rn(kv, w.x, -ph), __fmul_rn(kv, w.y));
+                a = min(a, r);
+                b = max(b, r);
+            }
+            Kf[i] = kv;
+            Kwh[i] = ph;
+            Kwl[i] = pl;
+        }
+    }
+    a = __reduce_min_sync(FULL, a);
+    b = __reduce_max_sync(FULL, b);
+    if ((tid & 31) == 0 && b >= a) {
+        atomicMin(&band[0], a);
+        atomicMax(&band[1], b);
+    }
+    __syncthreads();
+    const int blo = band[0], bhi = band[1], r0 = blo & ~3;
+    const int nk = bhi >= blo ? (bhi - r0) / 4 + 1 : 0, nblk = nk * (nk + 1) / 2;
+    const int nr = bhi - blo + 1;
+    // the blocks (bi, bj >= bi), row after row; a thread a block of a pixel group
+    int bi = 0, bj = 0;
+    const int ng = nblk ? 256 / nblk : 0, grp = nblk ? tid / nblk : 0;
+    unsigned long long sh[4][2], sl[4][2];
+#pragma unroll
+    for (int x = 0; x < 4; x++) sh[x][0] = sh[x][1] = sl[x][0] = sl[x][1] = 0ULL;
+    const bool on = grp < ng;
+    if (on) {
+        int left = tid - grp * nblk;
+        while (left >= nk - bi) {
+            left -= nk - bi;
+            bi++;
+        }
+        bj = bi + left;
+        const int oi = r0 + 4 * bi, oj = r0 + 4 * bj;
+        for (int pp = grp; pp < np; pp += ng) {
+            const float4 h = *(const float4 *)(Kwh + pp * n4 + oi), l = *(const float4 *)(Kwl + pp * n4 + oi);
+            const ulonglong2 f = *(const ulonglong2 *)(Kf + pp * n4 + oj);
+            const float hx[4] = {h.x, h.y, h.z, h.w}, lx[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const unsigned long long xh = f32x2(hx[x], hx[x]), nxh = f32x2(-hx[x], -hx[x]),
+                                         nxl = f32x2(-lx[x], -lx[x]);
+                ff_madd2(sh[x][0], sl[x][0], xh, nxh, nxl, f.x);
+                ff_madd2(sh[x][1], sl[x][1], xh, nxh, nxl, f.y);
+            }
+        }
+    }
+    // the right-hand side: a ring of a pixel group a thread
+    const int ngr = nr > 0 ? 256 / nr : 0, grr = nr > 0 ? tid / nr : 0;
+    if (grr < ngr) {
+        const int r = blo + tid - grr * nr;
+        float uh = 0.0f, ul = 0.0f;
+        for (int pp = grr; pp < np; pp += ngr) ff_madd(uh, ul, wyh[pp], wyl[pp], Kf[pp * n4 + r]);
+        hsum[tid] = make_float2(uh, ul);
+    }
+    __syncthreads();                                        // (the maps are done with: the sums take their place)
+    float2 *const red = (float2 *)gsm;                      // 16 x 256 (a thread's 16 sums)
+    if (on) {
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+#pragma unroll
+            for (int y = 0; y < 2; y++) {
+                float h0, h1, l0, l1;
+                f32x2_get(sh[x][y], h0, h1);
+                f32x2_get(sl[x][y], l0, l1);
+                red[(4 * x + 2 * y) * 256 + tid] = make_float2(h0, l0);
+                red[(4 * x + 2 * y + 1) * 256 + tid] = make_float2(h1, l1);
+            }
+    }
+    __syncthreads();
+    for (int e = tid; e < nent; e += 256) {
+        const int i = ent_i[e], j = ent_j[e];
+        const bool in = i >= blo && max(i, j) <= bhi;       // (an entry outside the tile's rings sums to zero)
+        double acc = 0.0;
+        if (in) {
+            const int ci = (i - r0) >> 2, cj = (j - r0) >> 2;
+            const float2 *q = j >= 0 ? red + (4 * (i & 3) + (j & 3)) * 256 + ci * nk - ci * (ci - 1) / 2 + cj - ci
+                                     : hsum + i - blo;
+            const int step = j >= 0 ? nblk : nr, m = j >= 0 ? ng : ngr;
+            float uh = 0.0f, ul = 0.0f;
+            for (int g = 0; g < m; g++) {
+                const float2 v = q[g * step];
+                ff_madd(uh, ul, v.x, v.y, 1.0f);
+            }
+            acc = (double)uh + (double)ul;
+        }
+        part[((size_t)k * gridDim.x + t) * nent + e] = acc;
+    }
+}
+
+// the same of float64 maps (a single system: a thread an entry), float64 FMAs over the band of rings that overlap
+__global__ void __launch_bounds__(256) k_prof_gram(const double *__restrict__ K, ProfBox box,
+                                                   const int *__restrict__ pix, const double *__restrict__ wpix,
+                                                   const double *__restrict__ wy, int npix_used,
+                                                   const int *__restrict__ ent_i, const int *__restrict__ ent_j,
+                                                   int nent, double *__restrict__ part, KRows kr) {
+    extern __shared__ __align__(16) double gsm[];
+    const int n = box.nrp;
+    double *Kd = gsm;                                       // GRAM_TP x n maps
+    double *Kw = Kd + GRAM_TP * n;                          // GRAM_TP x n maps x pixel weight
+    double *wys = Kw + GRAM_TP * n;                         // GRAM_TP weighted data
+    int *lo = (int *)(wys + GRAM_TP), *hi = lo + GRAM_TP;   // rings not zero: lo .. hi
+    __shared__ int srow[GRAM_TP];                           // the row whose K holds each pixel
+    const int k = blockIdx.y, t = blockIdx.x;
+    const int p0 = t * GRAM_TP;
+    const int np = min(GRAM_TP, npix_used - p0);
+    if (!gram_rows(box, pix, kr, k, t, p0, np, srow)) return;
+    __syncthreads();
     for (int i = threadIdx.x; i < np * n; i += blockDim.x) {
         const int pp = i / n, r = i - pp * n;
         const long long q = pix ? pix[p0 + pp] : p0 + pp;
-        const T kv = K[((size_t)srow[pp] * box.npix + q) * n + r];
-        const double w = wpix ? wpix[p0 + pp] : 1.0;
-        if constexpr (FF) {
-            // kv x w in float-float: kv x wh exactly (TwoProduct), plus kv x wl rounded
-            const float wh = (float)w, wl = (float)(w - (double)wh);
-            const float ph = __fmul_rn(kv, wh);
-            Kf[i] = kv;
-            Kwh[i] = ph;
-            Kwl[i] = __fadd_rn(__fmaf_rn(kv, wh, -ph), __fmul_rn(kv, wl));
-        } else {
-            Kd[i] = (double)kv;
-            Kw[i] = (double)kv * w;
-        }
+        const double kv = K[((size_t)srow[pp] * box.npix + q) * n + r];
+        Kd[i] = kv;
+        Kw[i] = kv * (wpix ? wpix[p0 + pp] : 1.0);
     }
-    for (int i = threadIdx.x; i < np; i += blockDim.x) {
-        if constexpr (FF) {
-            const double y = wy[p0 + i];
-            const float yh = (float)y;
-            wyh[i] = yh;
-            wyl[i] = (float)(y - (double)yh);
-        } else {
-            wys[i] = wy[p0 + i];
-        }
-    }
+    for (int i = threadIdx.x; i < np; i += blockDim.x) wys[i] = wy[p0 + i];
     __syncthreads();
     __shared__ int band[2];                                 // the tile's rings: band[0] .. band[1]
     if (threadIdx.x == 0) { band[0] = n; band[1] = -1; }
@@ -316,7 +450,7 @@ __global__ void __launch_bounds__(256) k_prof_gram(const T *__restrict__ K, Prof
     for (int pp = threadIdx.x; pp < np; pp += blockDim.x) {
         int a = n, b = -1;
         for (int r = 0; r < n; r++)
-            if (FF ? Kf[pp * n + r] != 0.0f : Kd[pp * n + r] != 0.0) {
+            if (Kd[pp * n + r] != 0.0) {
                 a = min(a, r);
                 b = r;
             }
@@ -333,21 +467,6 @@ __global__ void __launch_bounds__(256) k_prof_gram(const T *__restrict__ K, Prof
     for (int e = threadIdx.x; e < nent; e += blockDim.x) {
         const int i = ent_i[e], j = ent_j[e];
         double acc = 0.0;
-        if constexpr (FF) {
-            float sh = 0.0f, sl = 0.0f;
-            if (j >= 0) {
-                if (i >= blo && j <= bhi)
-                    for (int pp = 0; pp < np; pp++)
-                        if (lo[pp] <= i && j <= hi[pp])
-                            ff_madd(sh, sl, Kwh[pp * n + i], Kwl[pp * n + i], Kf[pp * n + j]);
-            } else {
-                if (i >= blo && i <= bhi)
-                    for (int pp = 0; pp < np; pp++)
-                        if (lo[pp] <= i && i <= hi[pp]) ff_madd(sh, sl, wyh[pp], wyl[pp], Kf[pp * n + i]);
-            }
-            out_entry(part, k, t, nent, e, (double)sh + (double)sl);
-            continue;
-        }
         if (j >= 0) {
             if (i >= blo && j <= bhi)                       // (an entry outside the tile's rings sums to zero)
                 for (int pp = 0; pp < np; pp++)
@@ -924,29 +1043,27 @@ void launch_prof_gather(cudaStream_t s, const double *xu, const int *stu, const 
 
 int prof_gram_tiles(int npix_used) { return (npix_used + GRAM_TP - 1) / GRAM_TP; }
 
-template <class T>
-static void prof_gram(cudaStream_t s, const T *K, const ProfBox &box, const int *pix, const double *wpix,
+void launch_prof_gram(cudaStream_t s, const float *K, const ProfBox &box, const int *pix, const double *wpix,
                       const double *wy, int npix_used, const int *ent_i, const int *ent_j, int nent, int nb,
                       double *part, double *gh, KRows kr) {
     const int nt = prof_gram_tiles(npix_used);
     if (nb == 0 || nt == 0) return;
-    const size_t smem = sizeof(T) == 4
-                            ? (size_t)(3 * GRAM_TP * box.nrp + 2 * GRAM_TP) * sizeof(float) + 2 * GRAM_TP * sizeof(int)
-                            : (size_t)(2 * GRAM_TP * box.nrp + GRAM_TP) * sizeof(double) + 2 * GRAM_TP * sizeof(int);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_prof_gram<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_prof_gram<T><<<dim3(nt, nb), 256, smem, s>>>(K, box, pix, wpix, wy, npix_used, ent_i, ent_j, nent, part, kr);
+    // (the maps, or the sums of 256 threads in their place)
+    const size_t smem = std::max((size_t)(3 * GRAM_TP * ((box.nrp + 3) & ~3) + 2 * GRAM_TP) * sizeof(float),
+                                 (size_t)256 * 16 * sizeof(double));
+    cudaFuncSetAttribute(k_prof_gram_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_prof_gram_ff<<<dim3(nt, nb), 256, smem, s>>>(K, box, pix, wpix, wy, npix_used, ent_i, ent_j, nent, part, kr);
     k_prof_gram_reduce<<<dim3((nent + 127) / 128, nb), 128, 0, s>>>(part, nt, nent, gh, kr.ktab ? kr.gflag : nullptr);
-}
-
-void launch_prof_gram(cudaStream_t s, const float *K, const ProfBox &box, const int *pix, const double *wpix,
-                      const double *wy, int npix_used, const int *ent_i, const int *ent_j, int nent, int nb,
-                      double *part, double *gh, KRows kr) {
-    prof_gram<float>(s, K, box, pix, wpix, wy, npix_used, ent_i, ent_j, nent, nb, part, gh, kr);
 }
 
 void launch_prof_gram64(cudaStream_t s, const double *A, const ProfBox &box, const double *b, int m, const int *ent_i,
                         const int *ent_j, int nent, double *part, double *gh) {
-    prof_gram<double>(s, A, box, nullptr, nullptr, b, m, ent_i, ent_j, nent, 1, part, gh, KRows{});
+    const int nt = prof_gram_tiles(m);
+    if (nt == 0) return;
+    const size_t smem = (size_t)(2 * GRAM_TP * box.nrp + GRAM_TP) * sizeof(double) + 2 * GRAM_TP * sizeof(int);
+    if (smem > 48 * 1024) cudaFuncSetAttribute(k_prof_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_prof_gram<<<dim3(nt, 1), 256, smem, s>>>(A, box, nullptr, nullptr, b, m, ent_i, ent_j, nent, part, KRows{});
+    k_prof_gram_reduce<<<dim3((nent + 127) / 128, 1), 128, 0, s>>>(part, nt, nent, gh, nullptr);
 }
 
 size_t prof_solve_smem(int n) {

@@ -1196,7 +1196,7 @@ void launch_an_model(cudaStream_t s, const GridDev &g, const AnSub *subs, int ns
     const long long nw = ntot;
     if (nw == 0 || nseg == 0) return;
     const size_t smem = an_smem_bytes(g.nz, g.nlines);
-    cudaFuncSetAttribute(k_an_model, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_an_model, smem);
     k_an_model<<<(unsigned)((nw + AN_WPB - 1) / AN_WPB), AN_WPB * 32, smem, s>>>(
         g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, astart, (const int4 *)aseg, nseg, ntot, zq,
         wq, zqf, vedges, cd2i, ptab, mem, (unsigned long long *)out64, mstride, skip_fast);
@@ -1210,7 +1210,7 @@ void launch_an_model_fast(cudaStream_t s, const GridDev &g, const AnSub *subs, i
     if (ntot == 0 || nseg == 0) return;
     const long long per = 32 * ANF_WPB;
     const size_t smem = ANF_WPB * (32 * sizeof(AnfSample) + ANF_RUNS * sizeof(int2)) + (PHI_N + (size_t)ANF_WPB * g.nz) * 4;
-    cudaFuncSetAttribute(k_an_model_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_an_model_fast, smem);
     k_an_model_fast<<<(unsigned)((ntot + per - 1) / per), ANF_WPB * 32, smem, s>>>(
         g, subs, nsub, sbase, ssub, (const double2 *)cs, (const float2 *)csf, (const float4 *)csff, astart,
         (const int4 *)aseg, nseg, ntot, zq, zqf, wqf, (const float2 *)vef, cd2if, ptabf, mem,
@@ -1248,7 +1248,7 @@ void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int n
     float *const top = amp + na;
     k_an_amps<<<(unsigned)((na + 255) / 256), 256, 0, s>>>(subs, nsub, mem, klist, n3, ng, chg, nchw, amp, top);
     const size_t smem = (size_t)2 * nsub * (ANR_MG + 1) * sizeof(float);
-    cudaFuncSetAttribute(k_an_replay, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_an_replay, smem);
     int per = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_an_replay, 256, smem);
     const int nc = std::max(1, std::min(152 * std::max(per, 1) / ng, (ntask + 7) / 8));
@@ -1290,7 +1290,7 @@ void launch_ant_pixel(cudaStream_t s, int nz, const int *pix0, int kfirst, int n
     const int nw = ant_warps(nz);
     if (nk <= 0 || npix <= 0 || !nw) return;
     const size_t smem = ant_smem(nz, nw);
-    cudaFuncSetAttribute(k_ant_pixel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_ant_pixel, smem);
     int per = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ant_pixel, 32 * nw, smem);
     k_ant_pixel<<<std::min((npix + nw - 1) / nw, 152 * std::max(per, 1)), 32 * nw, smem, s>>>(

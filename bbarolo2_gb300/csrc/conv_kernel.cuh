@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
                                                        float *__restrict__ smoothed, int do_conv, int do_resid,
                                                        double *__restrict__ partial, int npart, TileSrc ts) {
     extern __shared__ float sm[];
+    const bool all = do_conv & CONV_ALL_ROWS;
+    do_conv &= ~CONV_ALL_ROWS;
     constexpr int W = TO + KXW - 1;
     constexpr int TOY = TO * (32 / ZB);     // tile rows: 32 / ZB groups of lanes, 16 rows each
     const int k = blockIdx.x;
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
             v |= (q.x | q.y | q.z | q.w) << 1;
         }
         const bool some = __any_sync(0xffffffffu, v != 0);
-        if (lane == 0) rowf[r] = some;
+        if (lane == 0) rowf[r] = some || all;
         any |= some;
     }
     const int nonempty = __syncthreads_or(any);
@@ -295,11 +297,7 @@ void launch_t(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, in
     size_t smem = (size_t)(TOY + kye - 1) * (TO + KXW - 1) * ZB * sizeof(float) +
                   (size_t)(kye + 1) * ((KXW + 1) & ~1) * sizeof(float2) +
                   (size_t)(TOY + kye - 1) * sizeof(int);
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        cudaFuncSetAttribute(k_conv_resid<KXW, ZB, TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        configured = smem;
-    }
+    allow_smem((const void *)k_conv_resid<KXW, ZB, TS>, smem);
     dim3 grid(nb, maxt, nzb);
     k_conv_resid<KXW, ZB, TS><<<grid, 256, smem, s>>>(g, mem, model, mstride, nz, taps, ky, kx, smoothed, do_conv,
                                                  do_resid, partial, npart, ts);

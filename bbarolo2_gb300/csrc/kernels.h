@@ -49,6 +49,15 @@ struct ZigDev {
     double wn[128];
 };
 
+// Dynamic shared memory above 48 KB: the function's limit is set to all that its static arrays leave of the 227 KB of a
+// CTA, whatever this launch takes, so that host threads that launch one kernel with different sizes do not lower each
+// other's limit.
+inline void allow_smem(const void *f, size_t smem) {
+    cudaFuncAttributes a;
+    if (smem > 48 * 1024 && cudaFuncGetAttributes(&a, f) == cudaSuccess && a.maxDynamicSharedSizeBytes < (int)smem)
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
+}
+
 // ---- MC (mc.cu)
 // For every (member, cloud): its pixel in the member's box (or -1) and the count of clouds per tile.
 // Tile lists are split by pixel (NOWN per tile, tiles of at most 64 pixels): list index = (tile_off + tile) * NOWN
@@ -141,6 +150,7 @@ struct TileSrc {
     int *kout;
     int kstride;
 };
+#define CONV_ALL_ROWS 8      // (or-ed to do_conv: the rows of zeros are not left out)
 void launch_conv_resid(cudaStream_t s, const GridDev &g, const MemberDev *mem, const MemberDev *mem_host, int nb,
                        const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
                        float *smoothed, int do_conv, int do_resid, double *partial, TileSrc ts = TileSrc{nullptr, 0, 0, nullptr, 0});

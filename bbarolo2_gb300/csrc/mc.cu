@@ -1486,18 +1486,8 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
     if (maxt == 0 || nb == 0 || (klist && nk == 0)) return;
     size_t smem = (size_t)tx * ty * g.nz * sizeof(unsigned long long) + 16 + (size_t)8 * DEPTH * WB * sizeof(float) +
                   (size_t)g.nz * sizeof(float);
-    static size_t configured = 0;
-    if (smem > 48 * 1024 && smem > configured) {
-        cudaFuncSetAttribute(k_mc_deposit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        configured = smem;
-    }
     dim3 grid(klist ? nk : nb, maxt);
     if (lean && !model64) {
-        static size_t cfg_lean = 0;
-        if (smem > 48 * 1024 && smem > cfg_lean) {
-            cudaFuncSetAttribute(k_mc_deposit_lean, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            cfg_lean = smem;
-        }
         const int TP = tx * ty;
         if (TP == 64 || TP == 32) {
             // pixel-owned deposit: 8 (TP 64) or 4 (TP 32) pixels per warp
@@ -1511,11 +1501,7 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
             // 0.73 ms with 20, 1.05 ms with 32)
 #define PX(LPP, SPL)                                                                                                  \
     {                                                                                                                 \
-        static size_t cfg = 0;                                                                                        \
-        if (smem_px > 48 * 1024 && smem_px > cfg) {                                                                   \
-            cudaFuncSetAttribute(k_mc_deposit_px<LPP, SPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_px);\
-            cfg = smem_px;                                                                                            \
-        }                                                                                                             \
+        allow_smem((const void *)k_mc_deposit_px<LPP, SPL>, smem_px);                                                 \
         k_mc_deposit_px<LPP, SPL><<<grid, 256, smem_px, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count,             \
                                                              (const Entry *)bucket, zig, cd2if, model, mstride,       \
                                                              klist, delta, b64, tsrc, rp, err);                       \
@@ -1531,10 +1517,12 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
 #undef PX
             return;
         }
+        allow_smem((const void *)k_mc_deposit_lean, smem);
         k_mc_deposit_lean<<<grid, 256, smem, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count, (const Entry *)bucket,
                                                  zig, cd2if, model, mstride, err);
         return;
     }
+    allow_smem((const void *)k_mc_deposit, smem);
     k_mc_deposit<<<grid, 256, smem, s>>>(g, L, sub, nsub, mem, tx, ty, offset, count, (const Entry *)bucket, zig, cd2if,
                                         cd2i, model, mstride, model64, err);
 }

@@ -10,9 +10,9 @@
 //   k_maps_to_f32    x mean(cd2i) sum(relint) x scale factor, float32 (then the beam convolution of
 //                    k_conv_resid with the rings as channels);
 //   k_prof_gram_ff   the normal equations of the weighted least squares: G = A^T A, h = A^T b over the pixels
-//                    used (A = maps / rms), exact float64 products of the float32 maps, fixed-order sums;
+//                    used (A = maps / rms), float-float products and sums of the float32 maps in a fixed order;
 //   k_prof_solve     one CTA per member: solve_profile's two non-negative least-squares solves with the
-//                    smoothness prior, Lawson-Hanson on the normal equations (Cholesky of the passive set),
+//                    smoothness prior, Lawson-Hanson on the normal equations (L D L^T of the passive set),
 //                    warm-started from a passive set;
 //   k_mc_dens        the densities of the model's sub-rings (ring weights) into the MC sub-ring constants
 //                    (flux per sub-cloud, fixed-point deposits and exponent), checking the cloud layout;
@@ -20,7 +20,7 @@
 //
 // The maps need float32 accuracy only: the system is well conditioned (cond(A) ~ 1e2 on the 160x160x128
 // workload) and float32 map errors move the densities by ~1e-8; the Gram matrix squares the condition number
-// and is therefore accumulated in float64.
+// and is therefore accumulated with about 46 bits.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -1051,7 +1051,7 @@ void launch_prof_gram(cudaStream_t s, const float *K, const ProfBox &box, const 
     // (the maps, or the sums of 256 threads in their place)
     const size_t smem = std::max((size_t)(3 * GRAM_TP * ((box.nrp + 3) & ~3) + 2 * GRAM_TP) * sizeof(float),
                                  (size_t)256 * 16 * sizeof(double));
-    cudaFuncSetAttribute(k_prof_gram_ff, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_prof_gram_ff, smem);
     k_prof_gram_ff<<<dim3(nt, nb), 256, smem, s>>>(K, box, pix, wpix, wy, npix_used, ent_i, ent_j, nent, part, kr);
     k_prof_gram_reduce<<<dim3((nent + 127) / 128, nb), 128, 0, s>>>(part, nt, nent, gh, kr.ktab ? kr.gflag : nullptr);
 }
@@ -1061,7 +1061,7 @@ void launch_prof_gram64(cudaStream_t s, const double *A, const ProfBox &box, con
     const int nt = prof_gram_tiles(m);
     if (nt == 0) return;
     const size_t smem = (size_t)(2 * GRAM_TP * box.nrp + GRAM_TP) * sizeof(double) + 2 * GRAM_TP * sizeof(int);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_prof_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_prof_gram, smem);
     k_prof_gram<<<dim3(nt, 1), 256, smem, s>>>(A, box, nullptr, nullptr, b, m, ent_i, ent_j, nent, part, KRows{});
     k_prof_gram_reduce<<<dim3((nent + 127) / 128, 1), 128, 0, s>>>(part, nt, nent, gh, nullptr);
 }
@@ -1075,7 +1075,7 @@ void launch_prof_solve(cudaStream_t s, const double *gh, const ProfConst &pc, co
                        int *status) {
     if (nb == 0) return;
     const size_t smem = prof_solve_smem(pc.n);
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_prof_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem((const void *)k_prof_solve, smem);
     k_prof_solve<<<nb, PS_THREADS, smem, s>>>(gh, pc, lc, lv, ord, near, p0, x, pout, status);
 }
 

@@ -10,18 +10,17 @@
 //   k_wind_rawbox    one warp per cell: the pixels and channels that its points reach (windmodel.py:291-319), from the
 //                    extreme positions and velocities;
 //   (host)           offsets of the raw boxes and of the beam-grown boxes: one read of ncell x 6 integers;
-//   k_wind_deposit   one warp per point, lanes over channels: the channel-integrated line (the tabulated normal
-//                    CDF) times the bilinear weights of the four nearest pixels, added to the raw box of the cell
-//                    (float64 atomics; windmodel.py:322-366);
-//   k_wind_conv_*    one thread per voxel of a box: the beam convolution of each raw box into its grown box, as
-//                    two 1D passes for a separable beam, else with the 2D kernel, each sum in the reference's order
-//                    (windmodel.py:369-423);
+//   k_wind_deposit_cell  a CTA per cell, a thread per point: the channel-integrated line (the tabulated normal CDF)
+//                    times the bilinear weights of the four nearest pixels, added to the raw box of the cell in shared
+//                    memory (64-bit fixed point; windmodel.py:322-366), a box too large for it in global memory;
+//   k_wind_conv_*    the beam convolution of each raw box into its grown box in float-float, as two 1D passes with
+//                    eight outputs a thread for a separable beam, else with the 2D kernel (windmodel.py:369-423);
 //   k_wind_lists     the voxel lists of the reference (windmodel.py:477-527): the entries (A != 0, |A| >= rel x
 //                    the peak of the column, W != 0) counted per voxel, offsets by a scan, then written;
-//   k_wind_lists_gram  one warp per voxel: b[k] += A_k Wd and G[k, l] += W A_k A_l over the pairs of its entries
-//                    (windmodel.py:530-554), float64 atomics.
-// Everything is float64, as the reference. The sums differ from the reference's sequential sums by rounding only
-// (the deposits' order is not fixed, and the reductions are trees).
+//   k_wind_lists_gram  b[k] += A_k Wd and G[k, l] += W A_k A_l over the pairs of a voxel's entries, the pairs over the
+//                    lanes (windmodel.py:530-554), float64 atomics.
+// Everything is float64, as the reference, but the convolution (float-float, about 1e-14). The sums differ from the
+// reference's sequential sums by rounding only (the reductions are trees).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

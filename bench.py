@@ -694,7 +694,7 @@ def galwind_leg(args, dist, world, cpu=True):
     """GALWIND WTYPE 1 (the Monte-Carlo shells of a bi-cone, ``galwind.GalWindMC``) on a 128x128x64 cube of 4"
     pixels and 10 km/s channels: CONELEN 240" (80 shells 3" apart), OPENANG 60, VWIND 300, VDISP 20 km/s, DENS 10,
     CDENS 20, NV 20, INC 60, PHI 45, 16 chunks of shells (THREADS 16): the model's wall time through the public API
-    (streams parsed on host threads, clouds placed and deposited on the device, the cube read back). The CPU leg: the
+    (streams followed on the device, clouds placed and deposited there, the cube read back). The CPU leg: the
     oracle (the reference's _galmod_wind restated in C, one thread) over the same chunks; parity: the two models."""
     from bbarolo2_gb300.cube import Cube, Params
     from bbarolo2_gb300.galwind import GalWindMC, GalWindPars

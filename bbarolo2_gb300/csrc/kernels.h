@@ -49,12 +49,13 @@ struct ZigDev {
     double wn[128];
 };
 
-// Dynamic shared memory above 48 KB: the function's limit is set to all that its static arrays leave of the 227 KB of a
-// CTA, whatever this launch takes, so that host threads that launch one kernel with different sizes do not lower each
-// other's limit.
+// A launch with smem bytes of dynamic shared memory: above 48 KB with the function's static arrays, its limit is set to
+// all that they leave of the 227 KB of a CTA, whatever this launch takes, so that host threads that launch one kernel
+// with different sizes do not lower each other's limit.
 inline void allow_smem(const void *f, size_t smem) {
     cudaFuncAttributes a;
-    if (smem > 48 * 1024 && cudaFuncGetAttributes(&a, f) == cudaSuccess && a.maxDynamicSharedSizeBytes < (int)smem)
+    if (smem > 4 * 1024 && cudaFuncGetAttributes(&a, f) == cudaSuccess && a.sharedSizeBytes + smem > 48 * 1024 &&
+        a.maxDynamicSharedSizeBytes < 227 * 1024 - (int)a.sharedSizeBytes)
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
 }
 

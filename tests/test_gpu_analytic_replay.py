@@ -8,15 +8,20 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nz, nb", [(1, 10), (31, 10), (32, 17), (33, 18), (64, 34), (100, 12)])
-@pytest.mark.parametrize("z0, nr", [(12., 8), (4., 1), (25., 3)])
+@pytest.mark.parametrize("z0, nr", [(12., 8), (4., 1), (25., 3), (6., 90)])
 def test_replayed_members(gpu_lib, nz, nb, z0, nr):
     from bbarolo2_gb300 import _lib, configs, engine
     from bbarolo2_gb300.cube import Cube, Params
     from bbarolo2_gb300.galmod import ring_rows_batch
+    from bbarolo2_gb300.rings import Rings
     par = Params(CDENS=10, ISEED=1, LTYPE=2, galmodtype="ANALYTIC")
     cube = Cube.empty(37, 41, nz, [-10. / 3600., 10. / 3600., 5.], beam=30. / 3600., par=par,
                       crpix=[19., 21., nz / 2 + 1.], crval=[60., 0., 1000.], cunit=("deg", "deg", "km/s"))
     _, rings = configs.classic64(galmodtype="ANALYTIC")
+    if nr > rings.nr:                                        # (amplitudes that take more than 48 KB of shared memory)
+        r = 4. + 8. * np.arange(nr)
+        rings = Rings().setRings(radii=r, vsys=1000., vrot=150. * (1 - np.exp(-r / 40.)), vdisp=10., inc=55., phi=45.,
+                                 dens=np.exp(-r / 60.))
     rings = rings.subset(list(range(nr)))
     rings.xpos[:], rings.ypos[:], rings.z0[:] = 18., 20., z0
     dm = engine.DiskModel(cube)
@@ -29,6 +34,7 @@ def test_replayed_members(gpu_lib, nz, nb, z0, nr):
         for k in range(4, nb):
             rows[k, 12 if k % 2 else 13, k % nr] += 3.       # (INC or PA of one ring)
     sr, nv, descs, boxes = like.prepare(rows, rings, seed=1)
+    assert nr <= 8 or sr.shape[2] > 75
     out = {}
     try:
         for share in (0, 1):

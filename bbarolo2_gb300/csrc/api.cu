@@ -1517,15 +1517,15 @@ static bool conv_tc_ok(const bbgpu_ctx *ctx, int v, const TileSrc &ts) {
            (!ts.tsrc || ts.shx >= 3) && !ts.kout;
 }
 
-static int conv_run(bbgpu_ctx *ctx, cudaStream_t s, int v, bool conv, bool do_resid, TileSrc ts, int flags = 0);
+static int conv_run(bbgpu_ctx *ctx, cudaStream_t s, int v, bool conv, bool do_resid, TileSrc ts);
 
 // The variant of the batch convolution: the option's, or (option -1) the autotuner's for this kernel and these
 // channels. The autotuner runs the batch's convolution with each candidate (float32; tf32x3 where the kernel and the
 // channels qualify) on the batch in hand, twice each, times the second run with events, and keeps the faster for the
-// context's lifetime: every later batch with the same kernel shape and channels gets the same arithmetic. The float32
-// kernel is timed with the rows of zeros that it would leave out (how many there are is the first batch's alone, the
-// choice is not) and a tenth is added: a shape's choice, and with it the bits of its results, stays what it was before
-// the kernel staged its tiles a row at a time (1.0 to 1.25 times faster where both qualify).
+// context's lifetime: every later batch with the same kernel shape and channels gets the same arithmetic. What is
+// timed is what runs. For these shapes the float32 kernel is the one without ROWS: with ROWS it is up to 1.25 times
+// faster and has the same bits, but the choice moved (73 of 1904 shapes of 32 to 200 pixels, 32 to 160 channels and
+// kernels of 9x7 to 15x15, log L off by 1e-6), and a shape keeps the arithmetic that it had.
 static int conv_variant_of(bbgpu_ctx *ctx, cudaStream_t s, bool conv, bool do_resid, TileSrc ts, int &v) {
     v = ctx->conv_variant;
     if (v >= 0 || !conv) {
@@ -1550,7 +1550,7 @@ static int conv_variant_of(bbgpu_ctx *ctx, cudaStream_t s, bool conv, bool do_re
         float ms = 0.f;
         for (int rep = 0; rep < 2 && !rc; rep++) {
             cudaEventRecord(e0, s);
-            rc = conv_run(ctx, s, cand, conv, do_resid, ts, CONV_ALL_ROWS);
+            rc = conv_run(ctx, s, cand, conv, do_resid, ts);
             cudaEventRecord(e1, s);
         }
         if (rc) break;
@@ -1559,9 +1559,8 @@ static int conv_variant_of(bbgpu_ctx *ctx, cudaStream_t s, bool conv, bool do_re
             break;
         }
         ctx->tune_ms[cand] = ms;
-        const float cost = cand ? ms : 1.1f * ms;
-        if (cost < bms) {
-            bms = cost;
+        if (ms < bms) {
+            bms = ms;
             best = cand;
         }
     }
@@ -1583,15 +1582,15 @@ static int conv_batch(bbgpu_ctx *ctx, cudaStream_t s, bool conv, bool do_resid, 
 }
 
 // the convolution with variant v: on the tensor cores (1 bf16x3, 2 tf32x3) when the kernel, the channels and the tile
-// table qualify, else the float32 kernel
-static int conv_run(bbgpu_ctx *ctx, cudaStream_t s, int v, bool conv, bool do_resid, TileSrc ts, int flags) {
+// table qualify, else the float32 kernel (ROWS where there is no choice by time to make)
+static int conv_run(bbgpu_ctx *ctx, cudaStream_t s, int v, bool conv, bool do_resid, TileSrc ts) {
     const GridDev &g = ctx->g;
     float *smoothed = ctx->keep_smoothed ? ctx->d_smooth : nullptr;
     const bool tc = conv && conv_tc_ok(ctx, v, ts);
     if (!tc) {
         launch_conv_resid(s, g, ctx->d_mem, ctx->mem_host.data(), ctx->nb, ctx->d_model, ctx->mstride, g.nz,
-                          ctx->d_taps, ctx->ky, ctx->kx, ctx->kxw, smoothed, conv ? 1 | flags : 0,
-                          do_resid ? 1 : 0, ctx->d_partial, ts);
+                          ctx->d_taps, ctx->ky, ctx->kx, ctx->kxw, smoothed, conv ? 1 : 0, do_resid ? 1 : 0,
+                          ctx->d_partial, ts, ctx->conv_variant >= 0 || !conv_tc_ok(ctx, 2, ts));
         CKL();
         ctx->npart_used = conv_resid_npart(ctx->mem_host.data(), ctx->nb, g.nz);
         ctx->conv_used = 0;

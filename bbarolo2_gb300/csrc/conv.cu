@@ -11,9 +11,10 @@
 // memory). The epilogue applies the reference's threshold (values below 1e-12 set to zero) and flux scale,
 // and, instead of writing the smoothed cube, compares it with the data: each CTA leaves the sum of squared
 // residuals of its voxels (and the sum of log-variances for a fractional model error), reduced in float64.
-// Input rows that are all zero in the tile's channels (each channel holds a part of the disk) are left out of the
-// sums; the two output rows of a thread are the halves of packed FMAs. 61 models of 101x97x75, kernel 15x15: 0.76 ->
-// 0.56 ms (packed FMAs alone 0.75); ring maps of 160 steps, 40 maps of 160x160, kernel 9x9 wide: 0.71 -> 0.58 ms.
+// With ROWS, input rows that are all zero in the tile's channels (each channel holds a part of the disk) are left out
+// of the sums and the two output rows of a thread are the halves of packed FMAs. 61 models of 101x97x75, kernel 15x15:
+// 0.76 -> 0.56 ms (packed FMAs alone 0.75); ring maps of 160 steps, 40 maps of 160x160, kernel 9x9 wide: 0.71 -> 0.58
+// ms. Without it: tiles that are all zero skip the convolution.
 
 #include "conv_kernel.cuh"
 
@@ -86,7 +87,7 @@ int conv_resid_npart(const MemberDev *mem_host, int nb, int nz) {
 
 void launch_conv_resid(cudaStream_t s, const GridDev &g, const MemberDev *mem, const MemberDev *mem_host, int nb,
                        const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
-                       float *smoothed, int do_conv, int do_resid, double *partial, TileSrc ts) {
+                       float *smoothed, int do_conv, int do_resid, double *partial, TileSrc ts, bool rows) {
     int maxt, nzb;
     conv_grid(mem_host, nb, nz, maxt, nzb);
     if (nb == 0 || maxt == 0) return;
@@ -94,29 +95,14 @@ void launch_conv_resid(cudaStream_t s, const GridDev &g, const MemberDev *mem, c
     if (!do_conv) kxw = 1;
     const bool z16 = conv_zb(nz) == 16;
     if (kxw == 0) {            // a kernel wider than the templates: taps (ky, kx) in global memory
-        launch_conv_wide(s, g, mem, nb, maxt, nzb, z16, model, mstride, nz, taps, ky, kx, smoothed,
-                         do_conv & ~CONV_ALL_ROWS, do_resid, partial, npart, ts);
+        launch_conv_wide(s, g, mem, nb, maxt, nzb, z16, model, mstride, nz, taps, ky, kx, smoothed, do_conv, do_resid,
+                         partial, npart, ts);
         return;
     }
-    if (ts.tsrc) {
-        launch_conv_table(s, g, mem, nb, maxt, nzb, z16, model, mstride, nz, taps, ky, kx, kxw, smoothed, do_conv,
-                          do_resid, partial, npart, ts);
-        return;
-    }
-#define CASE(W)                                                                                                    \
-    case W:                                                                                                        \
-        if (z16)                                                                                                   \
-            launch_t<W, 16, false>(s, g, mem, nb, maxt, nzb, model, mstride, nz, taps, ky, kx, smoothed, do_conv,  \
-                                   do_resid, partial, npart, ts);                                                  \
-        else                                                                                                       \
-            launch_t<W, 32, false>(s, g, mem, nb, maxt, nzb, model, mstride, nz, taps, ky, kx, smoothed, do_conv,  \
-                                   do_resid, partial, npart, ts);                                                  \
-        break;
-    switch (kxw) {
-        CASE(1) CASE(3) CASE(5) CASE(7) CASE(9) CASE(11) CASE(13) CASE(15) CASE(17) CASE(21) CASE(25) CASE(31)
-        default: break;
-    }
-#undef CASE
+    auto launch = ts.tsrc ? (rows ? launch_conv_table : launch_conv_timed_table)
+                          : (rows ? launch_widths<false, true> : launch_conv_timed);
+    launch(s, g, mem, nb, maxt, nzb, z16, model, mstride, nz, taps, ky, kx, kxw, smoothed, do_conv, do_resid, partial,
+           npart, ts);
 }
 
 void launch_reduce_partials(cudaStream_t s, const double *partial, int npart, int nb, double *out2) {

@@ -28,16 +28,17 @@ __device__ __forceinline__ void cp_async_zfill4(float *dst, const float *src, bo
 
 // TS: the model of a pixel is looked up in a tile table (TileSrc): the table entries of the CTA's input region
 // are staged in shared memory, and when they all name one member the tile is read from that member's model.
+// ROWS: the tile is staged a row a warp and its rows of zeros are left out of the sums, two output rows a packed FMA.
+// The same sums in the same order without it, and the same bits; without it are the shapes whose float32 kernel is
+// chosen by its time against the tensor cores' (launch_conv_resid).
 #define TS_MAX 256
-template <int KXW, int ZB, bool TS>
+template <int KXW, int ZB, bool TS, bool ROWS>
 __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDev *__restrict__ mem,
                                                        const float *__restrict__ model, long long mstride, int nz,
                                                        const float *__restrict__ taps, int ky, int kx,
                                                        float *__restrict__ smoothed, int do_conv, int do_resid,
                                                        double *__restrict__ partial, int npart, TileSrc ts) {
     extern __shared__ float sm[];
-    const bool all = do_conv & CONV_ALL_ROWS;
-    do_conv &= ~CONV_ALL_ROWS;
     constexpr int W = TO + KXW - 1;
     constexpr int TOY = TO * (32 / ZB);     // tile rows: 32 / ZB groups of lanes, 16 rows each
     const int k = blockIdx.x;
@@ -54,21 +55,28 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
     const int hy = ky_eff / 2, hx = kx_eff / 2;
     const int H = TOY + ky_eff - 1, ncol = TO + kx_eff - 1;
     float *S = sm;                          // H x W x ZB
-    // row i: (tap of kernel row i, tap of kernel row i - 1) for i = 0 .. ky, KXWP pairs a row (16-byte rows)
+    // the taps, ky x KXW; with ROWS row i: (tap of kernel row i, tap of kernel row i - 1) for i = 0 .. ky, KXWP pairs a
+    // row (16-byte rows)
     constexpr int KXWP = (KXW + 1) & ~1;
-    float2 *sk = (float2 *)(sm + (size_t)H * W * ZB);
-    int *rowf = (int *)(sk + (ky_eff + 1) * KXWP);          // H flags: the row has a value other than zero
+    float *sk1 = sm + (size_t)H * W * ZB;
+    float2 *sk = (float2 *)sk1;
+    int *rowf = (int *)(sk + (ky_eff + 1) * KXWP);          // (ROWS) H flags: the row has a value other than zero
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ch = lane % ZB, grp = lane / ZB;
     const int y0 = (t / ntx) * TOY, x0 = (t % ntx) * TO;
     const int z = zb * ZB + ch;
     const bool zok = z < nz;
-    if (do_conv)
-        for (int i = threadIdx.x; i < (ky + 1) * KXWP; i += blockDim.x) {
-            const int r = i / KXWP, b = i - r * KXWP;
-            sk[i] = b >= KXW ? make_float2(0.0f, 0.0f)
-                             : make_float2(r < ky ? taps[r * KXW + b] : 0.0f, r > 0 ? taps[(r - 1) * KXW + b] : 0.0f);
-        }
+    if (do_conv) {
+        if constexpr (ROWS)
+            for (int i = threadIdx.x; i < (ky + 1) * KXWP; i += blockDim.x) {
+                const int r = i / KXWP, b = i - r * KXWP;
+                sk[i] = b >= KXW
+                            ? make_float2(0.0f, 0.0f)
+                            : make_float2(r < ky ? taps[r * KXW + b] : 0.0f, r > 0 ? taps[(r - 1) * KXW + b] : 0.0f);
+            }
+        else
+            for (int i = threadIdx.x; i < ky * KXW; i += blockDim.x) sk1[i] = taps[i];
+    }
     const float *mk = model + (size_t)k * mstride;
     // the model of the pixel (yy, xx): the member's own, or, with a tile table, that of the member whose model
     // holds the pixel's deposit tile (member 0's for the tiles a member shares with it)
@@ -115,24 +123,44 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
         return model + (size_t)(i < TS_MAX ? tsm[i] : __ldg(&ts.tsrc[M.tile_off + (yy >> ts.shy) * M.ntx +
                                                                        (xx >> ts.shx)])) * mstride;
     };
-    // the input tile with its halo, asynchronously, a row a warp at a time: 16-byte copies of 4 channels when the
-    // rows of channels are 16-byte aligned (nz a multiple of 4), else 4-byte copies; zeros outside the box and past nz
+    // the input tile with its halo, asynchronously (ROWS: a row a warp at a time): 16-byte copies of 4 channels when
+    // the rows of channels are 16-byte aligned (nz a multiple of 4), else 4-byte copies; zeros outside the box and past
+    // nz
     const bool vec = (nz & 3) == 0 && (((uintptr_t)mk) & 15) == 0;
-    const int lpx = vec ? ZB / 4 : ZB, ppi = 32 / lpx;      // lanes a pixel, pixels an instruction
-    const int zl = vec ? 4 * (lane % lpx) : lane % lpx, c0 = lane / lpx;
-    const bool zin = zb * ZB + zl < nz;
-    for (int r = warp; r < H; r += NW) {
-        const int yy = y0 - hy + r;
-        const bool rok = zin && yy >= 0 && yy < M.by;
-        const long long off = ((long long)yy * M.bx + x0 - hx) * nz + zb * ZB + zl;
-        float *dst = S + (size_t)r * W * ZB + zl;
+    if constexpr (ROWS) {
+        const int lpx = vec ? ZB / 4 : ZB, ppi = 32 / lpx;      // lanes a pixel, pixels an instruction
+        const int zl = vec ? 4 * (lane % lpx) : lane % lpx, c0 = lane / lpx;
+        const bool zin = zb * ZB + zl < nz;
+        for (int r = warp; r < H; r += NW) {
+            const int yy = y0 - hy + r;
+            const bool rok = zin && yy >= 0 && yy < M.by;
+            const long long off = ((long long)yy * M.bx + x0 - hx) * nz + zb * ZB + zl;
+            float *dst = S + (size_t)r * W * ZB + zl;
 #pragma unroll 4
-        for (int col = c0; col < W; col += ppi) {
-            const int xx = x0 - hx + col;
-            const bool ok = rok && col < ncol && xx >= 0 && xx < M.bx;
-            const float *from = ok ? src(yy, xx) + off + (long long)col * nz : mk;
-            if (vec) cp_async_zfill16(dst + col * ZB, from, ok);
-            else cp_async_zfill4(dst + col * ZB, from, ok);
+            for (int col = c0; col < W; col += ppi) {
+                const int xx = x0 - hx + col;
+                const bool ok = rok && col < ncol && xx >= 0 && xx < M.bx;
+                const float *from = ok ? src(yy, xx) + off + (long long)col * nz : mk;
+                if (vec) cp_async_zfill16(dst + col * ZB, from, ok);
+                else cp_async_zfill4(dst + col * ZB, from, ok);
+            }
+        }
+    } else if (vec) {
+        for (int c = threadIdx.x; c < H * W * (ZB / 4); c += blockDim.x) {
+            const int q = c & (ZB / 4 - 1), rc = c / (ZB / 4);
+            const int r = rc / W, col = rc - r * W;
+            const int yy = y0 - hy + r, xx = x0 - hx + col, zz = zb * ZB + 4 * q;
+            const bool ok = col < ncol && yy >= 0 && yy < M.by && xx >= 0 && xx < M.bx && zz < nz;
+            cp_async_zfill16(S + (size_t)rc * ZB + 4 * q, ok ? src(yy, xx) + ((size_t)yy * M.bx + xx) * nz + zz : mk,
+                             ok);
+        }
+    } else {
+        for (int c = threadIdx.x; c < H * W * ZB; c += blockDim.x) {
+            const int l = c & (ZB - 1), rc = c / ZB;
+            const int r = rc / W, col = rc - r * W;
+            const int yy = y0 - hy + r, xx = x0 - hx + col, zz = zb * ZB + l;
+            const bool ok = col < ncol && yy >= 0 && yy < M.by && xx >= 0 && xx < M.bx && zz < nz;
+            cp_async_zfill4(S + c, ok ? src(yy, xx) + ((size_t)yy * M.bx + xx) * nz + zz : mk, ok);
         }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -151,18 +179,33 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
         }
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncwarp();
-    // the rows that are all zero (empty channels, the outside of the disk): they add nothing to the sums
+    // the rows (without ROWS: the tile) that are all zero (empty channels, the outside of the disk): they add nothing
+    // to the sums
     bool any = false;
-    for (int r = warp; r < H; r += NW) {
-        unsigned v = 0;
-        for (int c = lane; c < W * ZB / 4; c += 32) {
-            const uint4 q = *(const uint4 *)(S + (size_t)r * W * ZB + 4 * c);
-            v |= (q.x | q.y | q.z | q.w) << 1;
+    if constexpr (ROWS) {
+        __syncwarp();
+        for (int r = warp; r < H; r += NW) {
+            unsigned v = 0;
+            for (int c = lane; c < W * ZB / 4; c += 32) {
+                const uint4 q = *(const uint4 *)(S + (size_t)r * W * ZB + 4 * c);
+                v |= (q.x | q.y | q.z | q.w) << 1;
+            }
+            const bool some = __any_sync(0xffffffffu, v != 0);
+            if (lane == 0) rowf[r] = some;
+            any |= some;
         }
-        const bool some = __any_sync(0xffffffffu, v != 0);
-        if (lane == 0) rowf[r] = some || all;
-        any |= some;
+    } else {
+        __syncthreads();
+        unsigned v = 0;
+        if (vec) {
+            for (int c = threadIdx.x; c < H * W * (ZB / 4); c += blockDim.x) {
+                const uint4 q = *(const uint4 *)(S + (size_t)c * 4);
+                v |= (q.x | q.y | q.z | q.w) << 1;
+            }
+        } else {
+            for (int c = threadIdx.x; c < H * W * ZB; c += blockDim.x) v |= __float_as_uint(S[c]) << 1;
+        }
+        any = v != 0;
     }
     const int nonempty = __syncthreads_or(any);
     float acc[2][TO];
@@ -171,10 +214,33 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
 #pragma unroll
         for (int x = 0; x < TO; x++) acc[rr][x] = 0.0f;
     if (nonempty) {
-        if (do_conv) {
-            // input row ty0 + i feeds output row ty0 with kernel row i and output row ty0 + 1 with kernel row
-            // i - 1: each input row is read from shared memory once (the sums run over the kernel rows in order),
-            // and the two output rows are the halves of packed FMAs (the first and the last input row feed one)
+        // input row ty0 + i feeds output row ty0 with kernel row i and output row ty0 + 1 with kernel row i - 1: each
+        // input row is read from shared memory once (the sums run over the kernel rows in order)
+        if (do_conv && !ROWS) {
+            for (int i = 0; i <= ky; i++) {
+                const float *row = S + (size_t)((ty0 + i) * W) * ZB + ch;
+                float win[W];
+#pragma unroll
+                for (int j = 0; j < W; j++) win[j] = row[j * ZB];
+                if (i < ky) {
+#pragma unroll
+                    for (int b = 0; b < KXW; b++) {
+                        const float kv = sk1[i * KXW + b];
+#pragma unroll
+                        for (int x = 0; x < TO; x++) acc[0][x] = fmaf(kv, win[x + b], acc[0][x]);
+                    }
+                }
+                if (i > 0) {
+#pragma unroll
+                    for (int b = 0; b < KXW; b++) {
+                        const float kv = sk1[(i - 1) * KXW + b];
+#pragma unroll
+                        for (int x = 0; x < TO; x++) acc[1][x] = fmaf(kv, win[x + b], acc[1][x]);
+                    }
+                }
+            }
+        } else if (do_conv) {
+            // (the two output rows are the halves of packed FMAs; the first and the last input row feed one)
             const float *col = S + (size_t)(ty0 * W) * ZB + ch;
             auto filled = [&](int i) {
                 return ZB == 32 ? rowf[2 * warp + i] != 0 : (rowf[2 * warp + i] | rowf[16 + 2 * warp + i]) != 0;
@@ -288,19 +354,40 @@ __global__ void __launch_bounds__(256, 2) k_conv_resid(GridDev g, const MemberDe
     }
 }
 
-template <int KXW, int ZB, bool TS>
+template <int KXW, int ZB, bool TS, bool ROWS>
 void launch_t(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, int maxt, int nzb, const float *model,
               long long mstride, int nz, const float *taps, int ky, int kx, float *smoothed, int do_conv,
               int do_resid, double *partial, int npart, TileSrc ts) {
     const int kye = do_conv ? ky : 1;
     constexpr int TOY = TO * (32 / ZB);
     size_t smem = (size_t)(TOY + kye - 1) * (TO + KXW - 1) * ZB * sizeof(float) +
-                  (size_t)(kye + 1) * ((KXW + 1) & ~1) * sizeof(float2) +
-                  (size_t)(TOY + kye - 1) * sizeof(int);
-    allow_smem((const void *)k_conv_resid<KXW, ZB, TS>, smem);
+                  (ROWS ? (size_t)(kye + 1) * ((KXW + 1) & ~1) * sizeof(float2) + (size_t)(TOY + kye - 1) * sizeof(int)
+                        : (size_t)ky * KXW * sizeof(float));
+    allow_smem((const void *)k_conv_resid<KXW, ZB, TS, ROWS>, smem);
     dim3 grid(nb, maxt, nzb);
-    k_conv_resid<KXW, ZB, TS><<<grid, 256, smem, s>>>(g, mem, model, mstride, nz, taps, ky, kx, smoothed, do_conv,
-                                                 do_resid, partial, npart, ts);
+    k_conv_resid<KXW, ZB, TS, ROWS><<<grid, 256, smem, s>>>(g, mem, model, mstride, nz, taps, ky, kx, smoothed, do_conv,
+                                                           do_resid, partial, npart, ts);
+}
+
+// (kxw: a width of KXWS in conv.cu)
+template <bool TS, bool ROWS>
+void launch_widths(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, int maxt, int nzb, bool z16,
+                   const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
+                   float *smoothed, int do_conv, int do_resid, double *partial, int npart, TileSrc ts) {
+#define CASE(W)                                                                                                       \
+    case W:                                                                                                           \
+        if (z16)                                                                                                      \
+            launch_t<W, 16, TS, ROWS>(s, g, mem, nb, maxt, nzb, model, mstride, nz, taps, ky, kx, smoothed, do_conv,  \
+                                      do_resid, partial, npart, ts);                                                  \
+        else                                                                                                          \
+            launch_t<W, 32, TS, ROWS>(s, g, mem, nb, maxt, nzb, model, mstride, nz, taps, ky, kx, smoothed, do_conv,  \
+                                      do_resid, partial, npart, ts);                                                  \
+        break;
+    switch (kxw) {
+        CASE(1) CASE(3) CASE(5) CASE(7) CASE(9) CASE(11) CASE(13) CASE(15) CASE(17) CASE(21) CASE(25) CASE(31)
+        default: break;
+    }
+#undef CASE
 }
 
 }  // namespace

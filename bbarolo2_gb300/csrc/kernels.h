@@ -151,14 +151,22 @@ struct TileSrc {
     int *kout;
     int kstride;
 };
-#define CONV_ALL_ROWS 8      // (or-ed to do_conv: the rows of zeros are not left out)
+// (rows: the rows of zeros of a tile are left out, the kernel's ROWS)
 void launch_conv_resid(cudaStream_t s, const GridDev &g, const MemberDev *mem, const MemberDev *mem_host, int nb,
                        const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
-                       float *smoothed, int do_conv, int do_resid, double *partial, TileSrc ts = TileSrc{nullptr, 0, 0, nullptr, 0});
-// (the tile-table variant, conv_table.cu: maxt tiles and nzb channel blocks of ZB = 16 (z16) or 32 channels)
+                       float *smoothed, int do_conv, int do_resid, double *partial,
+                       TileSrc ts = TileSrc{nullptr, 0, 0, nullptr, 0}, bool rows = true);
+// (its variants with the tile table, conv_table.cu, and without rows, conv_timed.cu and conv_timed_table.cu: maxt tiles
+// and nzb channel blocks of ZB = 16 (z16) or 32 channels)
 void launch_conv_table(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, int maxt, int nzb, bool z16,
                        const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
                        float *smoothed, int do_conv, int do_resid, double *partial, int npart, TileSrc ts);
+void launch_conv_timed(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, int maxt, int nzb, bool z16,
+                       const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
+                       float *smoothed, int do_conv, int do_resid, double *partial, int npart, TileSrc ts);
+void launch_conv_timed_table(cudaStream_t s, const GridDev &g, const MemberDev *mem, int nb, int maxt, int nzb, bool z16,
+                             const float *model, long long mstride, int nz, const float *taps, int ky, int kx, int kxw,
+                             float *smoothed, int do_conv, int do_resid, double *partial, int npart, TileSrc ts);
 void launch_reduce_partials(cudaStream_t s, const double *partial, int npart, int nb, double *out2);
 // (conv_wide.cu: kernels wider than the templates, kxw = 0 in launch_conv_resid; the taps (ky, kx) flipped)
 void conv_wide_taps(const double *k, int ky, int kx, float *taps);

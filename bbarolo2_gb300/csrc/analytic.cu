@@ -1031,12 +1031,11 @@ __device__ __host__ inline int ant_pitch(int nz) { return (nz + 3) & ~1; }     /
 // The pixels of the members [kfirst, kfirst + nk) (numbered pix0[kfirst] .. pix0[kfirst + nk)), a pixel a warp:
 // persistent, so that the CDF table is read into shared memory once. 32 samples at a time are gathered a lane each; of
 // a sample, a lane takes an edge of the line (its upper edge is the next lane's: 31 channels a step), always of a
-// channel that is the lane's number modulo 32, so that no lane touches another's sums. Bound by issue (about 90
-// instructions a step): 256 members of 256x256x192 7.3 ms (8.8 ms with 4-byte writes), where tiles of pixels with
-// shared-memory atomics, the samples' edges laid end to end, took 8.9 ms. A pixel without samples, four in five, is only
-// written. base64:
-// member 0's sums in its box, written with base_out (by a launch of member 0 alone), else added to the members with
-// mbase >= 0.
+// channel that is the lane's number modulo 32, so that no lane adds to another's sums; the 16-byte writes take four
+// neighbouring sums a lane, behind a warp barrier. Bound by issue (about 90 instructions a step): 256 members of
+// 256x256x192 7.3 ms (8.8 ms with 4-byte writes), where tiles of pixels with shared-memory atomics, the samples' edges
+// laid end to end, took 8.9 ms. A pixel without samples, four in five, is only written. base64: member 0's sums in its
+// box, written with base_out (by a launch of member 0 alone), else added to the members with mbase >= 0.
 __global__ void __launch_bounds__(ANT_NT) k_ant_pixel(int nz, const int *__restrict__ pix0, int kfirst, int nk,
                                                       const int *__restrict__ offset, const int *__restrict__ count,
                                                       const int *__restrict__ order,
@@ -1090,6 +1089,7 @@ __global__ void __launch_bounds__(ANT_NT) k_ant_pixel(int nz, const int *__restr
                 }
             }
         }
+        __syncwarp();                                       // (a 16-byte write takes the sums of four lanes)
         const MemberDev &M = mem[k];
         const long long at = (long long)(t - pix0[k]) * nz;
         const long long *bas = !base_out && mbase[k] >= 0 ? base64 : nullptr;

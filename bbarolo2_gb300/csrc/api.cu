@@ -254,7 +254,7 @@ struct bbgpu_ctx {
     uint8_t *d_cmask = nullptr;
     double *d_cnoise = nullptr, *h_cpix = nullptr;
     size_t d_cdata_cap = 0, d_cmask_cap = 0, d_cnoise_cap = 0, h_cpix_cap = 0;
-    int cny = 0, cnx = 0;
+    int cny = 0, cnx = 0, cnz = 0;
     void *d_wsjump = nullptr;             // GALWIND's streams: the jumps of k_ws_gen, the ziggurat's fn
     CUtensorMap *d_tmaps = nullptr;       // per member: TMA descriptor of its model
     int *d_tcq = nullptr;                 // the next work item of a tensor-core convolution launch
@@ -785,6 +785,7 @@ extern "C" int bbgpu_set_grid(bbgpu_ctx *ctx, const bbgpu_grid *gr, const double
     ctx->zcache.clear();
     ctx->samp_key.clear();
     ctx->prof_set = ctx->prof_uploaded = false;
+    ctx->cny = ctx->cnx = ctx->cnz = 0;                  // (a CLASSIC fit's data are of the old grid)
     ctx->grid_set = true;
     ctx->uploaded = ctx->ran = false;
     return BBGPU_OK;
@@ -2816,6 +2817,7 @@ extern "C" int bbgpu_classic_set(bbgpu_ctx *ctx, const float *data, const uint8_
     CK(cudaSetDevice(ctx->device));
     const size_t n = (size_t)dny * dnx * nz;
     int rc;
+    ctx->cny = ctx->cnx = ctx->cnz = 0;                  // (until the new data are there)
     if ((rc = dgrow(ctx, &ctx->d_cdata, &ctx->d_cdata_cap, n)) || (rc = dgrow(ctx, &ctx->d_cmask, &ctx->d_cmask_cap, n)) ||
         (rc = dgrow(ctx, &ctx->d_cnoise, &ctx->d_cnoise_cap, (size_t)nz)))
         return rc;
@@ -2825,6 +2827,7 @@ extern "C" int bbgpu_classic_set(bbgpu_ctx *ctx, const float *data, const uint8_
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->cny = dny;
     ctx->cnx = dnx;
+    ctx->cnz = nz;
     return BBGPU_OK;
 }
 
@@ -2842,7 +2845,7 @@ extern "C" int bbgpu_classic_residual(bbgpu_ctx *ctx, const double *sr, int nsub
     const int bsx = bhi0 - blo0, bsy = bhi1 - blo1, nz = ctx->g.nz;
     if (!sr || !nv || !out || nsub < 0 || blo0 < 0 || blo1 < 0 || bsx < 0 || bsy < 0 || ky < 0 || kx < 0 || (ky && !kernel))
         return fail(ctx, BBGPU_ERR_ARG, "classic_residual: invalid arguments");
-    if (!ctx->d_cdata) return fail(ctx, BBGPU_ERR_STATE, "classic_residual before classic_set");
+    if (!ctx->cnz || ctx->cnz != nz) return fail(ctx, BBGPU_ERR_STATE, "classic_residual before classic_set of this grid");
     if (bhi0 > ctx->cnx || bhi1 > ctx->cny) return fail(ctx, BBGPU_ERR_ARG, "classic_residual: box outside the data");
     CK(cudaSetDevice(ctx->device));
     *out = INFINITY;

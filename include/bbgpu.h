@@ -137,7 +137,8 @@ int bbgpu_residuals_fracerr(bbgpu_ctx *ctx, const double *model, const float *da
                             int maskmode, const uint8_t *region, int nz, int ny, int nx, double sigma2,
                             double eps2, double *out2);
 /* CLASSIC evaluations of one fit (Galfit.getFuncValue, bbarolo/galfit.py:736-749): the data and mask (dny, dnx, nz)
- * and the channel noise, then per trial ring its MC model, sparse convolution and _norm in one call. */
+ * and the channel noise (of the grid in hand: set_grid drops them), then per trial ring its MC model, sparse convolution
+ * and _norm in one call. */
 int bbgpu_classic_set(bbgpu_ctx *ctx, const float *data, const uint8_t *mask, int dny, int dnx, int nz,
                       const double *chan_noise);
 int bbgpu_classic_residual(bbgpu_ctx *ctx, const double *sr, int nsub, uint64_t seed, const int64_t *nv, int blo0,

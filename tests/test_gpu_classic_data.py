@@ -1,0 +1,53 @@
+"""The data that a CLASSIC evaluation is compared with: those of the grid in hand and of the call."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _fit(seed):
+    from bbarolo2_gb300 import classic, configs
+    from golden.cases import galfit_par
+    cube, rings = configs.classic64()
+    g = np.random.default_rng(seed)
+    data = g.normal(0., 0.05, cube.array.shape).astype(np.float32)
+    data[20:44] += 0.2
+    cube.array = data
+    par = galfit_par()
+    par.NORM, par.NORMALCUBE = "LOCAL", False
+    return classic.ClassicFit(cube, rings, par, 0.05, g.random(data.shape) < 0.7)
+
+
+def test_data_of_another_grid_are_refused(gpu_lib):
+    from bbarolo2_gb300 import _lib
+    fit = _fit(1)
+    fit.run(rings=[])
+    st, ctx = fit.model.setup, fit.ctx
+    sr, nv = st.subrings(fit.inr)
+    sr, nv = np.ascontiguousarray(sr, np.float64), np.ascontiguousarray(nv, np.int64)
+
+    def residual():
+        out = np.zeros(1)
+        rc = ctx.L.bbgpu_classic_residual(ctx.h, _lib.ptr(sr), sr.shape[1], ctypes.c_uint64(1), _lib.ptr(nv), 0, 0, 64,
+                                          64, None, 0, 0, 1.0, 32., 32., 45., 60., 0., 10., 1., 0, 2, 0.05, 1., 0,
+                                          _lib.ptr(out))
+        return rc, out[0]
+
+    rc, value = residual()
+    assert rc == _lib.OK and np.isfinite(value)
+    grid = fit.model._grid()
+    edges = np.asarray(st._vedges_lines, float).reshape(-1)
+    args = [_lib.ptr(st.cd2i), _lib.ptr(st.lfreq0), _lib.ptr(st.relint), _lib.ptr(edges)]
+    ctx.check(ctx.L.bbgpu_set_grid(ctx.h, grid, *args))
+    assert residual()[0] == _lib.ERR_STATE                   # (the same grid set anew)
+    more = np.concatenate([st.cd2i, st.cd2i])
+    wide = np.concatenate([edges, edges[-1] + np.arange(1, st.nsubs + 1) * (edges[-1] - edges[-2])])
+    grid.nz = 2 * st.nsubs
+    ctx.check(ctx.L.bbgpu_set_grid(ctx.h, grid, _lib.ptr(more), args[1], args[2], _lib.ptr(wide)))
+    assert residual()[0] == _lib.ERR_STATE                   # (more channels than the data have)
+    fit.model.ctx.check(ctx.L.bbgpu_set_grid(ctx.h, fit.model._grid(), *args))
+    fit.run(rings=[])
+    rc, again = residual()
+    assert rc == _lib.OK and again == value

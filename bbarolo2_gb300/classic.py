@@ -286,6 +286,20 @@ class ClassicFit:
     def _residual(self, dring, data_yxz, noise, normtype):
         """The CLASSIC residual of the model of one ring (``Galfit.getFuncValue``, ``bbarolo/galfit.py:736-749``):
         its MC model and sparse convolution on the device, then ``_norm`` on the device."""
+        self._upload(data_yxz)
+        return self._trial(dring, data_yxz, noise, normtype)
+
+    def _upload(self, data_yxz):
+        """The data, mask and channel noise that the trials compare with, on the device (``run`` uploads them once)."""
+        data, mask = np.ascontiguousarray(data_yxz, np.float32), np.ascontiguousarray(self.mask_yxz, bool)
+        chan_noise = np.ascontiguousarray(self.chan_noise, np.float64)
+        if mask.size < data.size or chan_noise.size < data.shape[2]:
+            raise ValueError("the mask or the channel noise is smaller than the data")
+        self.ctx.check(self.ctx.L.bbgpu_classic_set(self.ctx.h, _lib.ptr(data), _lib.ptr(mask.view(np.uint8)),
+                                                    *data.shape, _lib.ptr(chan_noise)))
+
+    def _trial(self, dring, data_yxz, noise, normtype):
+        """``_residual`` against the data of the last ``_upload`` (data_yxz: the same)."""
         m, st, p = self.model, self.model.setup, self.par
         blo, bhi = m.box(dring)
         if st.galmodtype != "MC":
@@ -329,7 +343,7 @@ class ClassicFit:
         for i, k in enumerate(self.free):
             x[i] = into_bounds(k, x[i], self.limits[k], float(getattr(self.inr, k)[ir]), draw)
             getattr(dring, k)[:] = x[i]
-        value = self._residual(dring, data_yxz, noise, normtype)
+        value = self._trial(dring, data_yxz, noise, normtype)
         self.log[ir].append((x.copy(), value))
         return value, x
 
@@ -344,11 +358,7 @@ class ClassicFit:
             noise = noise * scaling
         data_yxz = np.ascontiguousarray(np.asarray(data, np.float32).transpose(1, 2, 0))
         normtype = NORMCODE[self.norms[stage - 1]]
-        dny, dnx, nz = data_yxz.shape
-        chan_noise = np.ascontiguousarray(self.chan_noise, np.float64)
-        self.ctx.check(self.ctx.L.bbgpu_classic_set(self.ctx.h, _lib.ptr(data_yxz),
-                                                    _lib.ptr(self.mask_yxz.view(np.uint8)), dny, dnx, nz,
-                                                    _lib.ptr(chan_noise)))
+        self._upload(data_yxz)
         nr = self.inr.nr
         start = self.par.STARTRAD if self.par.STARTRAD < nr else 0
         order = list(range(start, nr)) if rings is None else list(rings)

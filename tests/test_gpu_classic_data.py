@@ -51,3 +51,25 @@ def test_data_of_another_grid_are_refused(gpu_lib):
     fit.run(rings=[])
     rc, again = residual()
     assert rc == _lib.OK and again == value
+
+
+@pytest.mark.parametrize("change", ["data", "mask", "chan_noise"])
+def test_residual_takes_what_it_is_given(gpu_lib, change):
+    """Other data, another mask or noise than the last run's: the value of a fit that ran with them."""
+    from bbarolo2_gb300 import classic
+    a, b = _fit(1), _fit(2)
+    if change != "data":
+        b.cube.array = a.cube.array
+    if change != "mask":
+        b.mask_yxz, b.mask2d = a.mask_yxz, a.mask2d
+    if change == "chan_noise":
+        b.chan_noise = np.linspace(1., 3., 64)
+    ring = classic.ring_annulus(a.inr, 4)
+    yxz = [np.ascontiguousarray(f.cube.array.transpose(1, 2, 0)) for f in (a, b)]
+    for f in (a, b):
+        f.par.FTYPE = 1                                      # (the residual that the noise weights)
+        f.run(rings=[])
+    va, vb = a._residual(ring, yxz[0], 0.05, 0), b._residual(ring, yxz[1], 0.05, 0)
+    assert va != vb
+    a.mask_yxz, a.chan_noise = b.mask_yxz, b.chan_noise
+    assert a._residual(ring, yxz[1], 0.05, 0) == vb

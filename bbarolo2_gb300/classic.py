@@ -310,7 +310,7 @@ class ClassicFit:
                          self.chan_noise, noise, float(p.BWEIGHT), normtype, None, None, None, None, None, 0, 0.,
                          ctx=self.ctx)
         sr, nv = (a[0] for a in subrings_batch(st, dring, ring_rows_batch([dring])))
-        k = m.cfield
+        k = None if m.cfield is None else np.ascontiguousarray(m.cfield, np.float64)
         out = np.empty(1)
         self.ctx.check(self.ctx.L.bbgpu_classic_residual(
             self.ctx.h, _lib.ptr(sr), sr.shape[1], seed32(st.iseed) & 0xFFFFFFFFFFFFFFFF, _lib.ptr(nv), blo[0], blo[1],

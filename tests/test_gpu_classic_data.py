@@ -73,3 +73,20 @@ def test_residual_takes_what_it_is_given(gpu_lib, change):
     assert va != vb
     a.mask_yxz, a.chan_noise = b.mask_yxz, b.chan_noise
     assert a._residual(ring, yxz[1], 0.05, 0) == vb
+
+
+def test_kernel_of_any_layout(gpu_lib):
+    """A beam kernel that is not C-contiguous."""
+    from bbarolo2_gb300 import classic
+    fit = _fit(3)
+    k = np.array(fit.model.cfield)
+    k[0] *= 0.25                                             # (not its own transpose)
+    ring = classic.ring_annulus(fit.inr, 3)
+    data = np.ascontiguousarray(fit.cube.array.transpose(1, 2, 0))
+    fit.run(rings=[])
+    fit.model.cfield = k
+    want = fit._residual(ring, data, 0.05, 0)
+    fit.model.cfield = np.asfortranarray(k)
+    assert fit._residual(ring, data, 0.05, 0) == want
+    fit.model.cfield = k.T
+    assert fit._residual(ring, data, 0.05, 0) != want

@@ -2275,7 +2275,7 @@ static int wind_clouds_run(bbgpu_ctx *ctx, std::vector<WindClouds> &chunks, DevB
 // The clouds of the chunks with their streams followed on the device (galwind.cu), M draws a cloud: rounds of at most
 // WS_WORDS words (0.5 GB), a chunk that is longer continued in the next. The words asked for leave 4% for the
 // deviates that take more than one (3.6% on average); a chunk that needs more takes another round. Of the words 2.75%
-// leave the ziggurat's one-word path: room for 4%.
+// leave the ziggurat's one-word path: room for 4%. 1: the model is the host parse's to make (err of launch_ws_words).
 #define WS_WORDS (64 << 20)
 #define WS_MIN 20000
 static int wind_stream_run(bbgpu_ctx *ctx, const std::vector<WindClouds> &chunks,
@@ -2394,7 +2394,7 @@ static int wind_stream_run(bbgpu_ctx *ctx, const std::vector<WindClouds> &chunks
         CK(cudaMemcpyAsync(ends.data(), d_end, sizeof(WsStart) * njob, cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        if (err) return fail(ctx, BBGPU_ERR_KERNEL, "galmod_wind: a velocity deviate could not be followed");
+        if (err) return 1;
         left = false;
         for (int j = 0; j < njob; j++) {
             Point &p = pt[chunk[j]];
@@ -2444,11 +2444,13 @@ static int wind_mc_run(bbgpu_ctx *ctx, double *out, bool cube, const double *sr,
     if (!B.get(&R.acc, sizeof(uint64_t) * R.n) || !B.get(&d_out, cube ? sizeof(double) * R.n : 8))
         return fail(ctx, BBGPU_ERR_NOMEM, "galmod_wind: device allocation failed");
     CK(cudaMemsetAsync(R.acc, 0, sizeof(uint64_t) * R.n, s));
-    int rc = 0;
     // (from WS_MIN draws on the device's dozen launches cost less than the host's 15 ns a draw and its uploads)
+    int rc = 1;
     if (same && M <= WS_MAXM && ncl * M >= WS_MIN) {
         rc = wind_stream_run(ctx, W, first, law, seed0, M, B, R);
-    } else {
+        if (rc == 1) CK(cudaMemsetAsync(R.acc, 0, sizeof(uint64_t) * R.n, s));
+    }
+    if (rc == 1) {
         // the chunks' streams parsed on host threads (each chunk its own stream), then one device pass
         std::vector<int> err(nch, 0);
         const int nt = std::max(1, std::min(threads, nch));

@@ -17,10 +17,11 @@
 // Otherwise (other counts, a handful of draws) the host parses the stream into the clouds and their deviates
 // (bbh_wind_clouds) and k_wind_mc places them.
 //
-// A cloud is placed with the reference's float64 operations in its order, no contraction (from the host parse its
-// pixel is the reference's; from the device's sin and cos its position is within an ulp or two of it), and deposited
-// in 64-bit fixed point (units 2^(E-62), 2^E above the total flux of the clouds: exact sums, independent of their
-// order).
+// A cloud is placed with the reference's float64 operations in its order, no contraction, and deposited in 64-bit fixed
+// point (units 2^(E-62), 2^E above the total flux of the clouds: exact sums, independent of their order). From the host
+// parse its pixel and channels are the reference's. On the device sin, cos, log and exp are within two ulps of the C
+// library's: where that could move a pixel, a channel or a deviate's rejection, the launch says so (WS_NEAR) and the
+// host parse makes the model, so that the same holds (about one model of 2.2 M clouds in a hundred thousand).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -149,6 +150,16 @@ __global__ void __launch_bounds__(128) k_ws_gen(const WindJob *__restrict__ jobs
     if (seg0 + lane < nseg) nfail[seg0 + lane] = cnt;
 }
 
+// v within 2^-20 of the middle between two integers (|v| < 2^31: one addition leaves 20 bits of the fraction)
+__device__ __forceinline__ bool ws_close(double v) {
+    return ((unsigned)__double2loint(__dadd_rn(v, 6442450944.0)) & 0xfffffu) - 0x7ffffu <= 2u;
+}
+// ... within tol, for which sin and cos 3.4e-16 off the C library's are enough: they move a cloud of radius rad by less
+// than 5e-15 rad
+__device__ __noinline__ bool ws_near(double v, double pos, double rad, double cdelt) {
+    return fabs(__dsub_rn(__dsub_rn(v, floor(v)), 0.5)) < 1e-14 * (fabs(pos) + 4.0 * rad / fabs(cdelt));
+}
+
 // the positions of the failing words, in order: a thread a mask
 __global__ void k_ws_list(const unsigned *__restrict__ masks, int nmask, const int *__restrict__ foff,
                           unsigned *__restrict__ fpos, int cap, int *__restrict__ err) {
@@ -159,7 +170,7 @@ __global__ void k_ws_list(const unsigned *__restrict__ masks, int nmask, const i
     for (int q = 0; q < t; q++) o += __popc(masks[seg * (WS_SEG / 32) + q]);
     for (unsigned m = masks[i]; m; m &= m - 1, o++) {
         if (o < cap) fpos[o] = (unsigned)i * 32 + __ffs(m) - 1;
-        else *err = 1;
+        else atomicOr(err, WS_LOST);
     }
 }
 
@@ -176,6 +187,12 @@ __global__ void k_ws_slow(const unsigned *__restrict__ fpos, const int *__restri
     double val = 0.0;
     const unsigned end = min(nword, p + 200u);              // (a deviate beyond 200 words does not occur)
     auto next = [&]() { return q < end ? words[q++] : (q++, 0ULL); };
+    // (a < b of values that may each be a few ulps off)
+    bool near = false;
+    auto less = [&](double a, double b) {
+        near |= fabs(__dsub_rn(a, b)) <= 1e-14 * fabs(b);
+        return a < b;
+    };
     for (;;) {
         int hv;
         const bool fast = ws_fast(next(), zig->kn, hv);
@@ -188,17 +205,18 @@ __global__ void k_ws_slow(const unsigned *__restrict__ fpos, const int *__restri
             do {
                 xx = __dmul_rn(-log(__dsub_rn(1.0, ws_uniform(next()))), 0.2904764);
                 yy = -log(__dsub_rn(1.0, ws_uniform(next())));
-            } while (__dadd_rn(yy, yy) < __dmul_rn(xx, xx) && q <= end);
+            } while (less(__dadd_rn(yy, yy), __dmul_rn(xx, xx)) && q <= end);
             val = hv > 0 ? __dadd_rn(3.442620, xx) : __dsub_rn(-3.442620, xx);
             break;
         }
         const double f = __dadd_rn(fn[iz], __dmul_rn(ws_uniform(next()), __dsub_rn(fn[iz - 1], fn[iz])));
-        if (f < exp(__dmul_rn(__dmul_rn(-.5, x), x))) break;
+        if (less(f, exp(__dmul_rn(__dmul_rn(-.5, x), x)))) break;
     }
     fext[i] = (unsigned char)min(q - p - 1, 255u);
     fval[i] = val;
     // (the last words of the launch cannot be resolved; they are guard words, which no cloud that is placed reads)
-    if (q > end && end != nword) *err = 1;
+    if (q > end && end != nword) atomicOr(err, WS_LOST);
+    if (near && q <= end) atomicOr(err, WS_NEAR);
 }
 
 // per (block, place at its first word): the words beyond one a draw, and by how many words the last deviate runs over
@@ -354,7 +372,7 @@ __global__ void k_ws_flux(const WindShell *__restrict__ shells, int nshell, Grid
 // A thread a cloud. The channel of a sample in float-float (the float64 pipe runs at 1/64 of the float32 rate here)
 // where the channel map is linear: within 1e-6 of a channel boundary, and for further lines, the reference's float64
 // operations.
-__global__ void __launch_bounds__(256) k_ws_clouds(const WindJob *__restrict__ jobs, int njob, long long ncl, int M,
+__global__ void __launch_bounds__(256, 4) k_ws_clouds(const WindJob *__restrict__ jobs, int njob, long long ncl, int M,
                                                    const WsStart *__restrict__ ends,
                                                    const uint2 *__restrict__ cloud,
                                                    const unsigned long long *__restrict__ words,
@@ -404,10 +422,11 @@ __global__ void __launch_bounds__(256) k_ws_clouds(const WindJob *__restrict__ j
     const double R = __dmul_rn(rad, sphi), z = __dmul_rn(rad, cphi);
     const double x = __dmul_rn(R, caz);
     const double y = __dsub_rn(__dmul_rn(__dmul_rn(R, saz), s.cinc), __dmul_rn(z, s.sinc));
-    const long long g0 =
-        lround_ref(__dadd_rn(s.xpos, __ddiv_rn(__dsub_rn(__dmul_rn(x, s.spa), __dmul_rn(y, s.cpa)), g.cdelt0)));
-    const long long g1 =
-        lround_ref(__dadd_rn(s.ypos, __ddiv_rn(__dadd_rn(__dmul_rn(x, s.cpa), __dmul_rn(y, s.spa)), g.cdelt1)));
+    const double px = __dadd_rn(s.xpos, __ddiv_rn(__dsub_rn(__dmul_rn(x, s.spa), __dmul_rn(y, s.cpa)), g.cdelt0));
+    const double py = __dadd_rn(s.ypos, __ddiv_rn(__dadd_rn(__dmul_rn(x, s.cpa), __dmul_rn(y, s.spa)), g.cdelt1));
+    const long long g0 = lround_ref(px), g1 = lround_ref(py);
+    if ((ws_close(px) && ws_near(px, s.xpos, rad, g.cdelt0)) || (ws_close(py) && ws_near(py, s.ypos, rad, g.cdelt1)))
+        atomicOr(err, WS_NEAR);
     if (g0 < blo0 || g0 >= bhi0 || g1 < blo1 || g1 >= bhi1) return;
     // bbarolo/galmod.py:581-589
     const double geom = __dadd_rn(__dmul_rn(cphi, s.cinc), __dmul_rn(__dmul_rn(sphi, saz), s.sinc));
@@ -420,7 +439,7 @@ __global__ void __launch_bounds__(256) k_ws_clouds(const WindJob *__restrict__ j
     unsigned p = 3;
     for (int iv = 0; iv < M - 3; iv++) {
         if (at.x + p >= nword) {                            // (the guard words are more than any cloud takes)
-            *err = 1;
+            atomicOr(err, WS_LOST);
             return;
         }
         int hv;
@@ -447,7 +466,15 @@ __global__ void __launch_bounds__(256) k_ws_clouds(const WindJob *__restrict__ j
             long long kc = c;
             if (nl || c == -0x40000000) {
                 const double d = one ? __dmul_rn((double)hv, zig->wn[hv & 127]) : slow;
-                kc = lround_ref(velgrid_exact(__dadd_rn(vs, __dmul_rn(d, s.vdisp)), g, nl));
+                const double v = __dadd_rn(vs, __dmul_rn(d, s.vdisp)), ch = velgrid_exact(v, g, nl);
+                kc = lround_ref(ch);
+                if (ws_close(ch)) {
+                    // (the velocity is within dv of the one from the C library's functions)
+                    const double dv = 1e-14 * (fabs(s.vsys) + 4.0 * (fabs(s.vsph) + fabs(s.vrot)) + 16.0 * fabs(s.vdisp));
+                    if (lround_ref(velgrid_exact(__dsub_rn(v, dv), g, nl)) != kc ||
+                        lround_ref(velgrid_exact(__dadd_rn(v, dv), g, nl)) != kc)
+                        atomicOr(err, WS_NEAR);
+                }
             }
             if (kc < 0 || kc >= g.nz) continue;
             atomicAdd(o + kc, (unsigned long long)fx[(size_t)nl * g.nz + kc]);

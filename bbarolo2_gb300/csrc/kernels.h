@@ -366,8 +366,11 @@ struct WindJob {
     WsStart start;
     int seg0, blk0, nblk, grp0, shell0, nshell, ncl, pad;
 };
-// words, failing words and their deviates (cap of them; err set when there are more); then the clouds; jump: (32, 128)
-// pairs of bbh_stream_jumps(WS_SEG)
+// words, failing words and their deviates (cap of them); then the clouds; jump: (32, 128) pairs of
+// bbh_stream_jumps(WS_SEG). err: WS_LOST (more than cap failing words, or a deviate of more words than are followed) and
+// WS_NEAR (a pixel, channel or rejection that the last bits of sin, cos, log or exp decide): the host parse decides
+#define WS_LOST 1
+#define WS_NEAR 2
 void launch_ws_words(cudaStream_t st, const WindJob *jobs, int njob, int nseg, const void *jump, const ZigDev *zig,
                      const double *fn, unsigned long long *words, unsigned *masks, int *nfail, int *foff, int *fcur,
                      int *scratch, unsigned *fpos, unsigned char *fext, double *fval, int cap, int *err);

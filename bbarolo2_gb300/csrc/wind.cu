@@ -552,8 +552,8 @@ __global__ void __launch_bounds__(512) k_wind_deposit_cell(const long long *__re
         for (int j = threadIdx.x; j < size; j += blockDim.x) out[j] = (double)(long long)acc[j] * unit;
         return;
     }
-    // for the convolution (k_wind_to_ff): the sums times 2^-b, 2^b above the largest, as float-float (the leading 24
-    // bits and those of the rest, from the integers)
+    // for the convolution (k_wind_to_ff): the sums times 2^-b, 2^b above the largest, as float-float, from the integers:
+    // the leading 24 bits rounded to nearest and the rest, signed, so that the pair is within 2^-49 (truncated, 2^-48)
     unsigned long long m = 0;
     auto mag = [](unsigned long long v) { return (long long)v < 0 ? 0ull - v : v; };
     for (int j = threadIdx.x; j < size; j += blockDim.x) m = max(m, mag(acc[j]));
@@ -571,8 +571,9 @@ __global__ void __launch_bounds__(512) k_wind_deposit_cell(const long long *__re
         float2 v = make_float2(0.f, 0.f);
         if (q) {
             const unsigned long long l = q << (64 - sh);             // the leading bit at the top
-            const float h = (float)(unsigned)(l >> 40);              // 24 bits, exact
-            const float r = (float)(unsigned)((l >> 8) & 0xffffffffull);
+            const unsigned long long t = ((l >> 39) + 1) >> 1;       // 24 bits rounded (or 2^24), exact in float32
+            const float h = (float)(unsigned)t;
+            const float r = (float)(int)((long long)(l - (t << 40)) >> 8);   // (|l - t 2^40| <= 2^39, also modulo 2^64)
             const float s0 = scalbnf(1.0f, sh - b - 24);
             v = make_float2(h * s0, r * (s0 * 2.3283064365386963e-10f));
             if ((long long)acc[j] < 0) v = make_float2(-v.x, -v.y);

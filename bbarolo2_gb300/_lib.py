@@ -29,7 +29,7 @@ SYMBOLS = ("bbgpu_ctx_create", "bbgpu_ctx_destroy", "bbgpu_last_error", "bbgpu_v
            "bbgpu_subrings_rows", "bbgpu_conv_variant", "bbgpu_graph_stats", "bbgpu_mlp_create",
            "bbgpu_mlp_destroy", "bbgpu_mlp_nparams", "bbgpu_mlp_get_params", "bbgpu_mlp_set_params",
            "bbgpu_mlp_predict", "bbgpu_mlp_gradients", "bbgpu_mlp_train_step", "bbgpu_mlp_train",
-           "bbgpu_model_cube", "bbgpu_classic_set", "bbgpu_classic_residual",
+           "bbgpu_release_scratch", "bbgpu_model_cube", "bbgpu_classic_set", "bbgpu_classic_residual",
            "bbgpu_galmod_wind", "bbgpu_galwind_spherical", "bbgpu_galwind_cube",
            "bbgpu_wind_create", "bbgpu_wind_destroy", "bbgpu_wind_last_error", "bbgpu_wind_launch_count",
            "bbgpu_wind_set_cells", "bbgpu_wind_points", "bbgpu_wind_set_points", "bbgpu_wind_boxes",
@@ -135,6 +135,7 @@ def load(path=None):
         "bbgpu_eval_profile": (i, [vp, vp, vp]),
         "bbgpu_solve_profile": (i, [vp, vp, vp, i, i, vp, d, d, d, vp, vp]),
         "bbgpu_galmod_wind": (i, [vp, vp, vp, i, i, i, u64, d, vp, i, i, i, i]),
+        "bbgpu_release_scratch": (i, [vp]),
         "bbgpu_model_cube": (i, [vp, i, vp, vp, i, C.c_uint64, vp, i, i, i, i, i, d]),
         "bbgpu_classic_set": (i, [vp, vp, vp, i, i, i, vp]),
         "bbgpu_classic_residual": (i, [vp, vp, i, C.c_uint64, vp, i, i, i, i, vp, i, i] + [d] * 8 + [i, i, d, d, i, vp]),
@@ -214,6 +215,10 @@ class Context:
         a, b = np.zeros(1, np.int64), np.zeros(1, np.int64)
         self.check(self.L.bbgpu_transfer_bytes(self.h, ptr(a), ptr(b)))
         return int(a[0]), int(b[0])
+
+    def release_scratch(self):
+        """Gives back the device memory that the stand-alone calls (models, convolutions, winds) keep for the next."""
+        self.check(self.L.bbgpu_release_scratch(self.h))
 
     def set_option(self, opt, value):
         self.check(self.L.bbgpu_set_option(self.h, int(opt), int(value)))

@@ -1972,6 +1972,21 @@ extern "C" int bbgpu_eval_model(bbgpu_ctx *ctx, int k, int smoothed, float *out,
 }
 
 // ------------------------------------------------------------------------------------------- reference kernels
+#define POOL_SLACK ((size_t)64 << 20)
+// what the calls of whole cubes (POOL_CUBES and on: GALWIND, bbgpu_convolve, bbgpu_model_cube) may keep together: a
+// wind of 2.2 M clouds takes 0.5 GB, the convolution of a 160x160x128 cube 0.07
+#define POOL_CUBES 5
+#define POOL_KEEP ((size_t)1 << 30)
+
+// Frees the scratch of the stand-alone calls but that of call site `keep` (-1: none is kept).
+static void pool_release(bbgpu_ctx *ctx, int keep) {
+    for (int t = 0; t < (int)(sizeof ctx->pool / sizeof *ctx->pool); t++) {
+        if (t == keep) continue;
+        for (PoolBuf &b : ctx->pool[t]) cudaFree(b.p);
+        ctx->pool[t].clear();
+    }
+}
+
 // Scratch buffers of a stand-alone call: the i-th buffer of call site `tag` is kept in the context and reused by
 // the next call of that site (grown when too small), so that a call allocates nothing once warm (a cudaFree would
 // also wait for the whole device). The calls of a context run in order on its stream, so reuse is safe.
@@ -1990,10 +2005,17 @@ struct DevBufs {
             if (b.p) cudaFree(b.p);
             b.p = nullptr;
             b.cap = 0;
-            const size_t want = need + need / 4;
+            // (a little more than this call's; where that does not fit, this call's and no other call's)
+            size_t want = need + std::min(need / 4, POOL_SLACK);
             if (cudaMalloc(&b.p, want) != cudaSuccess) {
                 cudaGetLastError();
-                return false;
+                pool_release(ctx, tag);
+                want = need;
+                if (cudaMalloc(&b.p, want) != cudaSuccess) {
+                    cudaGetLastError();
+                    b.p = nullptr;
+                    return false;
+                }
             }
             b.cap = want;
         }
@@ -2061,17 +2083,37 @@ static int conv_dev(bbgpu_ctx *ctx, DevBufs &B, const float *a, float *b, int nz
     return 0;
 }
 
-// (what a large cube took goes back at the end of its call)
+// (what a large cube took goes back at the end of its call: its own, and the other cubes' where both are too much)
 struct PoolTrim {
-    std::vector<PoolBuf> &v;
-    ~PoolTrim() {
-        size_t sum = 0;
-        for (PoolBuf &b : v) sum += b.cap;
-        if (sum <= ((size_t)2 << 30)) return;
+    bbgpu_ctx *ctx;
+    int tag;
+    static void drop(std::vector<PoolBuf> &v) {
         for (PoolBuf &b : v) cudaFree(b.p);
         v.clear();
     }
+    ~PoolTrim() {
+        const int n = (int)(sizeof ctx->pool / sizeof *ctx->pool);
+        size_t own = 0, sum = 0;
+        for (int t = POOL_CUBES; t < n; t++)
+            for (PoolBuf &b : ctx->pool[t]) (t == tag ? own : sum) += b.cap;
+        if (own > POOL_KEEP) {
+            drop(ctx->pool[tag]);
+            own = 0;
+        }
+        if (own + sum > POOL_KEEP)
+            for (int t = POOL_CUBES; t < n; t++)
+                if (t != tag) drop(ctx->pool[t]);
+    }
 };
+
+// Gives the device memory of the stand-alone calls' scratch back.
+extern "C" int bbgpu_release_scratch(bbgpu_ctx *ctx) {
+    if (!ctx) return BBGPU_ERR_ARG;
+    CK(cudaSetDevice(ctx->device));
+    CK(cudaStreamSynchronize(ctx->stream));
+    pool_release(ctx, -1);
+    return BBGPU_OK;
+}
 
 extern "C" int bbgpu_convolve(bbgpu_ctx *ctx, const double *in, double *out, int nz, int ny, int nx, double scale,
                               int threshold) {
@@ -2081,7 +2123,7 @@ extern "C" int bbgpu_convolve(bbgpu_ctx *ctx, const double *in, double *out, int
     if (!ctx->kernel_set) return fail(ctx, BBGPU_ERR_STATE, "convolve before set_kernel");
     CK(cudaSetDevice(ctx->device));
     const size_t n = (size_t)nz * ny * nx;
-    PoolTrim trim{ctx->pool[6]};
+    PoolTrim trim{ctx, 6};
     DevBufs B(ctx, 6);
     double *d64 = nullptr;
     float *a = nullptr, *b = nullptr;
@@ -2439,7 +2481,7 @@ static int wind_mc_run(bbgpu_ctx *ctx, double *out, bool cube, const double *sr,
         return BBGPU_OK;
     }
     DevBufs B(ctx, 5);
-    PoolTrim trim{ctx->pool[5]};
+    PoolTrim trim{ctx, 5};
     double *d_out = nullptr;
     if (!B.get(&R.acc, sizeof(uint64_t) * R.n) || !B.get(&d_out, cube ? sizeof(double) * R.n : 8))
         return fail(ctx, BBGPU_ERR_NOMEM, "galmod_wind: device allocation failed");
@@ -2622,7 +2664,7 @@ extern "C" int bbgpu_model_cube(bbgpu_ctx *ctx, int galmodtype, double *out, con
     CK(cudaSetDevice(ctx->device));
     const int nz = ctx->g.nz, by = bhi1 - blo1, bx = bhi0 - blo0;
     const size_t n = (size_t)by * bx * nz;
-    PoolTrim trim{ctx->pool[7]};
+    PoolTrim trim{ctx, 7};
     DevBufs B(ctx, 7);
     double *d64 = nullptr;
     float *a = nullptr, *b = nullptr;

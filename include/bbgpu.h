@@ -93,6 +93,10 @@ int bbgpu_set_kernel(bbgpu_ctx *ctx, const double *kernel, int ky, int kx);
 int bbgpu_set_cube(bbgpu_ctx *ctx, const float *data, const uint8_t *mask, const uint8_t *region);
 
 /* ---- reference-kernel entry points (one model per call; host arrays in and out) ------------------------ */
+/* These calls keep their device scratch in the context for the next one (calls that take whole cubes, GALWIND,
+ * bbgpu_convolve and bbgpu_model_cube, at most 1 GB together; the others what their largest call took) until
+ * bbgpu_ctx_destroy, or until this call gives it back: */
+int bbgpu_release_scratch(bbgpu_ctx *ctx);
 /* out (bhi1-blo1, bhi0-blo0, nz) float64 is ACCUMULATED (out +=), as the reference kernels. */
 int bbgpu_galmod_mc(bbgpu_ctx *ctx, double *out, const double *sr, int nsub, int ring_lo, int ring_hi,
                     uint64_t seed, const int64_t *nv, int blo0, int blo1, int bhi0, int bhi1);

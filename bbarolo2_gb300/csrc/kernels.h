@@ -5,6 +5,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <map>
+#include <mutex>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -51,12 +54,29 @@ struct ZigDev {
 
 // A launch with smem bytes of dynamic shared memory: above 48 KB with the function's static arrays, its limit is set to
 // all that they leave of the 227 KB of a CTA, whatever this launch takes, so that host threads that launch one kernel
-// with different sizes do not lower each other's limit.
+// with different sizes do not lower each other's limit. Once for a function and device: the attributes of a function
+// cost a driver call, and a small batch is bound by its host calls.
 inline void allow_smem(const void *f, size_t smem) {
-    cudaFuncAttributes a;
-    if (smem > 4 * 1024 && cudaFuncGetAttributes(&a, f) == cudaSuccess && a.sharedSizeBytes + smem > 48 * 1024 &&
-        a.maxDynamicSharedSizeBytes < 227 * 1024 - (int)a.sharedSizeBytes)
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
+    if (smem <= 4 * 1024) return;
+    struct Known {
+        size_t arrays;                     // bytes of its static arrays
+        bool raised;
+    };
+    static std::mutex mu;
+    static std::map<std::pair<const void *, int>, Known> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find({f, dev});
+    if (it == known.end()) {
+        cudaFuncAttributes a;
+        if (cudaFuncGetAttributes(&a, f) != cudaSuccess) return;
+        it = known.insert({{f, dev}, Known{a.sharedSizeBytes, false}}).first;
+    }
+    Known &k = it->second;
+    if (!k.raised && k.arrays + smem > 48 * 1024)
+        k.raised = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        227 * 1024 - (int)k.arrays) == cudaSuccess;
 }
 
 // ---- MC (mc.cu)

@@ -1251,7 +1251,7 @@ void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int n
     allow_smem((const void *)k_an_replay, smem);
     int per = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_an_replay, 256, smem);
-    const int nc = std::max(1, std::min(152 * std::max(per, 1) / ng, (ntask + 7) / 8));
+    const int nc = std::max(1, std::min(sm_count() * std::max(per, 1) / ng, (ntask + 7) / 8));
     k_an_replay<<<nc * ng, 256, smem, s>>>(g.nz, ng, nzb, npix, ntask, 2 * nsub, count + ntask + 1, count,
                                            (const int4 *)runs, prof, kw, amp, top, klist, n3, mem, (const unsigned long long *)own, mstride,
                                            model);
@@ -1293,7 +1293,7 @@ void launch_ant_pixel(cudaStream_t s, int nz, const int *pix0, int kfirst, int n
     allow_smem((const void *)k_ant_pixel, smem);
     int per = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ant_pixel, 32 * nw, smem);
-    k_ant_pixel<<<std::min((npix + nw - 1) / nw, 152 * std::max(per, 1)), 32 * nw, smem, s>>>(
+    k_ant_pixel<<<std::min((npix + nw - 1) / nw, sm_count() * std::max(per, 1)), 32 * nw, smem, s>>>(
         nz, pix0, kfirst, nk, offset, count, order, (const AntSample *)rec, (const float2 *)vef, cd2if, ptabf, mem,
         model, model64, mstride, base64, base_out, mbase);
 }

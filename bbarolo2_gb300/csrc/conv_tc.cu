@@ -869,10 +869,7 @@ void launch_conv_tc(cudaStream_t s, int variant, const GridDev &g, const MemberD
     if (nb == 0 || ntxg == 0 || ntyg == 0) return;
     // persistent CTAs, one per SM; work items: strips split in runs of at most TC_MAX_TILES tiles, at least four
     // items per CTA where the batch allows
-    int nsm = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (nsm <= 0) nsm = 1;
+    const int nsm = sm_count();
     const int nzb = (nz + TC_M - 1) / TC_M;
     int nsy = 1;
     while (nsy < ntyg && (long long)nb * nzb * ntxg * nsy < 4LL * nsm) nsy++;

@@ -79,6 +79,14 @@ inline void allow_smem(const void *f, size_t smem) {
                                         227 * 1024 - (int)k.arrays) == cudaSuccess;
 }
 
+// The SMs of the current device: what a persistent grid or a split fills.
+inline int sm_count() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) cudaGetLastError();
+    return n > 0 ? n : 1;
+}
+
 // ---- MC (mc.cu)
 // For every (member, cloud): its pixel in the member's box (or -1) and the count of clouds per tile.
 // Tile lists are split by pixel (NOWN per tile, tiles of at most 64 pixels): list index = (tile_off + tile) * NOWN
@@ -96,8 +104,8 @@ void launch_mc_sums64(cudaStream_t s, const long long *sums, long long n, int nz
                       const float *cd2if, int e, double *out, float *model);
 // The CTAs that share a tile's clouds in the pixel-owned deposit of one member with ntile tiles (argument split;
 // they add their sums to base64, and no float32 model is written).
-// Measured: one ring of a 64x64x64 cube (9 tiles, 20 k clouds) 81 us with one CTA a tile, 20 us with 16; from 304
-// tiles on the chip is full (two CTAs per SM) and a split would only repeat the tiles' zeroing and output.
+// Measured: one ring of a 64x64x64 cube (9 tiles, 20 k clouds) 81 us with one CTA a tile, 20 us with 16; from two tiles
+// an SM on the chip is full (two CTAs per SM) and a split would only repeat the tiles' zeroing and output.
 int mc_deposit_split(int ntile);
 // Exclusive scan of n list counts into offsets (and cursors, where not null); scratch holds (n + 1023) / 1024 ints.
 void launch_scan_tiles(cudaStream_t s, const int *count, int *offset, int *cursor, int n, int *scratch);

@@ -1527,7 +1527,7 @@ void launch_mc_deposit(cudaStream_t s, const GridDev &g, const LayoutDev &L, con
                                         cd2i, model, mstride, model64, err);
 }
 
-int mc_deposit_split(int ntile) { return max(1, min(16, 304 / max(ntile, 1))); }
+int mc_deposit_split(int ntile) { return max(1, min(16, 2 * sm_count() / max(ntile, 1))); }
 
 void launch_mc_sums64(cudaStream_t s, const long long *sums, long long n, int nz, const double *cd2i,
                       const float *cd2if, int e, double *out, float *model) {

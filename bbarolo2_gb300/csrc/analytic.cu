@@ -1,15 +1,22 @@
 // The ANALYTIC GALMOD deposit and the ring maps on the device (the reference's _galmod_analytic and
 // _ring_maps_analytic, bbarolo/galmod.py:326-536).
 //
-// One warp per azimuthal sample (sub-ring, radial sample, azimuth). The warp computes the pixels of the
-// sample's vertical samples (lanes over heights), merges consecutive heights that fall in the same pixel
-// (lane 0, in order, as the reference), and deposits each merged run: for a model, the channel-integrated
-// line profile (lanes over channels, computed once per sample and line from the tabulated normal CDF), for
-// ring maps the run's weight. All arithmetic that decides an index or a value is the reference's float64,
-// each operation rounded once in its order (no contraction), so pixels and channels are bit-exact. The sums
-// are in 64-bit fixed point (units 2^-e, e per member from a bound on its total flux): integer atomics, exact
-// and independent of the order of the deposits, so the model is deterministic; it differs from the
-// reference's running float64 sum by rounding only.
+//   k_an_model       any line, axis and layer: a warp a sample (sub-ring, radial sample, azimuth), lanes over heights, the
+//                    runs of consecutive heights in one pixel found by ballots, their weights added in the
+//                    reference's order, then the (run, channel) pairs over the lanes;
+//   k_an_model_fast  sub-rings with one line on a linear axis (anfast), in float32: 32 samples set up a lane each;
+//   k_an_records, k_an_amps, k_an_replay
+//                    members that are member 0 but for the fluxes: its runs listed by pixel, read once for 16 members;
+//   k_ant_bin, k_ant_list, k_ant_pixel
+//                    thin disks (one height, anfast): the samples listed by pixel, a warp a pixel;
+//   k_an_maps        ring maps: a run's weight in place of the line profile;
+//   k_fix_to_model   fixed point to float32.
+// What decides an index is the reference's: pixels and centre channels in float32 or float-float with a rounding bound,
+// beyond it by the reference's float64 operations, each rounded once in its order (no contraction), so they are
+// bit-exact. Values: k_an_model's and k_an_maps's are the reference's float64 ones; the float32 path's are within 1e-5 of
+// the model's peak. The sums are in 64-bit fixed point (units 2^-e, e per member from a bound on its total flux):
+// integer additions, exact and independent of the order of the deposits, so the model is deterministic; it differs from
+// the reference's running float64 sum by rounding only.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

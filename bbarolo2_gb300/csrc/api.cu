@@ -189,6 +189,7 @@ struct bbgpu_ctx {
     uint8_t *h_atab = nullptr, *d_atab = nullptr;
     size_t h_atab_cap = 0, d_atab_cap = 0;
     cudaEvent_t ev_tab = nullptr;
+    cudaEvent_t ev_up = nullptr;          // the last batch has left the pinned arrays (pinned_wait)
     long long *d_astart = nullptr;
     int *d_aseg = nullptr, *d_mbase = nullptr, *d_apix0 = nullptr;
     std::vector<unsigned long long> h_chg; // per member: the sub-rings a replaying member deposits itself
@@ -604,6 +605,7 @@ extern "C" int bbgpu_ctx_destroy(bbgpu_ctx *ctx) {
         if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
     if (ctx->ev_tab) cudaEventDestroy(ctx->ev_tab);
+    if (ctx->ev_up) cudaEventDestroy(ctx->ev_up);
     if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
     if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -869,6 +871,18 @@ static int member_desc(bbgpu_ctx *ctx, int k, const bbgpu_eval_desc &d, int fix_
     return 0;
 }
 
+// The pinned arrays of a batch are written by the host and copied from on the stream, maybe behind earlier runs: the next
+// upload waits until the last one's copies are done (pinned_sent), not for the runs.
+static int pinned_sent(bbgpu_ctx *ctx) {
+    if (!ctx->ev_up) CK(cudaEventCreateWithFlags(&ctx->ev_up, cudaEventDisableTiming));
+    CK(cudaEventRecord(ctx->ev_up, ctx->stream));
+    return 0;
+}
+static int pinned_wait(bbgpu_ctx *ctx) {
+    if (ctx->ev_up) CK(cudaEventSynchronize(ctx->ev_up));
+    return 0;
+}
+
 // An ANALYTIC batch (bbarolo/galmod.py:326-465 per member): the sub-ring constants of every member on the host
 // (vertical grids shared through a cache), the azimuthal samples of the shared radii, all uploaded; the members
 // may differ in every ring value but the radii.
@@ -882,6 +896,7 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
         if (memcmp(sr + (size_t)k * BBGPU_NSR * nsub, sr, sizeof(double) * nsub))
             return fail(ctx, BBGPU_ERR_ARG, "eval: member %d has other radii: evaluate it in another batch", k);
     int rc;
+    if ((rc = pinned_wait(ctx))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_asub, &ctx->h_asub_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_mem, &ctx->h_mem_cap, (size_t)nb))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_reuse, &ctx->h_reuse_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
@@ -1031,7 +1046,7 @@ static int batch_prepare_analytic(bbgpu_ctx *ctx, int nb, int nsub, const double
     ctx->h2d += (long long)((sizeof(AnSub) + (nb > 1)) * (size_t)nb * nsub + sizeof(MemberDev) * (size_t)nb);
     ctx->uploaded = true;
     ctx->ran = false;
-    return 0;
+    return pinned_sent(ctx);
 }
 
 static int batch_prepare(bbgpu_ctx *ctx, int galmodtype, int nb, int nsub, const double *sr, const int64_t *nv,
@@ -1069,6 +1084,7 @@ static int batch_prepare(bbgpu_ctx *ctx, int galmodtype, int nb, int nsub, const
     int rc = get_layout(ctx, seed, nsub, nc0.data(), nv0.data(), R0.data(), &E);
     if (rc) return rc;
     ctx->cur = E;
+    if ((rc = pinned_wait(ctx))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_sub, &ctx->h_sub_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_mem, &ctx->h_mem_cap, (size_t)nb))) return rc;
     if ((rc = hgrow(ctx, &ctx->h_reuse, &ctx->h_reuse_cap, (size_t)nb * (nsub ? nsub : 1)))) return rc;
@@ -1139,7 +1155,7 @@ static int batch_prepare(bbgpu_ctx *ctx, int galmodtype, int nb, int nsub, const
     ctx->h2d = (long long)((sizeof(SubMC) + (nb > 1)) * (size_t)nb * nsub + sizeof(MemberDev) * (size_t)nb);
     ctx->uploaded = true;
     ctx->ran = false;
-    return 0;
+    return pinned_sent(ctx);
 }
 
 // The flux normalisation of the batch (bbarolo/bayesian/likelihood.py:595-596): ring maps, beam convolution,

@@ -1256,9 +1256,8 @@ void launch_an_replay(cudaStream_t s, const GridDev &g, const AnSub *subs, int n
     k_an_amps<<<(unsigned)((na + 255) / 256), 256, 0, s>>>(subs, nsub, mem, klist, n3, ng, chg, nchw, amp, top);
     const size_t smem = (size_t)2 * nsub * (ANR_MG + 1) * sizeof(float);
     allow_smem((const void *)k_an_replay, smem);
-    int per = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_an_replay, 256, smem);
-    const int nc = std::max(1, std::min(sm_count() * std::max(per, 1) / ng, (ntask + 7) / 8));
+    const int nc = std::max(1, std::min(sm_count() * resident_ctas((const void *)k_an_replay, 256, smem) / ng,
+                                        (ntask + 7) / 8));
     k_an_replay<<<nc * ng, 256, smem, s>>>(g.nz, ng, nzb, npix, ntask, 2 * nsub, count + ntask + 1, count,
                                            (const int4 *)runs, prof, kw, amp, top, klist, n3, mem, (const unsigned long long *)own, mstride,
                                            model);
@@ -1298,9 +1297,8 @@ void launch_ant_pixel(cudaStream_t s, int nz, const int *pix0, int kfirst, int n
     if (nk <= 0 || npix <= 0 || !nw) return;
     const size_t smem = ant_smem(nz, nw);
     allow_smem((const void *)k_ant_pixel, smem);
-    int per = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ant_pixel, 32 * nw, smem);
-    k_ant_pixel<<<std::min((npix + nw - 1) / nw, sm_count() * std::max(per, 1)), 32 * nw, smem, s>>>(
+    const int fill = sm_count() * resident_ctas((const void *)k_ant_pixel, 32 * nw, smem);
+    k_ant_pixel<<<std::min((npix + nw - 1) / nw, fill), 32 * nw, smem, s>>>(
         nz, pix0, kfirst, nk, offset, count, order, (const AntSample *)rec, (const float2 *)vef, cd2if, ptabf, mem,
         model, model64, mstride, base64, base_out, mbase);
 }

@@ -7,6 +7,7 @@
 
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -77,6 +78,28 @@ inline void allow_smem(const void *f, size_t smem) {
     if (!k.raised && k.arrays + smem > 48 * 1024)
         k.raised = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         227 * 1024 - (int)k.arrays) == cudaSuccess;
+}
+
+// The CTAs of f with `threads` threads and smem bytes of dynamic shared memory that an SM holds (asked once for a
+// function, device and size).
+inline int resident_ctas(const void *f, int threads, size_t smem) {
+    static std::mutex mu;
+    static std::map<std::tuple<const void *, int, int, size_t>, int> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    const auto key = std::make_tuple(f, dev, threads, smem);
+    auto it = known.find(key);
+    if (it == known.end()) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, threads, smem) != cudaSuccess) {
+            cudaGetLastError();
+            return 1;
+        }
+        if (known.size() >= 256) known.clear();
+        it = known.insert({key, n > 0 ? n : 1}).first;
+    }
+    return it->second;
 }
 
 // The SMs of the current device: what a persistent grid or a split fills.

@@ -21,7 +21,7 @@
 // point (units 2^(E-62), 2^E above the total flux of the clouds: exact sums, independent of their order). From the host
 // parse its pixel and channels are the reference's. On the device sin, cos, log and exp are within two ulps of the C
 // library's: where that could move a pixel, a channel or a deviate's rejection, the launch says so (WS_NEAR) and the
-// host parse makes the model, so that the same holds (about one model of 2.2 M clouds in a hundred thousand).
+// host parse makes the model, so that the same holds (about one model of 2.2 M clouds in ten thousand).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -371,7 +371,7 @@ __global__ void k_ws_flux(const WindShell *__restrict__ shells, int nshell, Grid
 
 // A thread a cloud. The channel of a sample in float-float (the float64 pipe runs at 1/64 of the float32 rate here)
 // where the channel map is linear: within 1e-6 of a channel boundary, and for further lines, the reference's float64
-// operations.
+// operations. Four CTAs an SM: at 68 registers a thread, three, the model of 2.2 M clouds took 2.29 ms for 2.22.
 __global__ void __launch_bounds__(256, 4) k_ws_clouds(const WindJob *__restrict__ jobs, int njob, long long ncl, int M,
                                                    const WsStart *__restrict__ ends,
                                                    const uint2 *__restrict__ cloud,
